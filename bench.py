@@ -724,8 +724,8 @@ def ours(args, rank, world):
 
 def batch_leg(args, rank, world, stream, barrier, max_over_ranks):
     """64 independent scenes, nx,ny,nz ~ U[32,160] (seed 4), blob masks, FP32
-    faces, mixed precision to 1e-6: one batched call (xfp_project_batch_f32,
-    tile height autotuned) against a loop of single-scene calls on the same
+    faces, mixed precision to 1e-6: one batched call (xfp_project_batch_f32)
+    against a loop of single-scene calls on the same
     inputs, both device-resident.  Across ranks the scenes are LPT-sharded
     (no collective on the data path); times are the max over ranks."""
     import ctypes as C
@@ -761,7 +761,6 @@ def batch_leg(args, rank, world, stream, barrier, max_over_ranks):
         return best, out
 
     o = _lib.default_options()
-    # single solves with their tile height tuned per grid shape (cached by the warm-up loop)
     o.precision, o.tol, o.max_iter, o.device_pointers, o.tile_k = _lib.PREC["mixed"], TOL, MAXIT, 1, 0
     o.stream = C.c_void_p(stream.cuda_stream)
     ctx = _lib.Context(o)
@@ -786,7 +785,7 @@ def batch_leg(args, rank, world, stream, barrier, max_over_ranks):
 
     loop(fresh())                       # warm-up
     ms_loop, it_loop = timed(loop, 2)
-    batched(fresh())                    # warm-up: tile height timed and cached
+    batched(fresh())                    # warm-up
     ms_batch, (ok, it_batch, (tile_k, graph)) = timed(batched, 3)
     ctx.close()
     bp.close()
@@ -1039,7 +1038,7 @@ def main():
     ap.add_argument("--profile-case", type=int, default=0, metavar="N",
                     help="only project the N^3 blob scene twice (mixed, device-resident) and exit: "
                          "the small case the ncu captures of the sweep kernels use")
-    ap.add_argument("--tile-k", type=int, default=8, help="sweep tile height of --profile-case (8, 15 or 16)")
+    ap.add_argument("--tile-k", type=int, default=8, help="options.tile_k of --profile-case (8, 15 or 16)")
     args = ap.parse_args()
     if args.particles_case:
         import torch

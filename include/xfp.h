@@ -73,7 +73,7 @@ typedef struct xfp_options {
   double timeout_ms;     /* bound on any device-side wait (0: 2000 ms) */
   int max_refine;        /* mixed: iterative-refinement cycles (0: 20) */
   double inner_tol;      /* mixed: relative residual reduction per cycle (0: 1e-4) */
-  int tile_k;            /* sweep tile height in k-lines: 8, 15 or 16; 0: timed on the first call per grid (or batch) shape and cached */
+  int tile_k;            /* 0, 8, 15 or 16; kept for callers that set it: the sweeps have one decomposition, and results do not depend on it */
   void* stream;          /* cudaStream_t to run on; NULL: the context's own stream */
   int matrix;            /* XFP_MATRIX_*: which pressure matrix the solve/project/apply entry points use */
 } xfp_options;
@@ -101,7 +101,7 @@ typedef struct xfp_stats {
                             serialises them) */
   int sweeps;            /* triangular-solve sweep launches timed in ms_sweeps */
   long long launches;    /* device kernels launched by this call */
-  int tile_k;            /* sweep tile height the call used (k-lines) */
+  int tile_k;            /* options.tile_k, or 8 where that is 0 */
   int graph;             /* 1: the PCG iterations ran as a CUDA graph; 0: launched one by one */
   double ms_vec[3];      /* device time of the PCG loop's vector kernels (CUDA events, sampled as
                             ms_sweeps is): SpMV + dot,
@@ -195,9 +195,7 @@ typedef struct xfp_scene {
  * tolerance test, iteration count and PCG scalars), but the MIC(0) sweeps of
  * all scenes run in one persistent launch and the PCG iteration is replayed
  * as a CUDA graph.  No reference counterpart: xFluid projects one grid per
- * call (FluidSimulator.cpp:501-509).  With options.tile_k == 0 the sweep tile
- * height is picked per batch shape by timing the candidate heights on the
- * first call (cached in the context).  stats, if not NULL, receives n entries.  Returns
+ * call (FluidSimulator.cpp:501-509).  stats, if not NULL, receives n entries.  Returns
  * XFP_OK when every scene converged, XFP_NOT_CONVERGED when one did not. */
 int xfp_project_batch_f32(xfp_ctx* ctx, int n, const xfp_scene* scenes, xfp_stats* stats);
 int xfp_project_batch_f64(xfp_ctx* ctx, int n, const xfp_scene* scenes, xfp_stats* stats);

@@ -46,7 +46,7 @@ class BatchProjector:
     ``v``, ``w`` face arrays (updated in place), optional ``wu/wv/ww`` and
     optional ``pressure`` (nk,nj,ni) output.  All arrays of one call are host
     numpy arrays or all CUDA torch tensors, all float32 or all float64.
-    ``tile_k=0`` lets the library time both sweep tile heights per batch shape.
+    ``tile_k`` (0, 8, 15 or 16) is accepted and changes nothing.
     """
 
     def __init__(self, precision: str = "mixed", tol: float = 1e-6, max_iter: int = 200, tile_k: int = 0,

@@ -14,13 +14,10 @@
 //   * the PCG iteration is captured once as a CUDA graph (check_every
 //     iterations: SpMV+dot, x/r update, forward, backward, rho/beta, s update)
 //     and replayed until every scene has converged or hit its cap.
-//   * the sweep tile height: with options.tile_k == 0 the heights 8, 15 and 16
-//     are timed on the first call for a batch shape and the fastest is cached.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <map>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -32,22 +29,20 @@ using namespace xfp;
 namespace xfp_host {
 
 struct BatchState {
-  DevBuf lines, lens, tile_active, scene_tile_lists, counters;
-  DevBuf segs, tiles, tile_scene, scal, scal2, part, tols, maxits;
+  DevBuf lines, lens, scene_tile_lists, counters;
+  DevBuf segs, tile_scene, scal, scal2, part, tols, maxits;
   DevBuf io, pdense;
   std::vector<BatchSeg> hsegs;
-  std::vector<long long> line_base, rows, nlines_act;
-  int n = 0, nw = 0, ntiles = 0, blocks_lines = 0, blocks_cells = 0, blocks_groups = 0;
+  std::vector<long long> rows, nlines_act;
+  int n = 0, ntiles = 0, blocks_lines = 0, blocks_cells = 0, blocks_groups = 0;
   long long M = 0;
-  std::map<std::string, int> tuned;   // batch shape -> sweep tile height
-  std::string layout_key;             // shape + tile height of the layout built last
   bool graph_used = false;
 };
 
 void batch_state_free(BatchState* b) {
   if (!b) return;
-  DevBuf* all[] = {&b->lines, &b->lens, &b->tile_active, &b->scene_tile_lists, &b->counters, &b->segs,
-                   &b->tiles, &b->tile_scene, &b->scal, &b->scal2, &b->part,
+  DevBuf* all[] = {&b->lines, &b->lens, &b->scene_tile_lists, &b->counters, &b->segs,
+                   &b->tile_scene, &b->scal, &b->scal2, &b->part,
                    &b->tols, &b->maxits, &b->io, &b->pdense};
   for (DevBuf* d : all) d->release();
   delete b;
@@ -65,84 +60,82 @@ struct DevScene {
   T* p;
 };
 
-std::string shape_key(int n, const xfp_scene* sc, int prec) {
-  std::string k = std::to_string(prec) + ":";
-  for (int s = 0; s < n; ++s)
-    k += std::to_string(sc[s].ni) + "x" + std::to_string(sc[s].nj) + "x" + std::to_string(sc[s].nk) + ",";
-  return k;
-}
-
-// Line tables, compact slices and the merged tile list for tile height nw.
+// Line and block tables, compact and sweep slices, and the merged tile list.
 template <typename T>
-int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S, int nw) {
+int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S) {
   cudaStream_t st = ctx->stream;
   const int n = (int)S.size();
-  std::vector<long long> tile_base(n + 1, 0);
-  B->line_base.assign(n + 1, 0);
+  std::vector<long long> line_base(n + 1, 0), blk_base(n + 1, 0);
   for (int s = 0; s < n; ++s) {
-    B->line_base[s + 1] = B->line_base[s] + (long long)S[s].nj * S[s].nk;
-    const long long NJt = (S[s].nj + 31) / 32, NKt = (S[s].nk + nw - 1) / nw;
-    tile_base[s + 1] = tile_base[s] + NJt * NKt;
+    line_base[s + 1] = line_base[s] + (long long)S[s].nj * S[s].nk;
+    blk_base[s + 1] = blk_base[s] + (long long)((S[s].nj + 7) / 8) * ((S[s].nk + 7) / 8);
   }
-  const long long nlines = B->line_base[n], ntile_slots = tile_base[n];
+  const long long nlines = line_base[n], nblk = blk_base[n];
   XFP_CUDA(ctx, B->lines.ensure(nlines * sizeof(Line)));
   XFP_CUDA(ctx, B->lens.ensure((nlines + n) * sizeof(int)));
-  XFP_CUDA(ctx, B->tile_active.ensure(ntile_slots));
-  XFP_CUDA(ctx, B->scene_tile_lists.ensure(ntile_slots * sizeof(int)));
-  XFP_CUDA(ctx, B->counters.ensure((size_t)n * 4 * sizeof(long long)));
+  XFP_CUDA(ctx, ctx->blks.ensure((size_t)nblk * sizeof(WBlk)));
+  XFP_CUDA(ctx, B->scene_tile_lists.ensure((size_t)nblk * sizeof(int2)));
+  XFP_CUDA(ctx, B->counters.ensure((size_t)n * 5 * sizeof(long long)));
   Line* lines = B->lines.as<Line>();
   for (int s = 0; s < n; ++s) {
-    LayoutDev L{lines + B->line_base[s], B->lens.as<int>() + B->line_base[s] + s,
-                B->tile_active.as<unsigned char>() + tile_base[s], B->scene_tile_lists.as<int>() + tile_base[s],
-                B->counters.as<long long>() + 4 * s};
-    XFP_CUDA(ctx, layout_build(S[s].mat, S[s].ni, S[s].nj, S[s].nk, nw, L, st));
+    LayoutDev L{lines + line_base[s], B->lens.as<int>() + line_base[s] + s, ctx->blks.as<WBlk>() + blk_base[s],
+                B->scene_tile_lists.as<int2>() + blk_base[s], B->counters.as<long long>() + 5 * s};
+    XFP_CUDA(ctx, layout_build(S[s].mat, S[s].ni, S[s].nj, S[s].nk, L, st));
   }
-  std::vector<long long> cnt((size_t)n * 4);
+  std::vector<long long> cnt((size_t)n * 5);
+  std::vector<int2> all_tiles((size_t)nblk);
   XFP_CUDA(ctx, cudaMemcpyAsync(cnt.data(), B->counters.p, cnt.size() * sizeof(long long), cudaMemcpyDeviceToHost,
                                 st));
+  XFP_CUDA(ctx, cudaMemcpyAsync(all_tiles.data(), B->scene_tile_lists.p, (size_t)nblk * sizeof(int2),
+                                cudaMemcpyDeviceToHost, st));
   XFP_CUDA(ctx, cudaStreamSynchronize(st));
-  // compact slices: scene s occupies [base_s, base_s + M_s); line offsets made global
-  std::vector<long long> base(n + 1, 0);
+  // compact slices: scene s occupies [base_s, base_s + M_s); line offsets made
+  // global.  Sweep slices: groups [group_base_s, ...).
+  std::vector<long long> base(n + 1, 0), group_base(n + 1, 0);
   B->rows.assign(n, 0);
   B->nlines_act.assign(n, 0);
   for (int s = 0; s < n; ++s) {
-    base[s + 1] = base[s] + cnt[4 * s];
-    B->rows[s] = cnt[4 * s + 1];
-    B->nlines_act[s] = cnt[4 * s + 2];
+    base[s + 1] = base[s] + cnt[5 * s];
+    B->rows[s] = cnt[5 * s + 1];
+    B->nlines_act[s] = cnt[5 * s + 2];
+    group_base[s + 1] = group_base[s] + cnt[5 * s + 4];
   }
   if (base[n] >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "batch too large: more than 2^31 stored cells");
+  if (group_base[n] * 256 >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "batch too large for the sweep layout");
   for (int s = 0; s < n; ++s)
-    XFP_CUDA(ctx, offset_lines(lines + B->line_base[s], B->line_base[s + 1] - B->line_base[s], base[s], st));
-  // cell -> line index (line numbers local to each scene's table; cells global)
-  XFP_CUDA(ctx, ctx->cell_line.ensure((std::max<long long>(base[n], 4) + 8) * sizeof(int)));
+    XFP_CUDA(ctx, offset_lines(lines + line_base[s], line_base[s + 1] - line_base[s], base[s], st));
+  // group -> line index (line numbers local to each scene's table; cells
+  // global) and group -> sweep element
   XFP_CUDA(ctx, ctx->group_line.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(int)));
-  for (int s = 0; s < n; ++s)
-    XFP_CUDA(ctx, build_cell_line(lines + B->line_base[s], B->line_base[s + 1] - B->line_base[s],
-                                  ctx->cell_line.as<int>(), ctx->group_line.as<int>(), st));
-  // merge the scenes' tile lists by wavefront level (each list is already in
+  XFP_CUDA(ctx, ctx->gperm.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(int)));
+  for (int s = 0; s < n; ++s) {
+    XFP_CUDA(ctx, build_group_line(lines + line_base[s], line_base[s + 1] - line_base[s], ctx->group_line.as<int>(),
+                                   st));
+    XFP_CUDA(ctx, gperm_build(ctx->group_line.as<int>() + base[s] / 4, lines + line_base[s], S[s].nj,
+                              ctx->blks.as<WBlk>() + blk_base[s], (S[s].nj + 7) / 8, base[s + 1] - base[s], base[s],
+                              group_base[s], ctx->gperm.as<int>() + base[s] / 4, st));
+  }
+  // merge the scenes' block lists by wavefront level (each list is already in
   // its own topological order, which the merge keeps)
-  std::vector<int> all_tiles(ntile_slots > 0 ? ntile_slots : 1);
-  if (ntile_slots > 0)
-    XFP_CUDA(ctx, cudaMemcpyAsync(all_tiles.data(), B->scene_tile_lists.p, ntile_slots * sizeof(int),
-                                  cudaMemcpyDeviceToHost, st));
-  XFP_CUDA(ctx, cudaStreamSynchronize(st));
-  struct Item {
-    int level, scene, idx, packed;
-  };
-  std::vector<Item> items;
-  for (int s = 0; s < n; ++s)
-    for (long long q = 0; q < cnt[4 * s + 3]; ++q) {
-      const int packed = all_tiles[tile_base[s] + q];
-      items.push_back({(packed & 0xffff) + (packed >> 16), s, (int)q, packed});
-    }
-  std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
-    return a.level != b.level ? a.level < b.level : a.scene != b.scene ? a.scene < b.scene : a.idx < b.idx;
-  });
-  const int nt = (int)items.size();
-  std::vector<int> tiles(std::max(nt, 1)), tscene(std::max(nt, 1));
-  for (int t = 0; t < nt; ++t) {
-    tiles[t] = items[t].packed;
-    tscene[t] = items[t].scene;
+  long long ntl = 0;
+  for (int s = 0; s < n; ++s) ntl += cnt[5 * s + 3];
+  const int nt = (int)ntl;
+  std::vector<int2> tiles;
+  std::vector<int> tscene;
+  tiles.reserve(std::max(nt, 1));
+  tscene.reserve(std::max(nt, 1));
+  std::vector<long long> at(n, 0);
+  for (int level = 0; (int)tiles.size() < nt; ++level)
+    for (int s = 0; s < n; ++s)
+      for (; at[s] < cnt[5 * s + 3]; ++at[s]) {
+        const int2 t = all_tiles[blk_base[s] + at[s]];
+        if (t.x + t.y != level) break;
+        tiles.push_back(t);
+        tscene.push_back(s);
+      }
+  if (nt == 0) {
+    tiles.push_back(int2{0, 0});
+    tscene.push_back(0);
   }
   // per-scene block decomposition of the vector kernels (as a single launch)
   B->hsegs.assign(n, BatchSeg{});
@@ -150,7 +143,7 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S,
   int bl = 0, bc = 0, bg = 0;
   for (int s = 0; s < n; ++s) {
     BatchSeg& g = B->hsegs[s];
-    const long long nl = (long long)S[s].nj * S[s].nk, Ms = cnt[4 * s];
+    const long long nl = (long long)S[s].nj * S[s].nk, Ms = cnt[5 * s];
     g.ni = S[s].ni; g.nj = S[s].nj; g.nk = S[s].nk;
     g.blk_lines = (int)std::max<long long>(1, std::min<long long>((nl + 7) / 8, NBLK_MAX));
     g.blk_lines_start = bl;
@@ -160,12 +153,13 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S,
     g.blk_cells_start = bc;
     g.blk_groups = (int)spmv_block_count(Ms, NBLK_MAX);
     g.blk_groups_start = bg;
-    g.tile_base = (int)tile_base[s];
+    g.blk_base = blk_base[s];
+    g.line_base = line_base[s];
+    g.group_base = group_base[s];
     g.base = base[s];
     g.M = Ms;
-    g.lines = lines + B->line_base[s];
+    g.lines = lines + line_base[s];
     g.partials = B->part.as<double>() + (size_t)s * NBLK_MAX;
-    g.line_base = B->line_base[s];
     bl += g.blk_lines;
     bc += g.blk_cells;
     bg += g.blk_groups;
@@ -174,119 +168,51 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S,
   B->blocks_cells = bc;
   B->blocks_groups = bg;
   XFP_CUDA(ctx, B->segs.ensure(n * sizeof(BatchSeg)));
-  XFP_CUDA(ctx, B->tiles.ensure(tiles.size() * sizeof(int)));
+  XFP_CUDA(ctx, ctx->tiles.ensure(tiles.size() * sizeof(int2)));
   XFP_CUDA(ctx, B->tile_scene.ensure(tscene.size() * sizeof(int)));
   XFP_CUDA(ctx, cudaMemcpyAsync(B->segs.p, B->hsegs.data(), n * sizeof(BatchSeg), cudaMemcpyHostToDevice, st));
-  XFP_CUDA(ctx, cudaMemcpyAsync(B->tiles.p, tiles.data(), tiles.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+  XFP_CUDA(ctx, cudaMemcpyAsync(ctx->tiles.p, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
   XFP_CUDA(ctx, cudaMemcpyAsync(B->tile_scene.p, tscene.data(), tscene.size() * sizeof(int),
                                 cudaMemcpyHostToDevice, st));
   // the host vectors above go out of scope: make the copies complete first
   XFP_CUDA(ctx, cudaStreamSynchronize(st));
   B->n = n;
-  B->nw = nw;
   B->ntiles = nt;
   B->M = base[n];
-  ctx->nw = nw;
-  ctx->bnd_ni = 0;
-  for (int s = 0; s < n; ++s) ctx->bnd_ni = std::max(ctx->bnd_ni, S[s].ni);
   ctx->M = B->M;
   ctx->ntiles = nt;
-  ctx->nlines_all = nlines;
-  // Sweep layout over the merged tile list: spans on the device, offsets
-  // scanned here, the (scene, K, J) -> tile map filled here, then the cell ->
-  // element map scene by scene.
-  ctx->Msw = 0;
-  if (nt > 0) {
-    XFP_CUDA(ctx, ctx->swt.ensure(nt * sizeof(SwTile)));
-    XFP_CUDA(ctx, sw_tiles_build_batch(B->tiles.as<int>(), B->tile_scene.as<int>(), B->segs.as<BatchSeg>(), nt, nw,
-                                       ctx->swt.as<SwTile>(), st));
-    std::vector<SwTile> sw(nt);
-    XFP_CUDA(ctx, cudaMemcpyAsync(sw.data(), ctx->swt.p, nt * sizeof(SwTile), cudaMemcpyDeviceToHost, st));
-    XFP_CUDA(ctx, cudaStreamSynchronize(st));
-    long long off = 0;
-    for (auto& e : sw) {
-      e.off = off;
-      off += (long long)nw * e.ng * 128;
-    }
-    if (off >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "batch too large for the sweep layout");
-    ctx->Msw = off;
-    std::vector<int> tpos(std::max<long long>(ntile_slots, 1), -1);
-    for (int t = 0; t < nt; ++t) {
-      const int sc = tscene[t], J = tiles[t] & 0xffff, K = tiles[t] >> 16;
-      tpos[tile_base[sc] + (long long)K * ((S[sc].nj + 31) / 32) + J] = t;
-    }
-    XFP_CUDA(ctx, ctx->tile_pos.ensure(tpos.size() * sizeof(int)));
-    XFP_CUDA(ctx, cudaMemcpyAsync(ctx->swt.p, sw.data(), nt * sizeof(SwTile), cudaMemcpyHostToDevice, st));
-    XFP_CUDA(ctx, cudaMemcpyAsync(ctx->tile_pos.p, tpos.data(), tpos.size() * sizeof(int), cudaMemcpyHostToDevice,
-                                  st));
-    XFP_CUDA(ctx, ctx->sw_perm.ensure((size_t)(std::max<long long>(B->M, 4) + 8) * sizeof(int)));
-    for (int sc = 0; sc < n; ++sc)
-      XFP_CUDA(ctx, sw_perm_build(ctx->cell_line.as<int>() + base[sc], lines + B->line_base[sc], S[sc].nj, nw,
-                                  (S[sc].nj + 31) / 32, ctx->tile_pos.as<int>() + tile_base[sc],
-                                  ctx->swt.as<SwTile>(), base[sc + 1] - base[sc], ctx->sw_perm.as<int>() + base[sc],
-                                  st, base[sc]));
-    XFP_CUDA(ctx, cudaStreamSynchronize(st));
-  }
+  ctx->Gsw = group_base[n];
+  ctx->nlines_all = line_base[n];
   return XFP_OK;
 }
 
-SweepGrid batch_grid(xfp_ctx* ctx, BatchState* B, PcgScalars* sc) {
-  SweepGrid g{};
-  g.ntiles = B->ntiles;
-  g.tiles = B->tiles.as<int>();
-  g.ctl = ctx->ctl.as<SweepCtl>();
-  g.spin_limit = spin_limit(ctx);
-  g.scal = nullptr;
-  g.trace = nullptr;
+WaveArgs batch_args(xfp_ctx* ctx, BatchState* B, PcgScalars* sc) {
+  WaveArgs g = wave_args(ctx);
   g.tile_scene = B->tile_scene.as<int>();
   g.segs = B->segs.as<BatchSeg>();
   g.scal_batch = sc;
-  g.stage = ctx->stage_solves;
   return g;
 }
 
-template <typename VT, typename IT, typename CT>
-cudaError_t batch_sweep(xfp_ctx* ctx, BatchState* B, int op, const SweepGrid& g, const SweepData<VT, IT, CT>& d) {
-  if (B->ntiles <= 0) return cudaSuccess;
-  const int maxg = sweep_max_grid(op, d, B->nw, g.stage);
-  if (maxg <= 0) return cudaErrorLaunchOutOfResources;
-  return sweep_launch(op, g, d, B->nw, std::min(maxg, B->ntiles), ctx->stream);
-}
-
-// Assembly of every scene into the shared compact arrays.
+// Assembly of every scene into the shared compact arrays and sweep layout.
 template <typename FT, typename AT>
 int batch_assemble(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<FT>>& S, AT* const A[5]) {
-  for (size_t s = 0; s < S.size(); ++s)
+  for (size_t s = 0; s < S.size(); ++s) {
+    const BatchSeg& g = B->hsegs[s];
     XFP_CUDA(ctx, (assemble<FT, AT>(S[s].mat, S[s].u, S[s].v, S[s].w, S[s].wu, S[s].wv, S[s].ww, S[s].ni, S[s].nj,
-                                    S[s].nk, B->hsegs[s].lines, A[0], A[1], A[2], A[3], A[4], ctx->stream)));
-  return XFP_OK;
-}
-
-// MIC(0) factor of every scene in one sweep launch.
-template <typename VT, typename IT, typename CT>
-int batch_factor(xfp_ctx* ctx, BatchState* B, const CT* const A[4], CT* const F[6], IT* inv, CT omega, CT ratio) {
-  const size_t M = (size_t)std::max<long long>(B->M, 1);
-  // the factorisation writes L only where a coupling exists: clear the three L arrays first
-  for (int q = 0; q < 3; ++q) XFP_CUDA(ctx, cudaMemsetAsync(F[q], 0, M * sizeof(CT), ctx->stream));
-  XFP_CUDA(ctx, cudaMemsetAsync(inv, 0, M * sizeof(IT), ctx->stream));
-  SweepData<VT, IT, CT> d;
-  d.diag = A[0]; d.ax = A[1]; d.ay = A[2]; d.az = A[3];
-  d.flx = F[0]; d.fly = F[1]; d.flz = F[2];
-  d.oinv = inv;
-  d.sy = ctx->sy.as<unsigned long long>();
-  d.sz = ctx->sz.as<unsigned long long>();
-  d.omega = omega; d.ratio = ratio;
-  XFP_CUDA(ctx, (batch_sweep<VT, IT, CT>(ctx, B, SWEEP_FACTOR, batch_grid(ctx, B, nullptr), d)));
+                                    S[s].nk, g.lines, A[0], A[1], A[2], A[3], A[4], ctx->stream,
+                                    XFP_MATRIX_VARIATIONAL, Force3(), nullptr, ctx->sw_sys.as<AT>(),
+                                    ctx->blks.as<WBlk>() + g.blk_base, g.group_base)));
+  }
   return XFP_OK;
 }
 
 // PCG (pcg_solver.h:243-285) on every scene at once.  Per-scene tolerance and
 // cap come from tol/maxit, or from the device arrays tols/maxits when given.
 // On return hsc holds each scene's final scalars.
-template <typename VT, typename IT, typename DT>
-int batch_pcg(xfp_ctx* ctx, BatchState* B, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT* z,
-              const VT* const L[3], const IT* inv, double tol, int maxit, const double* tols, const int* maxits,
-              PcgScalars* dsc, std::vector<PcgScalars>& hsc, int maxit_all) {
+template <typename VT, typename DT>
+int batch_pcg(xfp_ctx* ctx, BatchState* B, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT* z, double tol,
+              int maxit, const double* tols, const int* maxits, PcgScalars* dsc, std::vector<PcgScalars>& hsc, int maxit_all) {
   cudaStream_t st = ctx->stream;
   const int n = B->n;
   const size_t M = (size_t)std::max<long long>(B->M, 1);
@@ -297,40 +223,31 @@ int batch_pcg(xfp_ctx* ctx, BatchState* B, const VT* const A[4], const VT* b, VT
   XFP_CUDA(ctx, cudaMemsetAsync(dsc, 0, n * sizeof(PcgScalars), st));
   XFP_CUDA(ctx, copy_vec<VT>(b, r, (long long)M, st));
   XFP_CUDA(ctx, batch_absmax_init<VT>(segs, n, B->blocks_cells, r, dsc, tol, maxit, tols, maxits, st));
-  SweepData<VT, IT, DT> d;
-  d.r = r; d.y = z; d.lx = L[0]; d.ly = L[1]; d.lz = L[2]; d.inv = inv;
-  d.partials = ctx->tpartials.as<double>();
-  d.sy = ctx->sy.as<unsigned long long>();
-  d.sz = ctx->sz.as<unsigned long long>();
-  SweepGrid g = batch_grid(ctx, B, dsc);
-  // the solves stream the sweep layout (as single scenes do): factor and r
-  // copied in, z gathered back through perm
-  if ((rc0 = sweep_copies<VT, IT, DT>(ctx, L, inv, r, &g, 1, &d)) != XFP_OK) return rc0;
+  // the solves stream the sweep layout (as single scenes do): r copied in, z
+  // gathered back through gperm
+  if ((rc0 = sweep_rhs<VT>(ctx, r)) != XFP_OK) return rc0;
+  const WaveArgs g = batch_args(ctx, B, dsc);
   const bool swl = B->ntiles > 0;
   VT* rsw = swl ? ctx->sw_r.as<VT>() : nullptr;
   const VT* zsw = swl ? ctx->sw_y.as<VT>() : nullptr;
-  const int* perm = swl ? ctx->sw_perm.as<int>() : nullptr;
+  const int* gperm = swl ? ctx->gperm.as<int>() : nullptr;
   const double* lpart = ctx->tpartials.as<double>();
-  // lines of inactive tiles are never written: their partials stay zero
+  // lines of blocks without cells are never written: their partials stay zero
   XFP_CUDA(ctx, cudaMemsetAsync(ctx->tpartials.p, 0, std::max<long long>(ctx->nlines_all, 1) * sizeof(double), st));
-  XFP_CUDA(ctx, (batch_sweep<VT, IT, DT>(ctx, B, SWEEP_FWD, g, d)));
-  XFP_CUDA(ctx, (batch_sweep<VT, IT, DT>(ctx, B, SWEEP_BWD, g, d)));
+  XFP_CUDA(ctx, (wave_launch<VT, DT>(SWEEP_FWD, g, st)));
+  XFP_CUDA(ctx, (wave_launch<VT, DT>(SWEEP_BWD, g, st)));
   XFP_CUDA(ctx, batch_bwd_reduce<DT>(segs, n, lpart, dsc, 0, st));
-  if (swl) {
-    if ((rc0 = sweep_result<VT>(ctx, s)) != XFP_OK) return rc0;
-  } else {
-    XFP_CUDA(ctx, copy_vec<VT>(z, s, (long long)M, st));
-  }
+  if ((rc0 = sweep_result<VT>(ctx, s)) != XFP_OK) return rc0;
   auto iteration = [&]() -> cudaError_t {
     cudaError_t e;
     if ((e = batch_spmv_dot<VT, VT, DT>(segs, n, B->blocks_groups, A[0], A[1], A[2], A[3], s, z,
                                         ctx->group_line.as<int>(), dsc, 0, st)))
       return e;
-    if ((e = batch_update_xr<VT>(segs, n, B->blocks_cells, x, r, s, z, dsc, st, rsw, perm))) return e;
-    if ((e = batch_sweep<VT, IT, DT>(ctx, B, SWEEP_FWD, g, d))) return e;
-    if ((e = batch_sweep<VT, IT, DT>(ctx, B, SWEEP_BWD, g, d))) return e;
+    if ((e = batch_update_xr<VT>(segs, n, B->blocks_cells, x, r, s, z, dsc, st, rsw, gperm))) return e;
+    if ((e = wave_launch<VT, DT>(SWEEP_FWD, g, st))) return e;
+    if ((e = wave_launch<VT, DT>(SWEEP_BWD, g, st))) return e;
     if ((e = batch_bwd_reduce<DT>(segs, n, lpart, dsc, 1, st))) return e;
-    return batch_update_s<VT>(segs, n, B->blocks_cells, s, z, dsc, st, zsw, perm);
+    return batch_update_s<VT>(segs, n, B->blocks_cells, s, z, dsc, st, zsw, gperm);
   };
   const int K = ctx->opt.check_every > 0 ? ctx->opt.check_every : 8;
   const int per_iter = B->ntiles > 0 ? 6 : 4;
@@ -394,7 +311,7 @@ template <typename IOT>
 int batch_solve(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<IOT>>& S, std::vector<SceneResult>& out) {
   const int prec = ctx->opt.precision, n = B->n;
   cudaStream_t st = ctx->stream;
-  const double tol = ctx->opt.tol, omega = ctx->opt.omega, ratio = ctx->opt.min_diag_ratio;
+  const double tol = ctx->opt.tol;
   const int maxit = ctx->opt.max_iter;
   const long long M = std::max<long long>(B->M, 1);
   XFP_CUDA(ctx, B->scal.ensure(n * sizeof(PcgScalars)));
@@ -408,28 +325,20 @@ int batch_solve(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<IOT>>& S
       double* A[5];
       for (int q = 0; q < 5; ++q) A[q] = ctx->A64[q].as<double>();
       if ((rc = batch_assemble<IOT, double>(ctx, B, S, A))) return rc;
-      double* F[6];
-      for (int q = 0; q < 6; ++q) F[q] = ctx->F64[q].as<double>();
       const double* Ac[4] = {A[0], A[1], A[2], A[3]};
-      if ((rc = batch_factor<double, double, double>(ctx, B, Ac, F, ctx->inv64.as<double>(), omega, ratio))) return rc;
-      const double* Lc[3] = {F[0], F[1], F[2]};
-      rc = batch_pcg<double, double, double>(ctx, B, Ac, A[4], ctx->x64.as<double>(), ctx->r64.as<double>(),
-                                             ctx->s64.as<double>(), ctx->z64.as<double>(), Lc,
-                                             ctx->inv64.as<double>(), tol, maxit, nullptr, nullptr, dsc, hsc, maxit);
+      XFP_CUDA(ctx, (wave_launch<double, double>(SWEEP_FACTOR, batch_args(ctx, B, nullptr), st)));
+      rc = batch_pcg<double, double>(ctx, B, Ac, A[4], ctx->x64.as<double>(), ctx->r64.as<double>(),
+                                     ctx->s64.as<double>(), ctx->z64.as<double>(), tol, maxit, nullptr, nullptr, dsc,
+                                     hsc, maxit);
     } else {
       float* A[5];
       for (int q = 0; q < 5; ++q) A[q] = ctx->A32[q].as<float>();
       if ((rc = batch_assemble<IOT, float>(ctx, B, S, A))) return rc;
-      float* F[6];
-      for (int q = 0; q < 6; ++q) F[q] = ctx->F32[q].as<float>();
       const float* Ac[4] = {A[0], A[1], A[2], A[3]};
-      if ((rc = batch_factor<float, float, float>(ctx, B, Ac, F, ctx->inv32.as<float>(), (float)omega,
-                                                  (float)ratio)))
-        return rc;
-      const float* Lc[3] = {F[0], F[1], F[2]};
-      rc = batch_pcg<float, float, float>(ctx, B, Ac, A[4], ctx->x32.as<float>(), ctx->r32.as<float>(),
-                                          ctx->s32.as<float>(), ctx->z32.as<float>(), Lc, ctx->inv32.as<float>(),
-                                          tol, maxit, nullptr, nullptr, dsc, hsc, maxit);
+      XFP_CUDA(ctx, (wave_launch<float, float>(SWEEP_FACTOR, batch_args(ctx, B, nullptr), st)));
+      rc = batch_pcg<float, float>(ctx, B, Ac, A[4], ctx->x32.as<float>(), ctx->r32.as<float>(),
+                                   ctx->s32.as<float>(), ctx->z32.as<float>(), tol, maxit, nullptr, nullptr, dsc, hsc,
+                                   maxit);
     }
     if (rc < 0) return rc;
     for (int q = 0; q < n; ++q) {
@@ -451,14 +360,8 @@ int batch_solve(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<IOT>>& S
     A32[q] = ctx->A32[q].as<float>();
     XFP_CUDA(ctx, (convert<double, float>(A[q], A32[q], M, st)));
   }
-  double* F[6];
-  for (int q = 0; q < 6; ++q) F[q] = ctx->F64[q].as<double>();
-  const double* Ac[4] = {A[0], A[1], A[2], A[3]};
-  if ((rc = batch_factor<float, double, double>(ctx, B, Ac, F, ctx->inv64.as<double>(), omega, ratio))) return rc;
-  for (int q = 0; q < 3; ++q) XFP_CUDA(ctx, (convert<double, float>(F[q], ctx->L32[q].as<float>(), M, st)));
-  // FP64 pivots, streamed by the FP32 solves rounded to FP32 (as a single scene's mixed solve)
-  XFP_CUDA(ctx, (convert<double, float>(ctx->inv64.as<double>(), ctx->inv32.as<float>(), M, st)));
-  const float* Lc[3] = {ctx->L32[0].as<float>(), ctx->L32[1].as<float>(), ctx->L32[2].as<float>()};
+  // FP64 factor, streamed by the FP32 solves rounded to FP32 (as a single scene's mixed solve)
+  XFP_CUDA(ctx, (wave_launch<float, double>(SWEEP_FACTOR, batch_args(ctx, B, nullptr), st)));
   const float* A32c[4] = {A32[0], A32[1], A32[2], A32[3]};
   double* x64 = ctx->x64.as<double>();
   double* r64 = ctx->r64.as<double>();
@@ -512,9 +415,8 @@ int batch_solve(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<IOT>>& S
     float* b32 = ctx->A32[4].as<float>();
     XFP_CUDA(ctx, copy_vec<float>(ctx->r32.as<float>(), b32, M, st));
     std::vector<PcgScalars> hin;
-    rc = batch_pcg<float, float, double>(ctx, B, A32c, b32, ctx->x32.as<float>(), ctx->r32.as<float>(),
-                                         ctx->s32.as<float>(), ctx->z32.as<float>(), Lc, ctx->inv32.as<float>(),
-                                          0.5, maxit, B->tols.as<double>(), B->maxits.as<int>(), dsc, hin, maxit);
+    rc = batch_pcg<float, double>(ctx, B, A32c, b32, ctx->x32.as<float>(), ctx->r32.as<float>(),
+                                  ctx->s32.as<float>(), ctx->z32.as<float>(), 0.5, maxit, B->tols.as<double>(), B->maxits.as<int>(), dsc, hin, maxit);
     if (rc < 0) return rc;
     for (int q = 0; q < n; ++q)
       if (maxits[q] > 0) {
@@ -543,47 +445,6 @@ int batch_solve(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<IOT>>& S
     out[q].res = res[q];
   }
   return XFP_OK;
-}
-
-// Times one factor and one forward+backward pair over a built layout.
-template <typename IOT>
-int time_sweeps(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<IOT>>& S, float* ms) {
-  cudaStream_t st = ctx->stream;
-  const long long M = std::max<long long>(B->M, 1);
-  XFP_CUDA(ctx, B->scal.ensure(B->n * sizeof(PcgScalars)));
-  XFP_CUDA(ctx, cudaMemsetAsync(B->scal.p, 0, B->n * sizeof(PcgScalars), st));
-  float* A[5];
-  for (int q = 0; q < 5; ++q) A[q] = ctx->A32[q].as<float>();
-  int rc;
-  if ((rc = batch_assemble<IOT, float>(ctx, B, S, A))) return rc;
-  float* F[6];
-  for (int q = 0; q < 6; ++q) F[q] = ctx->F32[q].as<float>();
-  const float* Ac[4] = {A[0], A[1], A[2], A[3]};
-  if ((rc = batch_factor<float, float, float>(ctx, B, Ac, F, ctx->inv32.as<float>(), 0.97f, 0.25f))) return rc;
-  SweepData<float, float, float> d;
-  d.r = A[4]; d.y = ctx->z32.as<float>(); d.lx = F[0]; d.ly = F[1]; d.lz = F[2]; d.inv = ctx->inv32.as<float>();
-  d.partials = ctx->tpartials.as<double>();
-  d.sy = ctx->sy.as<unsigned long long>();
-  d.sz = ctx->sz.as<unsigned long long>();
-  SweepGrid g = batch_grid(ctx, B, B->scal.as<PcgScalars>());
-  const float* Lf[3] = {F[0], F[1], F[2]};
-  if ((rc = sweep_copies<float, float, float>(ctx, Lf, d.inv, d.r, &g, 1, &d))) return rc;
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  XFP_CUDA(ctx, (batch_sweep<float, float, float>(ctx, B, SWEEP_FWD, g, d)));   // warm-up
-  cudaEventRecord(e0, st);
-  for (int q = 0; q < 2; ++q) {
-    XFP_CUDA(ctx, (batch_sweep<float, float, float>(ctx, B, SWEEP_FWD, g, d)));
-    XFP_CUDA(ctx, (batch_sweep<float, float, float>(ctx, B, SWEEP_BWD, g, d)));
-  }
-  cudaEventRecord(e1, st);
-  XFP_CUDA(ctx, cudaStreamSynchronize(st));
-  cudaEventElapsedTime(ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  (void)M;
-  return check_sweep_error(ctx);
 }
 
 template <typename IOT>
@@ -672,31 +533,10 @@ int project_batch(xfp_ctx* ctx, int n, const xfp_scene* scenes, xfp_stats* stats
     }
   }
 
-  // ---- layout (tile height tuned per batch shape) ----
+  // ---- layout ----
   const int prec = ctx->opt.precision;
-  const std::string key = shape_key(n, scenes, prec);
-  int nw = ctx->opt.tile_k;
   int rc;
-  if (nw == 0) {
-    auto it = B->tuned.find(key);
-    if (it != B->tuned.end()) {
-      nw = it->second;
-    } else {
-      float best = 0;
-      int best_nw = 8;
-      for (int cand : {8, 15, 16}) {
-        if ((rc = batch_layout<IOT>(ctx, B, S, cand))) return rc;
-        if ((rc = ensure_compact(ctx, XFP_PREC_F32))) return rc;
-        float ms = 0;
-        if ((rc = time_sweeps<IOT>(ctx, B, S, &ms))) return rc;
-        if (cand == 8 || ms < best) { best = ms; best_nw = cand; }
-      }
-      B->tuned[key] = best_nw;
-      nw = best_nw;
-      B->layout_key.clear();
-    }
-  }
-  if ((rc = batch_layout<IOT>(ctx, B, S, nw))) return rc;
+  if ((rc = batch_layout<IOT>(ctx, B, S))) return rc;
   if ((rc = ensure_compact(ctx, prec))) return rc;
   cudaEventRecord(ev[1], st);
 
@@ -773,7 +613,7 @@ int project_batch(xfp_ctx* ctx, int n, const xfp_scene* scenes, xfp_stats* stats
       const double cells = (double)scenes[s].ni * scenes[s].nj * scenes[s].nk;
       o.bytes = bpr * (double)o.rows * o.iterations + 33.0 * cells + 24.0 * (double)o.rows + 29.0 * cells;
       o.launches = launches;
-      o.tile_k = B->nw;
+      o.tile_k = ctx->nw;
       o.graph = B->graph_used ? 1 : 0;
     }
   }

@@ -3,7 +3,7 @@
 // One call runs, on the context's stream:
 //   layout   line table + tile list of the material grid          (xfp_layout.cu)
 //   assemble the variational system into the compact layout      (xfp_ops.cu)
-//   factor   MIC(0) in natural order                              (xfp_sweep.cu)
+//   factor   MIC(0) in natural order                              (xfp_wave.cu)
 //   PCG      spmv+dot / x,r update / forward / backward+dot / s update per
 //            iteration, convergence read back every check_every iterations
 //   output   pressure scattered to the dense grid, velocity update (project)
@@ -50,71 +50,37 @@ int check_dims(xfp_ctx* ctx, int ni, int nj, int nk, const void* mat) {
 }
 
 // ---------------------------------------------------------------- layout
-int build_sweep_layout(xfp_ctx* ctx);
-
 int build_layout(xfp_ctx* ctx, const uint8_t* dmat, int ni, int nj, int nk) {
-  const int nw = ctx->nw;
   const long long nlines = (long long)nj * nk;
-  const int NJt = (nj + 31) / 32, NKt = (nk + nw - 1) / nw;
+  const int NJB = (nj + 7) / 8, NKB = (nk + 7) / 8;
   XFP_CUDA(ctx, ctx->lines.ensure(nlines * sizeof(Line)));
   XFP_CUDA(ctx, ctx->lens.ensure((nlines + 1) * sizeof(int)));
-  XFP_CUDA(ctx, ctx->tile_active.ensure((size_t)NJt * NKt));
-  XFP_CUDA(ctx, ctx->tiles.ensure((size_t)NJt * NKt * sizeof(int)));
-  XFP_CUDA(ctx, ctx->counters.ensure(4 * sizeof(long long)));
-  LayoutDev L{ctx->lines.as<Line>(), ctx->lens.as<int>(), ctx->tile_active.as<unsigned char>(),
-              ctx->tiles.as<int>(), ctx->counters.as<long long>()};
-  XFP_CUDA(ctx, layout_build(dmat, ni, nj, nk, nw, L, ctx->stream));
-  long long cnt[4];
+  XFP_CUDA(ctx, ctx->blks.ensure((size_t)NJB * NKB * sizeof(WBlk)));
+  XFP_CUDA(ctx, ctx->tiles.ensure((size_t)NJB * NKB * sizeof(int2)));
+  XFP_CUDA(ctx, ctx->counters.ensure(5 * sizeof(long long)));
+  LayoutDev L{ctx->lines.as<Line>(), ctx->lens.as<int>(), ctx->blks.as<WBlk>(), ctx->tiles.as<int2>(),
+              ctx->counters.as<long long>()};
+  XFP_CUDA(ctx, layout_build(dmat, ni, nj, nk, L, ctx->stream));
+  long long cnt[5];
   XFP_CUDA(ctx, cudaMemcpyAsync(cnt, ctx->counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, ctx->stream));
   XFP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->ni = ni; ctx->nj = nj; ctx->nk = nk;
-  ctx->bnd_ni = ni;
-  ctx->NJt = NJt; ctx->NKt = NKt;
-  ctx->M = cnt[0]; ctx->rows = cnt[1]; ctx->nlines_act = cnt[2]; ctx->ntiles = cnt[3];
+  ctx->NJB = NJB; ctx->NKB = NKB;
+  ctx->M = cnt[0]; ctx->rows = cnt[1]; ctx->nlines_act = cnt[2]; ctx->ntiles = cnt[3]; ctx->Gsw = cnt[4];
   ctx->nlines_all = nlines;
-  XFP_CUDA(ctx, ctx->cell_line.ensure((std::max<long long>(ctx->M, 4) + 8) * sizeof(int)));
+  if (ctx->Gsw * 256 >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "grid too large for the sweep layout");
   XFP_CUDA(ctx, ctx->group_line.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(int)));
-  XFP_CUDA(ctx, build_cell_line(ctx->lines.as<Line>(), nlines, ctx->cell_line.as<int>(), ctx->group_line.as<int>(),
-                                ctx->stream));
-  return build_sweep_layout(ctx);
-}
-
-// Tile table of the sweep layout: per-tile spans on the device, block offsets
-// scanned here (tile order), table uploaded again.
-int build_sweep_layout(xfp_ctx* ctx) {
-  const int nt = (int)ctx->ntiles;
-  XFP_CUDA(ctx, ctx->swt.ensure(std::max(nt, 1) * sizeof(SwTile)));
-  XFP_CUDA(ctx, ctx->tile_pos.ensure((size_t)std::max(ctx->NJt * ctx->NKt, 1) * sizeof(int)));
-  ctx->Msw = 0;
-  if (nt == 0) return XFP_OK;
-  XFP_CUDA(ctx, sw_tiles_build(ctx->lines.as<Line>(), ctx->tiles.as<int>(), nt, ctx->nj, ctx->nk, ctx->nw, ctx->NJt,
-                               ctx->swt.as<SwTile>(), ctx->tile_pos.as<int>(), ctx->stream));
-  std::vector<SwTile> t(nt);
-  XFP_CUDA(ctx, cudaMemcpyAsync(t.data(), ctx->swt.p, nt * sizeof(SwTile), cudaMemcpyDeviceToHost, ctx->stream));
-  XFP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  long long off = 0;
-  for (auto& e : t) {
-    e.off = off;
-    off += (long long)ctx->nw * e.ng * 128;
-  }
-  ctx->Msw = off;
-  if (off >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "grid too large for the sweep layout");
-  XFP_CUDA(ctx, cudaMemcpyAsync(ctx->swt.p, t.data(), nt * sizeof(SwTile), cudaMemcpyHostToDevice, ctx->stream));
-  XFP_CUDA(ctx, ctx->sw_perm.ensure((size_t)(std::max<long long>(ctx->M, 4) + 8) * sizeof(int)));
-  XFP_CUDA(ctx, sw_perm_build(ctx->cell_line.as<int>(), ctx->lines.as<Line>(), ctx->nj, ctx->nw, ctx->NJt,
-                              ctx->tile_pos.as<int>(), ctx->swt.as<SwTile>(), ctx->M, ctx->sw_perm.as<int>(),
-                              ctx->stream));
-  XFP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  XFP_CUDA(ctx, ctx->gperm.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(int)));
+  XFP_CUDA(ctx, build_group_line(ctx->lines.as<Line>(), nlines, ctx->group_line.as<int>(), ctx->stream));
+  XFP_CUDA(ctx, gperm_build(ctx->group_line.as<int>(), ctx->lines.as<Line>(), nj, ctx->blks.as<WBlk>(), NJB, ctx->M, 0,
+                            0, ctx->gperm.as<int>(), ctx->stream));
   return XFP_OK;
 }
-
 
 int ensure_compact(xfp_ctx* ctx, int prec) {
   const size_t M = (size_t)std::max<long long>(ctx->M, 4) + 8;
   if (prec == XFP_PREC_F64 || prec == XFP_PREC_MIXED) {
     for (auto& b : ctx->A64) XFP_CUDA(ctx, b.ensure(M * 8));
-    for (auto& b : ctx->F64) XFP_CUDA(ctx, b.ensure(M * 8));
-    XFP_CUDA(ctx, ctx->inv64.ensure(M * 8));
     XFP_CUDA(ctx, ctx->x64.ensure(M * 8));
     XFP_CUDA(ctx, ctx->r64.ensure(M * 8));
   }
@@ -125,16 +91,10 @@ int ensure_compact(xfp_ctx* ctx, int prec) {
   }
   if (prec == XFP_PREC_F32 || prec == XFP_PREC_MIXED) {
     for (auto& b : ctx->A32) XFP_CUDA(ctx, b.ensure(M * 4));
-    XFP_CUDA(ctx, ctx->inv32.ensure(M * 4));
     XFP_CUDA(ctx, ctx->x32.ensure(M * 4));
     XFP_CUDA(ctx, ctx->r32.ensure(M * 4));
     XFP_CUDA(ctx, ctx->s32.ensure(M * 4));
     XFP_CUDA(ctx, ctx->z32.ensure(M * 4));
-    for (auto& b : ctx->L32) XFP_CUDA(ctx, b.ensure(M * 4));
-  }
-  if (prec == XFP_PREC_F32) {
-    for (auto& b : ctx->F32) XFP_CUDA(ctx, b.ensure(M * 4));
-    XFP_CUDA(ctx, ctx->inv32.ensure(M * 4));
   }
   XFP_CUDA(ctx, ctx->ctl.ensure(sizeof(SweepCtl)));
   XFP_CUDA(ctx, ctx->scal.ensure(sizeof(PcgScalars)));
@@ -142,56 +102,24 @@ int ensure_compact(xfp_ctx* ctx, int prec) {
   XFP_CUDA(ctx, ctx->partials.ensure(NBLK_MAX * sizeof(double)));
   // z.r partials: one per x-line
   XFP_CUDA(ctx, ctx->tpartials.ensure(std::max<long long>(ctx->nlines_all, 1) * sizeof(double)));
-  // stamped tile-boundary words: 4 per cell; zeroed when (re)allocated so no
-  // stale word can carry a live generation
-  const size_t sbytes = M * 4 * sizeof(unsigned long long);
-  for (DevBuf* b : {&ctx->sy, &ctx->sz}) {
-    if (b->cap < sbytes || !b->p) {
-      XFP_CUDA(ctx, b->ensure(sbytes));
-      XFP_CUDA(ctx, cudaMemsetAsync(b->p, 0, b->cap, ctx->stream));
-    }
-  }
-  return XFP_OK;
+  return ensure_sweep(ctx, prec == XFP_PREC_F32 ? 4 : 8);
 }
 
-SweepGrid make_grid(xfp_ctx* ctx, PcgScalars* sc, int bwd_mode) {
-  SweepGrid g;
-  g.ni = ctx->ni; g.nj = ctx->nj; g.nk = ctx->nk;
-  g.NJt = ctx->NJt; g.NKt = ctx->NKt;
-  g.ntiles = (int)ctx->ntiles;
-  g.maxT = ctx->ni + ctx->nj + ctx->nk;
-  g.bwd_mode = bwd_mode;
-  g.lines = ctx->lines.as<Line>();
-  g.tiles = ctx->tiles.as<int>();
-  g.ctl = ctx->ctl.as<SweepCtl>();
-  g.spin_limit = spin_limit(ctx);
-  g.scal = sc;
-  g.trace = ctx->tracing ? ctx->trace.as<int>() : nullptr;
-  g.stage = ctx->stage_solves;
-  return g;
-}
-
-template <typename VT, typename IT, typename CT>
-int run_sweep(xfp_ctx* ctx, int op, const SweepGrid& g, const SweepData<VT, IT, CT>& d) {
+// One sweep on the context's stream (VT, CT: wave_launch).
+template <typename VT, typename CT>
+int run_sweep(xfp_ctx* ctx, int op, const WaveArgs& g) {
   if (g.ntiles <= 0) return XFP_OK;
-  int maxg = sweep_max_grid(op, d, ctx->nw, g.stage);
-  if (maxg <= 0) {
-    const cudaError_t e = cudaGetLastError();
-    return fail(ctx, XFP_ERR_CUDA, std::string("sweep kernel cannot be resident (op ") + std::to_string(op) +
-                                       ", tile height " + std::to_string(ctx->nw) + "): " + cudaGetErrorString(e));
-  }
-  int grid = std::min(maxg, g.ntiles);
   // the forward and backward solve of every event_every-th iteration
   const int ord = op != SWEEP_FACTOR ? ctx->sweep_ord++ : -1;
   const bool timed = ctx->event_every > 0 && ord >= 0 && (ord / 2) % ctx->event_every == 0 &&
                      ctx->sweep_ev_used + 2 <= (int)ctx->sweep_ev.size();
   if (timed) cudaEventRecord(ctx->sweep_ev[ctx->sweep_ev_used], ctx->stream);
-  SweepGrid gl = g;
+  WaveArgs gl = g;
   if (ctx->expire_next_sweep) {
     gl.expect_bias = 1;
     ctx->expire_next_sweep = false;
   }
-  XFP_CUDA(ctx, sweep_launch(op, gl, d, ctx->nw, grid, ctx->stream));
+  XFP_CUDA(ctx, (wave_launch<VT, CT>(op, gl, ctx->stream)));
   if (timed) {
     cudaEventRecord(ctx->sweep_ev[ctx->sweep_ev_used + 1], ctx->stream);
     ctx->sweep_work[ctx->sweep_ev_used / 2] = 1;
@@ -238,23 +166,6 @@ int check_sweep_error(xfp_ctx* ctx) {
   SweepCtl c;
   XFP_CUDA(ctx, cudaMemcpyAsync(&c, ctx->ctl.p, sizeof(c), cudaMemcpyDeviceToHost, ctx->stream));
   XFP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (c.err && ctx->tracing) {
-    std::vector<int> t(ctx->trace.cap / sizeof(int));
-    cudaMemcpy(t.data(), ctx->trace.p, ctx->trace.cap, cudaMemcpyDeviceToHost);
-    int blk = c.err_thread / ((ctx->nw + 1) * 32);
-    fprintf(stderr, "xfp trace: failing block %d, op %d, nw %d (site 0 = not waiting)\n", blk, c.err_op, ctx->nw);
-    for (int b = 0; b < 1024; ++b) {
-      bool any = false;
-      for (int w = 0; w <= ctx->nw; ++w) any |= t[((size_t)b * (ctx->nw + 1) + w) * 4] > 0;
-      if (!any && b != blk) continue;
-      fprintf(stderr, " block %d:", b);
-      for (int w = 0; w <= ctx->nw; ++w) {
-        const int* r = &t[((size_t)b * (ctx->nw + 1) + w) * 4];
-        fprintf(stderr, " w%d[site %d step %d lane %d pub %d]", w, r[0], r[1], r[3], r[2]);
-      }
-      fprintf(stderr, "\n");
-    }
-  }
   if (c.err) {
     char buf[256];
     snprintf(buf, sizeof buf,
@@ -271,32 +182,13 @@ int check_sweep_error(xfp_ctx* ctx) {
   return XFP_OK;
 }
 
-// ---------------------------------------------------------------- factor
-// Zero the factor scratch, then the lower sweep.
-template <typename VT, typename IT, typename CT>
-int factor(xfp_ctx* ctx, const CT* const A[4], CT* const F[6], IT* inv, CT omega, CT ratio) {
-  const size_t M = (size_t)ctx->M;
-  // the factorisation writes L only where a coupling exists: clear the three L arrays first
-  for (int q = 0; q < 3; ++q) XFP_CUDA(ctx, cudaMemsetAsync(F[q], 0, M * sizeof(CT), ctx->stream));
-  XFP_CUDA(ctx, cudaMemsetAsync(inv, 0, M * sizeof(IT), ctx->stream));
-  SweepData<VT, IT, CT> d;
-  d.diag = A[0]; d.ax = A[1]; d.ay = A[2]; d.az = A[3];
-  d.flx = F[0]; d.fly = F[1]; d.flz = F[2];
-  d.oinv = inv;
-  d.sy = ctx->sy.as<unsigned long long>();
-  d.sz = ctx->sz.as<unsigned long long>();
-  d.omega = omega; d.ratio = ratio;
-  SweepGrid g = make_grid(ctx, nullptr, 0);
-  return run_sweep<VT, IT, CT>(ctx, SWEEP_FACTOR, g, d);
-}
-
 // ---------------------------------------------------------------- PCG
-// pcg_solver.h:243-285 on the compact system.  A: coefficient arrays (VT),
-// b: rhs (VT), x: solution (VT), L/inv: factor.  DT: dot accumulation type.
-template <typename VT, typename IT, typename DT>
-int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT* z,
-        const VT* const L[3], const IT* inv, double tol, int maxit, PcgScalars* dsc,
-        PcgScalars* hsc) {
+// pcg_solver.h:243-285 on the compact system; the factor is in the sweep
+// layout.  A: coefficient arrays (VT), b: rhs (VT), x: solution (VT).  DT: dot
+// accumulation type.
+template <typename VT, typename DT>
+int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT* z, double tol, int maxit,
+        PcgScalars* dsc, PcgScalars* hsc) {
   const long long M = ctx->M;
   cudaStream_t st = ctx->stream;
   if (tol < 1e-30) tol = 1e-30;  // set_solver_parameters, pcg_solver.h:237
@@ -304,34 +196,26 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
   XFP_CUDA(ctx, cudaMemsetAsync(dsc, 0, sizeof(PcgScalars), st));
   XFP_CUDA(ctx, copy_vec<VT>(b, r, M, st));
   XFP_CUDA(ctx, absmax_init<VT>(r, M, dsc, ctx->partials.as<double>(), NBLK_MAX, tol, maxit, st));
-  // lines of inactive tiles are never written: their z.r partials stay zero
+  // lines of blocks without cells are never written: their z.r partials stay zero
   XFP_CUDA(ctx, cudaMemsetAsync(ctx->tpartials.p, 0, std::max<long long>(ctx->nlines_all, 1) * sizeof(double), st));
-  SweepData<VT, IT, DT> d;
-  d.r = r; d.y = z; d.lx = L[0]; d.ly = L[1]; d.lz = L[2]; d.inv = inv;
-  d.partials = ctx->tpartials.as<double>();
-  d.sy = ctx->sy.as<unsigned long long>();
-  d.sz = ctx->sz.as<unsigned long long>();
-  SweepGrid gs[2] = {make_grid(ctx, dsc, 0), make_grid(ctx, dsc, 1)};
   int rc;
-  if ((rc = sweep_copies<VT, IT, DT>(ctx, L, inv, r, gs, 2, &d)) != XFP_OK) return rc;
+  if ((rc = sweep_rhs<VT>(ctx, r)) != XFP_OK) return rc;
+  WaveArgs g0 = wave_args(ctx);
+  g0.scal = dsc;
+  WaveArgs g1 = g0;
+  g1.bwd_mode = 1;
   const int first_timed = ctx->sweep_ev_used / 2;
   const int first_kern = ctx->kern_ev_used / 2;
   ctx->sweep_ord = 0;
-  const SweepGrid& g0 = gs[0];
-  const SweepGrid& g1 = gs[1];
-  // with a sweep layout, r is kept in both layouts (update_xr writes both)
-  // and z lives in the sweep layout only (update_s reads it through perm)
+  // r is kept in both layouts (update_xr writes both) and z lives in the sweep
+  // layout only (update_s reads it through gperm)
   const bool swl = ctx->ntiles > 0;
   VT* rsw = swl ? ctx->sw_r.as<VT>() : nullptr;
   const VT* zsw = swl ? ctx->sw_y.as<VT>() : nullptr;
-  const int* perm = swl ? ctx->sw_perm.as<int>() : nullptr;
-  if ((rc = run_sweep<VT, IT, DT>(ctx, SWEEP_FWD, g0, d)) != XFP_OK) return rc;
-  if ((rc = run_sweep<VT, IT, DT>(ctx, SWEEP_BWD, g0, d)) != XFP_OK) return rc;
-  if (swl) {
-    if ((rc = sweep_result<VT>(ctx, s)) != XFP_OK) return rc;
-  } else {
-    XFP_CUDA(ctx, copy_vec<VT>(z, s, M, st));
-  }
+  const int* gperm = swl ? ctx->gperm.as<int>() : nullptr;
+  if ((rc = run_sweep<VT, DT>(ctx, SWEEP_FWD, g0)) != XFP_OK) return rc;
+  if ((rc = run_sweep<VT, DT>(ctx, SWEEP_BWD, g0)) != XFP_OK) return rc;
+  if ((rc = sweep_result<VT>(ctx, s)) != XFP_OK) return rc;
   const int K = ctx->opt.check_every > 0 ? ctx->opt.check_every : 8;
   DT* part = reinterpret_cast<DT*>(ctx->partials.p);
   for (int done_iters = 0;;) {
@@ -342,11 +226,11 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
                                     ctx->nj, ctx->nk, M, dsc, part, ctx->vec_blocks, 0, st);
       }));
       XFP_CUDA(ctx, timed_kernel(ctx, 1, it, [&] {
-        return update_xr<VT, DT>(x, r, s, z, M, dsc, ctx->partials.as<double>(), ctx->xr_blocks, st, rsw, perm);
+        return update_xr<VT, DT>(x, r, s, z, M, dsc, ctx->partials.as<double>(), ctx->xr_blocks, st, rsw, gperm);
       }));
-      if ((rc = run_sweep<VT, IT, DT>(ctx, SWEEP_FWD, g1, d)) != XFP_OK) return rc;
-      if ((rc = run_sweep<VT, IT, DT>(ctx, SWEEP_BWD, g1, d)) != XFP_OK) return rc;
-      XFP_CUDA(ctx, timed_kernel(ctx, 2, it, [&] { return update_s<VT>(s, z, M, dsc, st, zsw, perm, ctx->s_blocks); }));
+      if ((rc = run_sweep<VT, DT>(ctx, SWEEP_FWD, g1)) != XFP_OK) return rc;
+      if ((rc = run_sweep<VT, DT>(ctx, SWEEP_BWD, g1)) != XFP_OK) return rc;
+      XFP_CUDA(ctx, timed_kernel(ctx, 2, it, [&] { return update_s<VT>(s, z, M, dsc, st, zsw, gperm, ctx->s_blocks); }));
     }
     done_iters += K;
     XFP_CUDA(ctx, cudaMemcpyAsync(hsc, dsc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
@@ -380,86 +264,13 @@ float ev_ms(xfp_ctx* ctx, int a, int b) {
 // Assembles, factors and solves.  On return the solution is in x64 (F64,
 // MIXED) or x32 (F32) in compact layout.  rhs_from_adjoint: when non-null, the
 // assembled b is replaced by G^T g (backward pass) before solving.
-//
-// Tile height (options.tile_k == 0): the first solve of a grid shape builds
-// the layout at each candidate height, assembles and factors in FP32 and
-// times two forward+backward sweep pairs; the fastest height is cached in the
-// context for that shape and precision.
+
 // The compute stream waits for the face gather of the I/O stream (host-pointer
 // mode, face-sparse) before it first reads the velocities.
 int inputs_ready(xfp_ctx* ctx) {
   if (!ctx->io_pending) return XFP_OK;
   ctx->io_pending = false;
   XFP_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_io_in, 0));
-  return XFP_OK;
-}
-
-template <typename IOT>
-int tune_tile_height(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const IOT* du_, const IOT* dv,
-                     const IOT* dw, const IOT* dwu, const IOT* dwv, const IOT* dww) {
-  if (ctx->opt.tile_k != 0) {
-    ctx->nw = ctx->opt.tile_k;
-    return XFP_OK;
-  }
-  const std::string key = std::to_string(ni) + "x" + std::to_string(nj) + "x" + std::to_string(nk) + ":" +
-                          std::to_string(ctx->opt.precision);
-  auto it = ctx->tuned_nw.find(key);
-  if (it != ctx->tuned_nw.end()) {
-    ctx->nw = it->second;
-    return XFP_OK;
-  }
-  cudaStream_t st = ctx->stream;
-  float best = 0.f;
-  int best_nw = 8;
-  if (int rc0 = inputs_ready(ctx)) return rc0;
-  cudaEvent_t e0, e1;
-  XFP_CUDA(ctx, cudaEventCreate(&e0));
-  XFP_CUDA(ctx, cudaEventCreate(&e1));
-  int rc = XFP_OK;
-  for (int cand : {8, 15, 16}) {
-    ctx->nw = cand;
-    if ((rc = build_layout(ctx, dmat, ni, nj, nk)) != XFP_OK) break;
-    if ((rc = ensure_compact(ctx, XFP_PREC_F32)) != XFP_OK) break;
-    if (ctx->ntiles == 0) { best_nw = 8; break; }
-    float* A[5];
-    for (int q = 0; q < 5; ++q) A[q] = ctx->A32[q].as<float>();
-    if (assemble<IOT, float>(dmat, du_, dv, dw, dwu, dwv, dww, ni, nj, nk, ctx->lines.as<Line>(), A[0], A[1], A[2],
-                             A[3], A[4], st, ctx->opt.matrix) != cudaSuccess) { rc = fail(ctx, XFP_ERR_CUDA, "assembly failed"); break; }
-    float* F[6];
-    for (int q = 0; q < 6; ++q) F[q] = ctx->F32[q].as<float>();
-    const float* Ac[4] = {A[0], A[1], A[2], A[3]};
-    if ((rc = factor<float, float, float>(ctx, Ac, F, ctx->inv32.as<float>(), 0.97f, 0.25f)) != XFP_OK) break;
-    SweepData<float, float, float> d;
-    d.r = A[4]; d.y = ctx->z32.as<float>(); d.lx = F[0]; d.ly = F[1]; d.lz = F[2]; d.inv = ctx->inv32.as<float>();
-    d.partials = ctx->tpartials.as<double>();
-    d.sy = ctx->sy.as<unsigned long long>();
-    d.sz = ctx->sz.as<unsigned long long>();
-    SweepGrid g = make_grid(ctx, nullptr, 0);
-    const float* Lc[3] = {F[0], F[1], F[2]};
-    if ((rc = sweep_copies<float, float, float>(ctx, Lc, ctx->inv32.as<float>(), A[4], &g, 1, &d)) != XFP_OK) break;
-    const int maxg = std::min(sweep_max_grid(SWEEP_FWD, d, cand, g.stage),
-                              sweep_max_grid(SWEEP_BWD, d, cand, g.stage));
-    if (maxg <= 0) continue;
-    const int grid = std::min(maxg, (int)ctx->ntiles);
-    cudaError_t e = sweep_launch(SWEEP_FWD, g, d, cand, grid, st);   // warm-up
-    if (e == cudaSuccess) e = cudaEventRecord(e0, st);
-    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
-      e = sweep_launch(SWEEP_FWD, g, d, cand, grid, st);
-      if (e == cudaSuccess) e = sweep_launch(SWEEP_BWD, g, d, cand, grid, st);
-    }
-    if (e == cudaSuccess) e = cudaEventRecord(e1, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) { rc = fail(ctx, XFP_ERR_CUDA, std::string("tile height timing: ") + cudaGetErrorString(e)); break; }
-    if ((rc = check_sweep_error(ctx)) != XFP_OK) break;
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    if (cand == 8 || ms < best) { best = ms; best_nw = cand; }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (rc != XFP_OK) return rc;
-  ctx->tuned_nw[key] = best_nw;
-  ctx->nw = best_nw;
   return XFP_OK;
 }
 
@@ -471,7 +282,6 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
   cudaStream_t st = ctx->stream;
   int rc;
   ev_record(ctx, 0);
-  if ((rc = tune_tile_height<IOT>(ctx, ni, nj, nk, dmat, du_, dv, dw, dwu, dwv, dww)) != XFP_OK) return rc;
   ctx->sweep_ev_used = 0;
   ctx->kern_ev_used = 0;
   if ((rc = build_layout(ctx, dmat, ni, nj, nk)) != XFP_OK) return rc;
@@ -482,47 +292,41 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
   ctx->iters = 0; ctx->refinements = 0; ctx->res = 0; ctx->bnorm = 0;
   PcgScalars* dsc = ctx->scal.as<PcgScalars>();
   PcgScalars& hsc = ctx->host_sc;
-  const double tol = ctx->opt.tol, omega = ctx->opt.omega, ratio = ctx->opt.min_diag_ratio;
+  const double tol = ctx->opt.tol;
   const int maxit = ctx->opt.max_iter;
 
   if (prec == XFP_PREC_F64) {
     double* A[5];
     for (int q = 0; q < 5; ++q) A[q] = ctx->A64[q].as<double>();
     XFP_CUDA(ctx, (assemble<IOT, double>(dmat, du_, dv, dw, dwu, dwv, dww, ni, nj, nk, lines, A[0], A[1], A[2],
-                                         A[3], A[4], st, ctx->opt.matrix, ctx->force)));
+                                         A[3], A[4], st, ctx->opt.matrix, ctx->force, nullptr,
+                                         ctx->sw_sys.as<double>(), ctx->blks.as<WBlk>())));
     if (adj_gu) XFP_CUDA(ctx, (apply_pressure_T<IOT, double>(dmat, dwu, dwv, dww, adj_gu, adj_gv, adj_gw, ni, nj,
                                                              nk, lines, A[4], st)));
     ev_record(ctx, 1);
-    double* F[6];
-    for (int q = 0; q < 6; ++q) F[q] = ctx->F64[q].as<double>();
     const double* Ac[4] = {A[0], A[1], A[2], A[3]};
-    if ((rc = factor<double, double, double>(ctx, Ac, F, ctx->inv64.as<double>(), omega, ratio)) != XFP_OK) return rc;
+    if ((rc = run_sweep<double, double>(ctx, SWEEP_FACTOR, wave_args(ctx))) != XFP_OK) return rc;
     if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
     ev_record(ctx, 2);
-    const double* Lc[3] = {F[0], F[1], F[2]};
-    rc = pcg<double, double, double>(ctx, Ac, A[4], ctx->x64.as<double>(), ctx->r64.as<double>(),
-                                     ctx->s64.as<double>(), ctx->z64.as<double>(), Lc, ctx->inv64.as<double>(),
-                                     tol, maxit, dsc, &hsc);
+    rc = pcg<double, double>(ctx, Ac, A[4], ctx->x64.as<double>(), ctx->r64.as<double>(), ctx->s64.as<double>(),
+                             ctx->z64.as<double>(), tol, maxit, dsc, &hsc);
     ev_record(ctx, 3);
     ctx->iters = hsc.iters; ctx->res = hsc.res; ctx->bnorm = hsc.bnorm;
   } else if (prec == XFP_PREC_F32) {
     float* A[5];
     for (int q = 0; q < 5; ++q) A[q] = ctx->A32[q].as<float>();
     XFP_CUDA(ctx, (assemble<IOT, float>(dmat, du_, dv, dw, dwu, dwv, dww, ni, nj, nk, lines, A[0], A[1], A[2],
-                                        A[3], A[4], st, ctx->opt.matrix, ctx->force)));
+                                        A[3], A[4], st, ctx->opt.matrix, ctx->force, nullptr,
+                                        ctx->sw_sys.as<float>(), ctx->blks.as<WBlk>())));
     if (adj_gu) XFP_CUDA(ctx, (apply_pressure_T<IOT, float>(dmat, dwu, dwv, dww, adj_gu, adj_gv, adj_gw, ni, nj,
                                                             nk, lines, A[4], st)));
     ev_record(ctx, 1);
-    float* F[6];
-    for (int q = 0; q < 6; ++q) F[q] = ctx->F32[q].as<float>();
     const float* Ac[4] = {A[0], A[1], A[2], A[3]};
-    if ((rc = factor<float, float, float>(ctx, Ac, F, ctx->inv32.as<float>(), (float)omega, (float)ratio)) != XFP_OK)
-      return rc;
+    if ((rc = run_sweep<float, float>(ctx, SWEEP_FACTOR, wave_args(ctx))) != XFP_OK) return rc;
     if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
     ev_record(ctx, 2);
-    const float* Lc[3] = {F[0], F[1], F[2]};
-    rc = pcg<float, float, float>(ctx, Ac, A[4], ctx->x32.as<float>(), ctx->r32.as<float>(), ctx->s32.as<float>(),
-                                  ctx->z32.as<float>(), Lc, ctx->inv32.as<float>(), tol, maxit, dsc, &hsc);
+    rc = pcg<float, float>(ctx, Ac, A[4], ctx->x32.as<float>(), ctx->r32.as<float>(), ctx->s32.as<float>(),
+                           ctx->z32.as<float>(), tol, maxit, dsc, &hsc);
     ev_record(ctx, 3);
     ctx->iters = hsc.iters; ctx->res = hsc.res; ctx->bnorm = hsc.bnorm;
   } else {
@@ -533,20 +337,16 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
     for (int q = 0; q < 4; ++q) A32[q] = ctx->A32[q].as<float>();
     // the FP32 stencil comes out of the same assembly pass
     XFP_CUDA(ctx, (assemble<IOT, double>(dmat, du_, dv, dw, dwu, dwv, dww, ni, nj, nk, lines, A[0], A[1], A[2],
-                                         A[3], A[4], st, ctx->opt.matrix, ctx->force, A32)));
+                                         A[3], A[4], st, ctx->opt.matrix, ctx->force, A32,
+                                         ctx->sw_sys.as<double>(), ctx->blks.as<WBlk>())));
     if (adj_gu) XFP_CUDA(ctx, (apply_pressure_T<IOT, double>(dmat, dwu, dwv, dww, adj_gu, adj_gv, adj_gw, ni, nj,
                                                              nk, lines, A[4], st)));
     ev_record(ctx, 1);
-    double* F[6];
-    for (int q = 0; q < 6; ++q) F[q] = ctx->F64[q].as<double>();
-    const double* Ac[4] = {A[0], A[1], A[2], A[3]};
-    if ((rc = factor<float, double, double>(ctx, Ac, F, ctx->inv64.as<double>(), omega, ratio)) != XFP_OK) return rc;
+    // the factorisation runs in FP64; the FP32 solves stream its L and pivots
+    // rounded to FP32
+    if ((rc = run_sweep<float, double>(ctx, SWEEP_FACTOR, wave_args(ctx))) != XFP_OK) return rc;
     if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
-    for (int q = 0; q < 3; ++q) XFP_CUDA(ctx, (convert<double, float>(F[q], ctx->L32[q].as<float>(), M, st)));
-    // the pivots are computed in FP64 (above); the FP32 solves stream them rounded to FP32
-    XFP_CUDA(ctx, (convert<double, float>(ctx->inv64.as<double>(), ctx->inv32.as<float>(), M, st)));
     ev_record(ctx, 2);
-    const float* Lc[3] = {ctx->L32[0].as<float>(), ctx->L32[1].as<float>(), ctx->L32[2].as<float>()};
     const float* A32c[4] = {A32[0], A32[1], A32[2], A32[3]};
     double* x64 = ctx->x64.as<double>();
     double* r64 = ctx->r64.as<double>();
@@ -581,9 +381,8 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
         // inner rhs lives in s32 scratch's partner: use r32 as b, z32/s32/x32 work
         float* b32 = ctx->A32[4].as<float>();
         XFP_CUDA(ctx, copy_vec<float>(ctx->r32.as<float>(), b32, M, st));
-        int irc = pcg<float, float, double>(ctx, A32c, b32, ctx->x32.as<float>(), ctx->r32.as<float>(),
-                                            ctx->s32.as<float>(), ctx->z32.as<float>(), Lc,
-                                            ctx->inv32.as<float>(), inner, maxit - total, dsc, &hsc);
+        int irc = pcg<float, double>(ctx, A32c, b32, ctx->x32.as<float>(), ctx->r32.as<float>(),
+                                     ctx->s32.as<float>(), ctx->z32.as<float>(), inner, maxit - total, dsc, &hsc);
         if (irc < 0) return irc;
         total += hsc.iters;
         XFP_CUDA(ctx, refine_update(x64, ctx->x32.as<float>(), M, st));
@@ -1028,73 +827,66 @@ int dump_dense(xfp_ctx* ctx, const T* compact, double* host_out) {
   return XFP_OK;
 }
 
-// VT/IT/CT as in the solve of the context's precision; A: coefficients used by
-// the factor (CT) and by the SpMV (VT).  SIT: the inverse-pivot type the
-// triangular solves stream (the mixed form factors in FP64 and solves with an
-// FP32 copy, as its PCG does); the dumped inv is the factor's own.
-template <typename VT, typename IT, typename CT, typename SIT = IT>
-int debug_core(xfp_ctx* ctx, const CT* const Af[5], const VT* const Av[4], CT* const F[6], IT* inv,
-               const VT* const L[3], const double* dr, double* out[12]) {
+// VT/CT as in the solve of the context's precision (the mixed form factors in
+// FP64 and solves with an FP32 copy; the dumped factor is the FP64 one).  Af:
+// the system (CT), Av: the SpMV's coefficients (VT), F: line-layout scratch.
+template <typename VT, typename CT>
+int debug_core(xfp_ctx* ctx, const CT* const Af[5], const VT* const Av[4], const double* dr, double* out[12]) {
   int rc;
   const long long M = ctx->M;
   cudaStream_t st = ctx->stream;
-  if ((rc = factor<VT, IT, CT>(ctx, Af, F, inv, (CT)ctx->opt.omega, (CT)ctx->opt.min_diag_ratio))) return rc;
-  if (!std::is_same<VT, CT>::value)
-    for (int q = 0; q < 3; ++q) XFP_CUDA(ctx, (convert<CT, VT>(F[q], const_cast<VT*>(L[q]), M, st)));
-  // r -> compact (VT), sweeps, SpMV
-  VT* r = reinterpret_cast<VT*>(ctx->r32.p ? ctx->r32.p : ctx->r64.p);
-  VT* z = reinterpret_cast<VT*>(ctx->z32.p ? ctx->z32.p : ctx->z64.p);
-  VT* qv = reinterpret_cast<VT*>(ctx->s32.p ? ctx->s32.p : ctx->s64.p);
-  if (std::is_same<VT, double>::value) {
-    r = (VT*)ctx->r64.p; z = (VT*)ctx->z64.p; qv = (VT*)ctx->s64.p;
-  }
-  if (dr) {
-    XFP_CUDA(ctx, ctx->io_p.ensure(ncells(ctx->ni, ctx->nj, ctx->nk) * sizeof(double)));
-    XFP_CUDA(ctx, cudaMemcpyAsync(ctx->io_p.p, dr, ncells(ctx->ni, ctx->nj, ctx->nk) * sizeof(double),
-                                  cudaMemcpyHostToDevice, st));
-    XFP_CUDA(ctx, ctx->io_gv.ensure((M + 8) * sizeof(double)));
-    XFP_CUDA(ctx, gather_compact<double>(ctx->io_p.as<double>(), ctx->lines.as<Line>(), ctx->ni, ctx->nj, ctx->nk,
-                                         ctx->io_gv.as<double>(), st));
-    if (std::is_same<VT, double>::value)
-      XFP_CUDA(ctx, copy_vec<double>(ctx->io_gv.as<double>(), (double*)r, M, st));
-    else
-      XFP_CUDA(ctx, (convert<double, float>(ctx->io_gv.as<double>(), (float*)r, M, st)));
-    const SIT* sinv = reinterpret_cast<const SIT*>(inv);
-    if (!std::is_same<SIT, IT>::value) {
-      XFP_CUDA(ctx, ctx->inv32.ensure((M + 8) * sizeof(float)));
-      XFP_CUDA(ctx, (convert<IT, SIT>(inv, reinterpret_cast<SIT*>(ctx->inv32.p), M, st)));
-      sinv = reinterpret_cast<const SIT*>(ctx->inv32.p);
-    }
-    SweepData<VT, SIT, CT> d;
-    d.r = r; d.y = z; d.lx = L[0]; d.ly = L[1]; d.lz = L[2]; d.inv = sinv;
-    d.partials = ctx->tpartials.as<double>();
-    d.sy = ctx->sy.as<unsigned long long>();
-    d.sz = ctx->sz.as<unsigned long long>();
-    SweepGrid g = make_grid(ctx, nullptr, 0);
-    if ((rc = sweep_copies<VT, SIT, CT>(ctx, L, sinv, r, &g, 1, &d))) return rc;
-    if ((rc = run_sweep<VT, SIT, CT>(ctx, SWEEP_FWD, g, d))) return rc;
-    // the solve results are in the sweep layout: back to the line layout
-    if ((rc = sweep_result<VT>(ctx, z))) return rc;
-    XFP_CUDA(ctx, cudaStreamSynchronize(st));
-    if ((rc = dump_dense<VT>(ctx, z, out[9]))) return rc;
-    if ((rc = run_sweep<VT, SIT, CT>(ctx, SWEEP_BWD, g, d))) return rc;
-    if ((rc = sweep_result<VT>(ctx, z))) return rc;
-    XFP_CUDA(ctx, (spmv_dot<VT, VT, VT>(Av[0], Av[1], Av[2], Av[3], r, qv, ctx->lines.as<Line>(),
-                                        ctx->group_line.as<int>(), ctx->nj, ctx->nk, M, nullptr, (VT*)nullptr,
-                                        NBLK_MAX, 1, st)));
-  }
+  const WaveArgs g = wave_args(ctx);
+  if ((rc = run_sweep<CT, CT>(ctx, SWEEP_FACTOR, g))) return rc;
+  DevBuf Fb;
+  XFP_CUDA(ctx, Fb.ensure((size_t)(M + 8) * 4 * sizeof(CT)));
+  CT* F[4];
+  for (int q = 0; q < 4; ++q) F[q] = Fb.as<CT>() + (size_t)(M + 8) * q;
+  struct Release { DevBuf& b; ~Release() { b.release(); } } release{Fb};
+  if (ctx->ntiles > 0)
+    XFP_CUDA(ctx, factor_lines<CT>(ctx->sw_fac.as<CT>(), ctx->lines.as<Line>(), ctx->nj, ctx->nk,
+                                   ctx->blks.as<WBlk>(), ctx->NJB, F, st));
   XFP_CUDA(ctx, cudaStreamSynchronize(st));
   if ((rc = check_sweep_error(ctx))) return rc;
   for (int q = 0; q < 5; ++q)
     if ((rc = dump_dense<CT>(ctx, Af[q], out[q]))) return rc;
-  if ((rc = dump_dense<IT>(ctx, inv, out[5]))) return rc;
+  if ((rc = dump_dense<CT>(ctx, F[3], out[5]))) return rc;
   for (int q = 0; q < 3; ++q)
     if ((rc = dump_dense<CT>(ctx, F[q], out[6 + q]))) return rc;
-  if (dr) {
-    if ((rc = dump_dense<VT>(ctx, z, out[10]))) return rc;
-    if ((rc = dump_dense<VT>(ctx, qv, out[11]))) return rc;
+  if (!dr) return XFP_OK;
+  // r -> compact (VT), sweeps, SpMV
+  VT *r, *z, *qv;
+  if (std::is_same<VT, double>::value) {
+    r = (VT*)ctx->r64.p; z = (VT*)ctx->z64.p; qv = (VT*)ctx->s64.p;
+  } else {
+    r = (VT*)ctx->r32.p; z = (VT*)ctx->z32.p; qv = (VT*)ctx->s32.p;
   }
-  return XFP_OK;
+  XFP_CUDA(ctx, ctx->io_p.ensure(ncells(ctx->ni, ctx->nj, ctx->nk) * sizeof(double)));
+  XFP_CUDA(ctx, cudaMemcpyAsync(ctx->io_p.p, dr, ncells(ctx->ni, ctx->nj, ctx->nk) * sizeof(double),
+                                cudaMemcpyHostToDevice, st));
+  XFP_CUDA(ctx, ctx->io_gv.ensure((M + 8) * sizeof(double)));
+  XFP_CUDA(ctx, gather_compact<double>(ctx->io_p.as<double>(), ctx->lines.as<Line>(), ctx->ni, ctx->nj, ctx->nk,
+                                       ctx->io_gv.as<double>(), st));
+  if (std::is_same<VT, double>::value)
+    XFP_CUDA(ctx, copy_vec<double>(ctx->io_gv.as<double>(), (double*)r, M, st));
+  else
+    XFP_CUDA(ctx, (convert<double, float>(ctx->io_gv.as<double>(), (float*)r, M, st)));
+  if (!std::is_same<VT, CT>::value)
+    if ((rc = run_sweep<VT, CT>(ctx, SWEEP_FACTOR, g))) return rc;
+  if ((rc = sweep_rhs<VT>(ctx, r))) return rc;
+  if ((rc = run_sweep<VT, CT>(ctx, SWEEP_FWD, g))) return rc;
+  // the solve results are in the sweep layout: back to the line layout
+  if ((rc = sweep_result<VT>(ctx, z))) return rc;
+  XFP_CUDA(ctx, cudaStreamSynchronize(st));
+  if ((rc = dump_dense<VT>(ctx, z, out[9]))) return rc;
+  if ((rc = run_sweep<VT, CT>(ctx, SWEEP_BWD, g))) return rc;
+  if ((rc = sweep_result<VT>(ctx, z))) return rc;
+  XFP_CUDA(ctx, (spmv_dot<VT, VT, VT>(Av[0], Av[1], Av[2], Av[3], r, qv, ctx->lines.as<Line>(),
+                                      ctx->group_line.as<int>(), ctx->nj, ctx->nk, M, nullptr, (VT*)nullptr,
+                                      NBLK_MAX, 1, st)));
+  XFP_CUDA(ctx, cudaStreamSynchronize(st));
+  if ((rc = check_sweep_error(ctx))) return rc;
+  if ((rc = dump_dense<VT>(ctx, z, out[10]))) return rc;
+  return dump_dense<VT>(ctx, qv, out[11]);
 }
 
 // ---------------------------------------------------------------- steps either side
@@ -1288,17 +1080,11 @@ int xfp_create(xfp_ctx** out, const xfp_options* opt) {
   ctx->kern_kind.assign(1536, -1);
   ctx->kern_iter.assign(1536, 0);
   for (auto& e : ctx->kern_ev) cudaEventCreate(&e);
-  if (const char* e = getenv("XFP_STAGE_SOLVES")) ctx->stage_solves = atoi(e) != 0;
   if (const char* e = getenv("XFP_VEC_BLOCKS")) ctx->vec_blocks = std::max(148, std::min(xfp_host::NBLK_MAX, atoi(e)));
   if (const char* e = getenv("XFP_KERNEL_EVENTS")) ctx->event_every = std::max(0, atoi(e));
   if (const char* e = getenv("XFP_XR_BLOCKS")) ctx->xr_blocks = std::max(148, std::min(xfp_host::NBLK_MAX, atoi(e)));
   if (const char* e = getenv("XFP_S_BLOCKS")) ctx->s_blocks = std::max(148, std::min(148 * 32, atoi(e)));
   if (const char* e = getenv("XFP_HOST_FACES")) ctx->host_sparse_ok = strcmp(e, "full") != 0;
-  if (getenv("XFP_TRACE")) {
-    ctx->tracing = true;
-    ctx->trace.ensure(1024 * 40 * 4 * sizeof(int));
-    cudaMemset(ctx->trace.p, 0xff, ctx->trace.cap);
-  }
   if (ctx->ctl.ensure(sizeof(SweepCtl)) != cudaSuccess) { xfp_destroy(ctx); return XFP_ERR_NOMEM; }
   SweepCtl c0{};
   c0.gen = 1;
@@ -1313,18 +1099,15 @@ int xfp_destroy(xfp_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   DevBuf* all[] = {&ctx->io_mat, &ctx->io_u, &ctx->io_v, &ctx->io_w, &ctx->io_wu, &ctx->io_wv, &ctx->io_ww,
                    &ctx->io_p, &ctx->io_gu, &ctx->io_gv, &ctx->io_gw, &ctx->lines, &ctx->lens,
-                   &ctx->tile_active, &ctx->tiles, &ctx->counters, &ctx->cell_line, &ctx->group_line, &ctx->inv64, &ctx->inv32, &ctx->x64,
+                   &ctx->blks, &ctx->tiles, &ctx->counters, &ctx->group_line, &ctx->gperm, &ctx->x64,
                    &ctx->r64, &ctx->x32, &ctx->r32, &ctx->s32, &ctx->z32, &ctx->s64, &ctx->z64, &ctx->dense,
-                   &ctx->sy, &ctx->sz, &ctx->bnd, &ctx->ctl, &ctx->scal, &ctx->scal2, &ctx->partials,
+                   &ctx->sw_sys, &ctx->sw_fac, &ctx->sw_r, &ctx->sw_y, &ctx->edge, &ctx->ctl, &ctx->scal, &ctx->scal2, &ctx->partials,
                    &ctx->tpartials};
   for (DevBuf* b : all) b->release();
   batch_state_free(ctx->batch);
   ctx->batch = nullptr;
   for (auto& b : ctx->A64) b.release();
   for (auto& b : ctx->A32) b.release();
-  for (auto& b : ctx->F64) b.release();
-  for (auto& b : ctx->F32) b.release();
-  for (auto& b : ctx->L32) b.release();
   for (auto& e : ctx->ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : ctx->sweep_ev)
@@ -1426,40 +1209,34 @@ int xfp_debug_stages(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* materi
     double* A[5];
     for (int k = 0; k < 5; ++k) A[k] = ctx->A64[k].as<double>();
     XFP_CUDA(ctx, (assemble<double, double>(dmat, du_, dv, dw, dwu, dwv, dww, ni, nj, nk, lines, A[0], A[1], A[2],
-                                            A[3], A[4], st, ctx->opt.matrix)));
-    double* F[6];
-    for (int k = 0; k < 6; ++k) F[k] = ctx->F64[k].as<double>();
+                                            A[3], A[4], st, ctx->opt.matrix, Force3(), nullptr,
+                                            ctx->sw_sys.as<double>(), ctx->blks.as<WBlk>())));
     const double* Af[5] = {A[0], A[1], A[2], A[3], A[4]};
     const double* Av[4] = {A[0], A[1], A[2], A[3]};
-    const double* L[3] = {F[0], F[1], F[2]};
-    return debug_core<double, double, double>(ctx, Af, Av, F, ctx->inv64.as<double>(), L, r, out);
+    return debug_core<double, double>(ctx, Af, Av, r, out);
   } else if (prec == XFP_PREC_F32) {
     float* A[5];
     for (int k = 0; k < 5; ++k) A[k] = ctx->A32[k].as<float>();
     XFP_CUDA(ctx, (assemble<double, float>(dmat, du_, dv, dw, dwu, dwv, dww, ni, nj, nk, lines, A[0], A[1], A[2],
-                                           A[3], A[4], st, ctx->opt.matrix)));
-    float* F[6];
-    for (int k = 0; k < 6; ++k) F[k] = ctx->F32[k].as<float>();
+                                           A[3], A[4], st, ctx->opt.matrix, Force3(), nullptr,
+                                           ctx->sw_sys.as<float>(), ctx->blks.as<WBlk>())));
     const float* Af[5] = {A[0], A[1], A[2], A[3], A[4]};
     const float* Av[4] = {A[0], A[1], A[2], A[3]};
-    const float* L[3] = {F[0], F[1], F[2]};
-    return debug_core<float, float, float>(ctx, Af, Av, F, ctx->inv32.as<float>(), L, r, out);
+    return debug_core<float, float>(ctx, Af, Av, r, out);
   } else {
     double* A[5];
     for (int k = 0; k < 5; ++k) A[k] = ctx->A64[k].as<double>();
     XFP_CUDA(ctx, (assemble<double, double>(dmat, du_, dv, dw, dwu, dwv, dww, ni, nj, nk, lines, A[0], A[1], A[2],
-                                            A[3], A[4], st, ctx->opt.matrix)));
+                                            A[3], A[4], st, ctx->opt.matrix, Force3(), nullptr,
+                                            ctx->sw_sys.as<double>(), ctx->blks.as<WBlk>())));
     float* A32[4];
     for (int k = 0; k < 4; ++k) {
       A32[k] = ctx->A32[k].as<float>();
       XFP_CUDA(ctx, (convert<double, float>(A[k], A32[k], ctx->M, st)));
     }
-    double* F[6];
-    for (int k = 0; k < 6; ++k) F[k] = ctx->F64[k].as<double>();
     const double* Af[5] = {A[0], A[1], A[2], A[3], A[4]};
     const float* Av[4] = {A32[0], A32[1], A32[2], A32[3]};
-    const float* L[3] = {ctx->L32[0].as<float>(), ctx->L32[1].as<float>(), ctx->L32[2].as<float>()};
-    return debug_core<float, double, double, float>(ctx, Af, Av, F, ctx->inv64.as<double>(), L, r, out);
+    return debug_core<float, double>(ctx, Af, Av, r, out);
   }
 }
 

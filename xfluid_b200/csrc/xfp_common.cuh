@@ -44,18 +44,31 @@ struct Force3 {
   __host__ __device__ bool axis_on(int a) const { return on && (d[a] > 1e-10 || d[a] < -1e-10); }
 };
 
-// Sweep-ordered copy ("sweep layout") of the arrays the triangular solves
-// stream.  For every active tile, compute warp (k) and group g of 4 forward
-// wavefront steps (steps 4g..4g+3) it holds a block of 32 lanes x 4 cells:
-// element [off + (w*ng + g - g0)*128 + lane*4 + e] is the cell of line
-// (j0+lane, k0+w) at forward step 4g+e, or zero where that line has no cell.
-// A warp's group access is then 512 contiguous bytes (4-byte values) instead
-// of 32 scattered 16-byte pieces.  g0/ng: the tile's first group and group
-// count (its step span, both sweep directions); off: its first element.
-struct __align__(16) SwTile {
-  long long off;
-  int g0, ng;
+// Sweep layout: the arrays the MIC(0) sweeps stream, in the order they use
+// them.  The lines are cut into blocks of 8 x 8 (j, k); a block's cells are kept
+// by groups of 4 wavefront steps t = i+j+k, group g holding steps 4g..4g+3.
+// Element [(goff + g - g0)*256 + wave_line_slot(j, k) + (t & 3)] is line (j,k)'s
+// cell of step t, zero where the line has none.  g0/ng: the block's first
+// group and group count; goff: its first group in the arrays (scene-relative
+// in a batch: BatchSeg::group_base).  ng = 0: no cells.
+struct __align__(16) WBlk {
+  int goff, g0, ng, pad;
 };
+// The factor (px, py, pz, inv) and the factorisation's system (diag and the
+// couplings to the higher cells) keep four values per cell, 1024 per group:
+// value a of line (j,k)'s cell of step 4g+e, so that a warp's step reads whole
+// 16-byte units of consecutive cells and each half of a block (k & 4) is contiguous.
+template <typename T>
+__host__ __device__ __forceinline__ int wave_cell_slot(int j, int k, int e, int a) {
+  constexpr int V = 16 / (int)sizeof(T), U = 4 / V;   // values per unit, units per cell
+  return (((((k & 7) >> 2) * 4 + e) * U + a / V) * 32 + (k & 3) * 8 + (j & 7)) * V + a % V;
+}
+// The wavefront kernel's clusters: WAVE_TJ x 2 CTAs of two blocks along k, a tile
+// of WAVE_TJ x WAVE_TK blocks (32 x 32 lines)
+constexpr int WAVE_TJ = 4, WAVE_TK = 4, WAVE_CLUSTER = 8;
+__host__ __device__ __forceinline__ int wave_line_slot(int j, int k) {
+  return (k & 1) * 128 + (((k & 7) >> 1) * 8 + (j & 7)) * 4;
+}
 
 // Control block of the persistent sweep kernels (one per context).
 struct SweepCtl {
@@ -65,7 +78,8 @@ struct SweepCtl {
   unsigned int err_where;  // which wait ran out first (diagnostics)
   int err_tile, err_tau, err_thread, err_op;
   unsigned long long err_word;   // the word the failed wait last saw
-  unsigned int err_expect, err_pad;
+  unsigned int err_expect;
+  unsigned int ticket;           // tiles handed out in the current launch
 };
 
 // One scene of a batch: its grid, its slice [base, base+M) of the compact
@@ -76,38 +90,64 @@ struct BatchSeg {
   int blk_lines, blk_lines_start;   // line-based kernels (residual)
   int blk_cells, blk_cells_start;   // cell-based kernels (updates, norms)
   int blk_groups, blk_groups_start; // the SpMV (one thread per 4-cell group)
-  int tile_base;                    // first slot of this scene's (K, J) -> tile map
+  long long blk_base, group_base;   // first entry of this scene's block table, first group of its sweep slice
+  long long line_base;              // its first line among all scenes'
   long long base, M;
   const Line* lines;
   double* partials;                 // this scene's reduction slots
-  long long line_base;              // first line of this scene in the batch's line table
 };
 
-// z.r from one partial per x-line, in an order that depends only on the
-// number of lines (never on the sweep's tile shape): 256 contiguous chunks,
-// each summed in line order, then a fixed pairwise tree.  Called by every
-// thread of a block of at least 256 threads; the sum is returned to all.
-template <bool F32>
-__device__ __forceinline__ double line_sum(const double* __restrict__ part, long long n, double* s) {
-  const int t = threadIdx.x;
-  if (t < 256) {
-    const long long C = (n + 255) / 256, a = (long long)t * C, b = a + C < n ? a + C : n;
-    double acc = 0.0;
-    float accf = 0.f;
-    for (long long q = a; q < b; ++q) {
-      const double v = ((volatile const double*)part)[q];
-      if (F32) accf = __fadd_rn(accf, (float)v); else acc = __dadd_rn(acc, v);
+// The sum of n per-line partials, in a fixed order: 256 chunks of C consecutive
+// lines, each summed in line order, then a fixed tree.  A lane's chain of C
+// additions is what it costs, so the chunks go to as many warps as there are:
+// a warp takes NCH chunks from `first` on (lane q's sum in lane q), P lines of
+// each at a time through buf, NCH * (P + 1) words of its own.
+template <bool F32, int NCH, int P>
+__device__ __forceinline__ double chunk_sums(const double* __restrict__ part, long long n, int first, double* buf) {
+  const int lane = threadIdx.x & 31;
+  const long long C = (n + 255) / 256;
+  double acc = 0.0;
+  float accf = 0.f;
+  for (long long o = 0; o < C; o += P) {
+    double v[NCH * P / 32];
+#pragma unroll
+    for (int i = 0; i < NCH * P / 32; ++i) {
+      const int e = i * 32 + lane;
+      const long long w = o + e % P, q = (first + e / P) * C + w;
+      v[i] = w < C && q < n ? __ldcg(part + q) : 0.0;
     }
-    s[t] = F32 ? (double)accf : acc;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NCH * P / 32; ++i) {
+      const int e = i * 32 + lane;
+      buf[(e / P) * (P + 1) + e % P] = v[i];
+    }
+    __syncwarp();
+    if (lane < NCH) {
+      const int m = C - o < P ? (int)(C - o) : P;
+#pragma unroll 8
+      for (int w = 0; w < m; ++w) {
+        const double x = buf[lane * (P + 1) + w];
+        if (F32) accf = __fadd_rn(accf, (float)x); else acc = __dadd_rn(acc, x);
+      }
+    }
   }
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if (t < h) s[t] = F32 ? (double)__fadd_rn((float)s[t], (float)s[t + h]) : __dadd_rn(s[t], s[t + h]);
-    __syncthreads();
-  }
-  const double r = s[0];
-  __syncthreads();
-  return r;
+  return F32 ? (double)accf : acc;
+}
+// the tree over the 256 chunk sums, by one warp; returned to lane 0
+template <bool F32>
+__device__ __forceinline__ double chunk_tree(const double* s) {
+  auto add = [](double a, double b) { return F32 ? (double)__fadd_rn((float)a, (float)b) : __dadd_rn(a, b); };
+  double v[8];
+#pragma unroll
+  for (int m = 0; m < 8; ++m) v[m] = s[(threadIdx.x & 31) + 32 * m];
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int m = 0; m < h; ++m) v[m] = add(v[m], v[m + h]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v[0] = add(v[0], __shfl_down_sync(XFP_FULL, v[0], o));
+  return v[0];
 }
 
 // Scalars of one PCG solve, resident on the device.

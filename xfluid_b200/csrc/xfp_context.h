@@ -4,7 +4,6 @@
 #pragma once
 
 #include <algorithm>
-#include <map>
 #include <string>
 #include <vector>
 
@@ -55,27 +54,21 @@ struct xfp_ctx {
   // I/O staging (host-pointer mode)
   DevBuf io_mat, io_u, io_v, io_w, io_wu, io_wv, io_ww, io_p, io_gu, io_gv, io_gw;
   // layout
-  DevBuf lines, lens, tile_active, tiles, counters, cell_line, group_line;
+  DevBuf lines, lens, blks, tiles, counters, group_line;
   // compact arrays
   DevBuf A64[5];                  // diag, ax, ay, az, b (FP64)
   DevBuf A32[5];                  // same in FP32
-  DevBuf F64[6], F32[6];          // factor scratch: L and missing per direction
-  DevBuf inv64, inv32, L32[3];
   DevBuf x64, r64, x32, r32, s32, z32, s64, z64, dense;
   // control
-  DevBuf ctl, scal, scal2, partials, tpartials, sy, sz, trace;
+  DevBuf ctl, scal, scal2, partials, tpartials;
   // particle steps (xfp_particles.cu): staged particles and field, bin keys,
   // indices, boxes, positions, bin starts, box spans, sort/scan scratch
   DevBuf part_io, phi_io, part_key, part_idx, part_box, part_pos, part_sbox, part_spos, part_start, part_span,
       part_tmp;
-  // sweep layout (SwTile): tile table, (K,J) -> tile map, cell -> element map
-  // and the copies the solves stream (lx, ly, lz, inv, r, y; 8 bytes per
-  // element covers every precision)
-  DevBuf swt, tile_pos, sw_perm, sw_l[3], sw_inv, sw_r, sw_y;
-  // the triangular solves' tile-boundary rows (SweepData::bk, bj), and the
-  // largest ni of the layout, which sets the rows per tile
-  DevBuf bnd;
-  int bnd_ni = 0;
+  // sweep layout (WBlk), Gsw groups: the factorisation's operands, the factor,
+  // r and y/z, the line-group -> element map, and the block-edge words (zeroed
+  // when (re)allocated so no stale word can carry a live generation)
+  DevBuf sw_sys, sw_fac, sw_r, sw_y, gperm, edge;
   // host-pointer mode: fluid span per x-line and the two byte counters of
   // the sparse face transfer; bytes moved by the current call; whether its
   // velocities went face-sparse; XFP_HOST_FACES=full turns the sparse
@@ -97,12 +90,7 @@ struct xfp_ctx {
   xfp::Force3 force;
   int step_layers = 0;
   DevBuf xmarker;
-  long long Msw = 0;
-  bool tracing = false;
-  // FP32/mixed triangular solves stage their group blocks through shared
-  // memory with cp.async (1, the default) or load them into registers (0,
-  // XFP_STAGE_SOLVES=0)
-  int stage_solves = 1;
+  long long Gsw = 0, nlines_all = 0;   // groups and x-lines (one scene, or the whole batch)
   // block cap of the PCG loop's SpMV: 148 x 4 measured best at 256^3 (37.4 us
   // per launch, against 38.7 at 148 x 8 and 54.5 at 148 x 2).  XFP_VEC_BLOCKS
   // overrides, within [148, NBLK_MAX]; the dot's reduction order follows it.
@@ -125,9 +113,9 @@ struct xfp_ctx {
   // per thread).  XFP_S_BLOCKS overrides, within [148, 148 x 32].
   int s_blocks = 148 * 8;
   // sizes of the current layout
-  int ni = 0, nj = 0, nk = 0, NJt = 0, NKt = 0, nw = 8;
+  int ni = 0, nj = 0, nk = 0, NJB = 0, NKB = 0;
+  int nw = 8;                     // options.tile_k as reported in the stats
   long long M = 0, rows = 0, nlines_act = 0, ntiles = 0;
-  long long nlines_all = 0;       // lines of the layout (nj*nk, or the whole batch's)
   xfp::PcgScalars host_sc{};
   // stats
   double ms_setup = 0, ms_factor = 0, ms_solve = 0, ms_apply = 0;
@@ -149,8 +137,6 @@ struct xfp_ctx {
   long long launches = 0;
   // batched scenes (xfp_project_batch_*): buffers, tables and tuning cache
   xfp_host::BatchState* batch = nullptr;
-  // single scenes with options.tile_k == 0: tile height picked per grid shape
-  std::map<std::string, int> tuned_nw;
   // xfp_debug_expire_next_sweep: the next sweep launch's boundary waits run out
   bool expire_next_sweep = false;
 };
@@ -194,51 +180,32 @@ int ensure_compact(xfp_ctx* ctx, int prec);
 int check_sweep_error(xfp_ctx* ctx);
 
 
-// Sweep-layout copies of the factor (after it is final in the solve type)
-// and of r; element slots of lanes without a cell stay zero.
-template <typename VT, typename IT, typename CT>
-int sweep_copies(xfp_ctx* ctx, const VT* const L[3], const IT* inv, const VT* r, xfp::SweepGrid* gs, int ng,
-                 xfp::SweepData<VT, IT, CT>* d) {
+// Sweep-layout buffers of the current layout: the factorisation's operands
+// (zeroed: cells that lines do not have stay zero), the factor, r (zeroed) and
+// y in 8 bytes a value, and the block-edge words.
+inline int ensure_sweep(xfp_ctx* ctx, size_t sys_bytes) {
   if (ctx->ntiles == 0) return XFP_OK;
-  const size_t bytes = (size_t)(ctx->Msw + 8) * 8;
-  for (auto& b : ctx->sw_l) XFP_CUDA(ctx, b.ensure(bytes));
-  XFP_CUDA(ctx, ctx->sw_inv.ensure(bytes));
-  XFP_CUDA(ctx, ctx->sw_r.ensure(bytes));
-  XFP_CUDA(ctx, ctx->sw_y.ensure(bytes));
-  cudaStream_t st = ctx->stream;
-  const int* perm = ctx->sw_perm.as<int>();
-  for (int q = 0; q < 3; ++q) {
-    XFP_CUDA(ctx, cudaMemsetAsync(ctx->sw_l[q].p, 0, (size_t)ctx->Msw * sizeof(VT), st));
-    XFP_CUDA(ctx, xfp::sw_permute<VT>(const_cast<VT*>(L[q]), ctx->sw_l[q].as<VT>(), perm, ctx->M, 0, st));
+  const size_t n = (size_t)ctx->Gsw * 256;
+  XFP_CUDA(ctx, ctx->sw_sys.ensure(n * 4 * 8));
+  XFP_CUDA(ctx, ctx->sw_fac.ensure(n * 4 * 8));
+  XFP_CUDA(ctx, ctx->sw_r.ensure(n * 8));
+  XFP_CUDA(ctx, ctx->sw_y.ensure(n * 8));
+  XFP_CUDA(ctx, cudaMemsetAsync(ctx->sw_sys.p, 0, n * 4 * sys_bytes, ctx->stream));
+  const size_t words = (size_t)ctx->Gsw * 2 * xfp::WAVE_EDGE;
+  if (ctx->edge.cap < words * 8 || !ctx->edge.p) {
+    XFP_CUDA(ctx, ctx->edge.ensure(words * 8));
+    XFP_CUDA(ctx, cudaMemsetAsync(ctx->edge.p, 0, ctx->edge.cap, ctx->stream));
   }
-  XFP_CUDA(ctx, cudaMemsetAsync(ctx->sw_inv.p, 0, (size_t)ctx->Msw * sizeof(IT), st));
-  XFP_CUDA(ctx, xfp::sw_permute<IT>(const_cast<IT*>(inv), ctx->sw_inv.as<IT>(), perm, ctx->M, 0, st));
-  XFP_CUDA(ctx, cudaMemsetAsync(ctx->sw_r.p, 0, (size_t)ctx->Msw * sizeof(VT), st));
-  XFP_CUDA(ctx, xfp::sw_permute<VT>(const_cast<VT*>(r), ctx->sw_r.as<VT>(), perm, ctx->M, 0, st));
-  d->lxs = ctx->sw_l[0].as<VT>();
-  d->lys = ctx->sw_l[1].as<VT>();
-  d->lzs = ctx->sw_l[2].as<VT>();
-  d->invs = ctx->sw_inv.as<IT>();
-  d->rs = ctx->sw_r.as<VT>();
-  d->ys = ctx->sw_y.as<VT>();
-  // boundary rows: per active tile, one row per wavefront step it can span,
-  // 32 k-edge words and nw j-edge words of P 64-bit words each; zeroed when
-  // (re)allocated so no stale word can carry a live generation
-  const int P = (int)(sizeof(VT) / 4);
-  const long long rows = (long long)ctx->bnd_ni + ctx->nw + 36;
-  const size_t kwords = (size_t)ctx->ntiles * rows * 32 * P, jwords = (size_t)ctx->ntiles * rows * ctx->nw * P;
-  const size_t bbytes = (kwords + jwords) * sizeof(unsigned long long);
-  if (ctx->bnd.cap < bbytes || !ctx->bnd.p) {
-    XFP_CUDA(ctx, ctx->bnd.ensure(bbytes));
-    XFP_CUDA(ctx, cudaMemsetAsync(ctx->bnd.p, 0, ctx->bnd.cap, st));
-  }
-  d->bk = ctx->bnd.as<unsigned long long>();
-  d->bj = d->bk + kwords;
-  for (int q = 0; q < ng; ++q) {
-    gs[q].swt = ctx->swt.as<xfp::SwTile>();
-    gs[q].tile_pos = ctx->tile_pos.as<int>();
-    gs[q].brows = (int)rows;
-  }
+  return XFP_OK;
+}
+
+// r into the sweep layout, ready for the solves.
+template <typename VT>
+int sweep_rhs(xfp_ctx* ctx, const VT* r) {
+  if (ctx->ntiles == 0) return XFP_OK;
+  XFP_CUDA(ctx, cudaMemsetAsync(ctx->sw_r.p, 0, (size_t)ctx->Gsw * 256 * sizeof(VT), ctx->stream));
+  XFP_CUDA(ctx, xfp::sw_permute<VT>(const_cast<VT*>(r), ctx->sw_r.as<VT>(), ctx->gperm.as<int>(), ctx->M, 0,
+                                    ctx->stream));
   return XFP_OK;
 }
 
@@ -247,8 +214,33 @@ int sweep_copies(xfp_ctx* ctx, const VT* const L[3], const IT* inv, const VT* r,
 template <typename VT>
 int sweep_result(xfp_ctx* ctx, VT* out) {
   if (ctx->ntiles == 0) return XFP_OK;
-  XFP_CUDA(ctx, xfp::sw_permute<VT>(out, ctx->sw_y.as<VT>(), ctx->sw_perm.as<int>(), ctx->M, 1, ctx->stream));
+  XFP_CUDA(ctx, xfp::sw_permute<VT>(out, ctx->sw_y.as<VT>(), ctx->gperm.as<int>(), ctx->M, 1, ctx->stream));
   return XFP_OK;
+}
+
+// The operands every sweep of the current layout shares.
+inline xfp::WaveArgs wave_args(xfp_ctx* ctx) {
+  xfp::WaveArgs g;
+  g.nj = ctx->nj;
+  g.nk = ctx->nk;
+  g.NJB = ctx->NJB;
+  g.NKB = ctx->NKB;
+  g.ntiles = (int)ctx->ntiles;
+  g.tiles = ctx->tiles.as<int2>();
+  g.blks = ctx->blks.as<xfp::WBlk>();
+  g.ctl = ctx->ctl.as<xfp::SweepCtl>();
+  g.spin_limit = spin_limit(ctx);
+  g.omega = ctx->opt.omega;
+  g.ratio = ctx->opt.min_diag_ratio;
+  g.sys = ctx->sw_sys.p;
+  g.fac_out = ctx->sw_fac.p;
+  g.fac = ctx->sw_fac.p;
+  g.r = ctx->sw_r.p;
+  g.y = ctx->sw_y.p;
+  g.partials = ctx->tpartials.as<double>();
+  g.bj = ctx->edge.as<unsigned long long>();
+  g.bk = g.bj + (size_t)ctx->Gsw * xfp::WAVE_EDGE;
+  return g;
 }
 
 }  // namespace xfp_host

@@ -14,126 +14,71 @@ enum { SWEEP_FACTOR = 0, SWEEP_FWD = 1, SWEEP_BWD = 2 };
 // launches); a call reports the difference across its own work.
 extern long long g_kernel_launches;
 
-// Static description of one sweep launch (tiles, progress words, control).
-struct SweepGrid {
-  int ni, nj, nk, NJt, NKt, ntiles, maxT;
-  int bwd_mode;                 // backward: 0 = initial rho, 1 = beta update
-  const Line* lines;            // [nk*nj]
-  const int* tiles;             // active tiles, topological order, J | K<<16
-  SweepCtl* ctl;
-  long long spin_limit;
-  PcgScalars* scal;             // forward/backward: skip when done; backward: rho/beta
-  int* trace;                   // optional: per (block, warp) {site, step, progress, tile} while waiting
+// One launch of the wavefront kernel (xfp_wave.cu): blocks, control, operands.
+struct WaveArgs {
+  int nj = 0, nk = 0;           // lines along j and k (one scene)
+  int NJB = 0, NKB = 0;         // 8 x 8-line blocks along j and k (one scene)
+  int ntiles = 0;
+  const int2* tiles = nullptr;  // active tiles (J, K), topological order
+  const WBlk* blks = nullptr;   // block table(s), [K * NJB + J]
+  SweepCtl* ctl = nullptr;
+  long long spin_limit = 0;
+  PcgScalars* scal = nullptr;   // forward/backward: skip when done; backward: rho/beta
+  int bwd_mode = 0;             // backward: 0 = initial rho, 1 = beta update
   // Batch of scenes (null for one scene): scene of each tile, per-scene
   // geometry and scalars.  Tiles of a converged scene are skipped, and the
   // backward dot partials are reduced per scene by batch_bwd_reduce.
   const int* tile_scene = nullptr;
   const BatchSeg* segs = nullptr;
   PcgScalars* scal_batch = nullptr;
-  // Diagnostic (xfp_debug_expire_next_sweep): the loaders expect boundary
-  // words stamped with generation + expect_bias, which no producer writes, so
-  // their bounded waits run out.  0 in normal operation.
+  // Diagnostic (xfp_debug_expire_next_sweep): edge words are expected with
+  // generation + expect_bias, which no producer writes, so the bounded waits
+  // run out.  0 in normal operation.
   unsigned expect_bias = 0;
-  // Sweep layout of the solve arrays (one entry per tile of `tiles`), or null:
-  // the solves then read the factor and write y in the line layout.
-  const SwTile* swt = nullptr;
-  // triangular solves of 4-byte types: stage the group blocks through shared
-  // memory with cp.async (1) or load them into registers (0)
-  int stage = 0;
-  // Triangular solves: (scene tile base + K * NJt + J) -> position in
-  // `tiles`, or -1 for an inactive tile; and the number of boundary rows per
-  // tile (one per wavefront step a tile can span: max ni + tile height + 36).
-  const int* tile_pos = nullptr;
-  int brows = 0;
-};
-
-// Arrays of one sweep.  VT: vector/L type of the solves, IT: invdiag type,
-// CT: factor arithmetic (and A input) type.
-template <typename VT, typename IT, typename CT>
-struct SweepData {
-  const VT* r = nullptr;        // forward: rhs r; backward: r for the fused z.r
-  VT* y = nullptr;              // forward: out y; backward: in y, out z (in place)
-  const VT* lx = nullptr;
-  const VT* ly = nullptr;
-  const VT* lz = nullptr;
-  const IT* inv = nullptr;
-  const CT* diag = nullptr;     // factor inputs
-  const CT* ax = nullptr;
-  const CT* ay = nullptr;
-  const CT* az = nullptr;
-  CT* flx = nullptr;            // factor outputs: L keyed by the higher cell,
-  CT* fly = nullptr;            // lx[c] = L(c,c-1), ly[c] = L(c,c-ni), lz[c] = L(c,c-nn)
-  CT* flz = nullptr;
-  IT* oinv = nullptr;
-  CT omega = CT(0.97), ratio = CT(0.25);
-  double* partials = nullptr;   // backward: one z.r partial per x-line (line table order)
-  // Tile-boundary values published for neighbouring tiles: per cell up to 4
-  // 64-bit words (32-bit payload chunk | launch generation << 32).
-  unsigned long long* sy = nullptr;  // to the j-neighbour tile
-  unsigned long long* sz = nullptr;  // to the k-neighbour tile
-  // Triangular solves: the same words kept by wavefront step instead of by
-  // cell, one row per step of the producing tile, so that a step's
-  // publication and a loader's poll each touch one contiguous row:
-  // bk[((tile * brows + row) * 32 + lane) * P + p] from the tile's k-edge warp,
-  // bj[((tile * brows + row) * NW + warp) * P + p] from its j-edge lanes.
+  double omega = 0.97, ratio = 0.25;
+  // sweep-layout arrays; the factor and the system keep four values per cell
+  // (wave_cell_slot): (px, py, pz, inv) and (diag, A(c+1,c), A(c+ni,c), A(c+nn,c))
+  const void* sys = nullptr;    // factor: the system, arithmetic type
+  void* fac_out = nullptr;      // factor: the result, solve type
+  const void* fac = nullptr;    // solves
+  const void* r = nullptr;      // solves: right-hand side (backward: for z.r)
+  void* y = nullptr;            // forward: out y; backward: in y, out z
+  double* partials = nullptr;   // backward: z.r per line, [k * nj + j]
+  unsigned long long* bj = nullptr;   // block-edge words of the J and K neighbours
   unsigned long long* bk = nullptr;
-  unsigned long long* bj = nullptr;
-  // Sweep-layout copies (used when SweepGrid::swt is set): the factor, r,
-  // and y, which the forward solve writes and the backward solve overwrites
-  // with z (the line-layout r and y are then not touched).
-  const VT* lxs = nullptr;
-  const VT* lys = nullptr;
-  const VT* lzs = nullptr;
-  const IT* invs = nullptr;
-  const VT* rs = nullptr;
-  VT* ys = nullptr;
 };
+// VT: the solves' value type and the stored factor's; CT: the factorisation's
+// arithmetic and the dot type of the backward solve.
+template <typename VT, typename CT>
+cudaError_t wave_launch(int op, const WaveArgs& g, cudaStream_t st);
+// 64-bit words of the J and K edges per group: 4 steps x 8 lines of up to 16
+// bytes (the factorisation's FP64 pair), 32 payload bits a word
+constexpr size_t WAVE_EDGE = 4 * 8 * 4;
 
-// Forward/backward solves (xfp_solve.cu); sweep_launch routes them there.
-template <typename VT, typename IT, typename CT>
-cudaError_t solve_launch(int op, const SweepGrid& g, const SweepData<VT, IT, CT>& d, int nw, int grid,
-                         cudaStream_t st);
-template <typename VT, typename IT, typename CT>
-int solve_max_grid(int op, int nw, int stage);
-
-#define XFP_SWEEP_DECL(VT, IT, CT)                                                             \
-  cudaError_t sweep_launch(int op, const SweepGrid& g, const SweepData<VT, IT, CT>& d, int nw, \
-                           int grid, cudaStream_t st);                                         \
-  int sweep_max_grid(int op, const SweepData<VT, IT, CT>& d, int nw, int stage = 0);
-XFP_SWEEP_DECL(double, double, double)
-XFP_SWEEP_DECL(float, float, float)
-XFP_SWEEP_DECL(float, double, double)   // mixed form: factorisation only
-XFP_SWEEP_DECL(float, float, double)    // mixed form: triangular solves only
-#undef XFP_SWEEP_DECL
-
-// ---- sweep layout (xfp_swlayout.cu) ----
-// Per-tile step spans of the active tiles (off left 0; the host scans them),
-// and the (K*NJt + J) -> tile position map.
-cudaError_t sw_tiles_build(const Line* lines, const int* tiles, int ntiles, int nj, int nk, int nw, int NJt,
-                           SwTile* swt, int* tile_pos, cudaStream_t st);
-// perm[c] = sweep-layout element of stored cell cell_base + c (c < M); the
-// line offsets count from cell 0 of the compact arrays.
-cudaError_t sw_perm_build(const int* cell_line, const Line* lines, int nj, int nw, int NJt, const int* tile_pos,
-                          const SwTile* swt, long long M, int* perm, cudaStream_t st, long long cell_base = 0);
-// Batch form of sw_tiles_build: spans of the merged tile list (tile t in scene tile_scene[t]).
-cudaError_t sw_tiles_build_batch(const int* tiles, const int* tile_scene, const BatchSeg* segs, int ntiles, int nw,
-                                 SwTile* swt, cudaStream_t st);
-// dir 0: sw[perm[c]] = line[c]; dir 1: line[c] = sw[perm[c]] for the M stored cells.
+// gperm[q] = sweep element of line-layout group q's first cell (M stored cells
+// from cell_base on; group_line of those cells, their scene's lines and blocks)
+cudaError_t gperm_build(const int* group_line, const Line* lines, int nj, const WBlk* blks, int NJB, long long M,
+                        long long cell_base, long long group_base, int* gperm, cudaStream_t st);
+// dir 0: sw[gperm] = line; dir 1: line = sw[gperm], for the M stored cells.
 template <typename T>
-cudaError_t sw_permute(T* line, T* sw, const int* perm, long long M, int dir, cudaStream_t st);
+cudaError_t sw_permute(T* line, T* sw, const int* gperm, long long M, int dir, cudaStream_t st);
+// The factor back in the line layout: F = lx, ly, lz (keyed by the higher cell), inv.
+template <typename T>
+cudaError_t factor_lines(const T* fac, const Line* lines, int nj, int nk, const WBlk* blks, int NJB, T* const F[4],
+                         cudaStream_t st);
 
 // ---- layout (xfp_layout.cu) ----
-// Builds the line table and the active-tile list for a material grid.
-// Returns on the host: stored cells M, unknown rows, active lines, active tiles.
+// Builds the line table, the block table and the active-tile list for a
+// material grid.  counters (device): stored cells M, unknown rows, active
+// lines, active tiles, sweep-layout groups.
 struct LayoutDev {
   Line* lines;               // [nk*nj]
   int* line_len_scan;        // scratch [nk*nj + 1]
-  unsigned char* tile_active;// [NKt*NJt]
-  int* tiles;                // [NKt*NJt]
-  long long* counters;       // [4] M, rows, lines, ntiles (device)
+  WBlk* blks;                // [ceil(nk/8) * ceil(nj/8)]
+  int2* tiles;               // active tiles (at most as many as blocks)
+  long long* counters;       // [5]
 };
-cudaError_t layout_build(const uint8_t* mat, int ni, int nj, int nk, int tile_k, LayoutDev L,
-                         cudaStream_t st);
+cudaError_t layout_build(const uint8_t* mat, int ni, int nj, int nk, LayoutDev L, cudaStream_t st);
 
 // ---- assembly / apply / vector kernels (xfp_ops.cu) ----
 template <typename FT, typename AT>
@@ -141,7 +86,9 @@ cudaError_t assemble(const uint8_t* mat, const FT* u, const FT* v, const FT* w, 
                      const FT* wv, const FT* ww, int ni, int nj, int nk, const Line* lines,
                      AT* diag, AT* ax, AT* ay, AT* az, AT* b, cudaStream_t st,
                      int matrix = XFP_MATRIX_VARIATIONAL, Force3 frc = Force3(),
-                     float* const A32[4] = nullptr);   // also write diag..az as FP32 (mixed form)
+                     float* const A32[4] = nullptr,    // also write diag..az as FP32 (mixed form)
+                     AT* sys = nullptr, const WBlk* blks = nullptr, long long group_base = 0);
+// sys: the factorisation's operands in the sweep layout (zeroed by the caller)
 
 template <typename T>
 cudaError_t scatter_dense(const T* x, const Line* lines, int ni, int nj, int nk, T* dense,
@@ -189,18 +136,17 @@ cudaError_t spmv_dot(const AT* diag, const AT* ax, const AT* ay, const AT* az, c
                      DT* partials, int nblk_max, int mode, cudaStream_t st);
 // SpMV blocks for M stored cells (the batch gives each scene the same count).
 long long spmv_block_count(long long M, int nblk_max);
-// cell_line[c] = index of the line storing cell c (for every cell of every
-// line); group_line[c / 4] the same per aligned 4-cell group.
-cudaError_t build_cell_line(const Line* lines, long long nlines, int* cell_line, int* group_line, cudaStream_t st);
-// rsw/perm (optional): the updated r is also stored at rsw[perm[c]].
+// group_line[c / 4] = index of the line storing the aligned 4-cell group of cell c.
+cudaError_t build_group_line(const Line* lines, long long nlines, int* group_line, cudaStream_t st);
+// rsw/gperm (optional): the updated r is also stored at rsw[gperm[c / 4]].
 template <typename VT, typename DT>
 cudaError_t update_xr(VT* x, VT* r, const VT* s, const VT* z, long long M, PcgScalars* sc,
                       double* partials, int nblk_max, cudaStream_t st, VT* rsw = nullptr,
-                      const int* perm = nullptr);
-// zsw/perm (optional): z is read from zsw[perm[c]] instead of z[c].
+                      const int* gperm = nullptr);
+// zsw/gperm (optional): z is read from zsw[gperm[c / 4]] instead of z[c].
 template <typename VT>
 cudaError_t update_s(VT* s, const VT* z, long long M, PcgScalars* sc, cudaStream_t st, const VT* zsw = nullptr,
-                     const int* perm = nullptr, int nblk_max = 148 * 16);
+                     const int* gperm = nullptr, int nblk_max = 148 * 16);
 template <typename VT>
 cudaError_t absmax_init(const VT* b, long long M, PcgScalars* sc, double* partials, int nblk_max,
                         double tol, int maxit, cudaStream_t st);
@@ -218,14 +164,14 @@ template <typename VT, typename AT, typename DT>
 cudaError_t batch_spmv_dot(const BatchSeg* segs, int nseg, int blocks, const AT* diag, const AT* ax,
                            const AT* ay, const AT* az, const VT* s, VT* z, const int* group_line, PcgScalars* sc,
                            int mode, cudaStream_t st);
-// rsw/perm, zsw/perm (optional): as update_xr / update_s, perm indexed by global cell
+// rsw/gperm, zsw/gperm (optional): as update_xr / update_s, gperm indexed by global group
 template <typename VT>
 cudaError_t batch_update_xr(const BatchSeg* segs, int nseg, int blocks, VT* x, VT* r, const VT* s,
                             const VT* z, PcgScalars* sc, cudaStream_t st, VT* rsw = nullptr,
-                            const int* perm = nullptr);
+                            const int* gperm = nullptr);
 template <typename VT>
 cudaError_t batch_update_s(const BatchSeg* segs, int nseg, int blocks, VT* s, const VT* z, PcgScalars* sc,
-                           cudaStream_t st, const VT* zsw = nullptr, const int* perm = nullptr);
+                           cudaStream_t st, const VT* zsw = nullptr, const int* gperm = nullptr);
 // tols/maxits: optional per-scene tolerance and iteration cap (else tol, maxit)
 template <typename VT>
 cudaError_t batch_absmax_init(const BatchSeg* segs, int nseg, int blocks, const VT* b, PcgScalars* sc,
@@ -233,8 +179,8 @@ cudaError_t batch_absmax_init(const BatchSeg* segs, int nseg, int blocks, const 
 cudaError_t batch_residual64(const BatchSeg* segs, int nseg, int blocks, const double* diag, const double* ax,
                              const double* ay, const double* az, const double* b, const double* x, double* r,
                              PcgScalars* sc, cudaStream_t st);
-// Per-scene z.r from the backward sweep's per-line partials (line_sum, the
-// single-scene order); mode 0: rho, mode 1: beta and rho.
+// Per-scene z.r from the backward sweep's line partials, in the single-scene
+// order; mode 0: rho, mode 1: beta and rho.
 template <typename DT>
 cudaError_t batch_bwd_reduce(const BatchSeg* segs, int nseg, const double* line_partials, PcgScalars* sc, int mode,
                              cudaStream_t st);

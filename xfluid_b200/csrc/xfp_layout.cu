@@ -112,37 +112,119 @@ __global__ void line_scan_kernel(Line* __restrict__ lines, const int* __restrict
   }
 }
 
-// Tile activity: a tile is a 32 (j) x tile_k (k) block of lines.
-__global__ void tile_active_kernel(const Line* __restrict__ lines, int nj, int nk, int tile_k,
-                                   int NJt, int NKt, unsigned char* __restrict__ act) {
-  const int t = blockIdx.x;
-  const int J = t % NJt, K = t / NJt;
-  int any = 0;
-  for (int q = threadIdx.x; q < 32 * tile_k; q += blockDim.x) {
-    const int j = J * 32 + (q & 31), k = K * tile_k + (q >> 5);
-    if (j < nj && k < nk && lines[(size_t)k * nj + j].len > 0) any = 1;
-  }
-  any = __syncthreads_or(any);
-  if (threadIdx.x == 0) act[t] = (unsigned char)any;
-}
-
-// Active tiles in topological order of the lower sweep: (J+K) ascending, then J.
-__global__ void tile_order_kernel(const unsigned char* __restrict__ act, int NJt, int NKt,
-                                  int* __restrict__ tiles, long long* __restrict__ counters) {
-  if (threadIdx.x != 0) return;
-  int n = 0;
-  for (int dsum = 0; dsum <= NJt + NKt - 2; ++dsum) {
-    const int jlo = max(0, dsum - (NKt - 1)), jhi = min(dsum, NJt - 1);
-    for (int J = jlo; J <= jhi; ++J) {
-      const int K = dsum - J;
-      if (act[(size_t)K * NJt + J]) tiles[n++] = J | (K << 16);
+// Sweep-layout blocks: one warp per block of 8 x 8 lines finds the span of
+// wavefront groups its cells cover (goff is scanned afterwards).
+__global__ void blk_span_kernel(const Line* __restrict__ lines, int nj, int nk, int NJB, long long nblk,
+                                WBlk* __restrict__ blks) {
+  const int lane = threadIdx.x & 31;
+  const long long b = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (b >= nblk) return;
+  const int jb = (int)(b % NJB), kb = (int)(b / NJB);
+  int lo = INT_MAX, hi = INT_MIN;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int j = jb * 8 + (lane & 7), k = kb * 8 + (lane >> 3) * 2 + h;
+    if (j < nj && k < nk) {
+      const Line L = lines[(size_t)k * nj + j];
+      if (L.len > 0) {
+        lo = min(lo, L.lo + j + k);
+        hi = max(hi, L.lo + L.len - 1 + j + k);
+      }
     }
   }
-  counters[3] = n;
+  lo = __reduce_min_sync(XFP_FULL, lo);
+  hi = __reduce_max_sync(XFP_FULL, hi);
+  if (lane == 0) {
+    WBlk w = {0, 0, 0, 0};
+    if (lo != INT_MAX) {
+      w.g0 = lo >> 2;   // lo may be negative (group padding): arithmetic shift
+      w.ng = (hi >> 2) - (lo >> 2) + 1;
+    }
+    blks[b] = w;
+  }
 }
 
-cudaError_t layout_build(const uint8_t* mat, int ni, int nj, int nk, int tile_k, LayoutDev L,
-                         cudaStream_t st) {
+// Inclusive scan of one value per thread over a block of 1024 threads.
+__device__ __forceinline__ long long scan1024(long long v, long long* sh) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long t = __shfl_up_sync(XFP_FULL, v, o);
+    if (lane >= o) v += t;
+  }
+  if (lane == 31) sh[w] = v;
+  __syncthreads();
+  if (w == 0) {
+    long long t = sh[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(XFP_FULL, t, o);
+      if (lane >= o) t += u;
+    }
+    sh[lane] = t;
+  }
+  __syncthreads();
+  const long long r = v + (w > 0 ? sh[w - 1] : 0);
+  __syncthreads();
+  return r;
+}
+
+// Block offsets (scan in block order) and the active tiles in topological
+// order of the lower sweep: (J+K) ascending, then J.  One CTA.
+__global__ void __launch_bounds__(1024) blk_scan_kernel(WBlk* __restrict__ blks, int NJB, int NKB, int NJT, int NKT,
+                                                        int2* __restrict__ tiles, long long* __restrict__ counters) {
+  __shared__ long long sh[32];
+  __shared__ long long s_tot;
+  const long long nblk = (long long)NJB * NKB, ntile = (long long)NJT * NKT;
+  long long carry = 0;
+  for (long long base = 0; base < nblk; base += 1024) {
+    const long long b = base + threadIdx.x;
+    const long long v = b < nblk ? blks[b].ng : 0;
+    const long long inc = scan1024(v, sh);
+    if (b < nblk) blks[b].goff = (int)(carry + inc - v);
+    if (threadIdx.x == 1023) s_tot = inc;
+    __syncthreads();
+    carry += s_tot;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) counters[4] = carry;
+  // tiles before diagonal d of an NJT x NKT grid
+  auto before = [&](long long d) -> long long {
+    const long long m = min(NJT, NKT), M = max(NJT, NKT);
+    if (d <= m) return d * (d + 1) / 2;
+    if (d <= M) return m * (m + 1) / 2 + (d - m) * m;
+    const long long left = m + M - 1 - d;   // diagonals from d on
+    return ntile - left * (left + 1) / 2;
+  };
+  carry = 0;
+  for (long long base = 0; base < ntile; base += 1024) {
+    const long long q = base + threadIdx.x;
+    int2 t = make_int2(0, 0);
+    long long act = 0;
+    if (q < ntile) {
+      long long lo = 0, hi = (long long)NJT + NKT - 2;   // the diagonal holding the q-th tile
+      while (lo < hi) {
+        const long long mid = (lo + hi + 1) >> 1;
+        if (before(mid) <= q) lo = mid; else hi = mid - 1;
+      }
+      const int J = (int)(max(0LL, lo - (NKT - 1)) + (q - before(lo)));
+      t = make_int2(J, (int)lo - J);
+      for (int a = 0; a < WAVE_TJ * WAVE_TK; ++a) {
+        const int jb = t.x * WAVE_TJ + a % WAVE_TJ, kb = t.y * WAVE_TK + a / WAVE_TJ;
+        if (jb < NJB && kb < NKB && blks[(long long)kb * NJB + jb].ng > 0) act = 1;
+      }
+    }
+    const long long inc = scan1024(act, sh);
+    if (act) tiles[carry + inc - 1] = t;
+    if (threadIdx.x == 1023) s_tot = inc;
+    __syncthreads();
+    carry += s_tot;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) counters[3] = carry;
+}
+
+cudaError_t layout_build(const uint8_t* mat, int ni, int nj, int nk, LayoutDev L, cudaStream_t st) {
   const long long nlines = (long long)nj * nk;
   const int wpb = 8;
   ++g_kernel_launches;
@@ -150,11 +232,13 @@ cudaError_t layout_build(const uint8_t* mat, int ni, int nj, int nk, int tile_k,
                                                                               L.line_len_scan);
   ++g_kernel_launches;
   line_scan_kernel<<<1, 1024, 0, st>>>(L.lines, L.line_len_scan, nlines, L.counters);
-  const int NJt = (nj + 31) / 32, NKt = (nk + tile_k - 1) / tile_k;
+  const int NJB = (nj + 7) / 8, NKB = (nk + 7) / 8;
+  const long long nblk = (long long)NJB * NKB;
   ++g_kernel_launches;
-  tile_active_kernel<<<NJt * NKt, 256, 0, st>>>(L.lines, nj, nk, tile_k, NJt, NKt, L.tile_active);
+  blk_span_kernel<<<(unsigned)((nblk + wpb - 1) / wpb), wpb * 32, 0, st>>>(L.lines, nj, nk, NJB, nblk, L.blks);
   ++g_kernel_launches;
-  tile_order_kernel<<<1, 32, 0, st>>>(L.tile_active, NJt, NKt, L.tiles, L.counters);
+  blk_scan_kernel<<<1, 1024, 0, st>>>(L.blks, NJB, NKB, (NJB + WAVE_TJ - 1) / WAVE_TJ, (NKB + WAVE_TK - 1) / WAVE_TK,
+                                      L.tiles, L.counters);
   return cudaGetLastError();
 }
 

@@ -45,7 +45,8 @@ __global__ void assemble_kernel(const uint8_t* __restrict__ mat, const FT* __res
                                 const Line* __restrict__ lines, AT* __restrict__ diag,
                                 AT* __restrict__ ax, AT* __restrict__ ay, AT* __restrict__ az,
                                 AT* __restrict__ b, int matrix, Force3 frc, float* __restrict__ d32,
-                                float* __restrict__ x32, float* __restrict__ y32, float* __restrict__ z32) {
+                                float* __restrict__ x32, float* __restrict__ y32, float* __restrict__ z32,
+                                AT* __restrict__ sys, const WBlk* __restrict__ blks, long long group_base) {
   const int lane = threadIdx.x & 31;
   const long long nlines = (long long)nj * nk;
   const size_t nn = (size_t)ni * nj;
@@ -54,11 +55,14 @@ __global__ void assemble_kernel(const uint8_t* __restrict__ mat, const FT* __res
     const Line L = lines[line];
     if (L.len == 0) continue;
     const int j = (int)(line % nj), k = (int)(line / nj);
+    WBlk blk = {0, 0, 0, 0};
+    if (sys != nullptr) blk = blks[(size_t)(k >> 3) * ((nj + 7) >> 3) + (j >> 3)];
     for (int q = lane; q < L.len; q += 32) {
       const int i = L.lo + q;
       const size_t c = (size_t)k * nn + (size_t)j * ni + i;
       const size_t o = (size_t)L.off + q;
       AT d = AT(0), bb = AT(0), ox = AT(0), oy = AT(0), oz = AT(0);
+      AT ux = AT(0), uy = AT(0), uz = AT(0);   // couplings to the higher cells (the matrix is symmetric)
       const uint8_t m = (i >= 0 && i < ni) ? mat[c] : MAT_AIR;
       if (m == MAT_FLUID || m == MAT_SOLID) {
         // neighbour (di,dj,dk), face value, weight, vsign
@@ -108,6 +112,9 @@ __global__ void assemble_kernel(const uint8_t* __restrict__ mat, const FT* __res
               if (nb == 1) ox = off;
               if (nb == 3) oy = off;
               if (nb == 5) oz = off;
+              if (nb == 0) ux = off;
+              if (nb == 2) uy = off;
+              if (nb == 4) uz = off;
             }
             d = AT(count);
           }
@@ -134,6 +141,9 @@ __global__ void assemble_kernel(const uint8_t* __restrict__ mat, const FT* __res
             if (nb == 1) ox = off;
             if (nb == 3) oy = off;
             if (nb == 5) oz = off;
+            if (nb == 0) ux = off;
+            if (nb == 2) uy = off;
+            if (nb == 4) uz = off;
           }
         } else {
           const int order[6] = {1, 3, 5, 4, 2, 0};
@@ -150,10 +160,22 @@ __global__ void assemble_kernel(const uint8_t* __restrict__ mat, const FT* __res
             if (nb == 1) ox = off;
             if (nb == 3) oy = off;
             if (nb == 5) oz = off;
+            if (nb == 0) ux = off;
+            if (nb == 2) uy = off;
+            if (nb == 4) uz = off;
           }
         }
       }
       diag[o] = d; ax[o] = ox; ay[o] = oy; az[o] = oz; b[o] = bb;
+      // the factorisation's operands, in the sweep layout
+      if (sys != nullptr) {
+        const int t = i + j + k;
+        AT* e = sys + (size_t)(group_base + blk.goff + (t >> 2) - blk.g0) * 1024;
+        e[wave_cell_slot<AT>(j, k, t & 3, 0)] = d;
+        e[wave_cell_slot<AT>(j, k, t & 3, 1)] = ux;
+        e[wave_cell_slot<AT>(j, k, t & 3, 2)] = uy;
+        e[wave_cell_slot<AT>(j, k, t & 3, 3)] = uz;
+      }
       // the mixed form's FP32 stencil, written by the assembly itself
       if (d32 != nullptr) {
         d32[o] = (float)d; x32[o] = (float)ox; y32[o] = (float)oy; z32[o] = (float)oz;
@@ -166,32 +188,36 @@ template <typename FT, typename AT>
 cudaError_t assemble(const uint8_t* mat, const FT* u, const FT* v, const FT* w, const FT* wu,
                      const FT* wv, const FT* ww, int ni, int nj, int nk, const Line* lines,
                      AT* diag, AT* ax, AT* ay, AT* az, AT* b, cudaStream_t st, int matrix, Force3 frc,
-                     float* const A32[4]) {
+                     float* const A32[4], AT* sys, const WBlk* blks, long long group_base) {
   const long long nlines = (long long)nj * nk;
   long long blocks = (nlines + 7) / 8;
   if (blocks > 65535 * 8) blocks = 65535 * 8;
   ++g_kernel_launches;
   assemble_kernel<FT, AT><<<(unsigned)blocks, 256, 0, st>>>(
       mat, u, v, w, wu, wv, ww, ni, nj, nk, lines, diag, ax, ay, az, b, matrix, frc, A32 ? A32[0] : nullptr,
-      A32 ? A32[1] : nullptr, A32 ? A32[2] : nullptr, A32 ? A32[3] : nullptr);
+      A32 ? A32[1] : nullptr, A32 ? A32[2] : nullptr, A32 ? A32[3] : nullptr, sys, blks, group_base);
   return cudaGetLastError();
 }
 template cudaError_t assemble<double, double>(const uint8_t*, const double*, const double*,
                                               const double*, const double*, const double*,
                                               const double*, int, int, int, const Line*, double*,
-                                              double*, double*, double*, double*, cudaStream_t, int, Force3, float* const*);
+                                              double*, double*, double*, double*, cudaStream_t, int, Force3, float* const*,
+                                             double*, const WBlk*, long long);
 template cudaError_t assemble<float, float>(const uint8_t*, const float*, const float*, const float*,
                                             const float*, const float*, const float*, int, int, int,
                                             const Line*, float*, float*, float*, float*, float*,
-                                            cudaStream_t, int, Force3, float* const*);
+                                            cudaStream_t, int, Force3, float* const*,
+                                             float*, const WBlk*, long long);
 template cudaError_t assemble<float, double>(const uint8_t*, const float*, const float*,
                                              const float*, const float*, const float*, const float*,
                                              int, int, int, const Line*, double*, double*, double*,
-                                             double*, double*, cudaStream_t, int, Force3, float* const*);
+                                             double*, double*, cudaStream_t, int, Force3, float* const*,
+                                             double*, const WBlk*, long long);
 template cudaError_t assemble<double, float>(const uint8_t*, const double*, const double*,
                                              const double*, const double*, const double*,
                                              const double*, int, int, int, const Line*, float*,
-                                             float*, float*, float*, float*, cudaStream_t, int, Force3, float* const*);
+                                             float*, float*, float*, float*, cudaStream_t, int, Force3, float* const*,
+                                             float*, const WBlk*, long long);
 
 // ---------------------------------------------------------------------------
 // Compact -> dense pressure grid: every cell written, 0 outside unknowns
@@ -769,13 +795,13 @@ template cudaError_t spmv_dot<float, float, double>(const float*, const float*, 
 // One thread per aligned 4-cell group, with 16-byte vector accesses (two for
 // FP64).  With a sweep layout the group's four cells sit at four consecutive
 // sweep-layout elements (consecutive forward steps, aligned to a group of 4),
-// so r goes there with one vector store at perm[c].
+// so r goes there with one vector store at gperm[c / 4].
 template <typename VT>
 __device__ __forceinline__ void update_xr_body(unsigned bid, unsigned nblk, VT* __restrict__ x,
                                                VT* __restrict__ r, const VT* __restrict__ s,
                                                const VT* __restrict__ z, long long M, PcgScalars* sc,
                                                double* __restrict__ partials, VT* __restrict__ rsw = nullptr,
-                                               const int* __restrict__ perm = nullptr) {
+                                               const int* __restrict__ gperm = nullptr) {
   __shared__ double sh[32];
   if (*(volatile int*)&sc->done) return;
   const VT alpha = (VT)sc->alpha;
@@ -795,7 +821,7 @@ __device__ __forceinline__ void update_xr_body(unsigned bid, unsigned nblk, VT* 
     ldg(B.r, r + c);
     ldg(B.s, s + c);
     ldg(B.z, z + c);
-    B.p = rsw != nullptr ? perm[c] : 0;
+    B.p = rsw != nullptr ? gperm[q] : 0;
   };
   auto finish = [&](Buf& B, long long q) {
     const long long c = 4 * q;
@@ -842,28 +868,28 @@ __global__ void __launch_bounds__(256) update_xr_kernel(VT* __restrict__ x, VT* 
                                                         const VT* __restrict__ s,
                                                         const VT* __restrict__ z, long long M,
                                                         PcgScalars* sc, double* __restrict__ partials,
-                                                        VT* __restrict__ rsw, const int* __restrict__ perm) {
-  update_xr_body<VT>(blockIdx.x, gridDim.x, x, r, s, z, M, sc, partials, rsw, perm);
+                                                        VT* __restrict__ rsw, const int* __restrict__ gperm) {
+  update_xr_body<VT>(blockIdx.x, gridDim.x, x, r, s, z, M, sc, partials, rsw, gperm);
 }
 template <typename VT>
 __global__ void __launch_bounds__(256) batch_update_xr_kernel(const BatchSeg* __restrict__ segs, int nseg,
                                                               VT* __restrict__ x, VT* __restrict__ r,
                                                               const VT* __restrict__ s, const VT* __restrict__ z,
                                                               PcgScalars* sc, VT* __restrict__ rsw,
-                                                              const int* __restrict__ perm) {
+                                                              const int* __restrict__ gperm) {
   const int q = batch_scene_of(segs, nseg, 0);
   const BatchSeg& S = segs[q];
   update_xr_body<VT>(blockIdx.x - S.blk_cells_start, S.blk_cells, x + S.base, r + S.base, s + S.base,
-                     z + S.base, S.M, sc + q, S.partials, rsw, perm ? perm + S.base : nullptr);
+                     z + S.base, S.M, sc + q, S.partials, rsw, gperm ? gperm + S.base / 4 : nullptr);
 }
 template <typename VT, typename DT>
 cudaError_t update_xr(VT* x, VT* r, const VT* s, const VT* z, long long M, PcgScalars* sc,
-                      double* partials, int nblk_max, cudaStream_t st, VT* rsw, const int* perm) {
+                      double* partials, int nblk_max, cudaStream_t st, VT* rsw, const int* gperm) {
   // 4-cell groups over at most nblk_max blocks
   int blocks = (int)std::min<long long>((M / 4 + 255) / 256, (long long)nblk_max);
   if (blocks < 1) blocks = 1;
   ++g_kernel_launches;
-  update_xr_kernel<VT><<<blocks, 256, 0, st>>>(x, r, s, z, M, sc, partials, rsw, perm);
+  update_xr_kernel<VT><<<blocks, 256, 0, st>>>(x, r, s, z, M, sc, partials, rsw, gperm);
   return cudaGetLastError();
 }
 template cudaError_t update_xr<double, double>(double*, double*, const double*, const double*, long long,
@@ -874,13 +900,13 @@ template cudaError_t update_xr<float, double>(float*, float*, const float*, cons
                                               PcgScalars*, double*, int, cudaStream_t, float*, const int*);
 
 // s = z + beta s  (add_scaled(beta, s, z) then swap, pcg_solver.h:280); one
-// thread per aligned 4-cell group, z read from the sweep layout at perm[c]
+// thread per aligned 4-cell group, z read from the sweep layout at gperm[c / 4]
 // (four consecutive elements) when there is one.
 template <typename VT>
 __device__ __forceinline__ void update_s_body(unsigned bid, unsigned nblk, VT* __restrict__ s,
                                               const VT* __restrict__ z, long long M, PcgScalars* sc,
                                               const VT* __restrict__ zsw = nullptr,
-                                              const int* __restrict__ perm = nullptr) {
+                                              const int* __restrict__ gperm = nullptr) {
   if (*(volatile int*)&sc->done) return;
   const VT beta = (VT)sc->beta;
   const long long G = M >> 2;
@@ -892,7 +918,7 @@ __device__ __forceinline__ void update_s_body(unsigned bid, unsigned nblk, VT* _
   auto load = [&](Buf& B, long long q) {
     const long long c = 4 * q;
     ldg(B.s, s + c);
-    ldg(B.z, zsw != nullptr ? zsw + perm[c] : z + c);
+    ldg(B.z, zsw != nullptr ? zsw + gperm[q] : z + c);
   };
   auto finish = [&](Buf& B, long long q) {
 #pragma unroll
@@ -913,27 +939,27 @@ __device__ __forceinline__ void update_s_body(unsigned bid, unsigned nblk, VT* _
 }
 template <typename VT>
 __global__ void update_s_kernel(VT* __restrict__ s, const VT* __restrict__ z, long long M,
-                                PcgScalars* sc, const VT* __restrict__ zsw, const int* __restrict__ perm) {
-  update_s_body<VT>(blockIdx.x, gridDim.x, s, z, M, sc, zsw, perm);
+                                PcgScalars* sc, const VT* __restrict__ zsw, const int* __restrict__ gperm) {
+  update_s_body<VT>(blockIdx.x, gridDim.x, s, z, M, sc, zsw, gperm);
 }
 template <typename VT>
 __global__ void batch_update_s_kernel(const BatchSeg* __restrict__ segs, int nseg, VT* __restrict__ s,
                                       const VT* __restrict__ z, PcgScalars* sc, const VT* __restrict__ zsw,
-                                      const int* __restrict__ perm) {
+                                      const int* __restrict__ gperm) {
   const int q = batch_scene_of(segs, nseg, 0);
   const BatchSeg& S = segs[q];
   update_s_body<VT>(blockIdx.x - S.blk_cells_start, S.blk_cells, s + S.base, z + S.base, S.M, sc + q, zsw,
-                    perm ? perm + S.base : nullptr);
+                    gperm ? gperm + S.base / 4 : nullptr);
 }
 template <typename VT>
 cudaError_t update_s(VT* s, const VT* z, long long M, PcgScalars* sc, cudaStream_t st, const VT* zsw,
-                     const int* perm, int nblk_max) {
+                     const int* gperm, int nblk_max) {
   // 4-cell groups over at most nblk_max blocks (one thread per group measured
   // slower at 256^3: more blocks, fewer groups per thread)
   int blocks = (int)std::min<long long>((M / 4 + 255) / 256, (long long)nblk_max);
   if (blocks < 1) blocks = 1;
   ++g_kernel_launches;
-  update_s_kernel<VT><<<blocks, 256, 0, st>>>(s, z, M, sc, zsw, perm);
+  update_s_kernel<VT><<<blocks, 256, 0, st>>>(s, z, M, sc, zsw, gperm);
   return cudaGetLastError();
 }
 template cudaError_t update_s<double>(double*, const double*, long long, PcgScalars*, cudaStream_t, const double*,
@@ -1129,32 +1155,30 @@ template cudaError_t batch_spmv_dot<float, float, double>(const BatchSeg*, int, 
                                                           const float*, const float*, const float*, float*,
                                                           const int*, PcgScalars*, int, cudaStream_t);
 
-// cell_line[c] = the line (index in its scene's table) that stores cell c;
-// group_line[c / 4] the same for every aligned 4-cell group (lines start at
-// multiples of 4 and hold multiples of 4 cells).
-__global__ void cell_line_kernel(const Line* __restrict__ lines, long long nlines, int* __restrict__ cell_line,
-                                 int* __restrict__ group_line) {
+// group_line[c / 4] = the line (index in its scene's table) that stores the
+// aligned 4-cell group of cell c (lines start at multiples of 4 and hold
+// multiples of 4 cells).
+__global__ void group_line_kernel(const Line* __restrict__ lines, long long nlines, int* __restrict__ group_line) {
   const int lane = threadIdx.x & 31;
   for (long long line = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); line < nlines;
        line += (long long)gridDim.x * (blockDim.x >> 5)) {
     const Line L = lines[line];
-    for (int q = lane; q < L.len; q += 32) cell_line[(size_t)L.off + q] = (int)line;
     for (int q = lane; q < (L.len >> 2); q += 32) group_line[((size_t)L.off >> 2) + q] = (int)line;
   }
 }
-cudaError_t build_cell_line(const Line* lines, long long nlines, int* cell_line, int* group_line, cudaStream_t st) {
+cudaError_t build_group_line(const Line* lines, long long nlines, int* group_line, cudaStream_t st) {
   if (nlines <= 0) return cudaSuccess;
   ++g_kernel_launches;
-  cell_line_kernel<<<(unsigned)std::min<long long>((nlines + 7) / 8, 65535LL * 8), 256, 0, st>>>(lines, nlines,
-                                                                                              cell_line, group_line);
+  group_line_kernel<<<(unsigned)std::min<long long>((nlines + 7) / 8, 65535LL * 8), 256, 0, st>>>(lines, nlines,
+                                                                                               group_line);
   return cudaGetLastError();
 }
 
 template <typename VT>
 cudaError_t batch_update_xr(const BatchSeg* segs, int nseg, int blocks, VT* x, VT* r, const VT* s,
-                            const VT* z, PcgScalars* sc, cudaStream_t st, VT* rsw, const int* perm) {
+                            const VT* z, PcgScalars* sc, cudaStream_t st, VT* rsw, const int* gperm) {
   ++g_kernel_launches;
-  batch_update_xr_kernel<VT><<<blocks, 256, 0, st>>>(segs, nseg, x, r, s, z, sc, rsw, perm);
+  batch_update_xr_kernel<VT><<<blocks, 256, 0, st>>>(segs, nseg, x, r, s, z, sc, rsw, gperm);
   return cudaGetLastError();
 }
 template cudaError_t batch_update_xr<double>(const BatchSeg*, int, int, double*, double*, const double*,
@@ -1164,9 +1188,9 @@ template cudaError_t batch_update_xr<float>(const BatchSeg*, int, int, float*, f
 
 template <typename VT>
 cudaError_t batch_update_s(const BatchSeg* segs, int nseg, int blocks, VT* s, const VT* z, PcgScalars* sc,
-                           cudaStream_t st, const VT* zsw, const int* perm) {
+                           cudaStream_t st, const VT* zsw, const int* gperm) {
   ++g_kernel_launches;
-  batch_update_s_kernel<VT><<<blocks, 256, 0, st>>>(segs, nseg, s, z, sc, zsw, perm);
+  batch_update_s_kernel<VT><<<blocks, 256, 0, st>>>(segs, nseg, s, z, sc, zsw, gperm);
   return cudaGetLastError();
 }
 template cudaError_t batch_update_s<double>(const BatchSeg*, int, int, double*, const double*, PcgScalars*,
@@ -1186,18 +1210,23 @@ template cudaError_t batch_absmax_init<double>(const BatchSeg*, int, int, const 
 template cudaError_t batch_absmax_init<float>(const BatchSeg*, int, int, const float*, PcgScalars*, double, int,
                                               const double*, const int*, cudaStream_t);
 
-// One block per scene: z.r from the scene's per-line partials with line_sum,
-// the same order the single-scene backward sweep's last CTA uses.
+// One CTA per scene: z.r from the scene's line partials, in the order the
+// single-scene backward sweep uses.
 template <typename DT>
-__global__ void __launch_bounds__(256) batch_bwd_reduce_kernel(const BatchSeg* __restrict__ segs,
-                                                               const double* __restrict__ lpart, PcgScalars* sc,
-                                                               int mode) {
-  __shared__ double s[256];
-  const int q = blockIdx.x;
+__global__ void __launch_bounds__(1024) batch_bwd_reduce_kernel(const BatchSeg* __restrict__ segs,
+                                                                 const double* __restrict__ lpart, PcgScalars* sc,
+                                                                 int mode) {
+  constexpr bool F32 = std::is_same<DT, float>::value;
+  __shared__ double sum[256], buf[32][8 * 17];
+  const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   PcgScalars* S = sc + q;
   if (*(volatile int*)&S->done) return;
   const BatchSeg& G = segs[q];
-  const double rho_new = line_sum<std::is_same<DT, float>::value>(lpart + G.line_base, (long long)G.nj * G.nk, s);
+  const double c = chunk_sums<F32, 8, 16>(lpart + G.line_base, (long long)G.nj * G.nk, warp * 8, buf[warp]);
+  if (lane < 8) sum[warp * 8 + lane] = c;
+  __syncthreads();
+  if (warp != 0) return;
+  const double rho_new = chunk_tree<F32>(sum);
   if (threadIdx.x != 0) return;
   if (mode == 0) {
     S->rho = rho_new;
@@ -1212,7 +1241,7 @@ template <typename DT>
 cudaError_t batch_bwd_reduce(const BatchSeg* segs, int nseg, const double* line_partials, PcgScalars* sc, int mode,
                              cudaStream_t st) {
   ++g_kernel_launches;
-  batch_bwd_reduce_kernel<DT><<<nseg, 256, 0, st>>>(segs, line_partials, sc, mode);
+  batch_bwd_reduce_kernel<DT><<<nseg, 1024, 0, st>>>(segs, line_partials, sc, mode);
   return cudaGetLastError();
 }
 template cudaError_t batch_bwd_reduce<double>(const BatchSeg*, int, const double*, PcgScalars*, int, cudaStream_t);
