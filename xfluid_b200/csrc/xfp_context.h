@@ -63,7 +63,7 @@ struct xfp_ctx {
   DevBuf ctl, scal, scal2, partials, tpartials;
   // particle steps (xfp_particles.cu): staged particles and field, bin keys,
   // indices, boxes, positions, bin starts, box spans, sort/scan scratch
-  DevBuf part_io, phi_io, part_key, part_idx, part_box, part_pos, part_sbox, part_spos, part_start, part_span,
+  DevBuf part_io, phi_io, part_key, part_idx, part_spos, part_start, part_span,
       part_tmp;
   // sweep layout (WBlk), Gsw groups: the factorisation's operands, the factor,
   // r and y/z, the line-group -> element map, and the block-edge words (zeroed

@@ -21,10 +21,9 @@
 // output gathers.  Particles are binned by the low corner of their own bounding
 // box (per face axis for the transfer, per cell for the field), clamped at 0,
 // with a stable radix sort, so a bin's particles are in index order.  An output
-// at index i is covered only by boxes with gmin <= i <= gmax, so it scans the
-// bins [i - maxspan, i] per axis (maxspan = the widest box, reduced from the
-// boxes themselves) and keeps the particles whose box holds it: exactly the
-// reference's set of contributions, no atomics, and a fixed summation order.
+// at index i is covered only by boxes with gmin <= i <= gmax, so it is covered
+// only from the bins [i - maxspan, i] per axis (maxspan = the widest box, reduced
+// from the boxes themselves): no atomics, and a fixed summation order.
 // That order is not the reference's particle order, so these sums agree with
 // the reference to FP64 rounding rather than bit for bit.
 //
@@ -278,10 +277,10 @@ struct BoxSpec {
   int ext[3];    // output grid extents
 };
 
-__device__ __forceinline__ void particle_box(const double* P, const BoxSpec& B, double dx, int lo[3], int hi[3],
-                                             V3* ps) {
-  const V3 p = vadd(v3(P[0], P[1], P[2]), v3(B.sh[0], B.sh[1], B.sh[2]));
-  *ps = p;
+__device__ __forceinline__ V3 shifted_pos(const double* P, const BoxSpec& B) {
+  return vadd(v3(P[0], P[1], P[2]), v3(B.sh[0], B.sh[1], B.sh[2]));
+}
+__device__ __forceinline__ void particle_box(V3 p, const BoxSpec& B, double dx, int lo[3], int hi[3]) {
   int a0, a1, a2, b0, b1, b2;
   pos2index(vadd(v3(-B.r, -B.r, -B.r), p), dx, &a0, &a1, &a2);
   pos2index(vadd(p, v3(B.r, B.r, B.r)), dx, &b0, &b1, &b2);
@@ -301,13 +300,12 @@ __device__ __forceinline__ void particle_box(const double* P, const BoxSpec& B, 
 // Key = bin of the box's low corner (clamped at 0, in cells), or nbins for
 // a box that covers no output; the widest box (in bins) goes to maxspan[q].
 __global__ void box_key_kernel(const double* __restrict__ parts, long long n, BoxSpec B, double dx, int nb0, int nb1,
-                               int nb2, long long nbins, unsigned* __restrict__ key, int* __restrict__ idx, int* __restrict__ box,
-                               double* __restrict__ pos, int* __restrict__ maxspan) {
+                               int nb2, long long nbins, unsigned* __restrict__ key, int* __restrict__ idx,
+                               int* __restrict__ maxspan) {
   int span[3] = {0, 0, 0};
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
     int lo[3], hi[3];
-    V3 p;
-    particle_box(parts + 6 * q, B, dx, lo, hi, &p);
+    particle_box(shifted_pos(parts + 6 * q, B), B, dx, lo, hi);
     bool hits = true;
     int bc[3];
     const int nb[3] = {nb0, nb1, nb2};
@@ -327,17 +325,12 @@ __global__ void box_key_kernel(const double* __restrict__ parts, long long n, Bo
         span[a] = max(span[a], sp);
       }
     }
-    int* bx = box + 6 * q;
-    bx[0] = lo[0]; bx[1] = hi[0]; bx[2] = lo[1]; bx[3] = hi[1]; bx[4] = lo[2]; bx[5] = hi[2];
-    pos[3 * q] = p.x;
-    pos[3 * q + 1] = p.y;
-    pos[3 * q + 2] = p.z;
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     int s = span[a];
     for (int o = 16; o > 0; o >>= 1) s = max(s, __shfl_xor_sync(0xffffffffu, s, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(&maxspan[a], s);
+    if ((threadIdx.x & 31) == 0 && s > *(volatile int*)&maxspan[a]) atomicMax(&maxspan[a], s);
   }
 }
 
@@ -347,19 +340,15 @@ __global__ void bin_count_kernel(const unsigned* __restrict__ key, long long n, 
     if ((long long)key[q] < nbins) atomicAdd(&count[key[q]], 1);
 }
 
-// sorted copies: box, shifted position and the carried value (velocity
-// component for the transfer, unused for the field)
-__global__ void bin_gather_kernel(const int* __restrict__ sidx, long long n, const int* __restrict__ box,
-                                  const double* __restrict__ pos, const double* __restrict__ parts, int vcomp,
-                                  int4* __restrict__ sbox_xy, int2* __restrict__ sbox_z,
-                                  double2* __restrict__ spos) {
+// sorted copies: shifted position and the carried value (velocity component
+// for the transfer, unused for the field)
+__global__ void bin_gather_kernel(const int* __restrict__ sidx, long long n, const double* __restrict__ parts,
+                                  BoxSpec B, int vcomp, double2* __restrict__ spos) {
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-    const int o = sidx[q];
-    const int* b = box + 6 * (size_t)o;
-    sbox_xy[q] = make_int4(b[0], b[1], b[2], b[3]);
-    sbox_z[q] = make_int2(b[4], b[5]);
-    spos[2 * q] = make_double2(pos[3 * (size_t)o], pos[3 * (size_t)o + 1]);
-    spos[2 * q + 1] = make_double2(pos[3 * (size_t)o + 2], vcomp >= 0 ? parts[6 * (size_t)o + 3 + vcomp] : 0.0);
+    const double* P = parts + 6 * (size_t)sidx[q];
+    const V3 p = shifted_pos(P, B);
+    spos[2 * q] = make_double2(p.x, p.y);
+    spos[2 * q + 1] = make_double2(p.z, vcomp >= 0 ? P[3 + vcomp] : 0.0);
   }
 }
 
@@ -374,45 +363,169 @@ __device__ __forceinline__ double poly_w(const Poly& W, double rs) {
   return sub_rn(add_rn(sub_rn(1.0, a), b), mul_rn(W.c2, rs));
 }
 
-// One output per thread: sum of the covering particles' weights (and
-// weighted values) over the bins [t/s - span, t/s] per axis, rows of bins
-// contiguous along x.  Transfer: out = value/weight where weight > 1e-7, else 0
+// A warp's outputs: sum of the covering particles' weights (and weighted
+// values).  Transfer: out = value/weight where weight > 1e-7, else 0
 // (:1010-1027).  Field: out = weight sum.
+//
+// A warp takes 4 x 4 x 2 outputs and walks the bins of all of them together, row
+// by row (rows of bins are contiguous along x): 32 candidates at a time, one per
+// lane, are tested against the box around the outputs, and the near ones are
+// queued in order in shared memory and added 64 at a time, all lanes reading the
+// same address.  The order in which an output meets its particles is that of its
+// own bins, and a particle that does not reach it adds nothing, so the sums are
+// those of a scan per output.  For the transfer every lane first marks the
+// particles near its own output (FP32, conservative) and then adds those alone:
+// an output needs an eighth of its warp's queue, where a field's needs three
+// tenths and the marking costs more than it saves (573 us against 528).
+//
+// What bounded a scan per output was every lane reading its own list: 13 passes
+// of the L1 pipeline a load, 83 % of a launch's time.  Now it is the issue of
+// instructions (28 for each particle near a warp's outputs: 940 of them for the
+// transfer at a radius of 1.5 cells and 8 particles a cell, 410 for the field with
+// two outputs a cell) and, at these sizes, the warps that finish last.  Measured at
+// 96^3, 1.3 M particles: transfer 1.14 -> 0.35 ms an axis (0.41 without the marks),
+// field 3.50 -> 0.53 ms.
+//
+// A particle's box holds every output within its radius (its bounds are whole
+// cells, half an output spacing and more beyond that), so a weight other than
+// zero needs no test of the box.  A velocity that is not finite does: it makes
+// every output of the box NaN, the zero weights' too.
+constexpr int GX = 4, GY = 4, GZ = 2, GWARPS = 4, GBATCH = 64;
+// a warp's queue: position and value, and the position from the middle of the warp's outputs in spacings
+struct GatherQueue {
+  float4 rel[GBATCH + 32];
+  double x[GBATCH + 32], y[GBATCH + 32], z[GBATCH + 32], v[GBATCH + 32];
+};
 template <bool FIELD>
-__global__ void gather_kernel(int e0, int e1, int e2, int s, double unit, int nb0, int nb1, int nb2, int sp0, int sp1,
-                              int sp2, const int* __restrict__ start, const int4* __restrict__ sbox_xy,
-                              const int2* __restrict__ sbox_z, const double2* __restrict__ spos, Poly W,
-                              double* __restrict__ out) {
-  const long long total = (long long)e0 * e1 * e2;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % e0), j = (int)((t / e0) % e1), k = (int)(t / ((long long)e0 * e1));
-    // output position: idx2Pos (xfluidutil.cpp:13-16) at this grid's spacing
-    const V3 g = v3(mul_rn(add_rn((double)i, 0.5), unit), mul_rn(add_rn((double)j, 0.5), unit),
-                    mul_rn(add_rn((double)k, 0.5), unit));
-    const int bi = min(i / s, nb0 - 1), bj = min(j / s, nb1 - 1), bk = min(k / s, nb2 - 1);
-    const int i0 = max(bi - sp0, 0), j0 = max(bj - sp1, 0), k0 = max(bk - sp2, 0);
-    double wsum = 0.0, vsum = 0.0;
-    for (int ck = k0; ck <= bk; ++ck)
-      for (int cj = j0; cj <= bj; ++cj) {
-        const long long row = ((long long)ck * nb1 + cj) * nb0;
-        const int qa = __ldg(&start[row + i0]), qb = __ldg(&start[row + bi + 1]);
-        for (int q = qa; q < qb; ++q) {
-          const int4 bxy = __ldg(&sbox_xy[q]);
-          const int2 bz = __ldg(&sbox_z[q]);
-          if (i < bxy.x || i > bxy.y || j < bxy.z || j > bxy.w || k < bz.x || k > bz.y) continue;
-          const double2 pxy = __ldg(&spos[2 * (size_t)q]), pzv = __ldg(&spos[2 * (size_t)q + 1]);
-          const V3 p = v3(pxy.x, pxy.y, pzv.x);
-          // transfer: curR = p - idx2Pos (:960); field: gp - p (:296)
-          const V3 d = FIELD ? vsub(g, p) : vsub(p, g);
-          const double cw = poly_w(W, vdot(d, d));
-          wsum = add_rn(wsum, cw);
-          if (!FIELD) vsum = add_rn(vsum, mul_rn(pzv.y, cw));
+__global__ void __launch_bounds__(32 * GWARPS, 7)
+    gather_kernel(BoxSpec B, double dx, double unit, int nb0, int nb1, int nb2, const int* __restrict__ maxspan,
+                  const int* __restrict__ start, const double2* __restrict__ spos, Poly W, float reach2, double* __restrict__ out) {
+  __shared__ GatherQueue queue[GWARPS];
+  const int lane = threadIdx.x & 31;
+  GatherQueue& Q = queue[threadIdx.x >> 5];
+  const int e0 = B.ext[0], e1 = B.ext[1], e2 = B.ext[2], s = B.s;
+  const unsigned n0 = (e0 + GX - 1) / GX, n1 = (e1 + GY - 1) / GY, n2 = (e2 + GZ - 1) / GZ;
+  const long long block = blockIdx.x * (long long)GWARPS + (threadIdx.x >> 5);
+  if (block >= (long long)n0 * n1 * n2) return;
+  const int ia = (int)(block % n0) * GX, ja = (int)(block / n0 % n1) * GY, ka = (int)(block / ((long long)n0 * n1)) * GZ;
+  const int ib = min(ia + GX, e0) - 1, jb = min(ja + GY, e1) - 1, kb = min(ka + GZ, e2) - 1;
+  const int i = ia + (lane & 3), j = ja + ((lane >> 2) & 3), k = ka + (lane >> 4);
+  // output position: idx2Pos (xfluidutil.cpp:13-16) at this grid's spacing
+  auto at = [&](int q) { return mul_rn(add_rn((double)q, 0.5), unit); };
+  const V3 g = v3(at(i), at(j), at(k));
+  const V3 ga = v3(at(ia), at(ja), at(ka)), gb = v3(at(ib), at(jb), at(kb));
+  const int bi = min(ib / s, nb0 - 1), bj = min(jb / s, nb1 - 1), bk = min(kb / s, nb2 - 1);
+  const int i0 = max(min(ia / s, nb0 - 1) - __ldg(maxspan), 0), j0 = max(min(ja / s, nb1 - 1) - __ldg(maxspan + 1), 0),
+            k0 = max(min(ka / s, nb2 - 1) - __ldg(maxspan + 2), 0);
+  const int nj = bj - j0 + 1, nr = nj * (bk - k0 + 1);
+  double wsum = 0.0, vsum = 0.0;
+  auto finite = [](double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; };
+  // the middle of the outputs, and this lane's output from there, in spacings
+  const V3 mid = v3(0.5 * (ga.x + gb.x), 0.5 * (ga.y + gb.y), 0.5 * (ga.z + gb.z));
+  const double per = 1.0 / unit;
+  const float gx = (float)((g.x - mid.x) * per), gy = (float)((g.y - mid.y) * per), gz = (float)((g.z - mid.z) * per);
+  int cnt = 0;
+  auto add_one = [&](V3 p, double v) {
+    // transfer: curR = p - idx2Pos (:960); field: gp - p (:296)
+    const V3 d = FIELD ? vsub(g, p) : vsub(p, g);
+    const double rs = vdot(d, d);
+    if (rs < W.r2) {
+      const double cw = poly_w(W, rs);
+      wsum = add_rn(wsum, cw);
+      if (!FIELD) vsum = add_rn(vsum, mul_rn(v, cw));
+    } else if (!FIELD && !finite(v)) {
+      int lo[3], hi[3];
+      particle_box(p, B, dx, lo, hi);
+      if (i >= lo[0] && i <= hi[0] && j >= lo[1] && j <= hi[1] && k >= lo[2] && k <= hi[2])
+        vsum = add_rn(vsum, mul_rn(v, 0.0));
+    }
+  };
+  auto add_queued = [&](int n) {   // the first n of the queue
+    if constexpr (FIELD) {
+#pragma unroll 4
+      for (int q = 0; q < n; ++q) add_one(v3(Q.x[q], Q.y[q], Q.z[q]), 0.0);
+      __syncwarp();
+      return;
+    }
+    unsigned mark[2] = {0u, 0u};
+    // (up to seven more are marked than queued, and cut off again)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int q = 0; q < 32; q += 8)
+        if (h * 32 + q < n)
+#pragma unroll
+          for (int o = q; o < q + 8; ++o) {
+            const float4 f = Q.rel[h * 32 + o];
+            const float dx = f.x - gx, dy = f.y - gy, dz = f.z - gz;
+            if (!(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) >= reach2)) mark[h] |= 1u << o;
+          }
+    if (n < 32) mark[0] &= (1u << n) - 1u;
+    if (n < 64) mark[1] &= n <= 32 ? 0u : (1u << (n - 32)) - 1u;
+    while ((mark[0] | mark[1]) != 0u) {
+      const bool low = mark[0] != 0u;
+      const unsigned m = low ? mark[0] : mark[1];
+      const int q = __ffs(m) - 1 + (low ? 0 : 32);
+      if (low) mark[0] = m & (m - 1u); else mark[1] = m & (m - 1u);
+      add_one(v3(Q.x[q], Q.y[q], Q.z[q]), Q.v[q]);
+    }
+    __syncwarp();
+  };
+  auto outside = [](double a, double p, double b) { return fmax(fmax(sub_rn(a, p), sub_rn(p, b)), 0.0); };
+  for (int r0 = 0; r0 < nr; r0 += 32) {
+    const int r = r0 + lane;
+    int qa = 0, qb = 0;
+    if (r < nr) {
+      const long long row = ((long long)(k0 + r / nj) * nb1 + j0 + r % nj) * nb0;
+      qa = __ldg(&start[row + i0]);
+      qb = __ldg(&start[row + bi + 1]);
+    }
+    for (unsigned live = __ballot_sync(XFP_FULL, qb > qa); live != 0; live &= live - 1) {
+      const int src = __ffs(live) - 1;
+      const unsigned last = __shfl_sync(XFP_FULL, qb, src);
+      for (unsigned c = __shfl_sync(XFP_FULL, qa, src) + lane; c - lane < last; c += 32) {
+        bool near = false;
+        double2 pxy = make_double2(0.0, 0.0), pzv = pxy;
+        if (c < last) {
+          pxy = __ldg(&spos[2 * (size_t)c]);
+          pzv = __ldg(&spos[2 * (size_t)c + 1]);
+          const V3 d = v3(outside(ga.x, pxy.x, gb.x), outside(ga.y, pxy.y, gb.y), outside(ga.z, pzv.x, gb.z));
+          near = vdot(d, d) < W.r2 || (!FIELD && !finite(pzv.y));
+        }
+        const unsigned m = __ballot_sync(XFP_FULL, near);
+        if (near) {
+          const int q = cnt + __popc(m & ((1u << lane) - 1u));
+          // (a value that is not finite is marked by every lane)
+          if (!FIELD)
+            Q.rel[q] = make_float4(!finite(pzv.y) ? NAN : (float)((pxy.x - mid.x) * per),
+                                   (float)((pxy.y - mid.y) * per), (float)((pzv.x - mid.z) * per), 0.f);
+          Q.x[q] = pxy.x;
+          Q.y[q] = pxy.y;
+          Q.z[q] = pzv.x;
+          if (!FIELD) Q.v[q] = pzv.y;
+        }
+        cnt += __popc(m);
+        __syncwarp();
+        if (cnt >= GBATCH) {
+          add_queued(GBATCH);
+          cnt -= GBATCH;
+          if (lane < cnt) {
+            if (!FIELD) Q.rel[lane] = Q.rel[GBATCH + lane];
+            Q.x[lane] = Q.x[GBATCH + lane];
+            Q.y[lane] = Q.y[GBATCH + lane];
+            Q.z[lane] = Q.z[GBATCH + lane];
+            if (!FIELD) Q.v[lane] = Q.v[GBATCH + lane];
+          }
+          __syncwarp();
         }
       }
-    if (FIELD) out[t] = wsum;
-    else out[t] = wsum > 0.0000001 ? div_rn(vsum, wsum) : 0.0;
+    }
   }
+  add_queued(cnt);
+  if (i > ib || j > jb || k > kb) return;
+  const size_t t = ((size_t)k * e1 + j) * e0 + i;
+  if (FIELD) out[t] = wsum;
+  else out[t] = wsum > 0.0000001 ? div_rn(vsum, wsum) : 0.0;
 }
 
 // _updateMaterial (:402-427)
@@ -497,25 +610,16 @@ int bin_and_gather(xfp_ctx* ctx, const double* dparts, long long n, const BoxSpe
   cudaStream_t st = ctx->stream;
   const int nb0 = (B.ext[0] + B.s - 1) / B.s, nb1 = (B.ext[1] + B.s - 1) / B.s, nb2 = (B.ext[2] + B.s - 1) / B.s;
   const long long nbins = (long long)nb0 * nb1 * nb2;
-  const long long total = (long long)B.ext[0] * B.ext[1] * B.ext[2];
   const size_t nn = (size_t)std::max<long long>(n, 1);
   XFP_CUDA(ctx, ctx->part_key.ensure(nn * 2 * sizeof(unsigned)));
   XFP_CUDA(ctx, ctx->part_idx.ensure(nn * 2 * sizeof(int)));
-  XFP_CUDA(ctx, ctx->part_box.ensure(nn * 6 * sizeof(int)));
-  XFP_CUDA(ctx, ctx->part_pos.ensure(nn * 3 * sizeof(double)));
-  XFP_CUDA(ctx, ctx->part_sbox.ensure(nn * (sizeof(int4) + sizeof(int2))));
   XFP_CUDA(ctx, ctx->part_spos.ensure(nn * 2 * sizeof(double2)));
   XFP_CUDA(ctx, ctx->part_start.ensure((size_t)(nbins + 2) * sizeof(int) * 2 + 16));
   unsigned* key = ctx->part_key.as<unsigned>();
   unsigned* key2 = key + nn;
   int* idx = ctx->part_idx.as<int>();
   int* idx2 = idx + nn;
-  int* box = ctx->part_box.as<int>();
-  double* pos = ctx->part_pos.as<double>();
-  // sorted copies for the gather: box as int4 (x, y) + int2 (z), position and
-  // carried value as two double2 -- four vector loads per candidate
-  int4* sbox_xy = ctx->part_sbox.as<int4>();
-  int2* sbox_z = reinterpret_cast<int2*>(sbox_xy + nn);
+  // sorted copies for the gather: position and carried value as two double2
   double2* spos = ctx->part_spos.as<double2>();
   int* count = ctx->part_start.as<int>();
   int* start = count + (nbins + 2);
@@ -526,8 +630,7 @@ int bin_and_gather(xfp_ctx* ctx, const double* dparts, long long n, const BoxSpe
   XFP_CUDA(ctx, cudaMemsetAsync(dspan, 0, 4 * sizeof(int), st));
   if (n > 0) {
     ++g_kernel_launches;
-    box_key_kernel<<<pgrid(n), 256, 0, st>>>(dparts, n, B, dx, nb0, nb1, nb2, nbins, key, idx, box, pos,
-                                               dspan);
+    box_key_kernel<<<pgrid(n), 256, 0, st>>>(dparts, n, B, dx, nb0, nb1, nb2, nbins, key, idx, dspan);
     XFP_CUDA(ctx, cudaGetLastError());
     // stable sort by bin (keys < nbins, no-cover key = nbins): a bin's
     // particles stay in index order
@@ -548,15 +651,16 @@ int bin_and_gather(xfp_ctx* ctx, const double* dparts, long long n, const BoxSpe
     XFP_CUDA(ctx, cub::DeviceScan::ExclusiveSum(ctx->part_tmp.p, tmp2, count, start, (int)(nbins + 1), st));
     g_kernel_launches += 2;
     ++g_kernel_launches;
-    bin_gather_kernel<<<pgrid(n), 256, 0, st>>>(idx2, n, box, pos, dparts, vcomp, sbox_xy, sbox_z, spos);
+    bin_gather_kernel<<<pgrid(n), 256, 0, st>>>(idx2, n, dparts, B, vcomp, spos);
     XFP_CUDA(ctx, cudaGetLastError());
   }
-  int span[4] = {0, 0, 0, 0};
-  XFP_CUDA(ctx, cudaMemcpyAsync(span, dspan, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
-  XFP_CUDA(ctx, cudaStreamSynchronize(st));
+  const long long blocks = (long long)((B.ext[0] + GX - 1) / GX) * ((B.ext[1] + GY - 1) / GY) * ((B.ext[2] + GZ - 1) / GZ);
+  // the FP32 test's reach in output spacings: the radius and more than its
+  // roundings, each a part in 2^24 of coordinates below the radius and a few spacings
+  const double reach = B.r / unit + 4e-6 * (B.r / unit + 8.0);
   ++g_kernel_launches;
-  gather_kernel<FIELD><<<pgrid(total), 256, 0, st>>>(B.ext[0], B.ext[1], B.ext[2], B.s, unit, nb0, nb1, nb2, span[0],
-                                                     span[1], span[2], start, sbox_xy, sbox_z, spos, W, out);
+  gather_kernel<FIELD><<<(unsigned)((blocks + GWARPS - 1) / GWARPS), 32 * GWARPS, 0, st>>>(
+      B, dx, unit, nb0, nb1, nb2, dspan, start, spos, W, (float)(reach * reach * (1.0 + 1e-6)), out);
   XFP_CUDA(ctx, cudaGetLastError());
   return XFP_OK;
 }
