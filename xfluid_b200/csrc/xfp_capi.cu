@@ -661,9 +661,8 @@ int project_impl(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* mat, IOT* 
     XFP_CUDA(ctx, (apply_pressure<IOT, IOT>(dmat, dwu, dwv, dww, dp, ni, nj, nk, mu, mv, mw, ctx->stream,
                                             ctx->opt.matrix, ctx->force)));
     if (ctx->step_layers > 0) {
-      const size_t nm = (size_t)(ni + 1) * (nj + 1) * (nk + 1);
-      XFP_CUDA(ctx, ctx->xmarker.ensure(nm * sizeof(short)));
-      XFP_CUDA(ctx, extrapolate<IOT>(dmat, ni, nj, nk, mu, mv, mw, ctx->step_layers, ctx->xmarker.as<short>(),
+      XFP_CUDA(ctx, ctx->xmarker.ensure(extrapolate_scratch(ni, nj, nk)));
+      XFP_CUDA(ctx, extrapolate<IOT>(dmat, ni, nj, nk, mu, mv, mw, ctx->step_layers, ctx->xmarker.as<unsigned>(),
                                      ctx->stream));
     }
   }
@@ -924,7 +923,7 @@ int forces_impl(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* mat, IOT* u
   return XFP_OK;
 }
 
-constexpr int kMaxLayers = 30000;   // the layer marker is 16-bit
+constexpr int kMaxLayers = 30000;   // a launch each
 
 template <typename IOT>
 int extrapolate_impl(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* mat, IOT* u, IOT* v, IOT* w,
@@ -940,9 +939,9 @@ int extrapolate_impl(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* mat, I
   if ((rc = stage_in<IOT>(ctx, ctx->io_u, u, nu(ni, nj, nk), &du_))) return rc;
   if ((rc = stage_in<IOT>(ctx, ctx->io_v, v, nv(ni, nj, nk), &dv))) return rc;
   if ((rc = stage_in<IOT>(ctx, ctx->io_w, w, nw_(ni, nj, nk), &dw))) return rc;
-  XFP_CUDA(ctx, ctx->xmarker.ensure((size_t)(ni + 1) * (nj + 1) * (nk + 1) * sizeof(short)));
+  XFP_CUDA(ctx, ctx->xmarker.ensure(extrapolate_scratch(ni, nj, nk)));
   XFP_CUDA(ctx, extrapolate<IOT>(dmat, ni, nj, nk, const_cast<IOT*>(du_), const_cast<IOT*>(dv),
-                                 const_cast<IOT*>(dw), layers, ctx->xmarker.as<short>(), ctx->stream));
+                                 const_cast<IOT*>(dw), layers, ctx->xmarker.as<unsigned>(), ctx->stream));
   if (!ctx->opt.device_pointers) {
     XFP_CUDA(ctx, cudaMemcpyAsync(u, du_, nu(ni, nj, nk) * sizeof(IOT), cudaMemcpyDeviceToHost, ctx->stream));
     XFP_CUDA(ctx, cudaMemcpyAsync(v, dv, nv(ni, nj, nk) * sizeof(IOT), cudaMemcpyDeviceToHost, ctx->stream));

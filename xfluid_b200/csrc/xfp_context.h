@@ -86,7 +86,7 @@ struct xfp_ctx {
   int host_sparse_ok = 1;
   // xfp_project_step_*: body force fused into assembly and apply, and the
   // extrapolation layers run after the apply (zero outside such a call);
-  // xmarker is the extrapolation's layer-marker scratch
+  // xmarker is the extrapolation's layer bits
   xfp::Force3 force;
   int step_layers = 0;
   DevBuf xmarker;

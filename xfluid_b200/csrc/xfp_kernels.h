@@ -111,10 +111,11 @@ template <typename FT>
 cudaError_t apply_forces(const uint8_t* mat, int ni, int nj, int nk, FT* u, FT* v, FT* w, Force3 frc,
                          cudaStream_t st);
 // FluidSimulator::_expolateVelocity(layers, axis) for the three axes
-// (FluidSimulator.cpp:521-650); marker: scratch of (ni+1)*(nj+1)*(nk+1) shorts.
+// (FluidSimulator.cpp:521-650); scratch: extrapolate_scratch bytes.
+size_t extrapolate_scratch(int ni, int nj, int nk);
 template <typename FT>
 cudaError_t extrapolate(const uint8_t* mat, int ni, int nj, int nk, FT* u, FT* v, FT* w, int layers,
-                        short* marker, cudaStream_t st);
+                        unsigned* scratch, cudaStream_t st);
 template <typename FT>
 cudaError_t divergence(const uint8_t* mat, int ni, int nj, int nk, const FT* u, const FT* v, const FT* w, FT* div,
                        cudaStream_t st);
