@@ -228,8 +228,8 @@ int batch_pcg(xfp_ctx* ctx, BatchState* B, const VT* const A[4], const VT* b, VT
   if ((rc0 = sweep_rhs<VT>(ctx, r)) != XFP_OK) return rc0;
   const WaveArgs g = batch_args(ctx, B, dsc);
   const bool swl = B->ntiles > 0;
-  VT* rsw = swl ? ctx->sw_r.as<VT>() : nullptr;
-  const VT* zsw = swl ? ctx->sw_y.as<VT>() : nullptr;
+  VT* rsw = swl ? ctx->sw.as<VT>() + WAVE_R : nullptr;
+  const VT* zsw = swl ? ctx->sw.as<VT>() + WAVE_Y : nullptr;
   const int* gperm = swl ? ctx->gperm.as<int>() : nullptr;
   const double* lpart = ctx->tpartials.as<double>();
   // lines of blocks without cells are never written: their partials stay zero

@@ -210,8 +210,8 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
   // r is kept in both layouts (update_xr writes both) and z lives in the sweep
   // layout only (update_s reads it through gperm)
   const bool swl = ctx->ntiles > 0;
-  VT* rsw = swl ? ctx->sw_r.as<VT>() : nullptr;
-  const VT* zsw = swl ? ctx->sw_y.as<VT>() : nullptr;
+  VT* rsw = swl ? ctx->sw.as<VT>() + WAVE_R : nullptr;
+  const VT* zsw = swl ? ctx->sw.as<VT>() + WAVE_Y : nullptr;
   const int* gperm = swl ? ctx->gperm.as<int>() : nullptr;
   if ((rc = run_sweep<VT, DT>(ctx, SWEEP_FWD, g0)) != XFP_OK) return rc;
   if ((rc = run_sweep<VT, DT>(ctx, SWEEP_BWD, g0)) != XFP_OK) return rc;
@@ -842,7 +842,7 @@ int debug_core(xfp_ctx* ctx, const CT* const Af[5], const VT* const Av[4], const
   for (int q = 0; q < 4; ++q) F[q] = Fb.as<CT>() + (size_t)(M + 8) * q;
   struct Release { DevBuf& b; ~Release() { b.release(); } } release{Fb};
   if (ctx->ntiles > 0)
-    XFP_CUDA(ctx, factor_lines<CT>(ctx->sw_fac.as<CT>(), ctx->lines.as<Line>(), ctx->nj, ctx->nk,
+    XFP_CUDA(ctx, factor_lines<CT>(ctx->sw.as<CT>(), ctx->lines.as<Line>(), ctx->nj, ctx->nk,
                                    ctx->blks.as<WBlk>(), ctx->NJB, F, st));
   XFP_CUDA(ctx, cudaStreamSynchronize(st));
   if ((rc = check_sweep_error(ctx))) return rc;
@@ -1100,7 +1100,7 @@ int xfp_destroy(xfp_ctx* ctx) {
                    &ctx->io_p, &ctx->io_gu, &ctx->io_gv, &ctx->io_gw, &ctx->lines, &ctx->lens,
                    &ctx->blks, &ctx->tiles, &ctx->counters, &ctx->group_line, &ctx->gperm, &ctx->x64,
                    &ctx->r64, &ctx->x32, &ctx->r32, &ctx->s32, &ctx->z32, &ctx->s64, &ctx->z64, &ctx->dense,
-                   &ctx->sw_sys, &ctx->sw_fac, &ctx->sw_r, &ctx->sw_y, &ctx->edge, &ctx->ctl, &ctx->scal, &ctx->scal2, &ctx->partials,
+                   &ctx->sw_sys, &ctx->sw, &ctx->edge, &ctx->ctl, &ctx->scal, &ctx->scal2, &ctx->partials,
                    &ctx->tpartials};
   for (DevBuf* b : all) b->release();
   batch_state_free(ctx->batch);

@@ -66,6 +66,11 @@ __host__ __device__ __forceinline__ int wave_cell_slot(int j, int k, int e, int 
 // The wavefront kernel's clusters: WAVE_TJ x 2 CTAs of two blocks along k, a tile
 // of WAVE_TJ x WAVE_TK blocks (32 x 32 lines)
 constexpr int WAVE_TJ = 4, WAVE_TK = 4, WAVE_CLUSTER = 8;
+// A group's row of the solves' array: the factor's four values of its 256 cells,
+// then r, then y (the backward solve's z).
+constexpr int WAVE_R = 4 * 256, WAVE_Y = 5 * 256, WAVE_ROW = 6 * 256;
+// element p = group * 256 + wave_line_slot of r or y, from the array's WAVE_R or WAVE_Y on
+__host__ __device__ __forceinline__ size_t wave_value(int p) { return (size_t)(p >> 8) * WAVE_ROW + (p & 255); }
 __host__ __device__ __forceinline__ int wave_line_slot(int j, int k) {
   return (k & 1) * 128 + (((k & 7) >> 1) * 8 + (j & 7)) * 4;
 }

@@ -68,7 +68,7 @@ struct xfp_ctx {
   // sweep layout (WBlk), Gsw groups: the factorisation's operands, the factor,
   // r and y/z, the line-group -> element map, and the block-edge words (zeroed
   // when (re)allocated so no stale word can carry a live generation)
-  DevBuf sw_sys, sw_fac, sw_r, sw_y, gperm, edge;
+  DevBuf sw_sys, sw, gperm, edge;
   // host-pointer mode: fluid span per x-line and the two byte counters of
   // the sparse face transfer; bytes moved by the current call; whether its
   // velocities went face-sparse; XFP_HOST_FACES=full turns the sparse
@@ -187,9 +187,7 @@ inline int ensure_sweep(xfp_ctx* ctx, size_t sys_bytes) {
   if (ctx->ntiles == 0) return XFP_OK;
   const size_t n = (size_t)ctx->Gsw * 256;
   XFP_CUDA(ctx, ctx->sw_sys.ensure(n * 4 * 8));
-  XFP_CUDA(ctx, ctx->sw_fac.ensure(n * 4 * 8));
-  XFP_CUDA(ctx, ctx->sw_r.ensure(n * 8));
-  XFP_CUDA(ctx, ctx->sw_y.ensure(n * 8));
+  XFP_CUDA(ctx, ctx->sw.ensure((size_t)ctx->Gsw * xfp::WAVE_ROW * 8));
   XFP_CUDA(ctx, cudaMemsetAsync(ctx->sw_sys.p, 0, n * 4 * sys_bytes, ctx->stream));
   const size_t words = (size_t)ctx->Gsw * 2 * xfp::WAVE_EDGE;
   if (ctx->edge.cap < words * 8 || !ctx->edge.p) {
@@ -203,8 +201,9 @@ inline int ensure_sweep(xfp_ctx* ctx, size_t sys_bytes) {
 template <typename VT>
 int sweep_rhs(xfp_ctx* ctx, const VT* r) {
   if (ctx->ntiles == 0) return XFP_OK;
-  XFP_CUDA(ctx, cudaMemsetAsync(ctx->sw_r.p, 0, (size_t)ctx->Gsw * 256 * sizeof(VT), ctx->stream));
-  XFP_CUDA(ctx, xfp::sw_permute<VT>(const_cast<VT*>(r), ctx->sw_r.as<VT>(), ctx->gperm.as<int>(), ctx->M, 0,
+  VT* const sr = ctx->sw.as<VT>() + xfp::WAVE_R;
+  XFP_CUDA(ctx, cudaMemset2DAsync(sr, xfp::WAVE_ROW * sizeof(VT), 0, 256 * sizeof(VT), (size_t)ctx->Gsw, ctx->stream));
+  XFP_CUDA(ctx, xfp::sw_permute<VT>(const_cast<VT*>(r), sr, ctx->gperm.as<int>(), ctx->M, 0,
                                     ctx->stream));
   return XFP_OK;
 }
@@ -214,7 +213,7 @@ int sweep_rhs(xfp_ctx* ctx, const VT* r) {
 template <typename VT>
 int sweep_result(xfp_ctx* ctx, VT* out) {
   if (ctx->ntiles == 0) return XFP_OK;
-  XFP_CUDA(ctx, xfp::sw_permute<VT>(out, ctx->sw_y.as<VT>(), ctx->gperm.as<int>(), ctx->M, 1, ctx->stream));
+  XFP_CUDA(ctx, xfp::sw_permute<VT>(out, ctx->sw.as<VT>() + xfp::WAVE_Y, ctx->gperm.as<int>(), ctx->M, 1, ctx->stream));
   return XFP_OK;
 }
 
@@ -233,10 +232,7 @@ inline xfp::WaveArgs wave_args(xfp_ctx* ctx) {
   g.omega = ctx->opt.omega;
   g.ratio = ctx->opt.min_diag_ratio;
   g.sys = ctx->sw_sys.p;
-  g.fac_out = ctx->sw_fac.p;
-  g.fac = ctx->sw_fac.p;
-  g.r = ctx->sw_r.p;
-  g.y = ctx->sw_y.p;
+  g.sw = ctx->sw.p;
   g.partials = ctx->tpartials.as<double>();
   g.bj = ctx->edge.as<unsigned long long>();
   g.bk = g.bj + (size_t)ctx->Gsw * xfp::WAVE_EDGE;

@@ -39,10 +39,8 @@ struct WaveArgs {
   // sweep-layout arrays; the factor and the system keep four values per cell
   // (wave_cell_slot): (px, py, pz, inv) and (diag, A(c+1,c), A(c+ni,c), A(c+nn,c))
   const void* sys = nullptr;    // factor: the system, arithmetic type
-  void* fac_out = nullptr;      // factor: the result, solve type
-  const void* fac = nullptr;    // solves
-  const void* r = nullptr;      // solves: right-hand side (backward: for z.r)
-  void* y = nullptr;            // forward: out y; backward: in y, out z
+  void* sw = nullptr;           // rows of WAVE_ROW values, solve type: the factor; r (backward: for
+                                // z.r); y (backward: in y, out z)
   double* partials = nullptr;   // backward: z.r per line, [k * nj + j]
   unsigned long long* bj = nullptr;   // block-edge words of the J and K neighbours
   unsigned long long* bk = nullptr;
@@ -59,7 +57,7 @@ constexpr size_t WAVE_EDGE = 4 * 8 * 4;
 // from cell_base on; group_line of those cells, their scene's lines and blocks)
 cudaError_t gperm_build(const int* group_line, const Line* lines, int nj, const WBlk* blks, int NJB, long long M,
                         long long cell_base, long long group_base, int* gperm, cudaStream_t st);
-// dir 0: sw[gperm] = line; dir 1: line = sw[gperm], for the M stored cells.
+// dir 0: sw[wave_value(gperm)] = line; dir 1: the way back, for the M stored cells.
 template <typename T>
 cudaError_t sw_permute(T* line, T* sw, const int* gperm, long long M, int dir, cudaStream_t st);
 // The factor back in the line layout: F = lx, ly, lz (keyed by the higher cell), inv.
@@ -139,12 +137,12 @@ cudaError_t spmv_dot(const AT* diag, const AT* ax, const AT* ay, const AT* az, c
 long long spmv_block_count(long long M, int nblk_max);
 // group_line[c / 4] = index of the line storing the aligned 4-cell group of cell c.
 cudaError_t build_group_line(const Line* lines, long long nlines, int* group_line, cudaStream_t st);
-// rsw/gperm (optional): the updated r is also stored at rsw[gperm[c / 4]].
+// rsw/gperm (optional): the updated r is also stored at rsw[wave_value(gperm[c / 4])].
 template <typename VT, typename DT>
 cudaError_t update_xr(VT* x, VT* r, const VT* s, const VT* z, long long M, PcgScalars* sc,
                       double* partials, int nblk_max, cudaStream_t st, VT* rsw = nullptr,
                       const int* gperm = nullptr);
-// zsw/gperm (optional): z is read from zsw[gperm[c / 4]] instead of z[c].
+// zsw/gperm (optional): z is read from zsw[wave_value(gperm[c / 4])] instead of z[c].
 template <typename VT>
 cudaError_t update_s(VT* s, const VT* z, long long M, PcgScalars* sc, cudaStream_t st, const VT* zsw = nullptr,
                      const int* gperm = nullptr, int nblk_max = 148 * 16);

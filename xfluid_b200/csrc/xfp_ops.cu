@@ -795,7 +795,7 @@ template cudaError_t spmv_dot<float, float, double>(const float*, const float*, 
 // One thread per aligned 4-cell group, with 16-byte vector accesses (two for
 // FP64).  With a sweep layout the group's four cells sit at four consecutive
 // sweep-layout elements (consecutive forward steps, aligned to a group of 4),
-// so r goes there with one vector store at gperm[c / 4].
+// so r goes there with one vector store at wave_value(gperm[c / 4]).
 template <typename VT>
 __device__ __forceinline__ void update_xr_body(unsigned bid, unsigned nblk, VT* __restrict__ x,
                                                VT* __restrict__ r, const VT* __restrict__ s,
@@ -833,7 +833,7 @@ __device__ __forceinline__ void update_xr_body(unsigned bid, unsigned nblk, VT* 
     }
     stg(x + c, B.x);
     stg(r + c, B.r);
-    if (rsw != nullptr) stg(rsw + B.p, B.r);
+    if (rsw != nullptr) stg(rsw + wave_value(B.p), B.r);
   };
   Buf A, B;
   long long q = (long long)bid * blockDim.x + threadIdx.x;
@@ -900,7 +900,7 @@ template cudaError_t update_xr<float, double>(float*, float*, const float*, cons
                                               PcgScalars*, double*, int, cudaStream_t, float*, const int*);
 
 // s = z + beta s  (add_scaled(beta, s, z) then swap, pcg_solver.h:280); one
-// thread per aligned 4-cell group, z read from the sweep layout at gperm[c / 4]
+// thread per aligned 4-cell group, z read from the sweep layout at wave_value(gperm[c / 4])
 // (four consecutive elements) when there is one.
 template <typename VT>
 __device__ __forceinline__ void update_s_body(unsigned bid, unsigned nblk, VT* __restrict__ s,
@@ -918,7 +918,7 @@ __device__ __forceinline__ void update_s_body(unsigned bid, unsigned nblk, VT* _
   auto load = [&](Buf& B, long long q) {
     const long long c = 4 * q;
     ldg(B.s, s + c);
-    ldg(B.z, zsw != nullptr ? zsw + gperm[q] : z + c);
+    ldg(B.z, zsw != nullptr ? zsw + wave_value(gperm[q]) : z + c);
   };
   auto finish = [&](Buf& B, long long q) {
 #pragma unroll

@@ -41,7 +41,9 @@
 // reports the groups it has taken, and no one writes a slot before that.
 //
 // Data.  Every block's cells lie in its own stream of groups of 4 steps (WBlk,
-// wave_line_slot, wave_cell_slot).  Cells that are absent hold zero in every
+// wave_line_slot, wave_cell_slot), a group's factor, r and y side by side, so
+// that one bulk copy of a few KB fills a slot (issuing two or three took the
+// helper warp longer than the steps take).  Cells that are absent hold zero in every
 // array, which makes their results zero without masks.
 //
 // Tiles are taken in topological order (J+K ascending): the first ones by
@@ -57,16 +59,18 @@
 // chunks (one CTA alone reads 65,536 partials at 256^3).
 //
 // Measured (device time of a launch, full box of 128^3 / 256^3 cells): a solve
-// takes 83 / 214 us in FP32 and 114 / 365 us in FP64 -- 0.43 (0.50) us per group
-// of four steps of the longest path, 13 us to start and end a launch, 2.5 (5) us
-// a block further in the cluster -- and the factorisation 0.24 / 0.75 ms.
+// takes 74 / 190 us in FP32 and 102 / 330 us in FP64 -- 0.31 (0.39) us per group
+// of four steps of a lone block, 0.05 more where it hands edges on, 12 us to start
+// and end a launch -- and the factorisation 0.23 / 0.68 ms.  (With an mbarrier each
+// for operands and edge values, acknowledgements by the compute warp and two or
+// three copies a group: 0.43 (0.50) us, 83 / 214 and 114 / 365 us.)
 // Before (one CTA per 32 x 15 lines, a CTA-wide barrier per step, tiles through
 // global memory): 263 us for the FP64 128^3 solve, 180 us for a half-full FP32
-// 256^3 one (now 112), 0.65 to 1.0 ms for the factorisation.  Tried on the way:
-// lockstep CTAs of 2 x 2 blocks (143 us where this takes 81), blocks that hand
-// over through L2 words only (117 to 134), per-step instead of per-group
-// hand-over in the cluster (367 cycles a step), one warp as helper and courier
-// with 4 slots a block (207).
+// 256^3 one (now 92), 0.65 to 1.0 ms for the factorisation.  Tried on the way:
+// lockstep CTAs of 2 x 2 blocks (143 us where the first form took 81), blocks that
+// hand over through L2 words only (117 to 134), per-step instead of per-group
+// hand-over in the cluster (367 cycles a step), one warp as helper and courier with
+// 4 slots a block (207).
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -87,7 +91,7 @@ template <int OP, typename VT, typename CT>
 struct WaveOp {
   using X = VT;
   using ST = VT;
-  static constexpr int HL = 2, IN = (OP == SWEEP_BWD ? 6 : 5) * GE, S = sizeof(VT) == 8 ? 4 : 8;
+  static constexpr int HL = 2, IN = (OP == SWEEP_BWD ? 6 : 5) * GE, S = 8;
 };
 template <typename VT, typename CT>
 struct WaveOp<SWEEP_FACTOR, VT, CT> {
@@ -111,11 +115,11 @@ template <int OP, typename VT, typename CT>
 struct __align__(128) UnitShared {
   static constexpr int S = WaveOp<OP, VT, CT>::S;
   Slot<OP, VT, CT> slot[S];
-  unsigned long long ops[S], edge[S];   // mbarriers: a slot's operands / edge values have landed
-  unsigned long long empty[S];          // mbarriers: the compute warp is done with a group
-  int limit[2];                         // the j / k consumer has room for this block's groups below
-  int done;                             // edge values taken (kept for a courier at work)
-  int broken;                           // a wait for a slot ran out: its mbarriers are not armed again
+  unsigned long long full[S];    // mbarriers: a slot's operands and edge values have landed
+  unsigned long long empty[S];   // mbarriers: the compute warp is done with a slot
+  int limit[2];                  // the j / k consumer has room for this block's groups below
+  int done;                      // slots given back (kept for a courier at work)
+  int broken;                    // a wait for a slot ran out: the unit does no more
 };
 
 // One value as stamped words.
@@ -145,22 +149,21 @@ struct EdgeWords {
     }
   }
 };
+// four steps' values of a line as stamped words (32-byte stores; every word counts by itself)
 template <typename X>
-__device__ __forceinline__ void publish(unsigned long long* a, unsigned stamp, const X& v) {
-  constexpr int P = Words<X>::P;
-  uint32_t w[P];
-  to_words(v, w);
-  if constexpr (P == 1) {
-    st_gpu64(a, stamped(stamp, w[0]));
-  } else {
+__device__ __forceinline__ void publish(unsigned long long* a, unsigned stamp, const X (&v)[4]) {
+  constexpr int N = 4 * Words<X>::P;
+  uint32_t w[N];
 #pragma unroll
-    for (int p = 0; p < P; p += 2)
-      asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};"
-                   ::"l"(a + p), "l"(stamped(stamp, w[p])), "l"(stamped(stamp, w[p + 1])) : "memory");
-  }
+  for (int s = 0; s < 4; ++s) to_words(v[s], w + s * Words<X>::P);
+#pragma unroll
+  for (int q = 0; q < N; q += 4)
+    asm volatile("st.relaxed.gpu.global.v4.u64 [%0], {%1, %2, %3, %4};"
+                 ::"l"(a + q), "l"(stamped(stamp, w[q])), "l"(stamped(stamp, w[q + 1])),
+                 "l"(stamped(stamp, w[q + 2])), "l"(stamped(stamp, w[q + 3])) : "memory");
 }
 // N 32-bit words to a slot in this cluster, counted by its mbarrier (both
-// shared::cluster addresses; 4, 8 or a multiple of 16 bytes, so aligned)
+// shared::cluster addresses, the slot's aligned to the store)
 template <int N>
 __device__ __forceinline__ void send(unsigned a, unsigned bar, const uint32_t (&w)[N]) {
   if constexpr (N == 1) {
@@ -186,18 +189,10 @@ __device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank) {
 __device__ __forceinline__ void st_cluster_u32(unsigned a, unsigned v) {
   asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
-__device__ __forceinline__ unsigned ld_shared_u32(unsigned a) {
-  unsigned v;
-  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-  return v;
-}
 __device__ __forceinline__ int ld_acquire_s32(const int* p) {
   int v;
   asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
   return v;
-}
-__device__ __forceinline__ void st_release_s32(int* p, int v) {
-  asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -291,29 +286,31 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
   auto rank_at = [&](int c, int kk) { return (kk / NW) * WAVE_TJ + c; };
   if (helper && lane == 0) {
     for (int q = 0; q < S; ++q) {
-      mbar_init(&sh.ops[q]);
-      mbar_init(&sh.edge[q]);
+      mbar_init(&sh.full[q]);
       mbar_init(&sh.empty[q]);
     }
     sh.broken = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // per slot: the parity of its mbarriers' next phase at the start of a tile
-  // (operands and empty: one per group q; edge values: one per u)
+  // (empty: one per group q; full: one per u)
   unsigned phase_q = 0, phase_u = 0;
+  bool first = true;
 
   for (int pos = blockIdx.x / WAVE_CLUSTER, turn = 0; pos < g.ntiles; turn ^= 1) {
     const int tpos = REV ? g.ntiles - 1 - pos : pos;
     if (helper && lane == 0) sh.done = 0;
     int NJB = g.NJB, NKB = g.NKB, lj = g.nj, lk = g.nk;
     long long gbase = 0, bbase = 0, lbase = 0;
-    bool skip = false;
+    // (a unit that gave up in an earlier tile does not arm its mbarriers again)
+    bool skip = !first && *(volatile int*)&sh.broken != 0;
+    first = false;
     if (g.tile_scene != nullptr) {
       const int sid = g.tile_scene[tpos];
       const BatchSeg& B = g.segs[sid];
       // a converged scene's tiles are skipped (its scalars only change between
       // launches, so every warp of this launch decides the same way)
-      skip = g.scal_batch != nullptr && *(volatile int*)&g.scal_batch[sid].done != 0;
+      skip |= g.scal_batch != nullptr && *(volatile int*)&g.scal_batch[sid].done != 0;
       lj = B.nj;
       lk = B.nk;
       lbase = B.line_base;
@@ -367,14 +364,12 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
       unsigned to_j = 0, bar_j = 0, to_k = 0, bar_k = 0;   // near consumers: slot 0
       if (near_nj) {
         to_j = cluster_addr(smem_u32(unit_at(kt)->slot[0].ej[HL * kl]), rank_at(cj + DIR, kt));
-        bar_j = cluster_addr(smem_u32(&unit_at(kt)->edge[0]), rank_at(cj + DIR, kt));
+        bar_j = cluster_addr(smem_u32(&unit_at(kt)->full[0]), rank_at(cj + DIR, kt));
       }
       if (near_nk) {
         to_k = cluster_addr(smem_u32(unit_at(kt + DIR)->slot[0].ek[jl]), rank_at(cj, kt + DIR));
-        bar_k = cluster_addr(smem_u32(&unit_at(kt + DIR)->edge[0]), rank_at(cj, kt + DIR));
+        bar_k = cluster_addr(smem_u32(&unit_at(kt + DIR)->full[0]), rank_at(cj, kt + DIR));
       }
-      const unsigned ack_j = near_pj ? cluster_addr(smem_u32(&unit_at(kt)->limit[0]), rank_at(cj - DIR, kt)) : 0u;
-      const unsigned ack_k = near_pk ? cluster_addr(smem_u32(&unit_at(kt - DIR)->limit[1]), rank_at(cj, kt - DIR)) : 0u;
       // this lane's cells in a group: factor/system values (r/y: lane * 4)
       const int cell = wave_cell_slot<ST>(jl, FACTOR ? half * 4 + kl : 2 * kl, 0, 0) - (FACTOR ? half * 2 * GE : 0);
       constexpr int CELL_H = 8 * (16 / (int)sizeof(ST));   // from line h = 0 to h = 1
@@ -382,34 +377,35 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
       // the range of own groups that each consumer takes, and how they travel
       const int lo_j = uj, hi_j = nj.ng > 0 ? min(me.ng - 1, uj + nj.ng) : INT_MIN;
       const int lo_k = uk, hi_k = nk.ng > 0 ? min(me.ng - 1, uk + nk.ng) : INT_MIN;
-      const bool far_in = (!near_pj && pj.ng > 0) || (!near_pk && pk.ng > 0);
       const bool far = (!near_nj && nj.ng > 0) || (!near_nk && nk.ng > 0);
       // ... as a lane's own count of groups it sends from lo on (0: none)
       const unsigned near_j = near_nj && edge_j && hi_j >= lo_j ? (unsigned)(hi_j - lo_j) + 1u : 0u;
       const unsigned near_k = near_nk && edge_k && hi_k >= lo_k ? (unsigned)(hi_k - lo_k) + 1u : 0u;
-      const bool ack_to_j = lane == 0 && near_pj, ack_to_k = lane == 0 && near_pk;
-      VT* res = static_cast<VT*>(FACTOR ? g.fac_out : g.y) + (mybase + (REV ? me.ng - 1 : 0)) * (FACTOR ? 4 * GE : GE) +
-                (FACTOR ? wave_cell_slot<VT>(jl, half * 4 + kl, 0, 0) : lane * 4);
+      VT* res = static_cast<VT*>(g.sw) + (mybase + (REV ? me.ng - 1 : 0)) * WAVE_ROW +
+                (FACTOR ? wave_cell_slot<VT>(jl, half * 4 + kl, 0, 0) : WAVE_Y + lane * 4);
 
-      // waits for a slot's mbarrier; on expiry the results are void from then on
-      // and the host reports the timeout
+      // waits for a slot's mbarrier; on expiry the results are void and the block
+      // ends (its helper finds the error flag), and the host reports the timeout
+      bool bad = false;
       auto wait = [&](unsigned long long* bar, unsigned parity, unsigned site, int n) {
         const unsigned b = smem_u32(bar);
         if (mbar_try(b, parity)) return;
         Spin sp;
+        bool gave_up = false;
         while (!mbar_try(b, parity)) {
           if (!sp.step(g.ctl, g.spin_limit)) {
             raise_timeout(g.ctl, site, tpos, n, OP, 0ull, parity);
             *(volatile int*)&sh.broken = 1;
+            gave_up = true;
             break;
           }
         }
-        __syncwarp();
+        bad = __any_sync(XFP_FULL, gave_up);
       };
       X ej[HL][4], ek[4];        // the producers' values of the group, in sweep order
       auto take_edges = [&](int u) {   // (zero where a producer has no such group: the helper's work)
         const int sl = u & (S - 1);
-        wait(&sh.edge[sl], parity_u(u), 3, u);
+        wait(&sh.full[sl], parity_u(u), 3, u);
         const SL& in = sh.slot[sl];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
@@ -417,14 +413,6 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
           for (int h = 0; h < HL; ++h) ej[h][s] = in.ej[HL * kl + h][s];
           ek[s] = in.ek[jl][s];
         }
-      };
-      // once the values are in registers, their slot is the producers' again:
-      // the groups that fit, in their numbering (all the rest at the end)
-      auto ack = [&](int u) {
-        const int fit = u == me.ng ? INT_MAX / 2 : u + 1 + S;
-        if (ack_to_j) st_cluster_u32(ack_j, (unsigned)(fit + aj));
-        if (ack_to_k) st_cluster_u32(ack_k, (unsigned)(fit + ak));
-        if (far_in && lane == 0) st_release_s32(&sh.done, u + 1);
       };
       ST v[4][HL][4];            // operands: [step in sweep order][line][value]
       VT rhs[HL][4];
@@ -435,30 +423,25 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
       auto load_rhs = [&](const SL& in) {
         if constexpr (!FACTOR) {
 #pragma unroll
-          for (int h = 0; h < HL; ++h) ldg(rhs[h], reinterpret_cast<const VT*>(in.ops) + 4 * GE + h * 128 + lane * 4);
+          for (int h = 0; h < HL; ++h) ldg(rhs[h], reinterpret_cast<const VT*>(in.ops) + (REV ? WAVE_Y : WAVE_R) + h * 128 + lane * 4);
         }
       };
       X ox[HL] = {}, oz_own = X{};               // this lane's previous step: x, and z for its other line
       X sy[HL] = {}, sz = X{};                   // the neighbour lanes' previous step
       X cj_[HL], ck_;                            // the producers' step before the group
       take_edges(0);
-      __syncwarp();
-      ack(0);
-      wait(&sh.ops[0], parity_q(0), 5, 0);
 #pragma unroll
       for (int s = 0; s < 4; ++s) load_step(sh.slot[0], s);
       load_rhs(sh.slot[0]);
 #pragma unroll
       for (int h = 0; h < HL; ++h) cj_[h] = ej[h][3];
       ck_ = ek[3];
-      for (int q = 0; q < me.ng; ++q) {
+      int room = 0;                              // (as last looked up)
+      for (int q = 0; q < me.ng && !bad; ++q) {
         // Four steps.  What the chain waits for (the shuffles of a step's
         // results) is issued before what it does not (the next group's operands,
-        // which take the registers of the step just done; reports; stores).
-        const int qn = q + 1 < me.ng ? q + 1 : q;   // the group whose operands are loaded here
-        const SL& nx = sh.slot[qn & (S - 1)];
-        const bool ready = mbar_try(smem_u32(&sh.ops[qn & (S - 1)]), parity_q(qn));
-        const int room = min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1]);
+        // which take the registers of the step just done; stores).
+        const SL& nx = sh.slot[(q + 1) & (S - 1)];   // (after the last group: whatever it holds)
         take_edges(q + 1);
         VT out[HL][4];
         X outj[HL][4], outk[4];
@@ -522,10 +505,6 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
 #pragma unroll
           for (int h = 0; h < HL; ++h) sy[h] = REV ? shfl_down_any(oy[h], 1) : shfl_up_any(oy[h], 1);
           sz = REV ? shfl_down_any(oz[up], 8) : shfl_up_any(oz[up], 8);
-          if (s == 0) {
-            if (!ready) wait(&sh.ops[qn & (S - 1)], parity_q(qn), 5, qn);
-            ack(q + 1);
-          }
           load_step(nx, s);
           if constexpr (FACTOR) {
             const VT f[4] = {(VT)ox[0].a, (VT)oy[0].a, (VT)oz[0].a, (VT)pivot};
@@ -538,8 +517,9 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
         // ---- edge values to the upper neighbours ----
         if (q >= room) {
           // a consumer's slot may not be free yet
-          Spin sp;
-          while (q >= min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1])) {
+          auto look = [&] { room = min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1]); };
+          look();
+          for (Spin sp; q >= room; look()) {
             if (!sp.step(g.ctl, g.spin_limit)) {
               raise_timeout(g.ctl, 4, tpos, q, OP, 0ull, (unsigned)room);
               break;
@@ -547,40 +527,34 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
           }
           __syncwarp();
         }
-        {
-          const unsigned d = (unsigned)(q - uj) & (S - 1);
-          const unsigned a = to_j + d * (unsigned)sizeof(SL), b = bar_j + d * 8;
-          uint32_t w[HL][4 * P];
+        const bool to_near_j = (unsigned)(q - lo_j) < near_j, to_near_k = (unsigned)(q - lo_k) < near_k;
+        if (to_near_j || to_near_k) {
+          if (to_near_j) {
+            const unsigned d = (unsigned)(q - uj) & (S - 1);
 #pragma unroll
-          for (int h = 0; h < HL; ++h)
+            for (int h = 0; h < HL; ++h) {
+              uint32_t w[4 * P];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) to_words(outj[h][s], w[h] + s * P);
-          if ((unsigned)(q - lo_j) < near_j) {
-#pragma unroll
-            for (int h = 0; h < HL; ++h) send(a + h * 4 * (unsigned)sizeof(X), b, w[h]);
+              for (int s = 0; s < 4; ++s) to_words(outj[h][s], w + s * P);
+              send(to_j + d * (unsigned)sizeof(SL) + h * 4 * (unsigned)sizeof(X), bar_j + d * 8, w);
+            }
           }
-        }
-        {
-          const unsigned d = (unsigned)(q - uk) & (S - 1);
-          const unsigned a = to_k + d * (unsigned)sizeof(SL), b = bar_k + d * 8;
-          uint32_t w[4 * P];
+          if (to_near_k) {
+            const unsigned d = (unsigned)(q - uk) & (S - 1);
+            uint32_t w[4 * P];
 #pragma unroll
-          for (int s = 0; s < 4; ++s) to_words(outk[s], w + s * P);
-          if ((unsigned)(q - lo_k) < near_k) send(a, b, w);
+            for (int s = 0; s < 4; ++s) to_words(outk[s], w + s * P);
+            send(to_k + d * (unsigned)sizeof(SL), bar_k + d * 8, w);
+          }
         }
         if (far) {
           if (!near_nj && edge_j && q >= lo_j && q <= hi_j) {
 #pragma unroll
-            for (int s = 0; s < 4; ++s)
-#pragma unroll
-              for (int h = 0; h < HL; ++h)
-                publish<X>(g.bj + ((size_t)(mybase + q) * 32 + s * 8 + half * 4 + HL * kl + h) * P, gen, outj[h][s]);
+            for (int h = 0; h < HL; ++h)
+              publish<X>(g.bj + ((size_t)(mybase + q) * 32 + (half * 4 + HL * kl + h) * 4) * P, gen, outj[h]);
           }
-          if (!near_nk && edge_k && q >= lo_k && q <= hi_k) {
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-              publish<X>(g.bk + ((size_t)(mybase + q) * 32 + s * 8 + jl) * P, gen, outk[s]);
-          }
+          if (!near_nk && edge_k && q >= lo_k && q <= hi_k)
+            publish<X>(g.bk + ((size_t)(mybase + q) * 32 + jl * 4) * P, gen, outk);
         }
         // ---- results (the backward solve's z also to its slot, for z.r) ----
         if constexpr (!FACTOR) {
@@ -588,81 +562,78 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
           for (int h = 0; h < HL; ++h) {
             stg(res + h * 128, out[h]);
             if constexpr (REV)
-              stg(reinterpret_cast<VT*>(sh.slot[q & (S - 1)].ops) + 4 * GE + h * 128 + lane * 4, out[h]);
+              stg(reinterpret_cast<VT*>(sh.slot[q & (S - 1)].ops) + WAVE_Y + h * 128 + lane * 4, out[h]);
           }
         }
-        res += DIR * (FACTOR ? 4 * GE : GE);
+        res += DIR * WAVE_ROW;
         load_rhs(nx);
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.empty[q & (S - 1)]);
       }
     } else if (!skip && me.ng > 0 && helper) {
       // ======================= helper warp =======================
-      auto row_of = [&](int q) -> long long { return mybase + (REV ? me.ng - 1 - q : q); };
-      auto fill_ops = [&](int q) {   // one lane
-        SL& d = sh.slot[q & (S - 1)];
-        unsigned long long* b = &sh.ops[q & (S - 1)];
-        mbar_expect(b, W::IN * (unsigned)sizeof(ST));
-        const long long e = row_of(q);
-        if constexpr (FACTOR) {
-          bulk_load(d.ops, static_cast<const ST*>(g.sys) + e * 4 * GE + half * 2 * GE, 2 * GE * sizeof(ST), b);
-        } else {
-          bulk_load(d.ops, static_cast<const ST*>(g.fac) + e * 4 * GE, 4 * GE * sizeof(ST), b);
-          bulk_load(d.ops + 4 * GE, static_cast<const ST*>(REV ? g.y : g.r) + e * GE, GE * sizeof(ST), b);
-          if constexpr (REV) bulk_load(d.ops + 5 * GE, static_cast<const ST*>(g.r) + e * GE, GE * sizeof(ST), b);
-        }
-      };
-      auto arm_edges = [&](int u) {   // the whole warp
-        SL& d = sh.slot[u & (S - 1)];
-        const bool have_j = (unsigned)(u + aj) < (unsigned)pj.ng, have_k = (unsigned)(u + ak) < (unsigned)pk.ng;
+      // operands of the next group to load
+      const long long e0 = mybase + (REV ? me.ng - 1 : 0);
+      const ST* src = FACTOR ? static_cast<const ST*>(g.sys) + e0 * 4 * GE + half * 2 * GE : static_cast<const ST*>(g.sw) + e0 * WAVE_ROW;
+      auto arm = [&](int n) {   // slot of group n, edge values u = n (the whole warp, n = 0, 1, ...)
+        SL& d = sh.slot[n & (S - 1)];
+        const bool have_j = (unsigned)(n + aj) < (unsigned)pj.ng, have_k = (unsigned)(n + ak) < (unsigned)pk.ng;
         // a producer without such a group sends nothing: its edge values are zero
-        if (!have_j)
-          for (int q = lane; q < (int)(sizeof(d.ej) / 16); q += 32) reinterpret_cast<uint4*>(&d.ej[0][0])[q] = make_uint4(0, 0, 0, 0);
-        if (!have_k)
-          for (int q = lane; q < (int)(sizeof(d.ek) / 16); q += 32) reinterpret_cast<uint4*>(&d.ek[0][0])[q] = make_uint4(0, 0, 0, 0);
-        __syncwarp();
-        if (lane == 0)
-          mbar_expect(&sh.edge[u & (S - 1)], (have_j ? (unsigned)sizeof(d.ej) : 0u) + (have_k ? (unsigned)sizeof(d.ek) : 0u));
+        // (and stay so, unless the slot's last use had some)
+        const bool clear_j = !have_j && (n < S || (unsigned)(n - S + aj) < (unsigned)pj.ng);
+        const bool clear_k = !have_k && (n < S || (unsigned)(n - S + ak) < (unsigned)pk.ng);
+        if (clear_j || clear_k) {
+          if (clear_j)
+            for (int q = lane; q < (int)(sizeof(d.ej) / 16); q += 32) reinterpret_cast<uint4*>(&d.ej[0][0])[q] = make_uint4(0, 0, 0, 0);
+          if (clear_k)
+            for (int q = lane; q < (int)(sizeof(d.ek) / 16); q += 32) reinterpret_cast<uint4*>(&d.ek[0][0])[q] = make_uint4(0, 0, 0, 0);
+          __syncwarp();
+        }
+        if (lane == 0) {
+          unsigned long long* b = &sh.full[n & (S - 1)];
+          mbar_expect(b, (have_j ? (unsigned)sizeof(d.ej) : 0u) + (have_k ? (unsigned)sizeof(d.ek) : 0u) +
+                             (n < me.ng ? W::IN * (unsigned)sizeof(ST) : 0u));
+          if (n < me.ng) bulk_load(d.ops, src, W::IN * sizeof(ST), b);
+        }
+        src += DIR * (FACTOR ? 4 * GE : WAVE_ROW);
       };
-      const bool ok = __all_sync(XFP_FULL, *(volatile int*)&sh.broken == 0);
-      if (ok) {
-        for (int q = 0; lane == 0 && q < S && q < me.ng; ++q) fill_ops(q);
-        __syncwarp();
-        for (int u = 0; u < S && u <= me.ng; ++u) arm_edges(u);
-      }
+      const unsigned ack_j = near_pj ? cluster_addr(smem_u32(&unit_at(kt)->limit[0]), rank_at(cj - DIR, kt)) : 0u;
+      const unsigned ack_k = near_pk ? cluster_addr(smem_u32(&unit_at(kt - DIR)->limit[1]), rank_at(cj, kt - DIR)) : 0u;
+      // who is told of a slot given back, a lane each: the producers in this
+      // cluster (in their numbering) and the courier
+      const bool far_in = (!near_pj && pj.ng > 0) || (!near_pk && pk.ng > 0);
+      const unsigned tell = lane == 0 ? ack_j : lane == 1 ? ack_k : cluster_addr(smem_u32(&sh.done), rank);
+      const int tell_ahead = lane == 0 ? S + aj : lane == 1 ? S + ak : 0;
+      const bool told = (lane == 0 && near_pj) || (lane == 1 && near_pk) || (lane == 2 && far_in);
+      for (int n = 0; n < S && n <= me.ng; ++n) arm(n);
       float dotf[2] = {0.f, 0.f};
       double dotd[2] = {0.0, 0.0};
-      for (int q = 0; ok && q < me.ng; ++q) {
+      for (int q = 0; q < me.ng; ++q) {
         const int sl = q & (S - 1);
-        // the compute warp is done with group q (and has taken the edge values of u = q + 1)
+        // the compute warp is done with group q
         const unsigned b = smem_u32(&sh.empty[sl]), parity = parity_q(q);
-        Spin sp;
-        bool out_of_time = false;
-        while (!__all_sync(XFP_FULL, mbar_try(b, parity))) {
-          // (its own waits are bounded; this one outlasts them)
-          sp.step(g.ctl, 8 * g.spin_limit);
-          if (sp.n >= 8 * g.spin_limit) {
+        if (!__all_sync(XFP_FULL, mbar_try(b, parity))) {
+          Spin sp;
+          // (the compute warp's own waits are bounded; this one outlasts them)
+          while (!mbar_try(b, parity) && sp.step(g.ctl, 8 * g.spin_limit)) {
+          }
+          if (!__all_sync(XFP_FULL, mbar_try(b, parity))) {
             raise_timeout(g.ctl, 7, tpos, q, OP, 0ull, parity);
-            out_of_time = true;
             break;
           }
         }
-        // (after a timeout the mbarriers are not armed again)
-        if (out_of_time || !__all_sync(XFP_FULL, *(volatile int*)&sh.broken == 0)) break;
         VT z[2][4], rr[2][4];
         if constexpr (REV) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            ldg(z[h], reinterpret_cast<const VT*>(sh.slot[sl].ops) + 4 * GE + h * 128 + lane * 4);
-            ldg(rr[h], reinterpret_cast<const VT*>(sh.slot[sl].ops) + 5 * GE + h * 128 + lane * 4);
+            ldg(z[h], reinterpret_cast<const VT*>(sh.slot[sl].ops) + WAVE_Y + h * 128 + lane * 4);
+            ldg(rr[h], reinterpret_cast<const VT*>(sh.slot[sl].ops) + WAVE_R + h * 128 + lane * 4);
           }
           __syncwarp();
         }
-        if (lane == 0 && q + S < me.ng) fill_ops(q + S);
-        __syncwarp();
-        if (q + 1 + S <= me.ng) arm_edges(q + 1 + S);
-        // u = 0 was taken before the first group: its slot is armed with u = 1's
-        if (q == 0 && S <= me.ng) arm_edges(S);
+        if (q + S <= me.ng) arm(q + S);
+        // the slot is the producers' again (all the rest at the end)
+        if (told) st_cluster_u32(tell, (unsigned)((q + 1 == me.ng ? INT_MAX / 2 : q + 1) + tell_ahead));
         if constexpr (REV) {
           // z.r, each line in cell order
 #pragma unroll
@@ -670,6 +641,7 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               if (DOT32) dotf[h] = __fadd_rn(dotf[h], __fmul_rn((float)z[h][s], (float)rr[h][s]));
+              else if (sizeof(VT) == 4) dotd[h] = __fma_rn((double)z[h][s], (double)rr[h][s], dotd[h]);   // (the product is exact)
               else dotd[h] = __dadd_rn(dotd[h], __dmul_rn((double)z[h][s], (double)rr[h][s]));
             }
         }
@@ -685,7 +657,7 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
       }
     } else if (!skip && me.ng > 0 && courier) {
       // ======================= courier warp =======================
-      // far producers: this block's u .. last, FB under way; lane = step * lines + line
+      // far producers: this block's u .. last, FB under way; lane = line * 4 + step
       const unsigned want = gen + g.expect_bias;   // bias != 0 only in the expired-wait diagnostic
       constexpr int LJ = HL * 4;                   // lines of this unit's j edge
       const bool use_j = lane < 4 * LJ;
@@ -705,11 +677,11 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
       range(fj, near_pj, aj, pj);
       range(fk, near_pk, ak, pk);
       const unsigned long long* src_j =
-          g.bj + ((size_t)(gbase + pj.goff) * 32 + (lane / LJ) * 8 + half * 4 + lane % LJ) * P;
+          g.bj + ((size_t)(gbase + pj.goff) * 32 + half * 16 + lane) * P;
       const unsigned long long* src_k = g.bk + ((size_t)(gbase + pk.goff) * 32 + lane) * P;
-      const unsigned to_j = cluster_addr(smem_u32(&sh.slot[0].ej[lane % LJ][(lane / LJ) & 3]), rank);
-      const unsigned to_k = cluster_addr(smem_u32(&sh.slot[0].ek[lane & 7][lane >> 3]), rank);
-      const unsigned bar = cluster_addr(smem_u32(&sh.edge[0]), rank);
+      const unsigned to_j = cluster_addr(smem_u32(&sh.slot[0].ej[(lane >> 2) % LJ][lane & 3]), rank);
+      const unsigned to_k = cluster_addr(smem_u32(&sh.slot[0].ek[lane >> 2][lane & 3]), rank);
+      const unsigned bar = cluster_addr(smem_u32(&sh.full[0]), rank);
       auto request = [&](Far& f, const unsigned long long* src, int a, bool use) {
 #pragma unroll
         for (int d = 0; d < FB; ++d)
@@ -883,9 +855,9 @@ __global__ void sw_permute_kernel(T* __restrict__ line, T* __restrict__ sw, cons
     T v[4];
     if (dir == 0) {
       ldg(v, line + 4 * q);
-      stg(sw + gperm[q], v);
+      stg(sw + wave_value(gperm[q]), v);
     } else {
-      ldg(v, sw + gperm[q]);
+      ldg(v, sw + wave_value(gperm[q]));
       stg(line + 4 * q, v);
     }
   }
@@ -905,7 +877,7 @@ __global__ void factor_lines_kernel(const T* __restrict__ fac, const Line* __res
     if ((unsigned)(i - L.lo) >= (unsigned)L.len) return T(0);
     const int t = i + j + k;
     const WBlk b = blks[(size_t)(k >> 3) * NJB + (j >> 3)];
-    return fac[(size_t)(b.goff + (t >> 2) - b.g0) * 4 * GE + wave_cell_slot<T>(j, k, t & 3, a)];
+    return fac[(size_t)(b.goff + (t >> 2) - b.g0) * WAVE_ROW + wave_cell_slot<T>(j, k, t & 3, a)];
   };
   for (long long line = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); line < nlines;
        line += (long long)gridDim.x * (blockDim.x >> 5)) {
