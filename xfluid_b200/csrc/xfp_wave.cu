@@ -35,10 +35,12 @@
 // A slot of the ring holds all that a block needs for one group -- its own
 // operands and its lower neighbours' edge values -- and one mbarrier counts
 // their bytes, so a compute warp waits once per group and then runs four steps
-// on registers and shuffles.  Two more warps keep the rest off its chain: a
-// helper refills the slots (bulk copies, S groups ahead) and sums z.r, and a
-// courier fetches the edge values that come through global memory.  A block
-// reports the groups it has taken, and no one writes a slot before that.
+// on registers and shuffles.  Three more warps keep the rest off its chain: a
+// sender takes the results from the slot to global memory and hands on the edges,
+// a helper refills the slots (bulk copies, S groups ahead) and reports the free
+// ones, without which no one writes to them, and a courier fetches the edge values
+// that come through global memory.  (The factorisation's step is long enough for
+// its compute warp to hand on its results itself.)
 //
 // Data.  Every block's cells lie in its own stream of groups of 4 steps (WBlk,
 // wave_line_slot, wave_cell_slot), a group's factor, r and y side by side, so
@@ -59,14 +61,17 @@
 // chunks (one CTA alone reads 65,536 partials at 256^3).
 //
 // Measured (device time of a launch, full box of 128^3 / 256^3 cells): a solve
-// takes 74 / 190 us in FP32 and 102 / 330 us in FP64 -- 0.31 (0.39) us per group
-// of four steps of a lone block, 0.05 more where it hands edges on, 12 us to start
-// and end a launch -- and the factorisation 0.23 / 0.68 ms.  (With an mbarrier each
-// for operands and edge values, acknowledgements by the compute warp and two or
-// three copies a group: 0.43 (0.50) us, 83 / 214 and 114 / 365 us.)
+// takes 62 / 164 us in FP32 and 92 / 290 us in FP64, the factorisation 0.24 / 0.68
+// ms; a launch costs 12 us to start and end, a group of four steps of a lone block
+// 0.25 (0.36) us, of which the steps are 0.13 (0.2) and the rest is waiting for a
+// slot, reading it and handing it on.
+// With the compute warp sending its edges and storing its results, as the
+// factorisation's does: 0.31 (0.39) us a group, 74 / 190 and 102 / 330 us.  With an
+// mbarrier each for operands and edge values, acknowledgements by the compute warp
+// and two or three copies a group: 0.43 (0.50) us, 83 / 214 and 114 / 365 us.
 // Before (one CTA per 32 x 15 lines, a CTA-wide barrier per step, tiles through
 // global memory): 263 us for the FP64 128^3 solve, 180 us for a half-full FP32
-// 256^3 one (now 92), 0.65 to 1.0 ms for the factorisation.  Tried on the way:
+// 256^3 one (now 80), 0.65 to 1.0 ms for the factorisation.  Tried on the way:
 // lockstep CTAs of 2 x 2 blocks (143 us where the first form took 81), blocks that
 // hand over through L2 words only (117 to 134), per-step instead of per-group
 // hand-over in the cluster (367 cycles a step), one warp as helper and courier with
@@ -99,6 +104,9 @@ struct WaveOp<SWEEP_FACTOR, VT, CT> {
   using ST = CT;
   static constexpr int HL = 1, IN = 2 * GE, S = 4;
 };
+// Warps for a unit: compute, helper, courier and, for the solves, sender.
+template <int OP>
+constexpr int roles_of() { return OP == SWEEP_FACTOR ? 3 : 4; }
 template <int OP>
 constexpr int warps_of() { return OP == SWEEP_FACTOR ? 4 : 2; }   // compute warps per CTA (two blocks)
 
@@ -116,9 +124,10 @@ struct __align__(128) UnitShared {
   static constexpr int S = WaveOp<OP, VT, CT>::S;
   Slot<OP, VT, CT> slot[S];
   unsigned long long full[S];    // mbarriers: a slot's operands and edge values have landed
-  unsigned long long empty[S];   // mbarriers: the compute warp is done with a slot
+  unsigned long long ready[S];   // mbarriers: a slot holds the group's results (solves)
+  unsigned long long empty[S];   // mbarriers: a slot can be filled again
   int limit[2];                  // the j / k consumer has room for this block's groups below
-  int done;                      // slots given back (kept for a courier at work)
+  int freed;                     // slots given back (kept for a courier at work)
   int broken;                    // a wait for a slot ran out: the unit does no more
 };
 
@@ -249,8 +258,26 @@ __device__ __forceinline__ void put_cell(double* p, int c, int e, const double (
   *reinterpret_cast<double2*>(p + c + e * 128 + 64) = make_double2(v[2], v[3]);
 }
 
+// z.r of a line in cell order (a backward group is taken from its last cell on),
+// in FP32 or in FP64
+template <typename VT, bool F32>
+struct LineDot {
+  float f = 0.f;
+  double d = 0.0;
+  __device__ __forceinline__ void add(const VT (&z)[4], const VT (&r)[4]) {
+#pragma unroll
+    for (int s = 3; s >= 0; --s) {
+      if (F32) f = __fadd_rn(f, __fmul_rn((float)z[s], (float)r[s]));
+      else if (sizeof(VT) == 4) d = __fma_rn((double)z[s], (double)r[s], d);   // (the product is exact)
+      else d = __dadd_rn(d, __dmul_rn((double)z[s], (double)r[s]));
+    }
+  }
+  __device__ __forceinline__ double sum() const { return F32 ? (double)f : d; }
+};
+
 template <int OP, typename VT, typename CT>
-__global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveArgs g) {
+__global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SWEEP_FACTOR && sizeof(VT) == 4 ? 2 : 1)
+    wave_kernel(WaveArgs g) {
   using W = WaveOp<OP, VT, CT>;
   using X = typename W::X;
   using ST = typename W::ST;
@@ -261,6 +288,7 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
   static_assert(S == 1 << LS, "slots are a power of two");
   constexpr bool DOT32 = std::is_same<CT, float>::value;   // plain FP32: a lane's z.r in FP32
   constexpr int DIR = REV ? -1 : 1;
+  constexpr int OUT = REV ? WAVE_Y : WAVE_R;               // a slot's results
   constexpr int NW = warps_of<OP>(), PER = NW / 2;         // compute warps per CTA, per block
   extern __shared__ __align__(128) unsigned char wave_smem[];
   U* const units = reinterpret_cast<U*>(wave_smem);
@@ -271,7 +299,7 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
   if (g.scal != nullptr && *(volatile int*)&g.scal->done != 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int unit = warp % NW;
-  const bool helper = warp / NW == 1, courier = warp / NW == 2;
+  const bool compute = warp < NW, helper = warp / NW == 1, courier = warp / NW == 2;
   U& sh = units[unit];
   const int jl = lane & 7, kl = lane >> 3;
   const int rank = blockIdx.x % WAVE_CLUSTER;
@@ -287,19 +315,20 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
   if (helper && lane == 0) {
     for (int q = 0; q < S; ++q) {
       mbar_init(&sh.full[q]);
+      mbar_init(&sh.ready[q]);
       mbar_init(&sh.empty[q]);
     }
     sh.broken = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // per slot: the parity of its mbarriers' next phase at the start of a tile
-  // (empty: one per group q; full: one per u)
+  // (ready and empty: one per group q; full: one per u)
   unsigned phase_q = 0, phase_u = 0;
   bool first = true;
 
   for (int pos = blockIdx.x / WAVE_CLUSTER, turn = 0; pos < g.ntiles; turn ^= 1) {
     const int tpos = REV ? g.ntiles - 1 - pos : pos;
-    if (helper && lane == 0) sh.done = 0;
+    if (helper && lane == 0) sh.freed = 0;
     int NJB = g.NJB, NKB = g.NKB, lj = g.nj, lk = g.nk;
     long long gbase = 0, bbase = 0, lbase = 0;
     // (a unit that gave up in an earlier tile does not arm its mbarriers again)
@@ -357,7 +386,27 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
 
     auto parity_q = [&](int q) { return ((phase_q >> (q & (S - 1))) ^ (unsigned)(q >> LS)) & 1u; };
     auto parity_u = [&](int u) { return ((phase_u >> (u & (S - 1))) ^ (unsigned)(u >> LS)) & 1u; };
-    if (!skip && me.ng > 0 && !helper && !courier) {
+    // waits for the phase of a mbarrier that another warp of this unit completes
+    // (whose own waits are bounded; this one outlasts them); false: it gave up
+    auto await = [&](unsigned long long* bar, int q, unsigned site) -> bool {
+      const unsigned b = smem_u32(bar), parity = parity_q(q);
+      if (__all_sync(XFP_FULL, mbar_try(b, parity))) return true;
+      Spin sp;
+      while (!mbar_try(b, parity) && sp.step(g.ctl, 8 * g.spin_limit)) {
+      }
+      if (__all_sync(XFP_FULL, mbar_try(b, parity))) return true;
+      raise_timeout(g.ctl, site, tpos, q, OP, 0ull, parity);
+      return false;
+    };
+    // z.r of this lane's line h of the block
+    auto put_dot = [&](int h, const LineDot<VT, DOT32>& d) {
+      const int j = jb * 8 + jl, k = kb * 8 + 2 * kl + h;
+      if (j < lj && k < lk) g.partials[lbase + (long long)k * lj + j] = d.sum();
+    };
+    // the range of own groups that each consumer takes
+    const int lo_j = uj, hi_j = nj.ng > 0 ? min(me.ng - 1, uj + nj.ng) : INT_MIN;
+    const int lo_k = uk, hi_k = nk.ng > 0 ? min(me.ng - 1, uk + nk.ng) : INT_MIN;
+    if (!skip && me.ng > 0 && compute) {
       // ======================= compute warp =======================
       const bool edge_j = jl == (REV ? 0 : 7), edge_k = kl == (REV ? 0 : 3);
       const bool in_j = jl == (REV ? 7 : 0), in_k = kl == (REV ? 3 : 0);
@@ -374,15 +423,11 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
       const int cell = wave_cell_slot<ST>(jl, FACTOR ? half * 4 + kl : 2 * kl, 0, 0) - (FACTOR ? half * 2 * GE : 0);
       constexpr int CELL_H = 8 * (16 / (int)sizeof(ST));   // from line h = 0 to h = 1
 
-      // the range of own groups that each consumer takes, and how they travel
-      const int lo_j = uj, hi_j = nj.ng > 0 ? min(me.ng - 1, uj + nj.ng) : INT_MIN;
-      const int lo_k = uk, hi_k = nk.ng > 0 ? min(me.ng - 1, uk + nk.ng) : INT_MIN;
       const bool far = (!near_nj && nj.ng > 0) || (!near_nk && nk.ng > 0);
       // ... as a lane's own count of groups it sends from lo on (0: none)
       const unsigned near_j = near_nj && edge_j && hi_j >= lo_j ? (unsigned)(hi_j - lo_j) + 1u : 0u;
       const unsigned near_k = near_nk && edge_k && hi_k >= lo_k ? (unsigned)(hi_k - lo_k) + 1u : 0u;
-      VT* res = static_cast<VT*>(g.sw) + (mybase + (REV ? me.ng - 1 : 0)) * WAVE_ROW +
-                (FACTOR ? wave_cell_slot<VT>(jl, half * 4 + kl, 0, 0) : WAVE_Y + lane * 4);
+      VT* res = static_cast<VT*>(g.sw) + mybase * WAVE_ROW + wave_cell_slot<VT>(jl, half * 4 + kl, 0, 0);   // (the factor)
 
       // waits for a slot's mbarrier; on expiry the results are void and the block
       // ends (its helper finds the error flag), and the host reports the timeout
@@ -442,7 +487,6 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
         // results) is issued before what it does not (the next group's operands,
         // which take the registers of the step just done; stores).
         const SL& nx = sh.slot[(q + 1) & (S - 1)];   // (after the last group: whatever it holds)
-        take_edges(q + 1);
         VT out[HL][4];
         X outj[HL][4], outk[4];
 #pragma unroll
@@ -505,6 +549,7 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
 #pragma unroll
           for (int h = 0; h < HL; ++h) sy[h] = REV ? shfl_down_any(oy[h], 1) : shfl_up_any(oy[h], 1);
           sz = REV ? shfl_down_any(oz[up], 8) : shfl_up_any(oz[up], 8);
+          if (s == 0) take_edges(q + 1);   // (the first step needs the last group's)
           load_step(nx, s);
           if constexpr (FACTOR) {
             const VT f[4] = {(VT)ox[0].a, (VT)oy[0].a, (VT)oz[0].a, (VT)pivot};
@@ -514,61 +559,59 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
 #pragma unroll
         for (int h = 0; h < HL; ++h) cj_[h] = ej[h][3];
         ck_ = ek[3];
-        // ---- edge values to the upper neighbours ----
-        if (q >= room) {
-          // a consumer's slot may not be free yet
-          auto look = [&] { room = min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1]); };
-          look();
-          for (Spin sp; q >= room; look()) {
-            if (!sp.step(g.ctl, g.spin_limit)) {
-              raise_timeout(g.ctl, 4, tpos, q, OP, 0ull, (unsigned)room);
-              break;
+        if constexpr (FACTOR) {
+          // ---- edge values to the upper neighbours ----
+          if (q >= room) {
+            // a consumer's slot may not be free yet
+            auto look = [&] { room = min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1]); };
+            look();
+            for (Spin sp; q >= room; look()) {
+              if (!sp.step(g.ctl, g.spin_limit)) {
+                raise_timeout(g.ctl, 4, tpos, q, OP, 0ull, (unsigned)room);
+                break;
+              }
             }
+            __syncwarp();
           }
-          __syncwarp();
-        }
-        const bool to_near_j = (unsigned)(q - lo_j) < near_j, to_near_k = (unsigned)(q - lo_k) < near_k;
-        if (to_near_j || to_near_k) {
-          if (to_near_j) {
-            const unsigned d = (unsigned)(q - uj) & (S - 1);
+          const bool to_near_j = (unsigned)(q - lo_j) < near_j, to_near_k = (unsigned)(q - lo_k) < near_k;
+          if (to_near_j || to_near_k) {
+            if (to_near_j) {
+              const unsigned d = (unsigned)(q - uj) & (S - 1);
 #pragma unroll
-            for (int h = 0; h < HL; ++h) {
+              for (int h = 0; h < HL; ++h) {
+                uint32_t w[4 * P];
+#pragma unroll
+                for (int s = 0; s < 4; ++s) to_words(outj[h][s], w + s * P);
+                send(to_j + d * (unsigned)sizeof(SL) + h * 4 * (unsigned)sizeof(X), bar_j + d * 8, w);
+              }
+            }
+            if (to_near_k) {
+              const unsigned d = (unsigned)(q - uk) & (S - 1);
               uint32_t w[4 * P];
 #pragma unroll
-              for (int s = 0; s < 4; ++s) to_words(outj[h][s], w + s * P);
-              send(to_j + d * (unsigned)sizeof(SL) + h * 4 * (unsigned)sizeof(X), bar_j + d * 8, w);
+              for (int s = 0; s < 4; ++s) to_words(outk[s], w + s * P);
+              send(to_k + d * (unsigned)sizeof(SL), bar_k + d * 8, w);
             }
           }
-          if (to_near_k) {
-            const unsigned d = (unsigned)(q - uk) & (S - 1);
-            uint32_t w[4 * P];
+          if (far) {
+            if (!near_nj && edge_j && q >= lo_j && q <= hi_j) {
 #pragma unroll
-            for (int s = 0; s < 4; ++s) to_words(outk[s], w + s * P);
-            send(to_k + d * (unsigned)sizeof(SL), bar_k + d * 8, w);
+              for (int h = 0; h < HL; ++h)
+                publish<X>(g.bj + ((size_t)(mybase + q) * 32 + (half * 4 + HL * kl + h) * 4) * P, gen, outj[h]);
+            }
+            if (!near_nk && edge_k && q >= lo_k && q <= hi_k)
+              publish<X>(g.bk + ((size_t)(mybase + q) * 32 + jl * 4) * P, gen, outk);
           }
-        }
-        if (far) {
-          if (!near_nj && edge_j && q >= lo_j && q <= hi_j) {
+          res += WAVE_ROW;
+        } else {
+          // the results to the slot, for the sender (forward: over r)
 #pragma unroll
-            for (int h = 0; h < HL; ++h)
-              publish<X>(g.bj + ((size_t)(mybase + q) * 32 + (half * 4 + HL * kl + h) * 4) * P, gen, outj[h]);
-          }
-          if (!near_nk && edge_k && q >= lo_k && q <= hi_k)
-            publish<X>(g.bk + ((size_t)(mybase + q) * 32 + jl * 4) * P, gen, outk);
+          for (int h = 0; h < HL; ++h)
+            stg(reinterpret_cast<VT*>(sh.slot[q & (S - 1)].ops) + OUT + h * 128 + lane * 4, out[h]);
         }
-        // ---- results (the backward solve's z also to its slot, for z.r) ----
-        if constexpr (!FACTOR) {
-#pragma unroll
-          for (int h = 0; h < HL; ++h) {
-            stg(res + h * 128, out[h]);
-            if constexpr (REV)
-              stg(reinterpret_cast<VT*>(sh.slot[q & (S - 1)].ops) + WAVE_Y + h * 128 + lane * 4, out[h]);
-          }
-        }
-        res += DIR * WAVE_ROW;
         load_rhs(nx);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sh.empty[q & (S - 1)]);
+        if (lane == 0) mbar_arrive(FACTOR ? &sh.empty[q & (S - 1)] : &sh.ready[q & (S - 1)]);
       }
     } else if (!skip && me.ng > 0 && helper) {
       // ======================= helper warp =======================
@@ -602,59 +645,26 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
       // who is told of a slot given back, a lane each: the producers in this
       // cluster (in their numbering) and the courier
       const bool far_in = (!near_pj && pj.ng > 0) || (!near_pk && pk.ng > 0);
-      const unsigned tell = lane == 0 ? ack_j : lane == 1 ? ack_k : cluster_addr(smem_u32(&sh.done), rank);
+      const unsigned tell = lane == 0 ? ack_j : lane == 1 ? ack_k : cluster_addr(smem_u32(&sh.freed), rank);
       const int tell_ahead = lane == 0 ? S + aj : lane == 1 ? S + ak : 0;
       const bool told = (lane == 0 && near_pj) || (lane == 1 && near_pk) || (lane == 2 && far_in);
       for (int n = 0; n < S && n <= me.ng; ++n) arm(n);
-      float dotf[2] = {0.f, 0.f};
-      double dotd[2] = {0.0, 0.0};
+      LineDot<VT, DOT32> dot;   // of the lines h = 1
       for (int q = 0; q < me.ng; ++q) {
         const int sl = q & (S - 1);
-        // the compute warp is done with group q
-        const unsigned b = smem_u32(&sh.empty[sl]), parity = parity_q(q);
-        if (!__all_sync(XFP_FULL, mbar_try(b, parity))) {
-          Spin sp;
-          // (the compute warp's own waits are bounded; this one outlasts them)
-          while (!mbar_try(b, parity) && sp.step(g.ctl, 8 * g.spin_limit)) {
-          }
-          if (!__all_sync(XFP_FULL, mbar_try(b, parity))) {
-            raise_timeout(g.ctl, 7, tpos, q, OP, 0ull, parity);
-            break;
-          }
-        }
-        VT z[2][4], rr[2][4];
+        if (!await(&sh.empty[sl], q, 7)) break;
+        VT z[4], rr[4];
         if constexpr (REV) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            ldg(z[h], reinterpret_cast<const VT*>(sh.slot[sl].ops) + WAVE_Y + h * 128 + lane * 4);
-            ldg(rr[h], reinterpret_cast<const VT*>(sh.slot[sl].ops) + WAVE_R + h * 128 + lane * 4);
-          }
+          ldg(z, reinterpret_cast<const VT*>(sh.slot[sl].ops) + WAVE_Y + 128 + lane * 4);
+          ldg(rr, reinterpret_cast<const VT*>(sh.slot[sl].ops) + WAVE_R + 128 + lane * 4);
           __syncwarp();
         }
         if (q + S <= me.ng) arm(q + S);
         // the slot is the producers' again (all the rest at the end)
         if (told) st_cluster_u32(tell, (unsigned)((q + 1 == me.ng ? INT_MAX / 2 : q + 1) + tell_ahead));
-        if constexpr (REV) {
-          // z.r, each line in cell order
-#pragma unroll
-          for (int s = 3; s >= 0; --s)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              if (DOT32) dotf[h] = __fadd_rn(dotf[h], __fmul_rn((float)z[h][s], (float)rr[h][s]));
-              else if (sizeof(VT) == 4) dotd[h] = __fma_rn((double)z[h][s], (double)rr[h][s], dotd[h]);   // (the product is exact)
-              else dotd[h] = __dadd_rn(dotd[h], __dmul_rn((double)z[h][s], (double)rr[h][s]));
-            }
-        }
+        if constexpr (REV) dot.add(z, rr);
       }
-      // ---- z.r of this block's lines ----
-      if constexpr (REV) {
-        const int j = jb * 8 + jl;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int k = kb * 8 + 2 * kl + h;
-          if (j < lj && k < lk) g.partials[lbase + (long long)k * lj + j] = DOT32 ? (double)dotf[h] : dotd[h];
-        }
-      }
+      if constexpr (REV) put_dot(1, dot);
     } else if (!skip && me.ng > 0 && courier) {
       // ======================= courier warp =======================
       // far producers: this block's u .. last, FB under way; lane = line * 4 + step
@@ -696,7 +706,7 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
           // its slot is free once group u - S is done with (one lane's look, so
           // that all lanes agree; a count, since the courier may be any number
           // of groups ahead, where a parity would be ambiguous)
-          if (f.u >= __shfl_sync(XFP_FULL, ld_acquire_s32(&sh.done), 0) + S) break;
+          if (f.u >= __shfl_sync(XFP_FULL, ld_acquire_s32(&sh.freed), 0) + S) break;
           if (use) {
             uint32_t w[P];
             to_words(f.w[0].value(), w);
@@ -725,6 +735,78 @@ __global__ void __launch_bounds__(3 * 32 * warps_of<OP>(), 1) wave_kernel(WaveAr
           if (!go) raise_timeout(g.ctl, 8, tpos, fj.u, OP, fj.w[0].w[0], want);
           break;
         }
+      }
+    }
+    if constexpr (!FACTOR) {
+      if (!skip && me.ng > 0 && warp >= 3 * NW) {
+        // ======================= sender warp =======================
+        // A lane each for the 8 lines of the j edge and the 8 of the k edge: the
+        // group's four values go to the consumer's slot or to global memory.
+        const bool is_j = lane < 8, is_edge = lane < 16;
+        const int line_j = is_j ? (REV ? 0 : 7) : lane & 7, line_k = is_j ? lane : (REV ? 0 : 7);
+        const int lo = is_j ? lo_j : lo_k, hi = is_j ? hi_j : hi_k;
+        const bool near = is_j ? near_nj : near_nk;
+        const unsigned count = is_edge && hi >= lo ? (unsigned)(hi - lo) + 1u : 0u;   // groups from lo on
+        unsigned to = 0, bar = 0;   // near: slot 0
+        if (near) {
+          SL& d = unit_at(is_j ? kt : kt + DIR)->slot[0];
+          const int r = is_j ? rank_at(cj + DIR, kt) : rank_at(cj, kt + DIR);
+          to = cluster_addr(smem_u32(is_j ? d.ej[lane & 7] : d.ek[lane & 7]), r);
+          bar = cluster_addr(smem_u32(&unit_at(is_j ? kt : kt + DIR)->full[0]), r);
+        }
+        unsigned long long* const pub = (is_j ? g.bj : g.bk) + ((size_t)mybase * 32 + (lane & 7) * 4) * P;
+        const volatile int* const limit = &sh.limit[is_j ? 0 : 1];
+        const int coef = wave_cell_slot<VT>(line_j, line_k, 0, is_j ? 1 : 2);
+        constexpr int CELL_E = 128;              // from one step's cells to the next's
+        const int edge_at = OUT + wave_line_slot(line_j, line_k);
+        VT* res = static_cast<VT*>(g.sw) + (mybase + (REV ? me.ng - 1 : 0)) * WAVE_ROW + WAVE_Y + lane * 4;
+        int room = 0;
+        LineDot<VT, DOT32> dot;   // of the lines h = 0 (the helper has h = 1)
+        for (int q = 0; q < me.ng; ++q) {
+          const int sl = q & (S - 1);
+          if (!await(&sh.ready[sl], q, 9)) break;
+          const VT* const ops = reinterpret_cast<const VT*>(sh.slot[sl].ops);
+          if ((unsigned)(q - lo) < count) {
+            VT y[4], w[4];
+            ldg(y, ops + edge_at);
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+              if (REV) w[s] = y[3 - s];
+              else w[s] = mul_rn(ops[coef + s * CELL_E], y[s]);   // L(m,c) y[c], as in the block
+            }
+            if (near) {
+              if (q >= room) {
+                // the consumer's slot may not be free yet
+                room = *limit;
+                for (Spin sp; q >= room; room = *limit) {
+                  if (!sp.step(g.ctl, g.spin_limit)) {
+                    raise_timeout(g.ctl, 4, tpos, q, OP, 0ull, (unsigned)room);
+                    break;
+                  }
+                }
+              }
+              const unsigned d = (unsigned)(q - lo) & (S - 1);
+              uint32_t m[4 * P];
+#pragma unroll
+              for (int s = 0; s < 4; ++s) to_words(w[s], m + s * P);
+              send(to + d * (unsigned)sizeof(SL), bar + d * 8, m);
+            } else {
+              publish<X>(pub + (size_t)q * 32 * P, gen, w);
+            }
+          }
+          __syncwarp();
+          VT z[2][4], rr[4];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) ldg(z[h], ops + OUT + h * 128 + lane * 4);
+          if constexpr (REV) ldg(rr, ops + WAVE_R + lane * 4);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.empty[sl]);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) stg(res + h * 128, z[h]);
+          res += DIR * WAVE_ROW;
+          if constexpr (REV) dot.add(z[0], rr);
+        }
+        if constexpr (REV) put_dot(0, dot);
       }
     }
     // slot n has carried the groups q = n, n + S, ... < ng and the edges u = n, n + S, ... <= ng
@@ -806,7 +888,7 @@ cudaError_t launch(const WaveArgs& g, cudaStream_t st) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeCooperative;
   attr[1].val.cooperative = 1;
-  cfg.blockDim = dim3(3 * 32 * NW);
+  cfg.blockDim = dim3(roles_of<OP>() * 32 * NW);
   cfg.gridDim = dim3(WAVE_CLUSTER);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
