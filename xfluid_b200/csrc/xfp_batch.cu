@@ -108,9 +108,10 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S)
   // global) and group -> sweep element
   XFP_CUDA(ctx, ctx->group_line.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->gperm.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(int)));
+  XFP_CUDA(ctx, ctx->group_nb.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(GroupNb)));
   for (int s = 0; s < n; ++s) {
-    XFP_CUDA(ctx, build_group_line(lines + line_base[s], line_base[s + 1] - line_base[s], ctx->group_line.as<int>(),
-                                   st));
+    XFP_CUDA(ctx, build_group_tables(lines + line_base[s], S[s].nj, S[s].nk, ctx->group_line.as<int>(),
+                                     ctx->group_nb.as<GroupNb>(), st));
     XFP_CUDA(ctx, gperm_build(ctx->group_line.as<int>() + base[s] / 4, lines + line_base[s], S[s].nj,
                               ctx->blks.as<WBlk>() + blk_base[s], (S[s].nj + 7) / 8, base[s + 1] - base[s], base[s],
                               group_base[s], ctx->gperm.as<int>() + base[s] / 4, st));
@@ -241,7 +242,7 @@ int batch_pcg(xfp_ctx* ctx, BatchState* B, const VT* const A[4], const VT* b, VT
   auto iteration = [&]() -> cudaError_t {
     cudaError_t e;
     if ((e = batch_spmv_dot<VT, VT, DT>(segs, n, B->blocks_groups, A[0], A[1], A[2], A[3], s, z,
-                                        ctx->group_line.as<int>(), dsc, 0, st)))
+                                        ctx->group_nb.as<GroupNb>(), dsc, 0, st)))
       return e;
     if ((e = batch_update_xr<VT>(segs, n, B->blocks_cells, x, r, s, z, dsc, st, rsw, gperm))) return e;
     if ((e = wave_launch<VT, DT>(SWEEP_FWD, g, st))) return e;

@@ -71,7 +71,9 @@ int build_layout(xfp_ctx* ctx, const uint8_t* dmat, int ni, int nj, int nk) {
   if (ctx->Gsw * 256 >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "grid too large for the sweep layout");
   XFP_CUDA(ctx, ctx->group_line.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->gperm.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(int)));
-  XFP_CUDA(ctx, build_group_line(ctx->lines.as<Line>(), nlines, ctx->group_line.as<int>(), ctx->stream));
+  XFP_CUDA(ctx, ctx->group_nb.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(GroupNb)));
+  XFP_CUDA(ctx, build_group_tables(ctx->lines.as<Line>(), nj, nk, ctx->group_line.as<int>(), ctx->group_nb.as<GroupNb>(),
+                                   ctx->stream));
   XFP_CUDA(ctx, gperm_build(ctx->group_line.as<int>(), ctx->lines.as<Line>(), nj, ctx->blks.as<WBlk>(), NJB, ctx->M, 0,
                             0, ctx->gperm.as<int>(), ctx->stream));
   return XFP_OK;
@@ -222,8 +224,8 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
     for (int q = 0; q < K; ++q) {
       const int it = done_iters + q + 1;   // this launch's PCG iteration (1-based)
       XFP_CUDA(ctx, timed_kernel(ctx, 0, it, [&] {
-        return spmv_dot<VT, VT, DT>(A[0], A[1], A[2], A[3], s, z, ctx->lines.as<Line>(), ctx->group_line.as<int>(),
-                                    ctx->nj, ctx->nk, M, dsc, part, ctx->vec_blocks, 0, st);
+        return spmv_dot<VT, VT, DT>(A[0], A[1], A[2], A[3], s, z, ctx->group_nb.as<GroupNb>(), M, dsc, part,
+                                    ctx->vec_blocks, 0, st);
       }));
       XFP_CUDA(ctx, timed_kernel(ctx, 1, it, [&] {
         return update_xr<VT, DT>(x, r, s, z, M, dsc, ctx->partials.as<double>(), ctx->xr_blocks, st, rsw, gperm);
@@ -879,9 +881,8 @@ int debug_core(xfp_ctx* ctx, const CT* const Af[5], const VT* const Av[4], const
   if ((rc = dump_dense<VT>(ctx, z, out[9]))) return rc;
   if ((rc = run_sweep<VT, CT>(ctx, SWEEP_BWD, g))) return rc;
   if ((rc = sweep_result<VT>(ctx, z))) return rc;
-  XFP_CUDA(ctx, (spmv_dot<VT, VT, VT>(Av[0], Av[1], Av[2], Av[3], r, qv, ctx->lines.as<Line>(),
-                                      ctx->group_line.as<int>(), ctx->nj, ctx->nk, M, nullptr, (VT*)nullptr,
-                                      NBLK_MAX, 1, st)));
+  XFP_CUDA(ctx, (spmv_dot<VT, VT, VT>(Av[0], Av[1], Av[2], Av[3], r, qv, ctx->group_nb.as<GroupNb>(), M, nullptr,
+                                      (VT*)nullptr, NBLK_MAX, 1, st)));
   XFP_CUDA(ctx, cudaStreamSynchronize(st));
   if ((rc = check_sweep_error(ctx))) return rc;
   if ((rc = dump_dense<VT>(ctx, z, out[10]))) return rc;
@@ -1098,7 +1099,7 @@ int xfp_destroy(xfp_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   DevBuf* all[] = {&ctx->io_mat, &ctx->io_u, &ctx->io_v, &ctx->io_w, &ctx->io_wu, &ctx->io_wv, &ctx->io_ww,
                    &ctx->io_p, &ctx->io_gu, &ctx->io_gv, &ctx->io_gw, &ctx->lines, &ctx->lens,
-                   &ctx->blks, &ctx->tiles, &ctx->counters, &ctx->group_line, &ctx->gperm, &ctx->x64,
+                   &ctx->blks, &ctx->tiles, &ctx->counters, &ctx->group_line, &ctx->group_nb, &ctx->gperm, &ctx->x64,
                    &ctx->r64, &ctx->x32, &ctx->r32, &ctx->s32, &ctx->z32, &ctx->s64, &ctx->z64, &ctx->dense,
                    &ctx->sw_sys, &ctx->sw, &ctx->edge, &ctx->ctl, &ctx->scal, &ctx->scal2, &ctx->partials,
                    &ctx->tpartials};

@@ -75,6 +75,13 @@ __host__ __device__ __forceinline__ int wave_line_slot(int j, int k) {
   return (k & 1) * 128 + (((k & 7) >> 1) * 8 + (j & 7)) * 4;
 }
 
+// Where the y and z neighbours (j -+ 1, k -+ 1) of a 4-cell group are stored: a
+// neighbour line holds the first of them in the quad before quad q and the last in
+// quad q, (q << 2) | (1: it stores the first quad) | (2: it stores the second).
+struct __align__(16) GroupNb {
+  unsigned ym, yp, zm, zp;
+};
+
 // Control block of the persistent sweep kernels (one per context).
 struct SweepCtl {
   unsigned int gen;        // launch generation; stamped words carry it in their high half

@@ -127,16 +127,15 @@ cudaError_t rhs_T(const uint8_t* mat, const FT* wu, const FT* wv, const FT* ww, 
                   const FT* gw, FT* du, FT* dv, FT* dw, cudaStream_t st);
 
 // PCG vector kernels over the compact arrays (length M).
-// z = A s with the fused dot s.z; one thread per aligned 4-cell group
-// (group_line maps a group to its line).
+// z = A s with the fused dot s.z; one thread per aligned 4-cell group.
 template <typename VT, typename AT, typename DT>
 cudaError_t spmv_dot(const AT* diag, const AT* ax, const AT* ay, const AT* az, const VT* s, VT* z,
-                     const Line* lines, const int* group_line, int nj, int nk, long long M, PcgScalars* sc,
-                     DT* partials, int nblk_max, int mode, cudaStream_t st);
+                     const GroupNb* group_nb, long long M, PcgScalars* sc, DT* partials, int nblk_max, int mode,
+                     cudaStream_t st);
 // SpMV blocks for M stored cells (the batch gives each scene the same count).
 long long spmv_block_count(long long M, int nblk_max);
-// group_line[c / 4] = index of the line storing the aligned 4-cell group of cell c.
-cudaError_t build_group_line(const Line* lines, long long nlines, int* group_line, cudaStream_t st);
+// Per aligned 4-cell group (c / 4): the line that stores it and its neighbours.
+cudaError_t build_group_tables(const Line* lines, int nj, int nk, int* group_line, GroupNb* group_nb, cudaStream_t st);
 // rsw/gperm (optional): the updated r is also stored at rsw[wave_value(gperm[c / 4])].
 template <typename VT, typename DT>
 cudaError_t update_xr(VT* x, VT* r, const VT* s, const VT* z, long long M, PcgScalars* sc,
@@ -161,7 +160,7 @@ cudaError_t copy_vec(const T* in, T* out, long long n, cudaStream_t st);
 // nseg scenes, per-scene scalars sc[nseg]); grid = the table's total blocks ----
 template <typename VT, typename AT, typename DT>
 cudaError_t batch_spmv_dot(const BatchSeg* segs, int nseg, int blocks, const AT* diag, const AT* ax,
-                           const AT* ay, const AT* az, const VT* s, VT* z, const int* group_line, PcgScalars* sc,
+                           const AT* ay, const AT* az, const VT* s, VT* z, const GroupNb* group_nb, PcgScalars* sc,
                            int mode, cudaStream_t st);
 // rsw/gperm, zsw/gperm (optional): as update_xr / update_s, gperm indexed by global group
 template <typename VT>

@@ -661,68 +661,79 @@ __device__ __forceinline__ DT partials_sum(const DT* partials, unsigned nblk, DT
 //
 // One thread per aligned group of 4 stored cells.  Lines start at multiples
 // of 4 and hold multiples of 4 cells, so a group never straddles two lines:
-// the thread reads its line once (group_line), loads s and the four
-// coefficient arrays as 16-byte vectors (two for FP64), takes its x
-// neighbours from the vectors (plus one cell either side), and finds its y/z
-// neighbours through the four neighbouring lines' records (shared by every
-// group of the line, so L1 hits).  Per cell the products are added in the
-// reference's column order, so the FP64 result is the reference's.
+// the thread loads s and the four coefficient arrays as 16-byte vectors (two for
+// FP64) and takes its x neighbours from them (plus one cell either side).  A
+// cell i sits at an address = i + j + k (mod 4), so the four y or z neighbours
+// start one cell before a quad or one cell into it: a vector and a single cell
+// each, found through the group's record (GroupNb).  Per cell the products are
+// added in the reference's column order, so the FP64 result is the reference's.
+//
+// What bounds it: latency at small sizes (record, s, the reduction), the loads'
+// instructions and L2 above.  Per launch, FP32 at 256^3 half full (3.2 M cells) /
+// FP64 dam at 128^3 (0.44 M) / FP64 at 24^3: 19 / 10.9 / 4.4 us; with five line
+// records a group and a scalar load per neighbour 30.5 / 14.8 / 5.8 us.
 // ---------------------------------------------------------------------------
 template <typename VT, typename AT, typename DT>
 __device__ __forceinline__ void spmv_dot_body(
     unsigned bid, unsigned nblk, const AT* __restrict__ diag, const AT* __restrict__ ax,
     const AT* __restrict__ ay, const AT* __restrict__ az, const VT* __restrict__ s, VT* __restrict__ z,
-    const Line* __restrict__ lines, const int* __restrict__ group_line, int nj, int nk, long long base, long long M,
-    PcgScalars* sc, DT* __restrict__ partials, int mode) {
+    const GroupNb* __restrict__ group_nb, long long base, long long M, PcgScalars* sc, DT* __restrict__ partials,
+    int mode) {
   static_assert(std::is_same<VT, AT>::value, "the vector and coefficient types agree");
   __shared__ DT sh[32];
   if (sc && *(volatile int*)&sc->done) return;
   DT acc = DT(0);
   const long long G = M >> 2;
+  // the group's four neighbours in a line before it (j or k - 1) / after it; 0 where there is none
+  auto before = [](const VT* __restrict__ p, unsigned nb, VT (&v)[4]) {
+    const size_t quad = (size_t)(nb >> 2) * 4;
+    VT w[4] = {VT(0), VT(0), VT(0), VT(0)};
+    v[0] = nb & 1u ? p[quad - 1] : VT(0);
+    if (nb & 2u) ldg(w, p + quad);
+    v[1] = w[0]; v[2] = w[1]; v[3] = w[2];
+  };
+  auto after = [](const VT* __restrict__ p, unsigned nb, VT (&v)[4]) {
+    const size_t quad = (size_t)(nb >> 2) * 4;
+    VT w[4] = {VT(0), VT(0), VT(0), VT(0)};
+    if (nb & 1u) ldg(w, p + quad - 4);
+    v[0] = w[1]; v[1] = w[2]; v[2] = w[3];
+    v[3] = nb & 2u ? p[quad] : VT(0);
+  };
   for (long long q = (long long)bid * blockDim.x + threadIdx.x; q < G; q += (long long)nblk * blockDim.x) {
     const long long c = base + 4 * q;
-    const int line = group_line[(base >> 2) + q];
-    const Line L = lines[line];
-    const int i0 = L.lo + (int)(c - L.off);
-    const int j = line % nj, k = line / nj;
+    const GroupNb nb = group_nb[(base >> 2) + q];
     VT sv[4], dv[4], xv[4], yv[4], zv[4];
     ldg(sv, s + c);
     ldg(dv, diag + c);
     ldg(xv, ax + c);
     ldg(yv, ay + c);
     ldg(zv, az + c);
-    // one cell either side of the group (when the line has it)
-    const VT sl = c > L.off ? s[c - 1] : VT(0);
-    const bool right = c + 4 < (long long)L.off + L.len;
+    // one cell either side of the group; the coefficient is 0 where the line
+    // ends (a line's first cell has no lower neighbour)
+    const VT sl = c > base ? s[c - 1] : VT(0);
+    const bool right = 4 * q + 4 < M;
     const VT sr = right ? s[c + 4] : VT(0);
     const VT xr = right ? ax[c + 4] : VT(0);
-    const Line Z = {0, 0, 0, 0};
-    const Line Lym = j > 0 ? lines[line - 1] : Z;
-    const Line Lyp = j + 1 < nj ? lines[line + 1] : Z;
-    const Line Lzm = k > 0 ? lines[line - nj] : Z;
-    const Line Lzp = k + 1 < nk ? lines[line + nj] : Z;
+    VT szm[4], sym[4], syp[4], szp[4], ayp[4], azp[4];
+    before(s, nb.zm, szm);
+    before(s, nb.ym, sym);
+    after(s, nb.yp, syp);
+    after(ay, nb.yp, ayp);
+    after(s, nb.zp, szp);
+    after(az, nb.zp, azp);
     VT out[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int i = i0 + e;
       VT a = VT(0);
-      // a nonzero lower coefficient means the neighbour is an unknown, stored in its line
-      if (zv[e] != VT(0)) a = add_rn(a, mul_rn(zv[e], s[(size_t)Lzm.off + (i - Lzm.lo)]));
-      if (yv[e] != VT(0)) a = add_rn(a, mul_rn(yv[e], s[(size_t)Lym.off + (i - Lym.lo)]));
+      // a nonzero coefficient means the neighbour is an unknown, stored in its line
+      if (zv[e] != VT(0)) a = add_rn(a, mul_rn(zv[e], szm[e]));
+      if (yv[e] != VT(0)) a = add_rn(a, mul_rn(yv[e], sym[e]));
       if (xv[e] != VT(0)) a = add_rn(a, mul_rn(xv[e], e == 0 ? sl : sv[e == 0 ? 0 : e - 1]));
       if (dv[e] != VT(0)) a = add_rn(a, mul_rn(dv[e], sv[e]));
       const VT cx = e < 3 ? xv[e < 3 ? e + 1 : 3] : xr;
       if (cx != VT(0)) a = add_rn(a, mul_rn(cx, e < 3 ? sv[e < 3 ? e + 1 : 3] : sr));
-      if ((unsigned)(i - Lyp.lo) < (unsigned)Lyp.len) {
-        const size_t n = (size_t)Lyp.off + (i - Lyp.lo);
-        const VT cy = ay[n];
-        if (cy != VT(0)) a = add_rn(a, mul_rn(cy, s[n]));
-      }
-      if ((unsigned)(i - Lzp.lo) < (unsigned)Lzp.len) {
-        const size_t n = (size_t)Lzp.off + (i - Lzp.lo);
-        const VT cz = az[n];
-        if (cz != VT(0)) a = add_rn(a, mul_rn(cz, s[n]));
-      }
+      if (ayp[e] != VT(0)) a = add_rn(a, mul_rn(ayp[e], syp[e]));
+      if (azp[e] != VT(0)) a = add_rn(a, mul_rn(azp[e], szp[e]));
       out[e] = a;
       if (mode == 0) acc = add_rn(acc, mul_rn((DT)sv[e], (DT)a));
     }
@@ -751,41 +762,37 @@ template <typename VT, typename AT, typename DT>
 __global__ void __launch_bounds__(256) spmv_dot_kernel(
     const AT* __restrict__ diag, const AT* __restrict__ ax, const AT* __restrict__ ay,
     const AT* __restrict__ az, const VT* __restrict__ s, VT* __restrict__ z,
-    const Line* __restrict__ lines, const int* __restrict__ group_line, int nj, int nk, long long M, PcgScalars* sc,
-    DT* __restrict__ partials, int mode) {
-  spmv_dot_body<VT, AT, DT>(blockIdx.x, gridDim.x, diag, ax, ay, az, s, z, lines, group_line, nj, nk, 0, M, sc,
-                            partials, mode);
+    const GroupNb* __restrict__ group_nb, long long M, PcgScalars* sc, DT* __restrict__ partials, int mode) {
+  spmv_dot_body<VT, AT, DT>(blockIdx.x, gridDim.x, diag, ax, ay, az, s, z, group_nb, 0, M, sc, partials, mode);
 }
 template <typename VT, typename AT, typename DT>
 __global__ void __launch_bounds__(256) batch_spmv_dot_kernel(
     const BatchSeg* __restrict__ segs, int nseg, const AT* __restrict__ diag, const AT* __restrict__ ax,
     const AT* __restrict__ ay, const AT* __restrict__ az, const VT* __restrict__ s, VT* __restrict__ z,
-    const int* __restrict__ group_line, PcgScalars* sc, int mode) {
+    const GroupNb* __restrict__ group_nb, PcgScalars* sc, int mode) {
   const int q = batch_scene_of(segs, nseg, 2);
   const BatchSeg& S = segs[q];
-  spmv_dot_body<VT, AT, DT>(blockIdx.x - S.blk_groups_start, S.blk_groups, diag, ax, ay, az, s, z, S.lines,
-                            group_line, S.nj, S.nk, S.base, S.M, sc + q, reinterpret_cast<DT*>(S.partials), mode);
+  spmv_dot_body<VT, AT, DT>(blockIdx.x - S.blk_groups_start, S.blk_groups, diag, ax, ay, az, s, z, group_nb, S.base,
+                            S.M, sc + q, reinterpret_cast<DT*>(S.partials), mode);
 }
 template <typename VT, typename AT, typename DT>
 cudaError_t spmv_dot(const AT* diag, const AT* ax, const AT* ay, const AT* az, const VT* s, VT* z,
-                     const Line* lines, const int* group_line, int nj, int nk, long long M, PcgScalars* sc,
-                     DT* partials, int nblk_max, int mode, cudaStream_t st) {
+                     const GroupNb* group_nb, long long M, PcgScalars* sc, DT* partials, int nblk_max, int mode,
+                     cudaStream_t st) {
   const int blocks = (int)spmv_block_count(M, nblk_max);
   ++g_kernel_launches;
-  spmv_dot_kernel<VT, AT, DT><<<blocks, 256, 0, st>>>(diag, ax, ay, az, s, z, lines, group_line, nj, nk, M, sc,
-                                                     partials, mode);
+  spmv_dot_kernel<VT, AT, DT><<<blocks, 256, 0, st>>>(diag, ax, ay, az, s, z, group_nb, M, sc, partials, mode);
   return cudaGetLastError();
 }
-template cudaError_t spmv_dot<double, double, double>(const double*, const double*, const double*,
-                                                      const double*, const double*, double*, const Line*,
-                                                      const int*, int, int, long long, PcgScalars*, double*, int,
-                                                      int, cudaStream_t);
+template cudaError_t spmv_dot<double, double, double>(const double*, const double*, const double*, const double*,
+                                                      const double*, double*, const GroupNb*, long long, PcgScalars*,
+                                                      double*, int, int, cudaStream_t);
 template cudaError_t spmv_dot<float, float, float>(const float*, const float*, const float*, const float*,
-                                                   const float*, float*, const Line*, const int*, int, int,
-                                                   long long, PcgScalars*, float*, int, int, cudaStream_t);
+                                                   const float*, float*, const GroupNb*, long long, PcgScalars*,
+                                                   float*, int, int, cudaStream_t);
 template cudaError_t spmv_dot<float, float, double>(const float*, const float*, const float*, const float*,
-                                                    const float*, float*, const Line*, const int*, int, int,
-                                                    long long, PcgScalars*, double*, int, int, cudaStream_t);
+                                                    const float*, float*, const GroupNb*, long long, PcgScalars*,
+                                                    double*, int, int, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // x += alpha s ; r += (-alpha) z ; |r|_inf  (pcg_solver.h:270-276).  The last
@@ -1137,40 +1144,62 @@ cudaError_t residual64(const double* diag, const double* ax, const double* ay, c
 // ---------------------------------------------------------------------------
 template <typename VT, typename AT, typename DT>
 cudaError_t batch_spmv_dot(const BatchSeg* segs, int nseg, int blocks, const AT* diag, const AT* ax,
-                           const AT* ay, const AT* az, const VT* s, VT* z, const int* group_line, PcgScalars* sc,
+                           const AT* ay, const AT* az, const VT* s, VT* z, const GroupNb* group_nb, PcgScalars* sc,
                            int mode, cudaStream_t st) {
   ++g_kernel_launches;
-  batch_spmv_dot_kernel<VT, AT, DT><<<blocks, 256, 0, st>>>(segs, nseg, diag, ax, ay, az, s, z, group_line, sc,
+  batch_spmv_dot_kernel<VT, AT, DT><<<blocks, 256, 0, st>>>(segs, nseg, diag, ax, ay, az, s, z, group_nb, sc,
                                                            mode);
   return cudaGetLastError();
 }
 template cudaError_t batch_spmv_dot<double, double, double>(const BatchSeg*, int, int, const double*,
                                                             const double*, const double*, const double*,
-                                                            const double*, double*, const int*, PcgScalars*, int,
+                                                            const double*, double*, const GroupNb*, PcgScalars*, int,
                                                             cudaStream_t);
 template cudaError_t batch_spmv_dot<float, float, float>(const BatchSeg*, int, int, const float*, const float*,
                                                          const float*, const float*, const float*, float*,
-                                                         const int*, PcgScalars*, int, cudaStream_t);
+                                                         const GroupNb*, PcgScalars*, int, cudaStream_t);
 template cudaError_t batch_spmv_dot<float, float, double>(const BatchSeg*, int, int, const float*, const float*,
                                                           const float*, const float*, const float*, float*,
-                                                          const int*, PcgScalars*, int, cudaStream_t);
+                                                          const GroupNb*, PcgScalars*, int, cudaStream_t);
 
-// group_line[c / 4] = the line (index in its scene's table) that stores the
-// aligned 4-cell group of cell c (lines start at multiples of 4 and hold
-// multiples of 4 cells).
-__global__ void group_line_kernel(const Line* __restrict__ lines, long long nlines, int* __restrict__ group_line) {
+// For the aligned 4-cell group of cell c, at c / 4: its line (index in its scene's
+// table; lines start at multiples of 4 and hold multiples of 4 cells) and where
+// its y and z neighbours are.
+__global__ void group_tables_kernel(const Line* __restrict__ lines, int nj, int nk, int* __restrict__ group_line,
+                                    GroupNb* __restrict__ group_nb) {
   const int lane = threadIdx.x & 31;
+  const long long nlines = (long long)nj * nk;
   for (long long line = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); line < nlines;
        line += (long long)gridDim.x * (blockDim.x >> 5)) {
     const Line L = lines[line];
-    for (int q = lane; q < (L.len >> 2); q += 32) group_line[((size_t)L.off >> 2) + q] = (int)line;
+    if (L.len == 0) continue;
+    const int j = (int)(line % nj), k = (int)(line / nj);
+    const Line Z = {0, 0, 0, 0};
+    const Line N[4] = {j > 0 ? lines[line - 1] : Z, j + 1 < nj ? lines[line + 1] : Z, k > 0 ? lines[line - nj] : Z,
+                       k + 1 < nk ? lines[line + nj] : Z};
+    for (int q = lane; q < (L.len >> 2); q += 32) {
+      const size_t at = ((size_t)L.off >> 2) + q;
+      unsigned nb[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        // the neighbour of the group's first cell; the quad after the one that
+        // holds it, and whether the line stores either
+        const int r = L.lo + 4 * q - N[n].lo;
+        const int quad = (r >> 2) + 1;
+        nb[n] = ((unsigned)((N[n].off >> 2) + quad) << 2) | ((unsigned)(r & ~3) < (unsigned)N[n].len ? 1u : 0u) |
+                ((unsigned)(4 * quad) < (unsigned)N[n].len ? 2u : 0u);
+      }
+      group_line[at] = (int)line;
+      group_nb[at] = {nb[0], nb[1], nb[2], nb[3]};
+    }
   }
 }
-cudaError_t build_group_line(const Line* lines, long long nlines, int* group_line, cudaStream_t st) {
+cudaError_t build_group_tables(const Line* lines, int nj, int nk, int* group_line, GroupNb* group_nb, cudaStream_t st) {
+  const long long nlines = (long long)nj * nk;
   if (nlines <= 0) return cudaSuccess;
   ++g_kernel_launches;
-  group_line_kernel<<<(unsigned)std::min<long long>((nlines + 7) / 8, 65535LL * 8), 256, 0, st>>>(lines, nlines,
-                                                                                               group_line);
+  group_tables_kernel<<<(unsigned)std::min<long long>((nlines + 7) / 8, 65535LL * 8), 256, 0, st>>>(
+      lines, nj, nk, group_line, group_nb);
   return cudaGetLastError();
 }
 
