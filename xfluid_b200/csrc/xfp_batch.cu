@@ -29,7 +29,7 @@ using namespace xfp;
 namespace xfp_host {
 
 struct BatchState {
-  DevBuf lines, lens, scene_tile_lists, counters;
+  DevBuf lines, scene_tile_lists, counters;
   DevBuf segs, tile_scene, scal, scal2, part, tols, maxits;
   DevBuf io, pdense;
   std::vector<BatchSeg> hsegs;
@@ -41,7 +41,7 @@ struct BatchState {
 
 void batch_state_free(BatchState* b) {
   if (!b) return;
-  DevBuf* all[] = {&b->lines, &b->lens, &b->scene_tile_lists, &b->counters, &b->segs,
+  DevBuf* all[] = {&b->lines, &b->scene_tile_lists, &b->counters, &b->segs,
                    &b->tile_scene, &b->scal, &b->scal2, &b->part,
                    &b->tols, &b->maxits, &b->io, &b->pdense};
   for (DevBuf* d : all) d->release();
@@ -72,13 +72,13 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S)
   }
   const long long nlines = line_base[n], nblk = blk_base[n];
   XFP_CUDA(ctx, B->lines.ensure(nlines * sizeof(Line)));
-  XFP_CUDA(ctx, B->lens.ensure((nlines + n) * sizeof(int)));
+  XFP_CUDA(ctx, ctx->line_sums.ensure(3 * LINE_CHUNKS * sizeof(long long)));
   XFP_CUDA(ctx, ctx->blks.ensure((size_t)nblk * sizeof(WBlk)));
   XFP_CUDA(ctx, B->scene_tile_lists.ensure((size_t)nblk * sizeof(int2)));
   XFP_CUDA(ctx, B->counters.ensure((size_t)n * 5 * sizeof(long long)));
   Line* lines = B->lines.as<Line>();
   for (int s = 0; s < n; ++s) {
-    LayoutDev L{lines + line_base[s], B->lens.as<int>() + line_base[s] + s, ctx->blks.as<WBlk>() + blk_base[s],
+    LayoutDev L{lines + line_base[s], ctx->line_sums.as<long long>(), ctx->blks.as<WBlk>() + blk_base[s],
                 B->scene_tile_lists.as<int2>() + blk_base[s], B->counters.as<long long>() + 5 * s};
     XFP_CUDA(ctx, layout_build(S[s].mat, S[s].ni, S[s].nj, S[s].nk, L, st));
   }

@@ -54,11 +54,11 @@ int build_layout(xfp_ctx* ctx, const uint8_t* dmat, int ni, int nj, int nk) {
   const long long nlines = (long long)nj * nk;
   const int NJB = (nj + 7) / 8, NKB = (nk + 7) / 8;
   XFP_CUDA(ctx, ctx->lines.ensure(nlines * sizeof(Line)));
-  XFP_CUDA(ctx, ctx->lens.ensure((nlines + 1) * sizeof(int)));
+  XFP_CUDA(ctx, ctx->line_sums.ensure(3 * LINE_CHUNKS * sizeof(long long)));
   XFP_CUDA(ctx, ctx->blks.ensure((size_t)NJB * NKB * sizeof(WBlk)));
   XFP_CUDA(ctx, ctx->tiles.ensure((size_t)NJB * NKB * sizeof(int2)));
   XFP_CUDA(ctx, ctx->counters.ensure(5 * sizeof(long long)));
-  LayoutDev L{ctx->lines.as<Line>(), ctx->lens.as<int>(), ctx->blks.as<WBlk>(), ctx->tiles.as<int2>(),
+  LayoutDev L{ctx->lines.as<Line>(), ctx->line_sums.as<long long>(), ctx->blks.as<WBlk>(), ctx->tiles.as<int2>(),
               ctx->counters.as<long long>()};
   XFP_CUDA(ctx, layout_build(dmat, ni, nj, nk, L, ctx->stream));
   long long cnt[5];
@@ -1098,7 +1098,7 @@ int xfp_destroy(xfp_ctx* ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   DevBuf* all[] = {&ctx->io_mat, &ctx->io_u, &ctx->io_v, &ctx->io_w, &ctx->io_wu, &ctx->io_wv, &ctx->io_ww,
-                   &ctx->io_p, &ctx->io_gu, &ctx->io_gv, &ctx->io_gw, &ctx->lines, &ctx->lens,
+                   &ctx->io_p, &ctx->io_gu, &ctx->io_gv, &ctx->io_gw, &ctx->lines, &ctx->line_sums,
                    &ctx->blks, &ctx->tiles, &ctx->counters, &ctx->group_line, &ctx->group_nb, &ctx->gperm, &ctx->x64,
                    &ctx->r64, &ctx->x32, &ctx->r32, &ctx->s32, &ctx->z32, &ctx->s64, &ctx->z64, &ctx->dense,
                    &ctx->sw_sys, &ctx->sw, &ctx->edge, &ctx->ctl, &ctx->scal, &ctx->scal2, &ctx->partials,

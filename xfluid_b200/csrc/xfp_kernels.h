@@ -69,9 +69,10 @@ cudaError_t factor_lines(const T* fac, const Line* lines, int nj, int nk, const 
 // Builds the line table, the block table and the active-tile list for a
 // material grid.  counters (device): stored cells M, unknown rows, active
 // lines, active tiles, sweep-layout groups.
+constexpr int LINE_CHUNKS = 1024;
 struct LayoutDev {
   Line* lines;               // [nk*nj]
-  int* line_len_scan;        // scratch [nk*nj + 1]
+  long long* sums;           // scratch [3 * LINE_CHUNKS]
   WBlk* blks;                // [ceil(nk/8) * ceil(nj/8)]
   int2* tiles;               // active tiles (at most as many as blocks)
   long long* counters;       // [5]

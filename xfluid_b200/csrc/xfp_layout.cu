@@ -5,6 +5,7 @@
 // and each solid neighbour of a fluid cell receives a row).  Every (j,k) x-line
 // stores its active span, rounded out to whole groups of XFP_ALIGN cells that
 // are aligned to the wavefront (see xfp_common.cuh).
+#include <algorithm>
 #include <climits>
 
 #include "xfp_common.cuh"
@@ -30,7 +31,7 @@ __device__ __forceinline__ bool is_unknown(const uint8_t* mat, int ni, int nj, i
 
 // One warp per x-line: span of unknowns and their count.
 __global__ void line_span_kernel(const uint8_t* __restrict__ mat, int ni, int nj, int nk,
-                                 Line* __restrict__ lines, int* __restrict__ lens) {
+                                 Line* __restrict__ lines) {
   const int lane = threadIdx.x & 31;
   const long long line = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (line >= (long long)nj * nk) return;
@@ -56,59 +57,86 @@ __global__ void line_span_kernel(const uint8_t* __restrict__ mat, int ni, int nj
       L.nrows = cnt;
     }
     lines[line] = L;
-    lens[line] = L.len;
   }
 }
 
-// Single-CTA exclusive scan of line lengths -> offsets; totals into counters.
-__global__ void line_scan_kernel(Line* __restrict__ lines, const int* __restrict__ lens,
-                                 long long nlines, long long* __restrict__ counters) {
-  __shared__ long long s_sum[1024];
-  __shared__ long long s_carry;
-  __shared__ long long s_rows, s_lines;
-  const int t = threadIdx.x, nt = blockDim.x;
-  if (t == 0) { s_carry = 0; s_rows = 0; s_lines = 0; }
+// Inclusive scan of one value per thread over a block of 1024 threads.
+__device__ __forceinline__ long long scan1024(long long v, long long* sh) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long t = __shfl_up_sync(XFP_FULL, v, o);
+    if (lane >= o) v += t;
+  }
+  if (lane == 31) sh[w] = v;
   __syncthreads();
-  long long rows = 0, act = 0;
-  for (long long base = 0; base < nlines; base += (long long)nt * 8) {
-    long long v[8];
-    long long local = 0;
+  if (w == 0) {
+    long long t = sh[lane];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      long long idx = base + (long long)t * 8 + q;
-      v[q] = idx < nlines ? lens[idx] : 0;
-      local += v[q];
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(XFP_FULL, t, o);
+      if (lane >= o) t += u;
     }
-    s_sum[t] = local;
-    __syncthreads();
-    for (int o = 1; o < nt; o <<= 1) {
-      long long add = t >= o ? s_sum[t - o] : 0;
-      __syncthreads();
-      s_sum[t] += add;
-      __syncthreads();
-    }
-    long long run = s_carry + s_sum[t] - local;
+    sh[lane] = t;
+  }
+  __syncthreads();
+  const long long r = v + (w > 0 ? sh[w - 1] : 0);
+  __syncthreads();
+  return r;
+}
+
+// Offsets of the lines (exclusive scan of their lengths) and the totals, in two
+// launches of at most LINE_CHUNKS CTAs with a chunk of lines each: every chunk's
+// sums, then the scan, each CTA adding up the chunks before its own.  (One CTA
+// alone took 65 us for the 16,384 lines of 128^3 and 155 us at 256^3; now 8 us.)
+__global__ void __launch_bounds__(1024) line_sum_kernel(const Line* __restrict__ lines, long long nlines,
+                                                        long long chunk, long long* __restrict__ sums) {
+  __shared__ long long sh[32];
+  const long long a = blockIdx.x * chunk, b = min(a + chunk, nlines);
+  long long v[3] = {0, 0, 0};   // cells, rows, active lines
+  for (long long l = a + threadIdx.x; l < b; l += 1024) {
+    const Line L = lines[l];
+    v[0] += L.len;
+    v[1] += L.nrows;
+    v[2] += L.len > 0;
+  }
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      long long idx = base + (long long)t * 8 + q;
-      if (idx < nlines) {
-        lines[idx].off = (int)run;
-        rows += lines[idx].nrows;
-        act += v[q] > 0;
-      }
-      run += v[q];
-    }
+  for (int n = 0; n < 3; ++n) {
+    const long long t = scan1024(v[n], sh);
+    if (threadIdx.x == 1023) sums[n * LINE_CHUNKS + blockIdx.x] = t;
+  }
+}
+__global__ void __launch_bounds__(1024) line_scan_kernel(Line* __restrict__ lines, long long nlines, long long chunk,
+                                                         const long long* __restrict__ sums,
+                                                         long long* __restrict__ counters) {
+  __shared__ long long sh[32];
+  __shared__ long long s_tot;
+  const long long a = blockIdx.x * chunk, b = min(a + chunk, nlines);
+  auto total = [&](int n, unsigned chunks) {   // of the first chunks (at most 1024)
+    const long long t = scan1024(threadIdx.x < chunks ? sums[n * LINE_CHUNKS + threadIdx.x] : 0, sh);
+    if (threadIdx.x == 1023) s_tot = t;
     __syncthreads();
-    if (t == nt - 1) s_carry += s_sum[t];
+    const long long r = s_tot;
+    __syncthreads();
+    return r;
+  };
+  long long carry = total(0, blockIdx.x);
+  for (long long base = a; base < b; base += 1024) {
+    const long long l = base + threadIdx.x;
+    const long long v = l < b ? lines[l].len : 0;
+    const long long inc = scan1024(v, sh);
+    if (l < b) lines[l].off = (int)(carry + inc - v);
+    if (threadIdx.x == 1023) s_tot = inc;
+    __syncthreads();
+    carry += s_tot;
     __syncthreads();
   }
-  atomicAdd((unsigned long long*)&s_rows, (unsigned long long)rows);
-  atomicAdd((unsigned long long*)&s_lines, (unsigned long long)act);
-  __syncthreads();
-  if (t == 0) {
-    counters[0] = s_carry;
-    counters[1] = s_rows;
-    counters[2] = s_lines;
+  if (blockIdx.x + 1 != gridDim.x) return;
+  const long long rows = total(1, gridDim.x), act = total(2, gridDim.x);
+  if (threadIdx.x == 0) {
+    counters[0] = carry;
+    counters[1] = rows;
+    counters[2] = act;
   }
 }
 
@@ -142,31 +170,6 @@ __global__ void blk_span_kernel(const Line* __restrict__ lines, int nj, int nk, 
     }
     blks[b] = w;
   }
-}
-
-// Inclusive scan of one value per thread over a block of 1024 threads.
-__device__ __forceinline__ long long scan1024(long long v, long long* sh) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const long long t = __shfl_up_sync(XFP_FULL, v, o);
-    if (lane >= o) v += t;
-  }
-  if (lane == 31) sh[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    long long t = sh[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long u = __shfl_up_sync(XFP_FULL, t, o);
-      if (lane >= o) t += u;
-    }
-    sh[lane] = t;
-  }
-  __syncthreads();
-  const long long r = v + (w > 0 ? sh[w - 1] : 0);
-  __syncthreads();
-  return r;
 }
 
 // Block offsets (scan in block order) and the active tiles in topological
@@ -228,10 +231,13 @@ cudaError_t layout_build(const uint8_t* mat, int ni, int nj, int nk, LayoutDev L
   const long long nlines = (long long)nj * nk;
   const int wpb = 8;
   ++g_kernel_launches;
-  line_span_kernel<<<(unsigned)((nlines + wpb - 1) / wpb), wpb * 32, 0, st>>>(mat, ni, nj, nk, L.lines,
-                                                                              L.line_len_scan);
+  line_span_kernel<<<(unsigned)((nlines + wpb - 1) / wpb), wpb * 32, 0, st>>>(mat, ni, nj, nk, L.lines);
+  const long long chunk = std::max<long long>(1024, (nlines + LINE_CHUNKS - 1) / LINE_CHUNKS);
+  const unsigned chunks = (unsigned)((nlines + chunk - 1) / chunk);
   ++g_kernel_launches;
-  line_scan_kernel<<<1, 1024, 0, st>>>(L.lines, L.line_len_scan, nlines, L.counters);
+  line_sum_kernel<<<chunks, 1024, 0, st>>>(L.lines, nlines, chunk, L.sums);
+  ++g_kernel_launches;
+  line_scan_kernel<<<chunks, 1024, 0, st>>>(L.lines, nlines, chunk, L.sums, L.counters);
   const int NJB = (nj + 7) / 8, NKB = (nk + 7) / 8;
   const long long nblk = (long long)NJB * NKB;
   ++g_kernel_launches;
