@@ -36,7 +36,6 @@ struct BatchState {
   std::vector<long long> rows, nlines_act;
   int n = 0, ntiles = 0, blocks_lines = 0, blocks_cells = 0, blocks_groups = 0;
   long long M = 0;
-  bool graph_used = false;
 };
 
 void batch_state_free(BatchState* b) {
@@ -239,66 +238,52 @@ int batch_pcg(xfp_ctx* ctx, BatchState* B, const VT* const A[4], const VT* b, VT
   XFP_CUDA(ctx, (wave_launch<VT, DT>(SWEEP_BWD, g, st)));
   XFP_CUDA(ctx, batch_bwd_reduce<DT>(segs, n, lpart, dsc, 0, st));
   if ((rc0 = sweep_result<VT>(ctx, s)) != XFP_OK) return rc0;
-  auto iteration = [&]() -> cudaError_t {
+  auto iteration = [&](cudaStream_t cs) -> cudaError_t {
     cudaError_t e;
     if ((e = batch_spmv_dot<VT, VT, DT>(segs, n, B->blocks_groups, A[0], A[1], A[2], A[3], s, z,
-                                        ctx->group_nb.as<GroupNb>(), dsc, 0, st)))
+                                        ctx->group_nb.as<GroupNb>(), dsc, 0, cs)))
       return e;
-    if ((e = batch_update_xr<VT>(segs, n, B->blocks_cells, x, r, s, z, dsc, st, rsw, gperm))) return e;
-    if ((e = wave_launch<VT, DT>(SWEEP_FWD, g, st))) return e;
-    if ((e = wave_launch<VT, DT>(SWEEP_BWD, g, st))) return e;
-    if ((e = batch_bwd_reduce<DT>(segs, n, lpart, dsc, 1, st))) return e;
-    return batch_update_s<VT>(segs, n, B->blocks_cells, s, z, dsc, st, zsw, gperm);
+    if ((e = batch_update_xr<VT>(segs, n, B->blocks_cells, x, r, s, z, dsc, cs, rsw, gperm))) return e;
+    if ((e = wave_launch<VT, DT>(SWEEP_FWD, g, cs))) return e;
+    if ((e = wave_launch<VT, DT>(SWEEP_BWD, g, cs))) return e;
+    if ((e = batch_bwd_reduce<DT>(segs, n, lpart, dsc, 1, cs))) return e;
+    return batch_update_s<VT>(segs, n, B->blocks_cells, s, z, dsc, cs, zsw, gperm);
   };
   const int K = ctx->opt.check_every > 0 ? ctx->opt.check_every : 8;
   const int per_iter = B->ntiles > 0 ? 6 : 4;
-  // capture K iterations as a graph; if capture is refused, launch directly
-  cudaGraphExec_t exec = nullptr;
-  {
-    cudaGraph_t graph = nullptr;
-    const long long before = g_kernel_launches;
-    cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-      cudaError_t le = cudaSuccess;
-      for (int q = 0; q < K && le == cudaSuccess; ++q) le = iteration();
-      e = cudaStreamEndCapture(st, &graph);
-      if (le != cudaSuccess) e = le;
-    }
-    if (e == cudaSuccess && graph) e = cudaGraphInstantiate(&exec, graph, 0);
-    if (graph) cudaGraphDestroy(graph);
-    if (e != cudaSuccess) {
-      if (exec) cudaGraphExecDestroy(exec);
-      exec = nullptr;
-      cudaGetLastError();
-    }
-    g_kernel_launches = before;   // counted per replay below
-  }
-  B->graph_used = exec != nullptr;
+  // iterations as a graph, read after every launch of it; if that is refused,
+  // launch directly
+  const int per = loop_iterations(ctx);
+  const bool graph = capture_iterations(ctx, per, iteration);
+  ctx->loop_graph = graph;
   hsc.assign(n, PcgScalars{});
   int rc = XFP_OK;
-  for (int done_iters = 0;;) {
-    if (exec) {
-      cudaError_t e = cudaGraphLaunch(exec, st);
-      if (e != cudaSuccess) { rc = fail(ctx, XFP_ERR_CUDA, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e)); break; }
-      g_kernel_launches += (long long)K * per_iter;
-    } else {
-      for (int q = 0; q < K; ++q) {
-        cudaError_t e = iteration();
-        if (e != cudaSuccess) { rc = fail(ctx, XFP_ERR_CUDA, std::string("batch iteration: ") + cudaGetErrorString(e)); break; }
-      }
-      if (rc) break;
-    }
-    done_iters += K;
-    cudaError_t e = cudaMemcpyAsync(hsc.data(), dsc, n * sizeof(PcgScalars), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) { rc = fail(ctx, XFP_ERR_CUDA, std::string("batch scalars: ") + cudaGetErrorString(e)); break; }
-    if ((rc = check_sweep_error(ctx)) != XFP_OK) break;
+  auto read = [&](cudaStream_t cs) -> cudaError_t {
+    const cudaError_t e = cudaMemcpyAsync(hsc.data(), dsc, n * sizeof(PcgScalars), cudaMemcpyDeviceToHost, cs);
+    if (e != cudaSuccess) return e;
+    return cudaMemcpyAsync(&ctx->loop_read->ctl, ctx->ctl.p, sizeof(SweepCtl), cudaMemcpyDeviceToHost, cs);
+  };
+  auto finished = [&](int& err, int& last) -> bool {
+    err = sweep_error(ctx, ctx->loop_read->ctl);
     bool all = true;
-    for (int q = 0; q < n; ++q) all &= hsc[q].done != 0;
-    if (all) break;
-    if (done_iters > maxit_all + 2 * K) { rc = fail(ctx, XFP_ERR_CUDA, "batch PCG loop did not terminate"); break; }
+    last = 0;
+    for (int q = 0; q < n; ++q) {
+      all &= hsc[q].done != 0;
+      last = std::max(last, hsc[q].iters);
+    }
+    return all;
+  };
+  if (graph) return replay_iterations(ctx, per, per_iter, maxit_all + 2 * K, read, finished);
+  for (int done_iters = 0;;) {
+    for (int q = 0; q < K; ++q) XFP_CUDA(ctx, iteration(st));
+    done_iters += K;
+    XFP_CUDA(ctx, read(st));
+    XFP_CUDA(ctx, cudaStreamSynchronize(st));
+    int last;
+    const bool end = finished(rc, last);
+    if (rc != XFP_OK || end) break;
+    if (done_iters > maxit_all + 2 * K) return fail(ctx, XFP_ERR_CUDA, "batch PCG loop did not terminate");
   }
-  if (exec) cudaGraphExecDestroy(exec);
   return rc;
 }
 
@@ -615,7 +600,7 @@ int project_batch(xfp_ctx* ctx, int n, const xfp_scene* scenes, xfp_stats* stats
       o.bytes = bpr * (double)o.rows * o.iterations + 33.0 * cells + 24.0 * (double)o.rows + 29.0 * cells;
       o.launches = launches;
       o.tile_k = ctx->nw;
-      o.graph = B->graph_used ? 1 : 0;
+      o.graph = ctx->loop_graph ? 1 : 0;
     }
   }
   return status;

@@ -165,9 +165,14 @@ double sweep_ms(xfp_ctx* ctx, int* n) {
 }
 
 int check_sweep_error(xfp_ctx* ctx) {
-  SweepCtl c;
+  SweepCtl& c = ctx->loop_read->ctl;
   XFP_CUDA(ctx, cudaMemcpyAsync(&c, ctx->ctl.p, sizeof(c), cudaMemcpyDeviceToHost, ctx->stream));
   XFP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  return sweep_error(ctx, c);
+}
+
+// Reports (and clears) the wait that ran out in a sweep, if one did.
+int sweep_error(xfp_ctx* ctx, const SweepCtl& c) {
   if (c.err) {
     char buf[256];
     snprintf(buf, sizeof buf,
@@ -185,12 +190,36 @@ int check_sweep_error(xfp_ctx* ctx) {
 }
 
 // ---------------------------------------------------------------- PCG
+// The loop's iterations as a graph, for the pcg calls with these arrays (captured
+// while the device factorises).  False: the loop launches directly.
+template <typename VT, typename DT>
+bool pcg_graph(xfp_ctx* ctx, const VT* const A[4], VT* x, VT* r, VT* s, VT* z, PcgScalars* dsc) {
+  if (ctx->event_every != 0 || wave_prepare<VT, DT>() != cudaSuccess) return false;
+  const bool swl = ctx->ntiles > 0;
+  WaveArgs g = wave_args(ctx);
+  g.scal = dsc;
+  g.bwd_mode = 1;
+  return capture_iterations(ctx, loop_iterations(ctx), [&](cudaStream_t cs) -> cudaError_t {
+    cudaError_t e;
+    if ((e = spmv_dot<VT, VT, DT>(A[0], A[1], A[2], A[3], s, z, ctx->group_nb.as<GroupNb>(), ctx->M, dsc,
+                                  reinterpret_cast<DT*>(ctx->partials.p), ctx->vec_blocks, 0, cs)))
+      return e;
+    if ((e = update_xr<VT, DT>(x, r, s, z, ctx->M, dsc, ctx->partials.as<double>(), ctx->xr_blocks, cs,
+                               swl ? ctx->sw.as<VT>() + WAVE_R : nullptr, swl ? ctx->gperm.as<int>() : nullptr)))
+      return e;
+    if ((e = wave_launch<VT, DT>(SWEEP_FWD, g, cs))) return e;
+    if ((e = wave_launch<VT, DT>(SWEEP_BWD, g, cs))) return e;
+    return update_s<VT>(s, z, ctx->M, dsc, cs, swl ? ctx->sw.as<VT>() + WAVE_Y : nullptr,
+                        swl ? ctx->gperm.as<int>() : nullptr, ctx->s_blocks);
+  });
+}
+
 // pcg_solver.h:243-285 on the compact system; the factor is in the sweep
 // layout.  A: coefficient arrays (VT), b: rhs (VT), x: solution (VT).  DT: dot
 // accumulation type.
 template <typename VT, typename DT>
 int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT* z, double tol, int maxit,
-        PcgScalars* dsc, PcgScalars* hsc) {
+        PcgScalars* dsc, PcgScalars* hsc, bool graph) {
   const long long M = ctx->M;
   cudaStream_t st = ctx->stream;
   if (tol < 1e-30) tol = 1e-30;  // set_solver_parameters, pcg_solver.h:237
@@ -220,7 +249,19 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
   if ((rc = sweep_result<VT>(ctx, s)) != XFP_OK) return rc;
   const int K = ctx->opt.check_every > 0 ? ctx->opt.check_every : 8;
   DT* part = reinterpret_cast<DT*>(ctx->partials.p);
-  for (int done_iters = 0;;) {
+  auto read = [&](cudaStream_t cs) -> cudaError_t {
+    const cudaError_t e = cudaMemcpyAsync(&ctx->loop_read->sc, dsc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, cs);
+    if (e != cudaSuccess) return e;
+    return cudaMemcpyAsync(&ctx->loop_read->ctl, ctx->ctl.p, sizeof(SweepCtl), cudaMemcpyDeviceToHost, cs);
+  };
+  auto finished = [&](int& err, int& last) -> bool {
+    *hsc = ctx->loop_read->sc;
+    last = hsc->iters;
+    err = sweep_error(ctx, ctx->loop_read->ctl);
+    return hsc->done != 0;
+  };
+  if (graph && (rc = replay_iterations(ctx, loop_iterations(ctx), g1.ntiles > 0 ? 5 : 3, maxit + 2 * K, read, finished)) != XFP_OK) return rc;
+  for (int done_iters = 0; !graph;) {
     for (int q = 0; q < K; ++q) {
       const int it = done_iters + q + 1;   // this launch's PCG iteration (1-based)
       XFP_CUDA(ctx, timed_kernel(ctx, 0, it, [&] {
@@ -235,10 +276,12 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
       XFP_CUDA(ctx, timed_kernel(ctx, 2, it, [&] { return update_s<VT>(s, z, M, dsc, st, zsw, gperm, ctx->s_blocks); }));
     }
     done_iters += K;
-    XFP_CUDA(ctx, cudaMemcpyAsync(hsc, dsc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
+    XFP_CUDA(ctx, read(st));
     XFP_CUDA(ctx, cudaStreamSynchronize(st));
-    if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
-    if (hsc->done) break;
+    int last;
+    const bool end = finished(rc, last);
+    if (rc != XFP_OK) return rc;
+    if (end) break;
     if (done_iters > maxit + 2 * K) return fail(ctx, XFP_ERR_CUDA, "PCG loop did not terminate");
   }
   // the preconditioner's two sweeps, then two per iteration but the last (the
@@ -286,6 +329,7 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
   ev_record(ctx, 0);
   ctx->sweep_ev_used = 0;
   ctx->kern_ev_used = 0;
+  ctx->loop_graph = false;
   if ((rc = build_layout(ctx, dmat, ni, nj, nk)) != XFP_OK) return rc;
   if ((rc = ensure_compact(ctx, prec)) != XFP_OK) return rc;
   if ((rc = inputs_ready(ctx)) != XFP_OK) return rc;
@@ -308,10 +352,13 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
     ev_record(ctx, 1);
     const double* Ac[4] = {A[0], A[1], A[2], A[3]};
     if ((rc = run_sweep<double, double>(ctx, SWEEP_FACTOR, wave_args(ctx))) != XFP_OK) return rc;
-    if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
     ev_record(ctx, 2);
+    const bool graph = pcg_graph<double, double>(ctx, Ac, ctx->x64.as<double>(), ctx->r64.as<double>(),
+                                                 ctx->s64.as<double>(), ctx->z64.as<double>(), dsc);
+    ctx->loop_graph = graph;
+    if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
     rc = pcg<double, double>(ctx, Ac, A[4], ctx->x64.as<double>(), ctx->r64.as<double>(), ctx->s64.as<double>(),
-                             ctx->z64.as<double>(), tol, maxit, dsc, &hsc);
+                             ctx->z64.as<double>(), tol, maxit, dsc, &hsc, graph);
     ev_record(ctx, 3);
     ctx->iters = hsc.iters; ctx->res = hsc.res; ctx->bnorm = hsc.bnorm;
   } else if (prec == XFP_PREC_F32) {
@@ -325,10 +372,13 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
     ev_record(ctx, 1);
     const float* Ac[4] = {A[0], A[1], A[2], A[3]};
     if ((rc = run_sweep<float, float>(ctx, SWEEP_FACTOR, wave_args(ctx))) != XFP_OK) return rc;
-    if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
     ev_record(ctx, 2);
+    const bool graph = pcg_graph<float, float>(ctx, Ac, ctx->x32.as<float>(), ctx->r32.as<float>(),
+                                               ctx->s32.as<float>(), ctx->z32.as<float>(), dsc);
+    ctx->loop_graph = graph;
+    if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
     rc = pcg<float, float>(ctx, Ac, A[4], ctx->x32.as<float>(), ctx->r32.as<float>(), ctx->s32.as<float>(),
-                           ctx->z32.as<float>(), tol, maxit, dsc, &hsc);
+                           ctx->z32.as<float>(), tol, maxit, dsc, &hsc, graph);
     ev_record(ctx, 3);
     ctx->iters = hsc.iters; ctx->res = hsc.res; ctx->bnorm = hsc.bnorm;
   } else {
@@ -347,9 +397,12 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
     // the factorisation runs in FP64; the FP32 solves stream its L and pivots
     // rounded to FP32
     if ((rc = run_sweep<float, double>(ctx, SWEEP_FACTOR, wave_args(ctx))) != XFP_OK) return rc;
-    if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
     ev_record(ctx, 2);
     const float* A32c[4] = {A32[0], A32[1], A32[2], A32[3]};
+    const bool graph = pcg_graph<float, double>(ctx, A32c, ctx->x32.as<float>(), ctx->r32.as<float>(),
+                                                ctx->s32.as<float>(), ctx->z32.as<float>(), dsc);
+    ctx->loop_graph = graph;
+    if ((rc = check_sweep_error(ctx)) != XFP_OK) return rc;
     double* x64 = ctx->x64.as<double>();
     double* r64 = ctx->r64.as<double>();
     PcgScalars* osc = ctx->scal2.as<PcgScalars>();
@@ -384,7 +437,7 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
         float* b32 = ctx->A32[4].as<float>();
         XFP_CUDA(ctx, copy_vec<float>(ctx->r32.as<float>(), b32, M, st));
         int irc = pcg<float, double>(ctx, A32c, b32, ctx->x32.as<float>(), ctx->r32.as<float>(),
-                                     ctx->s32.as<float>(), ctx->z32.as<float>(), inner, maxit - total, dsc, &hsc);
+                                     ctx->s32.as<float>(), ctx->z32.as<float>(), inner, maxit - total, dsc, &hsc, graph);
         if (irc < 0) return irc;
         total += hsc.iters;
         XFP_CUDA(ctx, refine_update(x64, ctx->x32.as<float>(), M, st));
@@ -472,6 +525,7 @@ void fill_stats(xfp_ctx* ctx, xfp_stats* s, int status, double ms_total) {
   }
   s->launches = g_kernel_launches - ctx->launches;
   s->tile_k = ctx->nw;
+  s->graph = ctx->loop_graph ? 1 : 0;
   s->h2d_bytes = ctx->h2d_bytes;
   s->d2h_bytes = ctx->d2h_bytes;
   s->host_faces = ctx->host_faces;
@@ -1085,6 +1139,11 @@ int xfp_create(xfp_ctx** out, const xfp_options* opt) {
   if (const char* e = getenv("XFP_XR_BLOCKS")) ctx->xr_blocks = std::max(148, std::min(xfp_host::NBLK_MAX, atoi(e)));
   if (const char* e = getenv("XFP_S_BLOCKS")) ctx->s_blocks = std::max(148, std::min(148 * 32, atoi(e)));
   if (const char* e = getenv("XFP_HOST_FACES")) ctx->host_sparse_ok = strcmp(e, "full") != 0;
+  if (cudaHostAlloc((void**)&ctx->loop_read, sizeof(*ctx->loop_read), cudaHostAllocDefault) != cudaSuccess) {
+    ctx->loop_read = nullptr;
+    xfp_destroy(ctx);
+    return XFP_ERR_NOMEM;
+  }
   if (ctx->ctl.ensure(sizeof(SweepCtl)) != cudaSuccess) { xfp_destroy(ctx); return XFP_ERR_NOMEM; }
   SweepCtl c0{};
   c0.gen = 1;
@@ -1120,6 +1179,11 @@ int xfp_destroy(xfp_ctx* ctx) {
   }
   for (cudaEvent_t e : {ctx->ev_io_mat, ctx->ev_io_in, ctx->ev_io_p})
     if (e) cudaEventDestroy(e);
+  if (ctx->loop_exec) cudaGraphExecDestroy(ctx->loop_exec);
+  for (cudaEvent_t e : ctx->loop_ev)
+    if (e) cudaEventDestroy(e);
+  if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
+  if (ctx->loop_read) cudaFreeHost(ctx->loop_read);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return XFP_OK;

@@ -49,6 +49,9 @@ struct WaveArgs {
 // arithmetic and the dot type of the backward solve.
 template <typename VT, typename CT>
 cudaError_t wave_launch(int op, const WaveArgs& g, cudaStream_t st);
+// What a first launch of the solves looks up, ahead of it (outside a capture).
+template <typename VT, typename CT>
+cudaError_t wave_prepare();
 // 64-bit words of the J and K edges per group: 4 steps x 8 lines of up to 16
 // bytes (the factorisation's FP64 pair), 32 payload bits a word
 constexpr size_t WAVE_EDGE = 4 * 8 * 4;

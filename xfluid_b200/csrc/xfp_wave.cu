@@ -875,41 +875,51 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
   atomicExch(&g.ctl->gen, gen + 1);
 }
 
+// A launch's configuration but for its grid and stream, and the clusters that the
+// current device holds at once (the kernel's attribute is per device too).
 template <int OP, typename VT, typename CT>
-cudaError_t launch(const WaveArgs& g, cudaStream_t st) {
-  // resident clusters, per device (the kernel's attribute is per device too)
-  static std::atomic<int> resident[64];
-  constexpr int NW = warps_of<OP>();
-  constexpr int smem = NW * (int)sizeof(UnitShared<OP, VT, CT>);
+struct WaveLaunch {
+  static constexpr int smem = warps_of<OP>() * (int)sizeof(UnitShared<OP, VT, CT>);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = WAVE_CLUSTER;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeCooperative;
-  attr[1].val.cooperative = 1;
-  cfg.blockDim = dim3(roles_of<OP>() * 32 * NW);
-  cfg.gridDim = dim3(WAVE_CLUSTER);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  int max_clusters = resident[dev & 63].load();
-  if (max_clusters == 0) {
-    int n = 0;
-    e = cudaFuncSetAttribute(wave_kernel<OP, VT, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, wave_kernel<OP, VT, CT>, &cfg);
+  int resident = 0;
+  cudaError_t prepare() {
+    static std::atomic<int> known[64];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = WAVE_CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
+    cfg.blockDim = dim3(roles_of<OP>() * 32 * warps_of<OP>());
+    cfg.gridDim = dim3(WAVE_CLUSTER);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (n < 1) return cudaErrorLaunchOutOfResources;
-    resident[dev & 63] = max_clusters = n;
+    resident = known[dev & 63].load();
+    if (resident == 0) {
+      int n = 0;
+      e = cudaFuncSetAttribute(wave_kernel<OP, VT, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, wave_kernel<OP, VT, CT>, &cfg);
+      if (e != cudaSuccess) return e;
+      if (n < 1) return cudaErrorLaunchOutOfResources;
+      known[dev & 63] = resident = n;
+    }
+    cfg.numAttrs = 2;
+    return cudaSuccess;
   }
-  cfg.gridDim = dim3(WAVE_CLUSTER * std::min(max_clusters, g.ntiles));
-  cfg.numAttrs = 2;
+};
+template <int OP, typename VT, typename CT>
+cudaError_t launch(const WaveArgs& g, cudaStream_t st) {
+  WaveLaunch<OP, VT, CT> L;
+  const cudaError_t e = L.prepare();
+  if (e != cudaSuccess) return e;
+  L.cfg.gridDim = dim3(WAVE_CLUSTER * std::min(L.resident, g.ntiles));
+  L.cfg.stream = st;
   ++g_kernel_launches;
-  return cudaLaunchKernelEx(&cfg, wave_kernel<OP, VT, CT>, g);
+  return cudaLaunchKernelEx(&L.cfg, wave_kernel<OP, VT, CT>, g);
 }
 
 // gperm[q] = sweep element of the first cell of line-layout group q (four
@@ -989,6 +999,14 @@ cudaError_t wave_launch(int op, const WaveArgs& g, cudaStream_t st) {
     default: return launch<SWEEP_BWD, VT, CT>(g, st);
   }
 }
+template <typename VT, typename CT>
+cudaError_t wave_prepare() {
+  const cudaError_t e = WaveLaunch<SWEEP_FWD, VT, CT>().prepare();
+  return e != cudaSuccess ? e : WaveLaunch<SWEEP_BWD, VT, CT>().prepare();
+}
+template cudaError_t wave_prepare<double, double>();
+template cudaError_t wave_prepare<float, float>();
+template cudaError_t wave_prepare<float, double>();
 template cudaError_t wave_launch<double, double>(int, const WaveArgs&, cudaStream_t);
 template cudaError_t wave_launch<float, float>(int, const WaveArgs&, cudaStream_t);
 template cudaError_t wave_launch<float, double>(int, const WaveArgs&, cudaStream_t);
