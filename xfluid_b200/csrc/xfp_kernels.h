@@ -14,6 +14,22 @@ enum { SWEEP_FACTOR = 0, SWEEP_FWD = 1, SWEEP_BWD = 2 };
 // launches); a call reports the difference across its own work.
 extern long long g_kernel_launches;
 
+// A launch of one of the PCG loop's kernels (start_next, wait_previous).
+template <typename... P, typename... A>
+cudaError_t launch_next(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ++g_kernel_launches;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // One launch of the wavefront kernel (xfp_wave.cu): blocks, control, operands.
 struct WaveArgs {
   int nj = 0, nk = 0;           // lines along j and k (one scene)

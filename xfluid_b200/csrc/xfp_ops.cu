@@ -763,6 +763,8 @@ __global__ void __launch_bounds__(256) spmv_dot_kernel(
     const AT* __restrict__ diag, const AT* __restrict__ ax, const AT* __restrict__ ay,
     const AT* __restrict__ az, const VT* __restrict__ s, VT* __restrict__ z,
     const GroupNb* __restrict__ group_nb, long long M, PcgScalars* sc, DT* __restrict__ partials, int mode) {
+  start_next();
+  wait_previous();
   spmv_dot_body<VT, AT, DT>(blockIdx.x, gridDim.x, diag, ax, ay, az, s, z, group_nb, 0, M, sc, partials, mode);
 }
 template <typename VT, typename AT, typename DT>
@@ -770,6 +772,8 @@ __global__ void __launch_bounds__(256) batch_spmv_dot_kernel(
     const BatchSeg* __restrict__ segs, int nseg, const AT* __restrict__ diag, const AT* __restrict__ ax,
     const AT* __restrict__ ay, const AT* __restrict__ az, const VT* __restrict__ s, VT* __restrict__ z,
     const GroupNb* __restrict__ group_nb, PcgScalars* sc, int mode) {
+  start_next();
+  wait_previous();
   const int q = batch_scene_of(segs, nseg, 2);
   const BatchSeg& S = segs[q];
   spmv_dot_body<VT, AT, DT>(blockIdx.x - S.blk_groups_start, S.blk_groups, diag, ax, ay, az, s, z, group_nb, S.base,
@@ -780,9 +784,7 @@ cudaError_t spmv_dot(const AT* diag, const AT* ax, const AT* ay, const AT* az, c
                      const GroupNb* group_nb, long long M, PcgScalars* sc, DT* partials, int nblk_max, int mode,
                      cudaStream_t st) {
   const int blocks = (int)spmv_block_count(M, nblk_max);
-  ++g_kernel_launches;
-  spmv_dot_kernel<VT, AT, DT><<<blocks, 256, 0, st>>>(diag, ax, ay, az, s, z, group_nb, M, sc, partials, mode);
-  return cudaGetLastError();
+  return launch_next(spmv_dot_kernel<VT, AT, DT>, blocks, 256, st, diag, ax, ay, az, s, z, group_nb, M, sc, partials, mode);
 }
 template cudaError_t spmv_dot<double, double, double>(const double*, const double*, const double*, const double*,
                                                       const double*, double*, const GroupNb*, long long, PcgScalars*,
@@ -876,6 +878,8 @@ __global__ void __launch_bounds__(256) update_xr_kernel(VT* __restrict__ x, VT* 
                                                         const VT* __restrict__ z, long long M,
                                                         PcgScalars* sc, double* __restrict__ partials,
                                                         VT* __restrict__ rsw, const int* __restrict__ gperm) {
+  start_next();
+  wait_previous();
   update_xr_body<VT>(blockIdx.x, gridDim.x, x, r, s, z, M, sc, partials, rsw, gperm);
 }
 template <typename VT>
@@ -884,6 +888,8 @@ __global__ void __launch_bounds__(256) batch_update_xr_kernel(const BatchSeg* __
                                                               const VT* __restrict__ s, const VT* __restrict__ z,
                                                               PcgScalars* sc, VT* __restrict__ rsw,
                                                               const int* __restrict__ gperm) {
+  start_next();
+  wait_previous();
   const int q = batch_scene_of(segs, nseg, 0);
   const BatchSeg& S = segs[q];
   update_xr_body<VT>(blockIdx.x - S.blk_cells_start, S.blk_cells, x + S.base, r + S.base, s + S.base,
@@ -895,9 +901,7 @@ cudaError_t update_xr(VT* x, VT* r, const VT* s, const VT* z, long long M, PcgSc
   // 4-cell groups over at most nblk_max blocks
   int blocks = (int)std::min<long long>((M / 4 + 255) / 256, (long long)nblk_max);
   if (blocks < 1) blocks = 1;
-  ++g_kernel_launches;
-  update_xr_kernel<VT><<<blocks, 256, 0, st>>>(x, r, s, z, M, sc, partials, rsw, gperm);
-  return cudaGetLastError();
+  return launch_next(update_xr_kernel<VT>, blocks, 256, st, x, r, s, z, M, sc, partials, rsw, gperm);
 }
 template cudaError_t update_xr<double, double>(double*, double*, const double*, const double*, long long,
                                                PcgScalars*, double*, int, cudaStream_t, double*, const int*);
@@ -947,12 +951,16 @@ __device__ __forceinline__ void update_s_body(unsigned bid, unsigned nblk, VT* _
 template <typename VT>
 __global__ void update_s_kernel(VT* __restrict__ s, const VT* __restrict__ z, long long M,
                                 PcgScalars* sc, const VT* __restrict__ zsw, const int* __restrict__ gperm) {
+  start_next();
+  wait_previous();
   update_s_body<VT>(blockIdx.x, gridDim.x, s, z, M, sc, zsw, gperm);
 }
 template <typename VT>
 __global__ void batch_update_s_kernel(const BatchSeg* __restrict__ segs, int nseg, VT* __restrict__ s,
                                       const VT* __restrict__ z, PcgScalars* sc, const VT* __restrict__ zsw,
                                       const int* __restrict__ gperm) {
+  start_next();
+  wait_previous();
   const int q = batch_scene_of(segs, nseg, 0);
   const BatchSeg& S = segs[q];
   update_s_body<VT>(blockIdx.x - S.blk_cells_start, S.blk_cells, s + S.base, z + S.base, S.M, sc + q, zsw,
@@ -965,9 +973,7 @@ cudaError_t update_s(VT* s, const VT* z, long long M, PcgScalars* sc, cudaStream
   // slower at 256^3: more blocks, fewer groups per thread)
   int blocks = (int)std::min<long long>((M / 4 + 255) / 256, (long long)nblk_max);
   if (blocks < 1) blocks = 1;
-  ++g_kernel_launches;
-  update_s_kernel<VT><<<blocks, 256, 0, st>>>(s, z, M, sc, zsw, gperm);
-  return cudaGetLastError();
+  return launch_next(update_s_kernel<VT>, blocks, 256, st, s, z, M, sc, zsw, gperm);
 }
 template cudaError_t update_s<double>(double*, const double*, long long, PcgScalars*, cudaStream_t, const double*,
                                       const int*, int);
@@ -1146,10 +1152,8 @@ template <typename VT, typename AT, typename DT>
 cudaError_t batch_spmv_dot(const BatchSeg* segs, int nseg, int blocks, const AT* diag, const AT* ax,
                            const AT* ay, const AT* az, const VT* s, VT* z, const GroupNb* group_nb, PcgScalars* sc,
                            int mode, cudaStream_t st) {
-  ++g_kernel_launches;
-  batch_spmv_dot_kernel<VT, AT, DT><<<blocks, 256, 0, st>>>(segs, nseg, diag, ax, ay, az, s, z, group_nb, sc,
+  return launch_next(batch_spmv_dot_kernel<VT, AT, DT>, blocks, 256, st, segs, nseg, diag, ax, ay, az, s, z, group_nb, sc,
                                                            mode);
-  return cudaGetLastError();
 }
 template cudaError_t batch_spmv_dot<double, double, double>(const BatchSeg*, int, int, const double*,
                                                             const double*, const double*, const double*,
@@ -1206,9 +1210,7 @@ cudaError_t build_group_tables(const Line* lines, int nj, int nk, int* group_lin
 template <typename VT>
 cudaError_t batch_update_xr(const BatchSeg* segs, int nseg, int blocks, VT* x, VT* r, const VT* s,
                             const VT* z, PcgScalars* sc, cudaStream_t st, VT* rsw, const int* gperm) {
-  ++g_kernel_launches;
-  batch_update_xr_kernel<VT><<<blocks, 256, 0, st>>>(segs, nseg, x, r, s, z, sc, rsw, gperm);
-  return cudaGetLastError();
+  return launch_next(batch_update_xr_kernel<VT>, blocks, 256, st, segs, nseg, x, r, s, z, sc, rsw, gperm);
 }
 template cudaError_t batch_update_xr<double>(const BatchSeg*, int, int, double*, double*, const double*,
                                              const double*, PcgScalars*, cudaStream_t, double*, const int*);
@@ -1218,9 +1220,7 @@ template cudaError_t batch_update_xr<float>(const BatchSeg*, int, int, float*, f
 template <typename VT>
 cudaError_t batch_update_s(const BatchSeg* segs, int nseg, int blocks, VT* s, const VT* z, PcgScalars* sc,
                            cudaStream_t st, const VT* zsw, const int* gperm) {
-  ++g_kernel_launches;
-  batch_update_s_kernel<VT><<<blocks, 256, 0, st>>>(segs, nseg, s, z, sc, zsw, gperm);
-  return cudaGetLastError();
+  return launch_next(batch_update_s_kernel<VT>, blocks, 256, st, segs, nseg, s, z, sc, zsw, gperm);
 }
 template cudaError_t batch_update_s<double>(const BatchSeg*, int, int, double*, const double*, PcgScalars*,
                                             cudaStream_t, const double*, const int*);
@@ -1247,6 +1247,8 @@ __global__ void __launch_bounds__(1024) batch_bwd_reduce_kernel(const BatchSeg* 
                                                                  int mode) {
   constexpr bool F32 = std::is_same<DT, float>::value;
   __shared__ double sum[256], buf[32][8 * 17];
+  start_next();
+  wait_previous();
   const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   PcgScalars* S = sc + q;
   if (*(volatile int*)&S->done) return;
@@ -1269,9 +1271,7 @@ __global__ void __launch_bounds__(1024) batch_bwd_reduce_kernel(const BatchSeg* 
 template <typename DT>
 cudaError_t batch_bwd_reduce(const BatchSeg* segs, int nseg, const double* line_partials, PcgScalars* sc, int mode,
                              cudaStream_t st) {
-  ++g_kernel_launches;
-  batch_bwd_reduce_kernel<DT><<<nseg, 1024, 0, st>>>(segs, line_partials, sc, mode);
-  return cudaGetLastError();
+  return launch_next(batch_bwd_reduce_kernel<DT>, nseg, 1024, st, segs, line_partials, sc, mode);
 }
 template cudaError_t batch_bwd_reduce<double>(const BatchSeg*, int, const double*, PcgScalars*, int, cudaStream_t);
 template cudaError_t batch_bwd_reduce<float>(const BatchSeg*, int, const double*, PcgScalars*, int, cudaStream_t);

@@ -296,7 +296,6 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
   // already writes the other
   __shared__ int s_next[2];
 
-  if (g.scal != nullptr && *(volatile int*)&g.scal->done != 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int unit = warp % NW;
   const bool compute = warp < NW, helper = warp / NW == 1, courier = warp / NW == 2;
@@ -305,7 +304,6 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
   const int rank = blockIdx.x % WAVE_CLUSTER;
   const int cj = rank % WAVE_TJ, ck = rank / WAVE_TJ;
   const int kt = ck * NW + unit;           // unit along k in the tile
-  const unsigned gen = ld_volatile_u32(&g.ctl->gen);
   const int nclusters = gridDim.x / WAVE_CLUSTER;
   // producers and consumers in this cluster (near) or in another (far)
   const bool near_pj = cj - DIR >= 0 && cj - DIR < WAVE_TJ, near_nj = cj + DIR >= 0 && cj + DIR < WAVE_TJ;
@@ -324,6 +322,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
   // per slot: the parity of its mbarriers' next phase at the start of a tile
   // (ready and empty: one per group q; full: one per u)
   unsigned phase_q = 0, phase_u = 0;
+  unsigned gen = 0;
   bool first = true;
 
   for (int pos = blockIdx.x / WAVE_CLUSTER, turn = 0; pos < g.ntiles; turn ^= 1) {
@@ -331,15 +330,10 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
     if (helper && lane == 0) sh.freed = 0;
     int NJB = g.NJB, NKB = g.NKB, lj = g.nj, lk = g.nk;
     long long gbase = 0, bbase = 0, lbase = 0;
-    // (a unit that gave up in an earlier tile does not arm its mbarriers again)
-    bool skip = !first && *(volatile int*)&sh.broken != 0;
-    first = false;
+    int sid = -1;
     if (g.tile_scene != nullptr) {
-      const int sid = g.tile_scene[tpos];
+      sid = g.tile_scene[tpos];
       const BatchSeg& B = g.segs[sid];
-      // a converged scene's tiles are skipped (its scalars only change between
-      // launches, so every warp of this launch decides the same way)
-      skip |= g.scal_batch != nullptr && *(volatile int*)&g.scal_batch[sid].done != 0;
       lj = B.nj;
       lk = B.nk;
       lbase = B.line_base;
@@ -369,6 +363,18 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
     // the consumers' u of this block's group q is q - uj, q - uk
     const WBlk nj = block_at(jb + DIR, ku), nk = block_at(jb, ku + DIR);
     const int uj = ahead(me, nj) - 1, uk = ahead(me, nk) - 1;
+    // the tables are the layout's; from here on, what the kernel before this one wrote
+    if (first) {
+      wait_previous();
+      if (g.scal != nullptr && *(volatile int*)&g.scal->done != 0) return;   // (changes between launches only)
+      gen = ld_volatile_u32(&g.ctl->gen);
+    }
+    // a unit that gave up in an earlier tile does not arm its mbarriers again; a
+    // converged scene's tiles are skipped (its scalars only change between
+    // launches, so every warp of this launch decides the same way)
+    const bool skip = (!first && *(volatile int*)&sh.broken != 0) ||
+                      (sid >= 0 && g.scal_batch != nullptr && *(volatile int*)&g.scal_batch[sid].done != 0);
+    first = false;
     if (helper && lane == 0) {
       sh.limit[0] = near_nj && nj.ng > 0 ? S + uj : INT_MAX;
       sh.limit[1] = near_nk && nk.ng > 0 ? S + uk : INT_MAX;
@@ -881,7 +887,7 @@ template <int OP, typename VT, typename CT>
 struct WaveLaunch {
   static constexpr int smem = warps_of<OP>() * (int)sizeof(UnitShared<OP, VT, CT>);
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   int resident = 0;
   cudaError_t prepare() {
     static std::atomic<int> known[64];
@@ -907,7 +913,9 @@ struct WaveLaunch {
       if (n < 1) return cudaErrorLaunchOutOfResources;
       known[dev & 63] = resident = n;
     }
-    cfg.numAttrs = 2;
+    attr[2].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[2].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 3;
     return cudaSuccess;
   }
 };
