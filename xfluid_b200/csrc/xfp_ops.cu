@@ -280,35 +280,23 @@ template cudaError_t gather_compact<float>(const float*, const Line*, int, int, 
 // :151-152); fluid|fluid and fluid|solid use both pressures, fluid|air uses the
 // ghost -p (:161-198); u -= 1.0*(p2-p1) (:200).  Faces with weight 0 are closed.
 // ---------------------------------------------------------------------------
+// One face: left and right cell, their materials and pressures (read where a cell
+// is in the grid), factor 1.
 template <typename PT>
-__device__ __forceinline__ bool face_dp(const uint8_t* mat, const PT* p, int ni, int nj, int nk,
-                                        int il, int jl, int kl, int ir, int jr, int kr, PT& dp) {
-  const size_t nn = (size_t)ni * nj;
-  const bool inl = il >= 0 && jl >= 0 && kl >= 0 && il < ni && jl < nj && kl < nk;
-  const bool inr = ir >= 0 && jr >= 0 && kr >= 0 && ir < ni && jr < nj && kr < nk;
-  const size_t cl = inl ? (size_t)kl * nn + (size_t)jl * ni + il : 0;
-  const size_t cr = inr ? (size_t)kr * nn + (size_t)jr * ni + ir : 0;
-  const uint8_t ml = inl ? mat[cl] : MAT_SOLID;
-  const uint8_t mr = inr ? mat[cr] : MAT_SOLID;
+__device__ __forceinline__ bool face_dp(uint8_t ml, uint8_t mr, bool inl, bool inr, PT pl, PT pr, PT& dp) {
   if (ml != MAT_FLUID && mr != MAT_FLUID) return false;
-  PT p1, p2;
-  if (ml == MAT_FLUID && mr == MAT_FLUID) {
-    p2 = p[cr]; p1 = p[cl];
-  } else if (ml == MAT_FLUID) {
-    p1 = p[cl];
-    if (mr == MAT_SOLID) {
-      if (!inr) return false;
-      p2 = p[cr];
-    } else {
-      p2 = -p1;
-    }
-  } else {
-    p2 = p[cr];
+  PT p1 = pl, p2 = pr;
+  if (ml != MAT_FLUID) {
     if (ml == MAT_SOLID) {
       if (!inl) return false;
-      p1 = p[cl];
     } else {
       p1 = -p2;
+    }
+  } else if (mr != MAT_FLUID) {
+    if (mr == MAT_SOLID) {
+      if (!inr) return false;
+    } else {
+      p2 = -p1;
     }
   }
   dp = sub_rn(p2, p1);
@@ -316,85 +304,93 @@ __device__ __forceinline__ bool face_dp(const uint8_t* mat, const PT* p, int ni,
 }
 
 // NormalPressureSolver::applyPressure (pressuresolver.cpp:109-212) for one face
-// with left cell l and right cell r (out of range counts as solid), factor 1:
-// fluid|solid takes p2 = p1 + f, solid|fluid p1 = p2 - f, a fluid|air face
-// takes 0 for the air side.  Returns false where no side is fluid.
+// (out of range counts as solid), factor 1: fluid|solid takes p2 = p1 + f,
+// solid|fluid p1 = p2 - f, a fluid|air face takes 0 for the air side.  Returns
+// false where no side is fluid.
 template <typename PT>
-__device__ __forceinline__ bool face_dp_normal(const uint8_t* __restrict__ mat, const PT* __restrict__ p, int ni,
-                                               int nj, int nk, int il, int jl, int kl, int ir, int jr, int kr, PT fv,
-                                               PT& dp) {
-  const size_t nn = (size_t)ni * nj;
-  const bool inl = il >= 0 && jl >= 0 && kl >= 0 && il < ni && jl < nj && kl < nk;
-  const bool inr = ir >= 0 && jr >= 0 && kr >= 0 && ir < ni && jr < nj && kr < nk;
-  const size_t cl = inl ? (size_t)kl * nn + (size_t)jl * ni + il : 0;
-  const size_t cr = inr ? (size_t)kr * nn + (size_t)jr * ni + ir : 0;
-  const uint8_t ml = inl ? mat[cl] : MAT_SOLID;
-  const uint8_t mr = inr ? mat[cr] : MAT_SOLID;
+__device__ __forceinline__ bool face_dp_normal(uint8_t ml, uint8_t mr, PT pl, PT pr, PT fv, PT& dp) {
   if (ml != MAT_FLUID && mr != MAT_FLUID) return false;
-  PT p1, p2;
-  if (ml == MAT_FLUID && mr == MAT_FLUID) {
-    p2 = p[cr]; p1 = p[cl];
-  } else if (ml == MAT_FLUID) {
-    p1 = p[cl];
-    p2 = mr == MAT_SOLID ? add_rn(p1, fv) : PT(0);
-  } else {
-    p2 = p[cr];
-    p1 = ml == MAT_SOLID ? sub_rn(p2, fv) : PT(0);
-  }
+  PT p1 = pl, p2 = pr;
+  if (ml == MAT_FLUID && mr != MAT_FLUID) p2 = mr == MAT_SOLID ? add_rn(p1, fv) : PT(0);
+  if (ml != MAT_FLUID) p1 = ml == MAT_SOLID ? sub_rn(p2, fv) : PT(0);
   dp = sub_rn(p2, p1);
   return true;
 }
 
+// One pass over the corner grid for the faces of all three axes, a warp per row
+// along x: they share the cell, its pressure and its material, and a row costs one
+// division.  Bound by the loads and stores of the faces next to fluid; other faces
+// are not read.  Half-full 256^3, FP32: 104 us (a launch per axis with 64-bit
+// divisions per face, reading every face: 292 us; one launch that takes the axes one
+// after the other: 152 us).
 template <typename FT, typename PT>
-__global__ void apply_kernel(const uint8_t* __restrict__ mat, const FT* __restrict__ wt,
-                             const PT* __restrict__ p, int ni, int nj, int nk, int axis,
-                             FT* __restrict__ f, int matrix, Force3 frc) {
-  const int si = ni + (axis == 0), sj = nj + (axis == 1), sk = nk + (axis == 2);
-  const size_t n = (size_t)si * sj * sk;
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(idx % si);
-    const int j = (int)((idx / si) % sj);
-    const int k = (int)(idx / ((size_t)si * sj));
-    // a body force first moves every face that borders fluid (_applyForces),
-    // then the pressure update uses the moved value
-    FT fv = f[idx];
-    bool changed = false;
-    if (frc.axis_on(axis)) {
-      const int il = i - (axis == 0), jl = j - (axis == 1), kl = k - (axis == 2);
-      const size_t nn = (size_t)ni * nj;
-      const bool fl = il >= 0 && jl >= 0 && kl >= 0 && mat[(size_t)kl * nn + (size_t)jl * ni + il] == MAT_FLUID;
-      const bool fr = i < ni && j < nj && k < nk && mat[(size_t)k * nn + (size_t)j * ni + i] == MAT_FLUID;
-      if (fl || fr) {
-        fv = add_rn(fv, (FT)frc.d[axis]);
-        changed = true;
+__global__ void __launch_bounds__(256) apply_kernel(const uint8_t* __restrict__ mat, const FT* __restrict__ wu,
+                                                    const FT* __restrict__ wv, const FT* __restrict__ ww,
+                                                    const PT* __restrict__ p, int ni, int nj, int nk,
+                                                    FT* __restrict__ u, FT* __restrict__ v, FT* __restrict__ w,
+                                                    int matrix, Force3 frc) {
+  const int lane = threadIdx.x & 31;
+  const size_t nn = (size_t)ni * nj;
+  const unsigned rows = (unsigned)(nj + 1) * (unsigned)(nk + 1);
+  for (unsigned row = blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8) {
+    const int k = (int)(row / (unsigned)(nj + 1)), j = (int)(row - (unsigned)k * (unsigned)(nj + 1));
+    for (int i = lane; i <= ni; i += 32) {
+      // the cell (3) and its lower neighbours by axis; then, all under way
+      // together, the pressures and faces that are needed
+      const size_t c = (size_t)k * nn + (size_t)j * ni + i, step[3] = {1, (size_t)ni, nn};
+      const bool here = i < ni && j < nj && k < nk;
+      const bool in[3] = {i > 0 && j < nj && k < nk, j > 0 && i < ni && k < nk, k > 0 && i < ni && j < nj};
+      const bool face[3] = {j < nj && k < nk, i < ni && k < nk, i < ni && j < nj};
+      const uint8_t m = here ? mat[c] : MAT_SOLID;
+      uint8_t ml[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) ml[a] = in[a] ? mat[c - step[a]] : MAT_SOLID;
+      const bool wet = m == MAT_FLUID || ml[0] == MAT_FLUID || ml[1] == MAT_FLUID || ml[2] == MAT_FLUID;
+      if (!wet) continue;
+      const PT pr = here ? p[c] : PT(0);
+      PT pl[3];
+      FT fv[3];
+      bool open[3];
+      size_t at[3];
+      FT* const f[3] = {u, v, w};
+      const FT* const wt[3] = {wu, wv, ww};
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        at[a] = ((size_t)k * (nj + (a == 1)) + j) * (ni + (a == 0)) + i;
+        const bool near = face[a] && (m == MAT_FLUID || ml[a] == MAT_FLUID);
+        pl[a] = near && in[a] ? p[c - step[a]] : PT(0);
+        fv[a] = near ? f[a][at[a]] : FT(0);
+        open[a] = near && (matrix == XFP_MATRIX_NORMAL || wt[a] == nullptr || wt[a][at[a]] != FT(0));
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (!face[a] || !(m == MAT_FLUID || ml[a] == MAT_FLUID)) continue;
+        // a body force first moves every face that borders fluid (_applyForces),
+        // then the pressure update uses the moved value
+        bool changed = false;
+        if (frc.axis_on(a)) {
+          fv[a] = add_rn(fv[a], (FT)frc.d[a]);
+          changed = true;
+        }
+        PT dp;
+        if (matrix == XFP_MATRIX_NORMAL ? face_dp_normal(ml[a], m, pl[a], pr, (PT)fv[a], dp)
+                                        : open[a] && face_dp(ml[a], m, in[a], here, pl[a], pr, dp)) {
+          fv[a] = sub_rn(fv[a], (FT)mul_rn(PT(1), dp));
+          changed = true;
+        }
+        if (changed) f[a][at[a]] = fv[a];
       }
     }
-    PT dp;
-    if (matrix == XFP_MATRIX_NORMAL) {
-      if (face_dp_normal(mat, p, ni, nj, nk, i - (axis == 0), j - (axis == 1), k - (axis == 2), i, j, k,
-                         (PT)fv, dp)) {
-        fv = sub_rn(fv, (FT)mul_rn(PT(1), dp));
-        changed = true;
-      }
-    } else if (!(wt && wt[idx] == FT(0)) &&
-               face_dp(mat, p, ni, nj, nk, i - (axis == 0), j - (axis == 1), k - (axis == 2), i, j, k, dp)) {
-      fv = sub_rn(fv, (FT)mul_rn(PT(1), dp));
-      changed = true;
-    }
-    if (changed) f[idx] = fv;
   }
 }
 template <typename FT, typename PT>
 cudaError_t apply_pressure(const uint8_t* mat, const FT* wu, const FT* wv, const FT* ww,
                            const PT* p, int ni, int nj, int nk, FT* u, FT* v, FT* w,
                            cudaStream_t st, int matrix, Force3 frc) {
-  for (int axis = 0; axis < 3; ++axis) {
-    size_t n = (size_t)(ni + (axis == 0)) * (nj + (axis == 1)) * (nk + (axis == 2));
-    unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 32);
-    ++g_kernel_launches;
-    apply_kernel<FT, PT><<<blocks, 256, 0, st>>>(mat, axis == 0 ? wu : axis == 1 ? wv : ww, p, ni, nj, nk,
-                                                axis, axis == 0 ? u : axis == 1 ? v : w, matrix, frc);
-  }
+  const long long rows = (long long)(nj + 1) * (nk + 1);
+  ++g_kernel_launches;
+  apply_kernel<FT, PT><<<(unsigned)std::min<long long>((rows + 7) / 8, 148LL * 64), 256, 0, st>>>(
+      mat, wu, wv, ww, p, ni, nj, nk, u, v, w, matrix, frc);
   return cudaGetLastError();
 }
 template cudaError_t apply_pressure<double, double>(const uint8_t*, const double*, const double*,
