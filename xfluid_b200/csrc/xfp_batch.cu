@@ -34,7 +34,7 @@ struct BatchState {
   DevBuf io, pdense;
   std::vector<BatchSeg> hsegs;
   std::vector<long long> rows, nlines_act;
-  int n = 0, ntiles = 0, blocks_lines = 0, blocks_cells = 0, blocks_groups = 0;
+  int n = 0, ntiles = 0, blocks_cells = 0, blocks_groups = 0;
   long long M = 0;
 };
 
@@ -140,15 +140,13 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S)
   // per-scene block decomposition of the vector kernels (as a single launch)
   B->hsegs.assign(n, BatchSeg{});
   XFP_CUDA(ctx, B->part.ensure((size_t)n * NBLK_MAX * sizeof(double)));
-  int bl = 0, bc = 0, bg = 0;
+  int bc = 0, bg = 0;
   for (int s = 0; s < n; ++s) {
     BatchSeg& g = B->hsegs[s];
-    const long long nl = (long long)S[s].nj * S[s].nk, Ms = cnt[5 * s];
+    const long long Ms = cnt[5 * s];
     g.ni = S[s].ni; g.nj = S[s].nj; g.nk = S[s].nk;
-    g.blk_lines = (int)std::max<long long>(1, std::min<long long>((nl + 7) / 8, NBLK_MAX));
-    g.blk_lines_start = bl;
-    // the cell-based kernels run one thread per 4-cell group (absmax_init and
-    // the residual stride over single cells with the same blocks)
+    // the cell-based kernels run one thread per 4-cell group (absmax_init strides
+    // over single cells with the same blocks)
     g.blk_cells = (int)std::max<long long>(1, std::min<long long>((Ms / 4 + 255) / 256, NBLK_MAX));
     g.blk_cells_start = bc;
     g.blk_groups = (int)spmv_block_count(Ms, NBLK_MAX);
@@ -160,11 +158,9 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S)
     g.M = Ms;
     g.lines = lines + line_base[s];
     g.partials = B->part.as<double>() + (size_t)s * NBLK_MAX;
-    bl += g.blk_lines;
     bc += g.blk_cells;
     bg += g.blk_groups;
   }
-  B->blocks_lines = bl;
   B->blocks_cells = bc;
   B->blocks_groups = bg;
   XFP_CUDA(ctx, B->segs.ensure(n * sizeof(BatchSeg)));
@@ -376,7 +372,8 @@ int batch_solve(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<IOT>>& S
   XFP_CUDA(ctx, B->maxits.ensure(n * sizeof(int)));
   for (int cyc = 0; cyc < max_ref; ++cyc) {
     if (cyc > 0) {
-      XFP_CUDA(ctx, batch_residual64(segs, n, B->blocks_lines, A[0], A[1], A[2], A[3], A[4], x64, r64, osc, st));
+      XFP_CUDA(ctx, batch_residual64(segs, n, B->blocks_groups, A[0], A[1], A[2], A[3], A[4], x64, r64,
+                                   ctx->group_nb.as<GroupNb>(), osc, st));
       XFP_CUDA(ctx, cudaMemcpyAsync(ho.data(), osc, n * sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
       XFP_CUDA(ctx, cudaStreamSynchronize(st));
       for (int q = 0; q < n; ++q) {
@@ -416,7 +413,8 @@ int batch_solve(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<IOT>>& S
   bool open = false;
   for (int q = 0; q < n; ++q) open |= !fin[q];
   if (open) {
-    XFP_CUDA(ctx, batch_residual64(segs, n, B->blocks_lines, A[0], A[1], A[2], A[3], A[4], x64, r64, osc, st));
+    XFP_CUDA(ctx, batch_residual64(segs, n, B->blocks_groups, A[0], A[1], A[2], A[3], A[4], x64, r64,
+                                   ctx->group_nb.as<GroupNb>(), osc, st));
     XFP_CUDA(ctx, cudaMemcpyAsync(ho.data(), osc, n * sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
     XFP_CUDA(ctx, cudaStreamSynchronize(st));
     for (int q = 0; q < n; ++q)

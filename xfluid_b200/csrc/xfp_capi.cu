@@ -422,7 +422,7 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
       status = XFP_NOT_CONVERGED;
       for (cycles = 0; cycles < max_ref && total < maxit; ++cycles) {
         if (cycles > 0) {
-          XFP_CUDA(ctx, residual64(A[0], A[1], A[2], A[3], A[4], x64, r64, lines, ni, nj, nk, M, osc,
+          XFP_CUDA(ctx, residual64(A[0], A[1], A[2], A[3], A[4], x64, r64, ctx->group_nb.as<GroupNb>(), M, osc,
                                    ctx->partials.as<double>(), NBLK_MAX, st));
           XFP_CUDA(ctx, cudaMemcpyAsync(&ho, osc, sizeof(ho), cudaMemcpyDeviceToHost, st));
           XFP_CUDA(ctx, cudaStreamSynchronize(st));
@@ -443,7 +443,7 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
         XFP_CUDA(ctx, refine_update(x64, ctx->x32.as<float>(), M, st));
       }
       if (status != XFP_OK) {
-        XFP_CUDA(ctx, residual64(A[0], A[1], A[2], A[3], A[4], x64, r64, lines, ni, nj, nk, M, osc,
+        XFP_CUDA(ctx, residual64(A[0], A[1], A[2], A[3], A[4], x64, r64, ctx->group_nb.as<GroupNb>(), M, osc,
                                  ctx->partials.as<double>(), NBLK_MAX, st));
         XFP_CUDA(ctx, cudaMemcpyAsync(&ho, osc, sizeof(ho), cudaMemcpyDeviceToHost, st));
         XFP_CUDA(ctx, cudaStreamSynchronize(st));

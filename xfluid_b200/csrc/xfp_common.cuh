@@ -108,9 +108,8 @@ struct SweepCtl {
 // kernels give it (line-based and cell-based grids, consecutive per scene).
 struct BatchSeg {
   int ni, nj, nk;
-  int blk_lines, blk_lines_start;   // line-based kernels (residual)
   int blk_cells, blk_cells_start;   // cell-based kernels (updates, norms)
-  int blk_groups, blk_groups_start; // the SpMV (one thread per 4-cell group)
+  int blk_groups, blk_groups_start; // the SpMV and the residual (one thread per 4-cell group)
   long long blk_base, group_base;   // first entry of this scene's block table, first group of its sweep slice
   long long line_base;              // its first line among all scenes'
   long long base, M;

@@ -196,7 +196,7 @@ cudaError_t batch_absmax_init(const BatchSeg* segs, int nseg, int blocks, const 
                               double tol, int maxit, const double* tols, const int* maxits, cudaStream_t st);
 cudaError_t batch_residual64(const BatchSeg* segs, int nseg, int blocks, const double* diag, const double* ax,
                              const double* ay, const double* az, const double* b, const double* x, double* r,
-                             PcgScalars* sc, cudaStream_t st);
+                             const GroupNb* group_nb, PcgScalars* sc, cudaStream_t st);
 // Per-scene z.r from the backward sweep's line partials, in the single-scene
 // order; mode 0: rho, mode 1: beta and rho.
 template <typename DT>
@@ -217,10 +217,9 @@ cudaError_t box_loss(const T* u, const T* v, const T* w, T* gu, T* gv, T* gw, in
 cudaError_t offset_lines(Line* lines, long long nlines, long long base, cudaStream_t st);
 
 // Mixed precision: r64 = b64 - A64 x64, |r|_inf and r32 = (float) r64 / scale.
-cudaError_t residual64(const double* diag, const double* ax, const double* ay, const double* az,
-                       const double* b, const double* x, double* r, const Line* lines, int ni,
-                       int nj, int nk, long long M, PcgScalars* sc, double* partials,
-                       int nblk_max, cudaStream_t st);
+cudaError_t residual64(const double* diag, const double* ax, const double* ay, const double* az, const double* b,
+                       const double* x, double* r, const GroupNb* group_nb, long long M, PcgScalars* sc,
+                       double* partials, int nblk_max, cudaStream_t st);
 cudaError_t refine_update(double* x64, const float* e32, long long M, cudaStream_t st);
 
 }  // namespace xfp

@@ -619,17 +619,15 @@ __device__ __forceinline__ bool last_block(PcgScalars* sc, unsigned nblk) {
 // Batch of scenes in one launch: block b belongs to the scene whose range of
 // blocks [start, start + count) holds it; the scene's blocks then run exactly
 // the decomposition a single-scene launch of `count` blocks would.
-// kind: which block range of the scene a block belongs to (0 cell-based
-// kernels, 1 line-based kernels, 2 the SpMV's 4-cell groups).
-__device__ __forceinline__ int batch_scene_of(const BatchSeg* __restrict__ segs, int nseg, int kind) {
+// groups: the block ranges of the kernels over 4-cell groups, not of the cell-based ones.
+__device__ __forceinline__ int batch_scene_of(const BatchSeg* __restrict__ segs, int nseg, bool groups) {
   __shared__ int s_seg;
   if (threadIdx.x == 0) {
     int lo = 0, hi = nseg - 1;
     const int b = (int)blockIdx.x;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      const int start = kind == 1 ? segs[mid].blk_lines_start
-                                  : kind == 2 ? segs[mid].blk_groups_start : segs[mid].blk_cells_start;
+      const int start = groups ? segs[mid].blk_groups_start : segs[mid].blk_cells_start;
       if (start <= b) lo = mid; else hi = mid - 1;
     }
     s_seg = lo;
@@ -669,6 +667,24 @@ __device__ __forceinline__ DT partials_sum(const DT* partials, unsigned nblk, DT
 // FP64 dam at 128^3 (0.44 M) / FP64 at 24^3: 19 / 10.9 / 4.4 us; with five line
 // records a group and a scalar load per neighbour 30.5 / 14.8 / 5.8 us.
 // ---------------------------------------------------------------------------
+// A group's four neighbours in a line before it (j or k - 1) / after it; 0 where
+// there is none.
+template <typename VT>
+__device__ __forceinline__ void nb_before(const VT* __restrict__ p, unsigned nb, VT (&v)[4]) {
+  const size_t quad = (size_t)(nb >> 2) * 4;
+  VT w[4] = {VT(0), VT(0), VT(0), VT(0)};
+  v[0] = nb & 1u ? p[quad - 1] : VT(0);
+  if (nb & 2u) ldg(w, p + quad);
+  v[1] = w[0]; v[2] = w[1]; v[3] = w[2];
+}
+template <typename VT>
+__device__ __forceinline__ void nb_after(const VT* __restrict__ p, unsigned nb, VT (&v)[4]) {
+  const size_t quad = (size_t)(nb >> 2) * 4;
+  VT w[4] = {VT(0), VT(0), VT(0), VT(0)};
+  if (nb & 1u) ldg(w, p + quad - 4);
+  v[0] = w[1]; v[1] = w[2]; v[2] = w[3];
+  v[3] = nb & 2u ? p[quad] : VT(0);
+}
 template <typename VT, typename AT, typename DT>
 __device__ __forceinline__ void spmv_dot_body(
     unsigned bid, unsigned nblk, const AT* __restrict__ diag, const AT* __restrict__ ax,
@@ -680,21 +696,6 @@ __device__ __forceinline__ void spmv_dot_body(
   if (sc && *(volatile int*)&sc->done) return;
   DT acc = DT(0);
   const long long G = M >> 2;
-  // the group's four neighbours in a line before it (j or k - 1) / after it; 0 where there is none
-  auto before = [](const VT* __restrict__ p, unsigned nb, VT (&v)[4]) {
-    const size_t quad = (size_t)(nb >> 2) * 4;
-    VT w[4] = {VT(0), VT(0), VT(0), VT(0)};
-    v[0] = nb & 1u ? p[quad - 1] : VT(0);
-    if (nb & 2u) ldg(w, p + quad);
-    v[1] = w[0]; v[2] = w[1]; v[3] = w[2];
-  };
-  auto after = [](const VT* __restrict__ p, unsigned nb, VT (&v)[4]) {
-    const size_t quad = (size_t)(nb >> 2) * 4;
-    VT w[4] = {VT(0), VT(0), VT(0), VT(0)};
-    if (nb & 1u) ldg(w, p + quad - 4);
-    v[0] = w[1]; v[1] = w[2]; v[2] = w[3];
-    v[3] = nb & 2u ? p[quad] : VT(0);
-  };
   for (long long q = (long long)bid * blockDim.x + threadIdx.x; q < G; q += (long long)nblk * blockDim.x) {
     const long long c = base + 4 * q;
     const GroupNb nb = group_nb[(base >> 2) + q];
@@ -711,12 +712,12 @@ __device__ __forceinline__ void spmv_dot_body(
     const VT sr = right ? s[c + 4] : VT(0);
     const VT xr = right ? ax[c + 4] : VT(0);
     VT szm[4], sym[4], syp[4], szp[4], ayp[4], azp[4];
-    before(s, nb.zm, szm);
-    before(s, nb.ym, sym);
-    after(s, nb.yp, syp);
-    after(ay, nb.yp, ayp);
-    after(s, nb.zp, szp);
-    after(az, nb.zp, azp);
+    nb_before(s, nb.zm, szm);
+    nb_before(s, nb.ym, sym);
+    nb_after(s, nb.yp, syp);
+    nb_after(ay, nb.yp, ayp);
+    nb_after(s, nb.zp, szp);
+    nb_after(az, nb.zp, azp);
     VT out[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -770,7 +771,7 @@ __global__ void __launch_bounds__(256) batch_spmv_dot_kernel(
     const GroupNb* __restrict__ group_nb, PcgScalars* sc, int mode) {
   start_next();
   wait_previous();
-  const int q = batch_scene_of(segs, nseg, 2);
+  const int q = batch_scene_of(segs, nseg, true);
   const BatchSeg& S = segs[q];
   spmv_dot_body<VT, AT, DT>(blockIdx.x - S.blk_groups_start, S.blk_groups, diag, ax, ay, az, s, z, group_nb, S.base,
                             S.M, sc + q, reinterpret_cast<DT*>(S.partials), mode);
@@ -886,7 +887,7 @@ __global__ void __launch_bounds__(256) batch_update_xr_kernel(const BatchSeg* __
                                                               const int* __restrict__ gperm) {
   start_next();
   wait_previous();
-  const int q = batch_scene_of(segs, nseg, 0);
+  const int q = batch_scene_of(segs, nseg, false);
   const BatchSeg& S = segs[q];
   update_xr_body<VT>(blockIdx.x - S.blk_cells_start, S.blk_cells, x + S.base, r + S.base, s + S.base,
                      z + S.base, S.M, sc + q, S.partials, rsw, gperm ? gperm + S.base / 4 : nullptr);
@@ -957,7 +958,7 @@ __global__ void batch_update_s_kernel(const BatchSeg* __restrict__ segs, int nse
                                       const int* __restrict__ gperm) {
   start_next();
   wait_previous();
-  const int q = batch_scene_of(segs, nseg, 0);
+  const int q = batch_scene_of(segs, nseg, false);
   const BatchSeg& S = segs[q];
   update_s_body<VT>(blockIdx.x - S.blk_cells_start, S.blk_cells, s + S.base, z + S.base, S.M, sc + q, zsw,
                     gperm ? gperm + S.base / 4 : nullptr);
@@ -1010,7 +1011,7 @@ template <typename VT>
 __global__ void batch_absmax_init_kernel(const BatchSeg* __restrict__ segs, int nseg, const VT* __restrict__ b,
                                          PcgScalars* sc, double tol, int maxit, const double* __restrict__ tols,
                                          const int* __restrict__ maxits) {
-  const int q = batch_scene_of(segs, nseg, 0);
+  const int q = batch_scene_of(segs, nseg, false);
   const BatchSeg& S = segs[q];
   absmax_init_body<VT>(blockIdx.x - S.blk_cells_start, S.blk_cells, b + S.base, S.M, sc + q, S.partials,
                        tols ? tols[q] : tol, maxits ? maxits[q] : maxit);
@@ -1059,43 +1060,43 @@ template cudaError_t copy_vec<float>(const float*, float*, long long, cudaStream
 __device__ __forceinline__ void residual64_body(
     unsigned bid, unsigned nblk, const double* __restrict__ diag, const double* __restrict__ ax,
     const double* __restrict__ ay, const double* __restrict__ az, const double* __restrict__ b,
-    const double* __restrict__ x, double* __restrict__ r, const Line* __restrict__ lines, int ni, int nj,
-    int nk, PcgScalars* sc, double* __restrict__ partials) {
+    const double* __restrict__ x, double* __restrict__ r, const GroupNb* __restrict__ group_nb, long long base,
+    long long M, PcgScalars* sc, double* __restrict__ partials) {
   __shared__ double sh[32];
-  const int lane = threadIdx.x & 31;
-  const long long nlines = (long long)nj * nk;
   double m = 0.0;
-  for (long long line = (long long)bid * (blockDim.x >> 5) + (threadIdx.x >> 5); line < nlines;
-       line += (long long)nblk * (blockDim.x >> 5)) {
-    const Line L = lines[line];
-    if (L.len == 0) continue;
-    const int j = (int)(line % nj), k = (int)(line / nj);
-    Line Lym = {0, 0, 0, 0}, Lyp = {0, 0, 0, 0}, Lzm = {0, 0, 0, 0}, Lzp = {0, 0, 0, 0};
-    if (j > 0) Lym = lines[line - 1];
-    if (j + 1 < nj) Lyp = lines[line + 1];
-    if (k > 0) Lzm = lines[line - nj];
-    if (k + 1 < nk) Lzp = lines[line + nj];
-    for (int q = lane; q < L.len; q += 32) {
-      const int i = L.lo + q;
-      const size_t c = (size_t)L.off + q;
+  for (long long q = (long long)bid * blockDim.x + threadIdx.x; q < M >> 2; q += (long long)nblk * blockDim.x) {
+    const long long c = base + 4 * q;
+    const GroupNb nb = group_nb[(base >> 2) + q];
+    double sv[4], dv[4], xv[4], yv[4], zv[4], bv[4], xzm[4], xym[4], xyp[4], xzp[4], ayp[4], azp[4], rv[4];
+    ldg(sv, x + c);
+    ldg(dv, diag + c);
+    ldg(xv, ax + c);
+    ldg(yv, ay + c);
+    ldg(zv, az + c);
+    ldg(bv, b + c);
+    const bool right = 4 * q + 4 < M;
+    const double sl = c > base ? x[c - 1] : 0.0, sr = right ? x[c + 4] : 0.0, xr = right ? ax[c + 4] : 0.0;
+    nb_before(x, nb.zm, xzm);
+    nb_before(x, nb.ym, xym);
+    nb_after(x, nb.yp, xyp);
+    nb_after(ay, nb.yp, ayp);
+    nb_after(x, nb.zp, xzp);
+    nb_after(az, nb.zp, azp);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const double cx = e < 3 ? xv[e < 3 ? e + 1 : 3] : xr;
       double a = 0.0;
-      if (az[c] != 0.0) a += az[c] * x[(size_t)Lzm.off + (i - Lzm.lo)];
-      if (ay[c] != 0.0) a += ay[c] * x[(size_t)Lym.off + (i - Lym.lo)];
-      if (ax[c] != 0.0) a += ax[c] * x[c - 1];
-      a += diag[c] * x[c];
-      if (q + 1 < L.len && ax[c + 1] != 0.0) a += ax[c + 1] * x[c + 1];
-      if ((unsigned)(i - Lyp.lo) < (unsigned)Lyp.len) {
-        const size_t n = (size_t)Lyp.off + (i - Lyp.lo);
-        if (ay[n] != 0.0) a += ay[n] * x[n];
-      }
-      if ((unsigned)(i - Lzp.lo) < (unsigned)Lzp.len) {
-        const size_t n = (size_t)Lzp.off + (i - Lzp.lo);
-        if (az[n] != 0.0) a += az[n] * x[n];
-      }
-      const double rv = b[c] - a;
-      r[c] = rv;
-      m = fmax(m, fabs(rv));
+      if (zv[e] != 0.0) a = __fma_rn(zv[e], xzm[e], a);
+      if (yv[e] != 0.0) a = __fma_rn(yv[e], xym[e], a);
+      if (xv[e] != 0.0) a = __fma_rn(xv[e], e == 0 ? sl : sv[e == 0 ? 0 : e - 1], a);
+      a = __fma_rn(dv[e], sv[e], a);
+      if (cx != 0.0) a = __fma_rn(cx, e < 3 ? sv[e < 3 ? e + 1 : 3] : sr, a);
+      if (ayp[e] != 0.0) a = __fma_rn(ayp[e], xyp[e], a);
+      if (azp[e] != 0.0) a = __fma_rn(azp[e], xzp[e], a);
+      rv[e] = bv[e] - a;
+      m = fmax(m, fabs(rv[e]));
     }
+    stg(r + c, rv);
   }
   double t = block_max(m, sh);
   if (threadIdx.x == 0) partials[bid] = t;
@@ -1109,35 +1110,32 @@ __device__ __forceinline__ void residual64_body(
 __global__ void __launch_bounds__(256) residual64_kernel(
     const double* __restrict__ diag, const double* __restrict__ ax, const double* __restrict__ ay,
     const double* __restrict__ az, const double* __restrict__ b, const double* __restrict__ x,
-    double* __restrict__ r, const Line* __restrict__ lines, int ni, int nj, int nk, PcgScalars* sc,
+    double* __restrict__ r, const GroupNb* __restrict__ group_nb, long long M, PcgScalars* sc,
     double* __restrict__ partials) {
-  residual64_body(blockIdx.x, gridDim.x, diag, ax, ay, az, b, x, r, lines, ni, nj, nk, sc, partials);
+  residual64_body(blockIdx.x, gridDim.x, diag, ax, ay, az, b, x, r, group_nb, 0, M, sc, partials);
 }
 __global__ void __launch_bounds__(256) batch_residual64_kernel(
     const BatchSeg* __restrict__ segs, int nseg, const double* __restrict__ diag, const double* __restrict__ ax,
     const double* __restrict__ ay, const double* __restrict__ az, const double* __restrict__ b,
-    const double* __restrict__ x, double* __restrict__ r, PcgScalars* sc) {
-  const int q = batch_scene_of(segs, nseg, 1);
+    const double* __restrict__ x, double* __restrict__ r, const GroupNb* __restrict__ group_nb, PcgScalars* sc) {
+  const int q = batch_scene_of(segs, nseg, true);
   const BatchSeg& S = segs[q];
-  residual64_body(blockIdx.x - S.blk_lines_start, S.blk_lines, diag, ax, ay, az, b, x, r, S.lines, S.ni, S.nj,
-                  S.nk, sc + q, S.partials);
+  residual64_body(blockIdx.x - S.blk_groups_start, S.blk_groups, diag, ax, ay, az, b, x, r, group_nb, S.base, S.M,
+                  sc + q, S.partials);
 }
 cudaError_t batch_residual64(const BatchSeg* segs, int nseg, int blocks, const double* diag, const double* ax,
                              const double* ay, const double* az, const double* b, const double* x, double* r,
-                             PcgScalars* sc, cudaStream_t st) {
+                             const GroupNb* group_nb, PcgScalars* sc, cudaStream_t st) {
   ++g_kernel_launches;
-  batch_residual64_kernel<<<blocks, 256, 0, st>>>(segs, nseg, diag, ax, ay, az, b, x, r, sc);
+  batch_residual64_kernel<<<blocks, 256, 0, st>>>(segs, nseg, diag, ax, ay, az, b, x, r, group_nb, sc);
   return cudaGetLastError();
 }
-cudaError_t residual64(const double* diag, const double* ax, const double* ay, const double* az,
-                       const double* b, const double* x, double* r, const Line* lines, int ni,
-                       int nj, int nk, long long M, PcgScalars* sc, double* partials,
-                       int nblk_max, cudaStream_t st) {
-  (void)M;
-  const long long nlines = (long long)nj * nk;
-  int blocks = (int)std::min<long long>((nlines + 7) / 8, (long long)nblk_max);
+cudaError_t residual64(const double* diag, const double* ax, const double* ay, const double* az, const double* b,
+                       const double* x, double* r, const GroupNb* group_nb, long long M, PcgScalars* sc,
+                       double* partials, int nblk_max, cudaStream_t st) {
   ++g_kernel_launches;
-  residual64_kernel<<<blocks, 256, 0, st>>>(diag, ax, ay, az, b, x, r, lines, ni, nj, nk, sc, partials);
+  residual64_kernel<<<(unsigned)spmv_block_count(M, nblk_max), 256, 0, st>>>(diag, ax, ay, az, b, x, r, group_nb, M, sc,
+                                                                            partials);
   return cudaGetLastError();
 }
 
