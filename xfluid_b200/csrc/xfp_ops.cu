@@ -1056,6 +1056,8 @@ template cudaError_t copy_vec<float>(const float*, float*, long long, cudaStream
 // ---------------------------------------------------------------------------
 // Mixed precision: FP64 residual r = b - A x with |r|_inf (into sc->res), on
 // the FP64 copy of A; and x64 += e32 after each FP32 inner solve.
+// A thread per 4-cell group, with the SpMV's vectors and neighbour records; bound by
+// its loads.  256^3 half full: 50 us (144 with a line per warp and single loads).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void residual64_body(
     unsigned bid, unsigned nblk, const double* __restrict__ diag, const double* __restrict__ ax,
