@@ -210,8 +210,10 @@ __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
-__device__ __forceinline__ double rsqrt_ref(double x) { return __ddiv_rn(1.0, __dsqrt_rn(x)); }
-__device__ __forceinline__ float rsqrt_ref(float x) { return __fdiv_rn(1.0f, __fsqrt_rn(x)); }
+// 1 / sqrt(x), both rounded as the reference rounds them: the reciprocal is the
+// correctly rounded quotient 1 / y, in fewer steps than a division
+__device__ __forceinline__ double rsqrt_ref(double x) { return __drcp_rn(__dsqrt_rn(x)); }
+__device__ __forceinline__ float rsqrt_ref(float x) { return __frcp_rn(__fsqrt_rn(x)); }
 
 // One group of XFP_ALIGN (4) consecutive cells of an array, from/to a
 // group-aligned index: one 16-byte access (FP32) or two (FP64).  Groups of 8
