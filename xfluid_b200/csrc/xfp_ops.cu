@@ -171,10 +171,13 @@ __global__ void assemble_kernel(const uint8_t* __restrict__ mat, const FT* __res
       if (sys != nullptr) {
         const int t = i + j + k;
         AT* e = sys + (size_t)(group_base + blk.goff + (t >> 2) - blk.g0) * 1024;
-        e[wave_cell_slot<AT>(j, k, t & 3, 0)] = d;
-        e[wave_cell_slot<AT>(j, k, t & 3, 1)] = ux;
-        e[wave_cell_slot<AT>(j, k, t & 3, 2)] = uy;
-        e[wave_cell_slot<AT>(j, k, t & 3, 3)] = uz;
+        AT* c0 = e + wave_cell_slot<AT>(j, k, t & 3, 0);
+        if constexpr (sizeof(AT) == 8) {   // two 16-byte units (wave_cell_slot)
+          *reinterpret_cast<double2*>(c0) = make_double2(d, ux);
+          *reinterpret_cast<double2*>(c0 + 64) = make_double2(uy, uz);
+        } else {
+          *reinterpret_cast<float4*>(c0) = make_float4(d, ux, uy, uz);
+        }
       }
       // the mixed form's FP32 stencil, written by the assembly itself
       if (d32 != nullptr) {
