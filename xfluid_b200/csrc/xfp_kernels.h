@@ -10,9 +10,9 @@ namespace xfp {
 
 enum { SWEEP_FACTOR = 0, SWEEP_FWD = 1, SWEEP_BWD = 2 };
 
-// Kernels launched by this library in this process (every launcher adds its
+// Kernels launched by this library in this thread (every launcher adds its
 // launches); a call reports the difference across its own work.
-extern long long g_kernel_launches;
+extern thread_local long long g_kernel_launches;
 
 // A launch of one of the PCG loop's kernels (start_next, wait_previous).
 template <typename... P, typename... A>

@@ -15,7 +15,7 @@
 
 namespace xfp {
 
-long long g_kernel_launches = 0;
+thread_local long long g_kernel_launches = 0;
 
 __device__ __forceinline__ size_t uix(int ni, int nj, int i, int j, int k) {
   return ((size_t)k * nj + j) * (size_t)(ni + 1) + i;
