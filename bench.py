@@ -489,8 +489,24 @@ def ours(args, rank, world):
     rows = int(last["rows"])
     iters = int(last["iterations"])
     launches = int(sum(s["launches"] for _, s in stats))
-    sweep_ms = sum(s["ms_sweeps"] for _, s in stats)
-    sweeps = sum(s["sweeps"] for _, s in stats)
+    # the roofline's kernel durations: CUDA events on every 16th PCG iteration of
+    # a few projections after the timed ones (with events the loop launches its
+    # kernels one by one, not as a graph)
+    had = os.environ.get("XFP_KERNEL_EVENTS")
+    os.environ["XFP_KERNEL_EVENTS"] = had or "16"
+    ctx_ev = ctx_for("mixed", 1)
+    if had is None:
+        del os.environ["XFP_KERNEL_EVENTS"]
+    ev_stats = []
+    for s in range(min(6, args.steps) + 1):
+        for dst, src in zip(copies[0], vel0):
+            dst.copy_(src)
+        st_ev = project_dev(ctx_ev, copies[0], pres)[1]
+        if s:
+            ev_stats.append(st_ev)
+    ctx_ev.close()
+    sweep_ms = sum(s["ms_sweeps"] for s in ev_stats)
+    sweeps = sum(s["sweeps"] for s in ev_stats)
     # algorithmic bytes of one sweep launch (mixed: FP32 vectors and L, the FP64
     # pivots streamed as FP32): forward r 4 + L 12 + invdiag 4 + y 4 = 24 B/row;
     # backward y 4 + L 12 + invdiag 4 + r 4 + z 4 = 28 B/row; launches
@@ -517,8 +533,8 @@ def ours(args, rank, world):
     # convergence excluded): algorithmic bytes per unknown row (FP32 vectors
     # and coefficients) -- SpMV s + 4 coefficients + z = 24; x/r update x, s,
     # r, z read + x, r written = 24; s update z, s read + s written = 12
-    vec_ms = [sum(s_["ms_vec"][k] for _, s_ in stats) for k in range(3)]
-    vec_n = [sum(s_["vec_launches"][k] for _, s_ in stats) for k in range(3)]
+    vec_ms = [sum(s_["ms_vec"][k] for s_ in ev_stats) for k in range(3)]
+    vec_n = [sum(s_["vec_launches"][k] for s_ in ev_stats) for k in range(3)]
     vk = {}
     for k, (name, bpr) in enumerate((("spmv_dot", 24.0), ("update_xr", 24.0), ("update_s", 12.0))):
         if vec_n[k] > 0 and vec_ms[k] > 0:
@@ -1018,12 +1034,6 @@ def particles_leg(stream, barrier, max_over_ranks, cpu=True):
 
 
 def main():
-    # The roofline's solve and vector-kernel durations come from CUDA events on
-    # every 16th PCG iteration of the timed projections, the preconditioner's
-    # first solve pair included (the library records none by default: an
-    # event between two launches serialises them, and events on every launch
-    # cost 6 % of a projection).
-    os.environ.setdefault("XFP_KERNEL_EVENTS", "16")
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=25)
