@@ -71,16 +71,18 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S)
   }
   const long long nlines = line_base[n], nblk = blk_base[n];
   XFP_CUDA(ctx, B->lines.ensure(nlines * sizeof(Line)));
-  XFP_CUDA(ctx, ctx->line_sums.ensure(3 * LINE_CHUNKS * sizeof(long long)));
+  XFP_CUDA(ctx, ctx->line_sums.ensure((size_t)std::min(n, LAYOUT_SCENES) * 3 * LINE_CHUNKS * sizeof(long long)));
   XFP_CUDA(ctx, ctx->blks.ensure((size_t)nblk * sizeof(WBlk)));
   XFP_CUDA(ctx, B->scene_tile_lists.ensure((size_t)nblk * sizeof(int2)));
   XFP_CUDA(ctx, B->counters.ensure((size_t)n * 5 * sizeof(long long)));
   Line* lines = B->lines.as<Line>();
-  for (int s = 0; s < n; ++s) {
-    LayoutDev L{lines + line_base[s], ctx->line_sums.as<long long>(), ctx->blks.as<WBlk>() + blk_base[s],
-                B->scene_tile_lists.as<int2>() + blk_base[s], B->counters.as<long long>() + 5 * s};
-    XFP_CUDA(ctx, layout_build(S[s].mat, S[s].ni, S[s].nj, S[s].nk, L, st));
-  }
+  std::vector<LayoutScene> layouts(n);
+  for (int s = 0; s < n; ++s)   // (the scratch is a launch's own)
+    layouts[s] = {S[s].mat, S[s].ni, S[s].nj, S[s].nk, lines + line_base[s],
+                  ctx->line_sums.as<long long>() + (size_t)(s % LAYOUT_SCENES) * 3 * LINE_CHUNKS,
+                  ctx->blks.as<WBlk>() + blk_base[s], B->scene_tile_lists.as<int2>() + blk_base[s],
+                  B->counters.as<long long>() + 5 * s};
+  XFP_CUDA(ctx, layout_build(layouts.data(), n, st));
   std::vector<long long> cnt((size_t)n * 5);
   std::vector<int2> all_tiles((size_t)nblk);
   XFP_CUDA(ctx, cudaMemcpyAsync(cnt.data(), B->counters.p, cnt.size() * sizeof(long long), cudaMemcpyDeviceToHost,
@@ -101,20 +103,16 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S)
   }
   if (base[n] >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "batch too large: more than 2^31 stored cells");
   if (group_base[n] * 256 >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "batch too large for the sweep layout");
-  for (int s = 0; s < n; ++s)
-    XFP_CUDA(ctx, offset_lines(lines + line_base[s], line_base[s + 1] - line_base[s], base[s], st));
   // group -> line index (line numbers local to each scene's table; cells
   // global) and group -> sweep element
   XFP_CUDA(ctx, ctx->group_line.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->gperm.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->group_nb.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(GroupNb)));
-  for (int s = 0; s < n; ++s) {
-    XFP_CUDA(ctx, build_group_tables(lines + line_base[s], S[s].nj, S[s].nk, ctx->group_line.as<int>(),
-                                     ctx->group_nb.as<GroupNb>(), st));
-    XFP_CUDA(ctx, gperm_build(ctx->group_line.as<int>() + base[s] / 4, lines + line_base[s], S[s].nj,
-                              ctx->blks.as<WBlk>() + blk_base[s], (S[s].nj + 7) / 8, base[s + 1] - base[s], base[s],
-                              group_base[s], ctx->gperm.as<int>() + base[s] / 4, st));
-  }
+  std::vector<TableScene> tables(n);
+  for (int s = 0; s < n; ++s)
+    tables[s] = {lines + line_base[s], ctx->blks.as<WBlk>() + blk_base[s], S[s].nj, S[s].nk, base[s], group_base[s]};
+  XFP_CUDA(ctx, layout_tables(tables.data(), n, ctx->group_line.as<int>(), ctx->group_nb.as<GroupNb>(),
+                              ctx->gperm.as<int>(), st));
   // merge the scenes' block lists by wavefront level (each list is already in
   // its own topological order, which the merge keeps)
   long long ntl = 0;

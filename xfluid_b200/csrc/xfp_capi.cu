@@ -58,9 +58,9 @@ int build_layout(xfp_ctx* ctx, const uint8_t* dmat, int ni, int nj, int nk) {
   XFP_CUDA(ctx, ctx->blks.ensure((size_t)NJB * NKB * sizeof(WBlk)));
   XFP_CUDA(ctx, ctx->tiles.ensure((size_t)NJB * NKB * sizeof(int2)));
   XFP_CUDA(ctx, ctx->counters.ensure(5 * sizeof(long long)));
-  LayoutDev L{ctx->lines.as<Line>(), ctx->line_sums.as<long long>(), ctx->blks.as<WBlk>(), ctx->tiles.as<int2>(),
-              ctx->counters.as<long long>()};
-  XFP_CUDA(ctx, layout_build(dmat, ni, nj, nk, L, ctx->stream));
+  const LayoutScene L{dmat, ni, nj, nk, ctx->lines.as<Line>(), ctx->line_sums.as<long long>(), ctx->blks.as<WBlk>(),
+                      ctx->tiles.as<int2>(), ctx->counters.as<long long>()};
+  XFP_CUDA(ctx, layout_build(&L, 1, ctx->stream));
   long long cnt[5];
   XFP_CUDA(ctx, cudaMemcpyAsync(cnt, ctx->counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, ctx->stream));
   XFP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -72,10 +72,9 @@ int build_layout(xfp_ctx* ctx, const uint8_t* dmat, int ni, int nj, int nk) {
   XFP_CUDA(ctx, ctx->group_line.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->gperm.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->group_nb.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(GroupNb)));
-  XFP_CUDA(ctx, build_group_tables(ctx->lines.as<Line>(), nj, nk, ctx->group_line.as<int>(), ctx->group_nb.as<GroupNb>(),
-                                   ctx->stream));
-  XFP_CUDA(ctx, gperm_build(ctx->group_line.as<int>(), ctx->lines.as<Line>(), nj, ctx->blks.as<WBlk>(), NJB, ctx->M, 0,
-                            0, ctx->gperm.as<int>(), ctx->stream));
+  const TableScene T{ctx->lines.as<Line>(), ctx->blks.as<WBlk>(), nj, nk, 0, 0};
+  XFP_CUDA(ctx, layout_tables(&T, 1, ctx->group_line.as<int>(), ctx->group_nb.as<GroupNb>(), ctx->gperm.as<int>(),
+                              ctx->stream));
   return XFP_OK;
 }
 

@@ -72,10 +72,6 @@ cudaError_t wave_prepare();
 // bytes (the factorisation's FP64 pair), 32 payload bits a word
 constexpr size_t WAVE_EDGE = 4 * 8 * 4;
 
-// gperm[q] = sweep element of line-layout group q's first cell (M stored cells
-// from cell_base on; group_line of those cells, their scene's lines and blocks)
-cudaError_t gperm_build(const int* group_line, const Line* lines, int nj, const WBlk* blks, int NJB, long long M,
-                        long long cell_base, long long group_base, int* gperm, cudaStream_t st);
 // dir 0: sw[wave_value(gperm)] = line; dir 1: the way back, for the M stored cells.
 template <typename T>
 cudaError_t sw_permute(T* line, T* sw, const int* gperm, long long M, int dir, cudaStream_t st);
@@ -89,14 +85,28 @@ cudaError_t factor_lines(const T* fac, const Line* lines, int nj, int nk, const 
 // material grid.  counters (device): stored cells M, unknown rows, active
 // lines, active tiles, sweep-layout groups.
 constexpr int LINE_CHUNKS = 1024;
-struct LayoutDev {
+constexpr int LAYOUT_SCENES = 16;   // grids a launch of the layout kernels takes
+struct LayoutScene {
+  const uint8_t* mat;
+  int ni, nj, nk;
   Line* lines;               // [nk*nj]
   long long* sums;           // scratch [3 * LINE_CHUNKS]
   WBlk* blks;                // [ceil(nk/8) * ceil(nj/8)]
   int2* tiles;               // active tiles (at most as many as blocks)
   long long* counters;       // [5]
 };
-cudaError_t layout_build(const uint8_t* mat, int ni, int nj, int nk, LayoutDev L, cudaStream_t st);
+cudaError_t layout_build(const LayoutScene* scenes, int n, cudaStream_t st);
+// Per aligned 4-cell group: the line that stores it, its neighbours and its place in
+// the sweep layout; the grids' cells follow one another from `base` on, their groups of
+// the sweep layout from group_base on.  Line offsets are made global.
+struct TableScene {
+  Line* lines;
+  const WBlk* blks;
+  int nj, nk;
+  long long base, group_base;
+};
+cudaError_t layout_tables(const TableScene* scenes, int n, int* group_line, GroupNb* group_nb, int* gperm,
+                          cudaStream_t st);
 
 // ---- assembly / apply / vector kernels (xfp_ops.cu) ----
 template <typename FT, typename AT>
@@ -154,8 +164,6 @@ cudaError_t spmv_dot(const AT* diag, const AT* ax, const AT* ay, const AT* az, c
                      cudaStream_t st);
 // SpMV blocks for M stored cells (the batch gives each scene the same count).
 long long spmv_block_count(long long M, int nblk_max);
-// Per aligned 4-cell group (c / 4): the line that stores it and its neighbours.
-cudaError_t build_group_tables(const Line* lines, int nj, int nk, int* group_line, GroupNb* group_nb, cudaStream_t st);
 // rsw/gperm (optional): the updated r is also stored at rsw[wave_value(gperm[c / 4])].
 template <typename VT, typename DT>
 cudaError_t update_xr(VT* x, VT* r, const VT* s, const VT* z, long long M, PcgScalars* sc,
@@ -212,9 +220,6 @@ cudaError_t advect_adjoint(const T* u, const T* v, const T* w, const T* gu, cons
 template <typename T>
 cudaError_t box_loss(const T* u, const T* v, const T* w, T* gu, T* gv, T* gw, int ni, int nj, int nk,
                      const double box[6], double* loss, cudaStream_t st);
-
-// Adds base[s] to the offsets of scene s's line table.
-cudaError_t offset_lines(Line* lines, long long nlines, long long base, cudaStream_t st);
 
 // Mixed precision: r64 = b64 - A64 x64, |r|_inf and r32 = (float) r64 / scale.
 cudaError_t residual64(const double* diag, const double* ax, const double* ay, const double* az, const double* b,

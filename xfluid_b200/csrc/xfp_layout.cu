@@ -29,9 +29,19 @@ __device__ __forceinline__ bool is_unknown(const uint8_t* mat, int ni, int nj, i
   return false;
 }
 
+// The layout kernels take up to LAYOUT_SCENES grids a launch, blockIdx.y being the
+// grid: a batch of 12 took 60 launches of 2 to 6 us for its line and block tables, and
+// 36 for its group tables.
+struct LayoutSet {
+  LayoutScene s[LAYOUT_SCENES];
+};
+
 // One warp per x-line: span of unknowns and their count.
-__global__ void line_span_kernel(const uint8_t* __restrict__ mat, int ni, int nj, int nk,
-                                 Line* __restrict__ lines) {
+__global__ void line_span_kernel(const __grid_constant__ LayoutSet set) {
+  const LayoutScene& G = set.s[blockIdx.y];
+  const uint8_t* __restrict__ mat = G.mat;
+  const int ni = G.ni, nj = G.nj, nk = G.nk;
+  Line* __restrict__ lines = G.lines;
   const int lane = threadIdx.x & 31;
   const long long line = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (line >= (long long)nj * nk) return;
@@ -89,10 +99,17 @@ __device__ __forceinline__ long long scan1024(long long v, long long* sh) {
 // launches of at most LINE_CHUNKS CTAs with a chunk of lines each: every chunk's
 // sums, then the scan, each CTA adding up the chunks before its own.  (One CTA
 // alone took 65 us for the 16,384 lines of 128^3 and 155 us at 256^3; now 8 us.)
-__global__ void __launch_bounds__(1024) line_sum_kernel(const Line* __restrict__ lines, long long nlines,
-                                                        long long chunk, long long* __restrict__ sums) {
+__device__ __forceinline__ long long line_chunk(long long nlines) {
+  return max(1024LL, (nlines + LINE_CHUNKS - 1) / LINE_CHUNKS);
+}
+__global__ void __launch_bounds__(1024) line_sum_kernel(const __grid_constant__ LayoutSet set) {
   __shared__ long long sh[32];
+  const LayoutScene& G = set.s[blockIdx.y];
+  const Line* __restrict__ lines = G.lines;
+  long long* __restrict__ sums = G.sums;
+  const long long nlines = (long long)G.nj * G.nk, chunk = line_chunk(nlines);
   const long long a = blockIdx.x * chunk, b = min(a + chunk, nlines);
+  if (a >= nlines) return;
   long long v[3] = {0, 0, 0};   // cells, rows, active lines
   for (long long l = a + threadIdx.x; l < b; l += 1024) {
     const Line L = lines[l];
@@ -106,14 +123,19 @@ __global__ void __launch_bounds__(1024) line_sum_kernel(const Line* __restrict__
     if (threadIdx.x == 1023) sums[n * LINE_CHUNKS + blockIdx.x] = t;
   }
 }
-__global__ void __launch_bounds__(1024) line_scan_kernel(Line* __restrict__ lines, long long nlines, long long chunk,
-                                                         const long long* __restrict__ sums,
-                                                         long long* __restrict__ counters) {
+__global__ void __launch_bounds__(1024) line_scan_kernel(const __grid_constant__ LayoutSet set) {
   __shared__ long long sh[32];
   __shared__ long long s_tot;
+  const LayoutScene& G = set.s[blockIdx.y];
+  Line* __restrict__ lines = G.lines;
+  const long long* __restrict__ sums = G.sums;
+  long long* __restrict__ counters = G.counters;
+  const long long nlines = (long long)G.nj * G.nk, chunk = line_chunk(nlines);
+  const unsigned chunks = (unsigned)((nlines + chunk - 1) / chunk);
   const long long a = blockIdx.x * chunk, b = min(a + chunk, nlines);
-  auto total = [&](int n, unsigned chunks) {   // of the first chunks (at most 1024)
-    const long long t = scan1024(threadIdx.x < chunks ? sums[n * LINE_CHUNKS + threadIdx.x] : 0, sh);
+  if (a >= nlines) return;
+  auto total = [&](int n, unsigned first) {   // of the first chunks (at most 1024)
+    const long long t = scan1024(threadIdx.x < first ? sums[n * LINE_CHUNKS + threadIdx.x] : 0, sh);
     if (threadIdx.x == 1023) s_tot = t;
     __syncthreads();
     const long long r = s_tot;
@@ -131,8 +153,8 @@ __global__ void __launch_bounds__(1024) line_scan_kernel(Line* __restrict__ line
     carry += s_tot;
     __syncthreads();
   }
-  if (blockIdx.x + 1 != gridDim.x) return;
-  const long long rows = total(1, gridDim.x), act = total(2, gridDim.x);
+  if (blockIdx.x + 1 != chunks) return;
+  const long long rows = total(1, chunks), act = total(2, chunks);
   if (threadIdx.x == 0) {
     counters[0] = carry;
     counters[1] = rows;
@@ -142,8 +164,12 @@ __global__ void __launch_bounds__(1024) line_scan_kernel(Line* __restrict__ line
 
 // Sweep-layout blocks: one warp per block of 8 x 8 lines finds the span of
 // wavefront groups its cells cover (goff is scanned afterwards).
-__global__ void blk_span_kernel(const Line* __restrict__ lines, int nj, int nk, int NJB, long long nblk,
-                                WBlk* __restrict__ blks) {
+__global__ void blk_span_kernel(const __grid_constant__ LayoutSet set) {
+  const LayoutScene& G = set.s[blockIdx.y];
+  const Line* __restrict__ lines = G.lines;
+  WBlk* __restrict__ blks = G.blks;
+  const int nj = G.nj, nk = G.nk, NJB = (nj + 7) / 8;
+  const long long nblk = (long long)NJB * ((nk + 7) / 8);
   const int lane = threadIdx.x & 31;
   const long long b = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (b >= nblk) return;
@@ -173,11 +199,16 @@ __global__ void blk_span_kernel(const Line* __restrict__ lines, int nj, int nk, 
 }
 
 // Block offsets (scan in block order) and the active tiles in topological
-// order of the lower sweep: (J+K) ascending, then J.  One CTA.
-__global__ void __launch_bounds__(1024) blk_scan_kernel(WBlk* __restrict__ blks, int NJB, int NKB, int NJT, int NKT,
-                                                        int2* __restrict__ tiles, long long* __restrict__ counters) {
+// order of the lower sweep: (J+K) ascending, then J.  One CTA per grid.
+__global__ void __launch_bounds__(1024) blk_scan_kernel(const __grid_constant__ LayoutSet set) {
   __shared__ long long sh[32];
   __shared__ long long s_tot;
+  const LayoutScene& G = set.s[blockIdx.y];
+  WBlk* __restrict__ blks = G.blks;
+  int2* __restrict__ tiles = G.tiles;
+  long long* __restrict__ counters = G.counters;
+  const int NJB = (G.nj + 7) / 8, NKB = (G.nk + 7) / 8;
+  const int NJT = (NJB + WAVE_TJ - 1) / WAVE_TJ, NKT = (NKB + WAVE_TK - 1) / WAVE_TK;
   const long long nblk = (long long)NJB * NKB, ntile = (long long)NJT * NKT;
   long long carry = 0;
   for (long long base = 0; base < nblk; base += 1024) {
@@ -227,25 +258,104 @@ __global__ void __launch_bounds__(1024) blk_scan_kernel(WBlk* __restrict__ blks,
   if (threadIdx.x == 0) counters[3] = carry;
 }
 
-cudaError_t layout_build(const uint8_t* mat, int ni, int nj, int nk, LayoutDev L, cudaStream_t st) {
+// For the aligned 4-cell group of cell c, at c / 4 (cells counted over all grids):
+// its line (index in its grid's table; lines start at multiples of 4 and hold
+// multiples of 4 cells), where its y and z neighbours are, and the sweep element of
+// its first cell (its four cells are four consecutive elements).
+struct TableSet {
+  TableScene s[LAYOUT_SCENES];
+};
+__global__ void group_tables_kernel(const __grid_constant__ TableSet set, int* __restrict__ group_line,
+                                    GroupNb* __restrict__ group_nb, int* __restrict__ gperm) {
+  const TableScene& G = set.s[blockIdx.y];
+  const Line* __restrict__ lines = G.lines;
+  const int nj = G.nj, nk = G.nk;
+  const int lane = threadIdx.x & 31;
   const long long nlines = (long long)nj * nk;
-  const int wpb = 8;
-  ++g_kernel_launches;
-  line_span_kernel<<<(unsigned)((nlines + wpb - 1) / wpb), wpb * 32, 0, st>>>(mat, ni, nj, nk, L.lines);
-  const long long chunk = std::max<long long>(1024, (nlines + LINE_CHUNKS - 1) / LINE_CHUNKS);
-  const unsigned chunks = (unsigned)((nlines + chunk - 1) / chunk);
-  ++g_kernel_launches;
-  line_sum_kernel<<<chunks, 1024, 0, st>>>(L.lines, nlines, chunk, L.sums);
-  ++g_kernel_launches;
-  line_scan_kernel<<<chunks, 1024, 0, st>>>(L.lines, nlines, chunk, L.sums, L.counters);
-  const int NJB = (nj + 7) / 8, NKB = (nk + 7) / 8;
-  const long long nblk = (long long)NJB * NKB;
-  ++g_kernel_launches;
-  blk_span_kernel<<<(unsigned)((nblk + wpb - 1) / wpb), wpb * 32, 0, st>>>(L.lines, nj, nk, NJB, nblk, L.blks);
-  ++g_kernel_launches;
-  blk_scan_kernel<<<1, 1024, 0, st>>>(L.blks, NJB, NKB, (NJB + WAVE_TJ - 1) / WAVE_TJ, (NKB + WAVE_TK - 1) / WAVE_TK,
-                                      L.tiles, L.counters);
-  return cudaGetLastError();
+  for (long long line = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); line < nlines;
+       line += (long long)gridDim.x * (blockDim.x >> 5)) {
+    const Line L = lines[line];
+    if (L.len == 0) continue;
+    const int j = (int)(line % nj), k = (int)(line / nj);
+    const Line Z = {0, 0, 0, 0};
+    const Line N[4] = {j > 0 ? lines[line - 1] : Z, j + 1 < nj ? lines[line + 1] : Z, k > 0 ? lines[line - nj] : Z,
+                       k + 1 < nk ? lines[line + nj] : Z};
+    const WBlk b = G.blks[(size_t)(k >> 3) * ((nj + 7) / 8) + (j >> 3)];
+    for (int q = lane; q < (L.len >> 2); q += 32) {
+      const size_t at = ((size_t)(G.base + L.off) >> 2) + q;
+      unsigned nb[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        // the neighbour of the group's first cell; the quad after the one that
+        // holds it, and whether the line stores either
+        const int r = L.lo + 4 * q - N[n].lo;
+        const int quad = (r >> 2) + 1;
+        nb[n] = ((unsigned)(((G.base + N[n].off) >> 2) + quad) << 2) |
+                ((unsigned)(r & ~3) < (unsigned)N[n].len ? 1u : 0u) | ((unsigned)(4 * quad) < (unsigned)N[n].len ? 2u : 0u);
+      }
+      const int t = L.lo + 4 * q + j + k;
+      group_line[at] = (int)line;
+      group_nb[at] = {nb[0], nb[1], nb[2], nb[3]};
+      gperm[at] = (int)((G.group_base + b.goff + (t >> 2) - b.g0) * 256 + wave_line_slot(j, k));
+    }
+  }
+}
+// Adds every grid's base to the offsets of its lines.
+__global__ void offset_lines_kernel(const __grid_constant__ TableSet set) {
+  const TableScene& G = set.s[blockIdx.y];
+  const long long nlines = (long long)G.nj * G.nk;
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nlines; q += (long long)gridDim.x * blockDim.x)
+    G.lines[q].off += (int)G.base;
+}
+
+cudaError_t layout_build(const LayoutScene* scenes, int n, cudaStream_t st) {
+  for (int first = 0; first < n; first += LAYOUT_SCENES) {
+    LayoutSet set = {};
+    const unsigned m = (unsigned)std::min(LAYOUT_SCENES, n - first);
+    long long nlines = 0, nblk = 0, chunks = 0;
+    for (unsigned q = 0; q < m; ++q) {
+      const LayoutScene& G = set.s[q] = scenes[first + q];
+      const long long l = (long long)G.nj * G.nk, chunk = std::max<long long>(1024, (l + LINE_CHUNKS - 1) / LINE_CHUNKS);
+      nlines = std::max(nlines, l);
+      chunks = std::max(chunks, (l + chunk - 1) / chunk);
+      nblk = std::max(nblk, (long long)((G.nj + 7) / 8) * ((G.nk + 7) / 8));
+    }
+    const int wpb = 8;
+    g_kernel_launches += 5;
+    line_span_kernel<<<dim3((unsigned)((nlines + wpb - 1) / wpb), m), wpb * 32, 0, st>>>(set);
+    line_sum_kernel<<<dim3((unsigned)chunks, m), 1024, 0, st>>>(set);
+    line_scan_kernel<<<dim3((unsigned)chunks, m), 1024, 0, st>>>(set);
+    blk_span_kernel<<<dim3((unsigned)((nblk + wpb - 1) / wpb), m), wpb * 32, 0, st>>>(set);
+    blk_scan_kernel<<<dim3(1, m), 1024, 0, st>>>(set);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t layout_tables(const TableScene* scenes, int n, int* group_line, GroupNb* group_nb, int* gperm,
+                          cudaStream_t st) {
+  for (int first = 0; first < n; first += LAYOUT_SCENES) {
+    TableSet set = {};
+    const unsigned m = (unsigned)std::min(LAYOUT_SCENES, n - first);
+    long long nlines = 0;
+    bool offset = false;
+    for (unsigned q = 0; q < m; ++q) {
+      set.s[q] = scenes[first + q];
+      nlines = std::max(nlines, (long long)set.s[q].nj * set.s[q].nk);
+      offset |= set.s[q].base != 0;
+    }
+    ++g_kernel_launches;
+    group_tables_kernel<<<dim3((unsigned)std::min<long long>((nlines + 7) / 8, 65535LL * 8), m), 256, 0, st>>>(
+        set, group_line, group_nb, gperm);
+    if (offset) {
+      ++g_kernel_launches;
+      offset_lines_kernel<<<dim3((unsigned)std::min<long long>((nlines + 255) / 256, 148LL * 8), m), 256, 0, st>>>(set);
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace xfp

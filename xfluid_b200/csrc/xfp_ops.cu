@@ -1165,47 +1165,6 @@ template cudaError_t batch_spmv_dot<float, float, double>(const BatchSeg*, int, 
                                                           const float*, const float*, const float*, float*,
                                                           const GroupNb*, PcgScalars*, int, cudaStream_t);
 
-// For the aligned 4-cell group of cell c, at c / 4: its line (index in its scene's
-// table; lines start at multiples of 4 and hold multiples of 4 cells) and where
-// its y and z neighbours are.
-__global__ void group_tables_kernel(const Line* __restrict__ lines, int nj, int nk, int* __restrict__ group_line,
-                                    GroupNb* __restrict__ group_nb) {
-  const int lane = threadIdx.x & 31;
-  const long long nlines = (long long)nj * nk;
-  for (long long line = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); line < nlines;
-       line += (long long)gridDim.x * (blockDim.x >> 5)) {
-    const Line L = lines[line];
-    if (L.len == 0) continue;
-    const int j = (int)(line % nj), k = (int)(line / nj);
-    const Line Z = {0, 0, 0, 0};
-    const Line N[4] = {j > 0 ? lines[line - 1] : Z, j + 1 < nj ? lines[line + 1] : Z, k > 0 ? lines[line - nj] : Z,
-                       k + 1 < nk ? lines[line + nj] : Z};
-    for (int q = lane; q < (L.len >> 2); q += 32) {
-      const size_t at = ((size_t)L.off >> 2) + q;
-      unsigned nb[4];
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        // the neighbour of the group's first cell; the quad after the one that
-        // holds it, and whether the line stores either
-        const int r = L.lo + 4 * q - N[n].lo;
-        const int quad = (r >> 2) + 1;
-        nb[n] = ((unsigned)((N[n].off >> 2) + quad) << 2) | ((unsigned)(r & ~3) < (unsigned)N[n].len ? 1u : 0u) |
-                ((unsigned)(4 * quad) < (unsigned)N[n].len ? 2u : 0u);
-      }
-      group_line[at] = (int)line;
-      group_nb[at] = {nb[0], nb[1], nb[2], nb[3]};
-    }
-  }
-}
-cudaError_t build_group_tables(const Line* lines, int nj, int nk, int* group_line, GroupNb* group_nb, cudaStream_t st) {
-  const long long nlines = (long long)nj * nk;
-  if (nlines <= 0) return cudaSuccess;
-  ++g_kernel_launches;
-  group_tables_kernel<<<(unsigned)std::min<long long>((nlines + 7) / 8, 65535LL * 8), 256, 0, st>>>(
-      lines, nj, nk, group_line, group_nb);
-  return cudaGetLastError();
-}
-
 template <typename VT>
 cudaError_t batch_update_xr(const BatchSeg* segs, int nseg, int blocks, VT* x, VT* r, const VT* s,
                             const VT* z, PcgScalars* sc, cudaStream_t st, VT* rsw, const int* gperm) {
@@ -1274,19 +1233,6 @@ cudaError_t batch_bwd_reduce(const BatchSeg* segs, int nseg, const double* line_
 }
 template cudaError_t batch_bwd_reduce<double>(const BatchSeg*, int, const double*, PcgScalars*, int, cudaStream_t);
 template cudaError_t batch_bwd_reduce<float>(const BatchSeg*, int, const double*, PcgScalars*, int, cudaStream_t);
-
-__global__ void offset_lines_kernel(Line* __restrict__ lines, long long nlines, long long base) {
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nlines;
-       q += (long long)gridDim.x * blockDim.x)
-    lines[q].off += (int)base;
-}
-cudaError_t offset_lines(Line* lines, long long nlines, long long base, cudaStream_t st) {
-  if (base == 0 || nlines <= 0) return cudaSuccess;
-  ++g_kernel_launches;
-  offset_lines_kernel<<<(unsigned)std::min<long long>((nlines + 255) / 256, 148LL * 8), 256, 0, st>>>(lines, nlines,
-                                                                                                   base);
-  return cudaGetLastError();
-}
 
 __global__ void refine_update_kernel(double* __restrict__ x64, const float* __restrict__ e32, long long M) {
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < M; c += (long long)gridDim.x * blockDim.x)

@@ -930,22 +930,6 @@ cudaError_t launch(const WaveArgs& g, cudaStream_t st) {
   return cudaLaunchKernelEx(&L.cfg, wave_kernel<OP, VT, CT>, g);
 }
 
-// gperm[q] = sweep element of the first cell of line-layout group q (four
-// consecutive cells of a line are four consecutive elements)
-__global__ void gperm_kernel(const int* __restrict__ group_line, const Line* __restrict__ lines, int nj,
-                             const WBlk* __restrict__ blks, int NJB, long long ngroups, long long cell_base,
-                             long long group_base, int* __restrict__ gperm) {
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < ngroups;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int l = group_line[q];
-    const int j = l % nj, k = l / nj;
-    const Line L = lines[l];
-    const int t = L.lo + (int)(cell_base + 4 * q - L.off) + j + k;
-    const WBlk b = blks[(size_t)(k >> 3) * NJB + (j >> 3)];
-    gperm[q] = (int)((group_base + b.goff + (t >> 2) - b.g0) * GE + wave_line_slot(j, k));
-  }
-}
-
 // one thread per group of 4 cells: dir 0 line -> sweep, dir 1 sweep -> line
 template <typename T>
 __global__ void sw_permute_kernel(T* __restrict__ line, T* __restrict__ sw, const int* __restrict__ gperm,
@@ -1018,15 +1002,6 @@ template cudaError_t wave_prepare<float, double>();
 template cudaError_t wave_launch<double, double>(int, const WaveArgs&, cudaStream_t);
 template cudaError_t wave_launch<float, float>(int, const WaveArgs&, cudaStream_t);
 template cudaError_t wave_launch<float, double>(int, const WaveArgs&, cudaStream_t);
-
-cudaError_t gperm_build(const int* group_line, const Line* lines, int nj, const WBlk* blks, int NJB, long long M,
-                        long long cell_base, long long group_base, int* gperm, cudaStream_t st) {
-  if (M <= 0) return cudaSuccess;
-  ++g_kernel_launches;
-  gperm_kernel<<<cap_blocks(M / 4), 256, 0, st>>>(group_line, lines, nj, blks, NJB, M / 4, cell_base, group_base,
-                                                  gperm);
-  return cudaGetLastError();
-}
 
 template <typename T>
 cudaError_t sw_permute(T* line, T* sw, const int* gperm, long long M, int dir, cudaStream_t st) {
