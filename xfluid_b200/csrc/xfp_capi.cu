@@ -10,6 +10,7 @@
 // Mixed precision wraps the FP32 PCG in FP64 iterative refinement.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -178,10 +179,10 @@ int sweep_error(xfp_ctx* ctx, const SweepCtl& c) {
              "device wait timed out (site %u, op %d, tile %d, step %d, thread %d, ntiles %lld, seen %016llx, "
              "expect %08x)",
              c.err_where, c.err_op, c.err_tile, c.err_tau, c.err_thread, ctx->ntiles, c.err_word, c.err_expect);
-    // clear so the context stays usable
-    SweepCtl z{};
-    z.gen = c.gen;
-    cudaMemcpyAsync(ctx->ctl.p, &z, sizeof(z), cudaMemcpyHostToDevice, ctx->stream);
+    // clear so the context stays usable: all but the generation, which launches
+    // that ran beside the read have advanced since (their stamps must not come again)
+    constexpr size_t keep = offsetof(SweepCtl, finished);
+    cudaMemsetAsync(static_cast<char*>(ctx->ctl.p) + keep, 0, sizeof(SweepCtl) - keep, ctx->stream);
     cudaStreamSynchronize(ctx->stream);
     return fail(ctx, XFP_ERR_TIMEOUT, buf);
   }
