@@ -86,7 +86,12 @@ namespace xfp {
 namespace {
 
 constexpr int GE = 256;   // cells of one block's group: 64 lines x 4 steps
-constexpr int FB = 4;     // groups of edge words a courier has under way per far edge
+// Groups of edge words a courier has under way per far edge.  Two cover a load's
+// way to L2 and back at a group's pace; every further one only lengthens a poll
+// and the queue of all couriers' polls.  Whole projections in ms with 1 / 2 / 3 / 4 /
+// 6: 128^3 FP64 8.60 8.51 8.63 8.72 9.11, 256^3 mixed 11.1 9.98 9.94 10.1 10.3,
+// 150 x 97 x 131 mixed 9.64 8.82 8.84 8.90 9.01.
+constexpr int FB = 2;
 
 // What a block hands to a neighbour per line and step (X): the factorisation
 // sends L(m,c) and the sum of the column's other two entries (the dropped
@@ -703,6 +708,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
         for (int d = 0; d < FB; ++d)
           if (use && f.u + d <= f.last && !f.w[d].ready(want)) f.w[d].load(src + (size_t)(f.u + d + a) * 32 * P);
       };
+      int room = S;   // (with a look at `freed` for every group: 128^3 FP64 8.43 ms against 8.35)
       auto forward = [&](Far& f, unsigned to, bool use) -> bool {
         bool moved = false;
 #pragma unroll
@@ -711,8 +717,10 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
           const unsigned at = (unsigned)f.u & (S - 1);
           // its slot is free once group u - S is done with (one lane's look, so
           // that all lanes agree; a count, since the courier may be any number
-          // of groups ahead, where a parity would be ambiguous)
-          if (f.u >= __shfl_sync(XFP_FULL, ld_acquire_s32(&sh.freed), 0) + S) break;
+          // of groups ahead, where a parity would be ambiguous); looked at again only
+          // when the last count is used up
+          if (f.u >= room) room = __shfl_sync(XFP_FULL, ld_acquire_s32(&sh.freed), 0) + S;
+          if (f.u >= room) break;
           if (use) {
             uint32_t w[P];
             to_words(f.w[0].value(), w);
