@@ -61,8 +61,8 @@
 // chunks (one CTA alone reads 65,536 partials at 256^3).
 //
 // Measured (device time of a launch, full box of 128^3 / 256^3 cells): a solve
-// takes 62 / 164 us in FP32 and 92 / 290 us in FP64, the factorisation 0.24 / 0.68
-// ms; a launch costs 12 us to start and end, a group of four steps of a lone block
+// takes 62 / 159 us in FP32 and 90 / 285 us in FP64, the factorisation 0.21 / 0.64
+// ms (FP64 0.22 / 0.69); a launch costs 12 us to start and end, a group of four steps of a lone block
 // 0.25 (0.36) us, of which the steps are 0.13 (0.2) and the rest is waiting for a
 // slot, reading it and handing it on.
 // With the compute warp sending its edges and storing its results, as the
