@@ -81,6 +81,7 @@
 #include <climits>
 
 #include "xfp_sweep_util.cuh"
+#include "xfp_warp_wait.h"
 
 namespace xfp {
 namespace {
@@ -397,17 +398,20 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
 
     auto parity_q = [&](int q) { return ((phase_q >> (q & (S - 1))) ^ (unsigned)(q >> LS)) & 1u; };
     auto parity_u = [&](int u) { return ((phase_u >> (u & (S - 1))) ^ (unsigned)(u >> LS)) & 1u; };
-    // waits for the phase of a mbarrier that another warp of this unit completes
-    // (whose own waits are bounded; this one outlasts them); false: it gave up
-    auto await = [&](unsigned long long* bar, int q, unsigned site) -> bool {
-      const unsigned b = smem_u32(bar), parity = parity_q(q);
-      if (__all_sync(XFP_FULL, mbar_try(b, parity))) return true;
+    // waits for a mbarrier's phase, all lanes together (a lane's own look may be
+    // ahead of another's, and full-warp shuffles follow); false: it gave up
+    auto vote = [](bool v) { return __all_sync(XFP_FULL, v) != 0; };
+    auto phase_of = [&](unsigned long long* bar, unsigned parity, long long limit, int n, unsigned site) -> bool {
+      const unsigned b = smem_u32(bar);
       Spin sp;
-      while (!mbar_try(b, parity) && sp.step(g.ctl, 8 * g.spin_limit)) {
-      }
-      if (__all_sync(XFP_FULL, mbar_try(b, parity))) return true;
-      raise_timeout(g.ctl, site, tpos, q, OP, 0ull, parity);
+      if (warp_wait([&] { return mbar_try(b, parity); }, vote, [&] { return sp.step(g.ctl, limit); })) return true;
+      raise_timeout(g.ctl, site, tpos, n, OP, 0ull, parity);
       return false;
+    };
+    // ... one that another warp of this unit completes (whose own waits are
+    // bounded; this one outlasts them)
+    auto await = [&](unsigned long long* bar, int q, unsigned site) -> bool {
+      return phase_of(bar, parity_q(q), 8 * g.spin_limit, q, site);
     };
     // z.r of this lane's line h of the block
     auto put_dot = [&](int h, const LineDot<VT, DOT32>& d) {
@@ -444,19 +448,8 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
       // ends (its helper finds the error flag), and the host reports the timeout
       bool bad = false;
       auto wait = [&](unsigned long long* bar, unsigned parity, unsigned site, int n) {
-        const unsigned b = smem_u32(bar);
-        if (mbar_try(b, parity)) return;
-        Spin sp;
-        bool gave_up = false;
-        while (!mbar_try(b, parity)) {
-          if (!sp.step(g.ctl, g.spin_limit)) {
-            raise_timeout(g.ctl, site, tpos, n, OP, 0ull, parity);
-            *(volatile int*)&sh.broken = 1;
-            gave_up = true;
-            break;
-          }
-        }
-        bad = __any_sync(XFP_FULL, gave_up);
+        bad = !phase_of(bar, parity, g.spin_limit, n, site);
+        if (bad) *(volatile int*)&sh.broken = 1;
       };
       X ej[HL][4], ek[4];        // the producers' values of the group, in sweep order
       auto take_edges = [&](int u) {   // (zero where a producer has no such group: the helper's work)
@@ -573,16 +566,16 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
         if constexpr (FACTOR) {
           // ---- edge values to the upper neighbours ----
           if (q >= room) {
-            // a consumer's slot may not be free yet
-            auto look = [&] { room = min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1]); };
-            look();
-            for (Spin sp; q >= room; look()) {
-              if (!sp.step(g.ctl, g.spin_limit)) {
-                raise_timeout(g.ctl, 4, tpos, q, OP, 0ull, (unsigned)room);
-                break;
-              }
-            }
-            __syncwarp();
+            // a consumer's slot may not be free yet (one lane's look, so that all
+            // lanes agree)
+            Spin sp;
+            if (!warp_wait(
+                    [&] {
+                      room = __shfl_sync(XFP_FULL, min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1]), 0);
+                      return q < room;
+                    },
+                    vote, [&] { return sp.step(g.ctl, g.spin_limit); }))
+              raise_timeout(g.ctl, 4, tpos, q, OP, 0ull, (unsigned)room);
           }
           const bool to_near_j = (unsigned)(q - lo_j) < near_j, to_near_k = (unsigned)(q - lo_k) < near_k;
           if (to_near_j || to_near_k) {
