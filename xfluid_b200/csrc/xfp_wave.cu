@@ -231,6 +231,9 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(b)) : "memory");
 }
 
+// orders what this thread knows of ordinary accesses to shared memory before its bulk copies
+__device__ __forceinline__ void fence_bulk() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 __device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
   asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
@@ -634,10 +637,14 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
             for (int q = lane; q < (int)(sizeof(d.ej) / 16); q += 32) reinterpret_cast<uint4*>(&d.ej[0][0])[q] = make_uint4(0, 0, 0, 0);
           if (clear_k)
             for (int q = lane; q < (int)(sizeof(d.ek) / 16); q += 32) reinterpret_cast<uint4*>(&d.ek[0][0])[q] = make_uint4(0, 0, 0, 0);
-          __syncwarp();
         }
+        __syncwarp();
         if (lane == 0) {
           unsigned long long* b = &sh.full[n & (S - 1)];
+          // The compute warp wrote its results over r or y here with ordinary stores,
+          // which reached this lane through `ready`, `empty` and the warp's barrier;
+          // without the fence the copy, of another proxy, would not be ordered after them
+          fence_bulk();
           mbar_expect(b, (have_j ? (unsigned)sizeof(d.ej) : 0u) + (have_k ? (unsigned)sizeof(d.ek) : 0u) +
                              (n < me.ng ? W::IN * (unsigned)sizeof(ST) : 0u));
           if (n < me.ng) bulk_load(d.ops, src, W::IN * sizeof(ST), b);
