@@ -70,7 +70,8 @@ typedef struct xfp_options {
   int device_pointers;   /* 1: array arguments are device pointers */
   int device;            /* CUDA device ordinal */
   int check_every;       /* PCG iterations per host convergence read (0: 8) */
-  double timeout_ms;     /* bound on any device-side wait (0: 2000 ms) */
+  double timeout_ms;     /* bound on the sweeps' waits for values of other thread-block clusters (0: 2000 ms); all
+                            other device-side waits end with these */
   int max_refine;        /* mixed: iterative-refinement cycles (0: 20) */
   double inner_tol;      /* mixed: relative residual reduction per cycle (0: 1e-4) */
   int tile_k;            /* 0, 8, 15 or 16; kept for callers that set it: the sweeps have one decomposition, and results do not depend on it */
@@ -233,10 +234,12 @@ int xfp_box_loss_f32(xfp_ctx* ctx, int ni, int nj, int nk, const float* u, const
  * launched on this context waits, at every tile hand-off, for a boundary word
  * that no producer writes.  Every such wait is bounded (options.timeout_ms):
  * the first to run out records where it gave up and raises the context's
- * error flag, every other wait then returns within a few hundred polls, and
- * the call returns XFP_ERR_TIMEOUT with the site in xfp_last_error().  The
- * context stays usable; nothing faults.  Needs a grid with more than one
- * sweep tile.  Used by the tests of the timeout path. */
+ * error flag, every other such wait then returns within a few hundred polls,
+ * the sweep goes on with void values to its end, and the call returns
+ * XFP_ERR_TIMEOUT with the site in xfp_last_error().  The context stays usable;
+ * nothing faults.  Called n times: the n-th sweep from here on (of a single
+ * scene: the factorisation, the first two solves, then the PCG loop's).  Needs
+ * a grid with more than one sweep tile.  Used by the tests of the timeout path. */
 int xfp_debug_expire_next_sweep(xfp_ctx* ctx);
 
 /* ---- The simulator steps either side of the projection ----

@@ -17,3 +17,15 @@ def test_slots_are_refilled_behind_a_proxy_fence():
         before = CODE[max(0, at - 500):at]
         assert "fence_bulk();" in before
         assert "__syncwarp();" in before[:before.rindex("fence_bulk();")]
+
+
+def test_an_expired_wait_leaves_no_copies_behind():
+    """Only a wait inside a cluster ends a loop early, and then the CTAs of the cluster
+    leave after the copies to their slots: the courier goes on, and no sleep stands
+    for a wait."""
+    courier = CODE[CODE.index("courier) {"):CODE.index("if constexpr (!FACTOR) {\n      if (!skip")]
+    expired = courier[courier.index("sp.step(g.ctl, g.spin_limit)"):]
+    assert "late = true;" in expired and "break;" not in expired
+    end = CODE[CODE.index("if (*(volatile int*)&s_broken != 0) {"):]
+    assert end.index("mbar_try(") < end.index("cluster_sync();") < end.index("break;")
+    assert "__nanosleep" not in CODE

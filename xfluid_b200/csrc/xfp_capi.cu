@@ -117,10 +117,7 @@ int run_sweep(xfp_ctx* ctx, int op, const WaveArgs& g) {
                      ctx->sweep_ev_used + 2 <= (int)ctx->sweep_ev.size();
   if (timed) cudaEventRecord(ctx->sweep_ev[ctx->sweep_ev_used], ctx->stream);
   WaveArgs gl = g;
-  if (ctx->expire_next_sweep) {
-    gl.expect_bias = 1;
-    ctx->expire_next_sweep = false;
-  }
+  if (ctx->expire_sweep > 0 && --ctx->expire_sweep == 0) gl.expect_bias = 1;
   XFP_CUDA(ctx, (wave_launch<VT, CT>(op, gl, ctx->stream)));
   if (timed) {
     cudaEventRecord(ctx->sweep_ev[ctx->sweep_ev_used + 1], ctx->stream);
@@ -199,6 +196,15 @@ bool pcg_graph(xfp_ctx* ctx, const VT* const A[4], VT* x, VT* r, VT* s, VT* z, P
   WaveArgs g = wave_args(ctx);
   g.scal = dsc;
   g.bwd_mode = 1;
+  int expire = ctx->expire_sweep - 2;   // (the loop's first two solves are launched, not captured)
+  auto sweep = [&](int op, cudaStream_t cs) {
+    WaveArgs gl = g;
+    if (expire > 0 && --expire == 0) {
+      gl.expect_bias = 1;
+      ctx->expire_sweep = 0;
+    }
+    return wave_launch<VT, DT>(op, gl, cs);
+  };
   return capture_iterations(ctx, loop_iterations(ctx), [&](cudaStream_t cs) -> cudaError_t {
     cudaError_t e;
     if ((e = spmv_dot<VT, VT, DT>(A[0], A[1], A[2], A[3], s, z, ctx->group_nb.as<GroupNb>(), ctx->M, dsc,
@@ -207,8 +213,8 @@ bool pcg_graph(xfp_ctx* ctx, const VT* const A[4], VT* x, VT* r, VT* s, VT* z, P
     if ((e = update_xr<VT, DT>(x, r, s, z, ctx->M, dsc, ctx->partials.as<double>(), ctx->xr_blocks, cs,
                                swl ? ctx->sw.as<VT>() + WAVE_R : nullptr, swl ? ctx->gperm.as<int>() : nullptr)))
       return e;
-    if ((e = wave_launch<VT, DT>(SWEEP_FWD, g, cs))) return e;
-    if ((e = wave_launch<VT, DT>(SWEEP_BWD, g, cs))) return e;
+    if ((e = sweep(SWEEP_FWD, cs))) return e;
+    if ((e = sweep(SWEEP_BWD, cs))) return e;
     return update_s<VT>(s, z, ctx->M, dsc, cs, swl ? ctx->sw.as<VT>() + WAVE_Y : nullptr,
                         swl ? ctx->gperm.as<int>() : nullptr, ctx->s_blocks);
   });
@@ -1314,7 +1320,7 @@ int xfp_project_backward_f32(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t
 
 extern "C" int xfp_debug_expire_next_sweep(xfp_ctx* ctx) {
   if (!ctx) return XFP_ERR_ARGS;
-  ctx->expire_next_sweep = true;
+  ++ctx->expire_sweep;
   return XFP_OK;
 }
 

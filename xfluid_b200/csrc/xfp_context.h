@@ -151,8 +151,9 @@ struct xfp_ctx {
   long long launches = 0;
   // batched scenes (xfp_project_batch_*): buffers, tables and tuning cache
   xfp_host::BatchState* batch = nullptr;
-  // xfp_debug_expire_next_sweep: the next sweep launch's boundary waits run out
-  bool expire_next_sweep = false;
+  // xfp_debug_expire_next_sweep: in the n-th sweep launch from here on (0: none) the
+  // waits for other clusters' edge words run out
+  int expire_sweep = 0;
 };
 
 namespace xfp_host {

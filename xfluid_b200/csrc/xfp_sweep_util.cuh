@@ -53,13 +53,17 @@ __device__ __forceinline__ void st_gpu64(unsigned long long* p, unsigned long lo
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v));
 }
 
+// Turns of a wait: false after `limit`, and with ctl once another wait has run out.
 struct Spin {
   long long n = 0;
-  __device__ __forceinline__ bool step(const SweepCtl* ctl, long long limit) {
+  __device__ __forceinline__ bool step(long long limit) {
     ++n;
     if (n > 256) __nanosleep(n > 8192 ? 256 : 20);
-    if ((n & 255) == 0 && ld_volatile_u32(&ctl->err)) return false;
     return n < limit;
+  }
+  __device__ __forceinline__ bool step(const SweepCtl* ctl, long long limit) {
+    if (!step(limit)) return false;
+    return (n & 255) != 0 || ld_volatile_u32(&ctl->err) == 0;
   }
 };
 

@@ -51,10 +51,16 @@
 // Tiles are taken in topological order (J+K ascending): the first ones by
 // cluster index (a cooperative launch, so all clusters are resident), the
 // others from a ticket counter, so a tile only ever waits on tiles that
-// resident clusters hold.  Every wait is bounded (spin_limit polls); on expiry
-// the kernel records SweepCtl::err, every other wait gives up quickly, the
-// clusters run to their ends (all copies are consumed) and the host reports
-// XFP_ERR_TIMEOUT.
+// resident clusters hold.
+//
+// Waits are bounded.  The one wait that depends on other clusters, a courier's for
+// edge words, runs out after spin_limit polls, or once another has: it records
+// SweepCtl::err and from there on hands over whatever the words hold.  The results
+// are void, but every group is still sent, waited for and freed, so that the tile
+// runs to its end as it always does, no copy is left under way, and the host reports
+// XFP_ERR_TIMEOUT.  The waits inside a cluster depend on nothing but that; they
+// outlast it eight times, and one that runs out all the same (give_up) ends the
+// cluster after its tile, once the copies to its slots have landed.
 //
 // z.r is summed as the solves always did: every lane its lines in cell order,
 // the lines in 256 chunks, a fixed tree; the last cluster's eight CTAs share the
@@ -134,7 +140,6 @@ struct __align__(128) UnitShared {
   unsigned long long empty[S];   // mbarriers: a slot can be filled again
   int limit[2];                  // the j / k consumer has room for this block's groups below
   int freed;                     // slots given back (kept for a courier at work)
-  int broken;                    // a wait for a slot ran out: the unit does no more
 };
 
 // One value as stamped words.
@@ -231,6 +236,11 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(b)) : "memory");
 }
 
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
 // orders what this thread knows of ordinary accesses to shared memory before its bulk copies
 __device__ __forceinline__ void fence_bulk() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -304,6 +314,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
   // the next tile, by tile parity: a CTA may still read one while the leader
   // already writes the other
   __shared__ int s_next[2];
+  __shared__ int s_broken;   // a wait inside the cluster ran out
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int unit = warp % NW;
@@ -319,13 +330,13 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
   const bool near_pk = kt - DIR >= 0 && kt - DIR < 2 * NW, near_nk = kt + DIR >= 0 && kt + DIR < 2 * NW;
   auto unit_at = [&](int kk) -> U* { return &units[kk % NW]; };
   auto rank_at = [&](int c, int kk) { return (kk / NW) * WAVE_TJ + c; };
+  if (threadIdx.x == 0) s_broken = 0;
   if (helper && lane == 0) {
     for (int q = 0; q < S; ++q) {
       mbar_init(&sh.full[q]);
       mbar_init(&sh.ready[q]);
       mbar_init(&sh.empty[q]);
     }
-    sh.broken = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // per slot: the parity of its mbarriers' next phase at the start of a tile
@@ -378,11 +389,9 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
       if (g.scal != nullptr && *(volatile int*)&g.scal->done != 0) return;   // (changes between launches only)
       gen = ld_volatile_u32(&g.ctl->gen);
     }
-    // a unit that gave up in an earlier tile does not arm its mbarriers again; a
-    // converged scene's tiles are skipped (its scalars only change between
+    // a converged scene's tiles are skipped (its scalars only change between
     // launches, so every warp of this launch decides the same way)
-    const bool skip = (!first && *(volatile int*)&sh.broken != 0) ||
-                      (sid >= 0 && g.scal_batch != nullptr && *(volatile int*)&g.scal_batch[sid].done != 0);
+    const bool skip = sid >= 0 && g.scal_batch != nullptr && *(volatile int*)&g.scal_batch[sid].done != 0;
     first = false;
     if (helper && lane == 0) {
       sh.limit[0] = near_nj && nj.ng > 0 ? S + uj : INT_MAX;
@@ -401,26 +410,28 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
 
     auto parity_q = [&](int q) { return ((phase_q >> (q & (S - 1))) ^ (unsigned)(q >> LS)) & 1u; };
     auto parity_u = [&](int u) { return ((phase_u >> (u & (S - 1))) ^ (unsigned)(u >> LS)) & 1u; };
+    // a wait inside the cluster ran out
+    auto give_up = [&](unsigned site, int n, unsigned expect) {
+      raise_timeout(g.ctl, site, tpos, n, OP, 0ull, expect);
+      for (int r = 0; r < WAVE_CLUSTER; ++r) st_cluster_u32(cluster_addr(smem_u32(&s_broken), r), 1u);
+    };
+    const long long near_limit = 8 * g.spin_limit;
     // waits for a mbarrier's phase, all lanes together (a lane's own look may be
     // ahead of another's, and full-warp shuffles follow); false: it gave up
     auto vote = [](bool v) { return __all_sync(XFP_FULL, v) != 0; };
-    auto phase_of = [&](unsigned long long* bar, unsigned parity, long long limit, int n, unsigned site) -> bool {
+    auto await = [&](unsigned long long* bar, unsigned parity, int n, unsigned site) -> bool {
       const unsigned b = smem_u32(bar);
       Spin sp;
-      if (warp_wait([&] { return mbar_try(b, parity); }, vote, [&] { return sp.step(g.ctl, limit); })) return true;
-      raise_timeout(g.ctl, site, tpos, n, OP, 0ull, parity);
+      if (warp_wait([&] { return mbar_try(b, parity); }, vote, [&] { return sp.step(near_limit); })) return true;
+      give_up(site, n, parity);
       return false;
-    };
-    // ... one that another warp of this unit completes (whose own waits are
-    // bounded; this one outlasts them)
-    auto await = [&](unsigned long long* bar, int q, unsigned site) -> bool {
-      return phase_of(bar, parity_q(q), 8 * g.spin_limit, q, site);
     };
     // z.r of this lane's line h of the block
     auto put_dot = [&](int h, const LineDot<VT, DOT32>& d) {
       const int j = jb * 8 + jl, k = kb * 8 + 2 * kl + h;
       if (j < lj && k < lk) g.partials[lbase + (long long)k * lj + j] = d.sum();
     };
+    int armed = 0;   // (the helper's) slots filled in this tile
     // the range of own groups that each consumer takes
     const int lo_j = uj, hi_j = nj.ng > 0 ? min(me.ng - 1, uj + nj.ng) : INT_MIN;
     const int lo_k = uk, hi_k = nk.ng > 0 ? min(me.ng - 1, uk + nk.ng) : INT_MIN;
@@ -447,17 +458,11 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
       const unsigned near_k = near_nk && edge_k && hi_k >= lo_k ? (unsigned)(hi_k - lo_k) + 1u : 0u;
       VT* res = static_cast<VT*>(g.sw) + mybase * WAVE_ROW + wave_cell_slot<VT>(jl, half * 4 + kl, 0, 0);   // (the factor)
 
-      // waits for a slot's mbarrier; on expiry the results are void and the block
-      // ends (its helper finds the error flag), and the host reports the timeout
       bool bad = false;
-      auto wait = [&](unsigned long long* bar, unsigned parity, unsigned site, int n) {
-        bad = !phase_of(bar, parity, g.spin_limit, n, site);
-        if (bad) *(volatile int*)&sh.broken = 1;
-      };
       X ej[HL][4], ek[4];        // the producers' values of the group, in sweep order
       auto take_edges = [&](int u) {   // (zero where a producer has no such group: the helper's work)
         const int sl = u & (S - 1);
-        wait(&sh.full[sl], parity_u(u), 3, u);
+        bad |= !await(&sh.full[sl], parity_u(u), u, 3);
         const SL& in = sh.slot[sl];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
@@ -577,8 +582,10 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
                       room = __shfl_sync(XFP_FULL, min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1]), 0);
                       return q < room;
                     },
-                    vote, [&] { return sp.step(g.ctl, g.spin_limit); }))
-              raise_timeout(g.ctl, 4, tpos, q, OP, 0ull, (unsigned)room);
+                    vote, [&] { return sp.step(near_limit); })) {
+              give_up(4, q, (unsigned)room);
+              break;
+            }
           }
           const bool to_near_j = (unsigned)(q - lo_j) < near_j, to_near_k = (unsigned)(q - lo_k) < near_k;
           if (to_near_j || to_near_k) {
@@ -659,18 +666,21 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
       const unsigned tell = lane == 0 ? ack_j : lane == 1 ? ack_k : cluster_addr(smem_u32(&sh.freed), rank);
       const int tell_ahead = lane == 0 ? S + aj : lane == 1 ? S + ak : 0;
       const bool told = (lane == 0 && near_pj) || (lane == 1 && near_pk) || (lane == 2 && far_in);
-      for (int n = 0; n < S && n <= me.ng; ++n) arm(n);
+      for (; armed < S && armed <= me.ng; ++armed) arm(armed);
       LineDot<VT, DOT32> dot;   // of the lines h = 1
       for (int q = 0; q < me.ng; ++q) {
         const int sl = q & (S - 1);
-        if (!await(&sh.empty[sl], q, 7)) break;
+        if (!await(&sh.empty[sl], parity_q(q), q, 7)) break;
         VT z[4], rr[4];
         if constexpr (REV) {
           ldg(z, reinterpret_cast<const VT*>(sh.slot[sl].ops) + WAVE_Y + 128 + lane * 4);
           ldg(rr, reinterpret_cast<const VT*>(sh.slot[sl].ops) + WAVE_R + 128 + lane * 4);
           __syncwarp();
         }
-        if (q + S <= me.ng) arm(q + S);
+        if (q + S <= me.ng) {
+          arm(q + S);
+          ++armed;
+        }
         // the slot is the producers' again (all the rest at the end)
         if (told) st_cluster_u32(tell, (unsigned)((q + 1 == me.ng ? INT_MAX / 2 : q + 1) + tell_ahead));
         if constexpr (REV) dot.add(z, rr);
@@ -708,12 +718,13 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
         for (int d = 0; d < FB; ++d)
           if (use && f.u + d <= f.last && !f.w[d].ready(want)) f.w[d].load(src + (size_t)(f.u + d + a) * 32 * P);
       };
+      bool late = false;   // a wait ran out: what the words hold will do
       int room = S;   // (with a look at `freed` for every group: 128^3 FP64 8.43 ms against 8.35)
       auto forward = [&](Far& f, unsigned to, bool use) -> bool {
         bool moved = false;
 #pragma unroll
         for (int d = 0; d < FB; ++d) {
-          if (f.u > f.last || !__all_sync(XFP_FULL, !use || f.w[0].ready(want))) break;
+          if (f.u > f.last || !__all_sync(XFP_FULL, late || !use || f.w[0].ready(want))) break;
           const unsigned at = (unsigned)f.u & (S - 1);
           // its slot is free once group u - S is done with (one lane's look, so
           // that all lanes agree; a count, since the courier may be any number
@@ -744,10 +755,16 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
           sp = Spin();
           continue;
         }
-        const bool go = sp.step(g.ctl, g.spin_limit);
-        if (!__all_sync(XFP_FULL, go)) {
-          if (!go) raise_timeout(g.ctl, 8, tpos, fj.u, OP, fj.w[0].w[0], want);
+        if (late) {   // only a slot is waited for
+          if (vote(sp.step(near_limit))) continue;
+          give_up(8, fj.u, want);
           break;
+        }
+        const bool go = sp.step(g.ctl, g.spin_limit);
+        if (!vote(go)) {
+          if (!go) raise_timeout(g.ctl, 8, tpos, fj.u, OP, fj.w[0].w[0], want);
+          late = true;
+          sp = Spin();
         }
       }
     }
@@ -760,7 +777,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
         const int line_j = is_j ? (REV ? 0 : 7) : lane & 7, line_k = is_j ? lane : (REV ? 0 : 7);
         const int lo = is_j ? lo_j : lo_k, hi = is_j ? hi_j : hi_k;
         const bool near = is_j ? near_nj : near_nk;
-        const unsigned count = is_edge && hi >= lo ? (unsigned)(hi - lo) + 1u : 0u;   // groups from lo on
+        unsigned count = is_edge && hi >= lo ? (unsigned)(hi - lo) + 1u : 0u;   // groups from lo on
         unsigned to = 0, bar = 0;   // near: slot 0
         if (near) {
           SL& d = unit_at(is_j ? kt : kt + DIR)->slot[0];
@@ -778,7 +795,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
         LineDot<VT, DOT32> dot;   // of the lines h = 0 (the helper has h = 1)
         for (int q = 0; q < me.ng; ++q) {
           const int sl = q & (S - 1);
-          if (!await(&sh.ready[sl], q, 9)) break;
+          if (!await(&sh.ready[sl], parity_q(q), q, 9)) break;
           const VT* const ops = reinterpret_cast<const VT*>(sh.slot[sl].ops);
           if ((unsigned)(q - lo) < count) {
             VT y[4], w[4];
@@ -793,17 +810,20 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
                 // the consumer's slot may not be free yet
                 room = *limit;
                 for (Spin sp; q >= room; room = *limit) {
-                  if (!sp.step(g.ctl, g.spin_limit)) {
-                    raise_timeout(g.ctl, 4, tpos, q, OP, 0ull, (unsigned)room);
+                  if (!sp.step(near_limit)) {
+                    give_up(4, q, (unsigned)room);
+                    count = 0;   // it is not free: nothing more goes there
                     break;
                   }
                 }
               }
-              const unsigned d = (unsigned)(q - lo) & (S - 1);
-              uint32_t m[4 * P];
+              if (count != 0) {
+                const unsigned d = (unsigned)(q - lo) & (S - 1);
+                uint32_t m[4 * P];
 #pragma unroll
-              for (int s = 0; s < 4; ++s) to_words(w[s], m + s * P);
-              send(to + d * (unsigned)sizeof(SL), bar + d * 8, m);
+                for (int s = 0; s < 4; ++s) to_words(w[s], m + s * P);
+                send(to + d * (unsigned)sizeof(SL), bar + d * 8, m);
+              }
             } else {
               publish<X>(pub + (size_t)q * 32 * P, gen, w);
             }
@@ -823,6 +843,22 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
         if constexpr (REV) put_dot(0, dot);
       }
     }
+    __syncwarp();
+    cluster_sync();   // every slot has been read; s_next and s_broken are set
+    if (*(volatile int*)&s_broken != 0) {
+      // Nothing more is sent.  What is under way to this CTA's slots lands before
+      // any CTA of the cluster leaves: a slot's mbarrier tells, unless a value that
+      // was never sent is missing from it too, for which 10 ms have to do.
+      if (helper) {
+        const unsigned long long t0 = now_ns();
+        for (int u = max(0, armed - S); u < armed; ++u)
+          (void)warp_wait([&] { return mbar_try(smem_u32(&sh.full[u & (S - 1)]), parity_u(u)); }, vote,
+                          [&] { return now_ns() - t0 < 10000000ull; });
+      }
+      __syncwarp();
+      cluster_sync();
+      break;
+    }
     // slot n has carried the groups q = n, n + S, ... < ng and the edges u = n, n + S, ... <= ng
     if (!skip && me.ng > 0)
 #pragma unroll
@@ -830,15 +866,9 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
         phase_q ^= (unsigned)(((me.ng - 1 - n + S) >> LS) & 1) << n;
         phase_u ^= (unsigned)(((me.ng - n + S) >> LS) & 1) << n;
       }
-    __syncwarp();
-    cluster_sync();   // every slot has been read; s_next is set
     pos = *(volatile int*)&s_next[turn];
   }
 
-  // a block that gave up on a slot outlives the copies and stores still under
-  // way to it (a few microseconds)
-  if (*(volatile int*)&sh.broken != 0)
-    for (int q = 0; q < 200; ++q) __nanosleep(1000);
   // ---------------- launch epilogue: the last cluster closes the generation ----------------
   unsigned last = 0;
   if (rank == 0 && threadIdx.x == 0) {
