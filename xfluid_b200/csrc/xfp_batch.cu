@@ -257,25 +257,18 @@ int batch_pcg(xfp_ctx* ctx, BatchState* B, const VT* const A[4], const VT* b, VT
     if (e != cudaSuccess) return e;
     return cudaMemcpyAsync(&ctx->loop_read->ctl, ctx->ctl.p, sizeof(SweepCtl), cudaMemcpyDeviceToHost, cs);
   };
-  auto finished = [&](int& err, int& last) -> bool {
-    err = sweep_error(ctx, ctx->loop_read->ctl);
+  auto done = [&] {
     bool all = true;
-    last = 0;
-    for (int q = 0; q < n; ++q) {
-      all &= hsc[q].done != 0;
-      last = std::max(last, hsc[q].iters);
-    }
+    for (int q = 0; q < n; ++q) all &= hsc[q].done != 0;
     return all;
   };
-  if (graph) return replay_iterations(ctx, per, per_iter, maxit_all + 2 * K, read, finished);
+  if (graph) return replay_iterations(ctx, per, per_iter, maxit_all + 2 * K, read, done);
   for (int done_iters = 0;;) {
     for (int q = 0; q < K; ++q) XFP_CUDA(ctx, iteration(st));
     done_iters += K;
     XFP_CUDA(ctx, read(st));
     XFP_CUDA(ctx, cudaStreamSynchronize(st));
-    int last;
-    const bool end = finished(rc, last);
-    if (rc != XFP_OK || end) break;
+    if ((rc = sweep_error(ctx, ctx->loop_read->ctl)) != XFP_OK || done()) break;
     if (done_iters > maxit_all + 2 * K) return fail(ctx, XFP_ERR_CUDA, "batch PCG loop did not terminate");
   }
   return rc;

@@ -260,13 +260,8 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
     if (e != cudaSuccess) return e;
     return cudaMemcpyAsync(&ctx->loop_read->ctl, ctx->ctl.p, sizeof(SweepCtl), cudaMemcpyDeviceToHost, cs);
   };
-  auto finished = [&](int& err, int& last) -> bool {
-    *hsc = ctx->loop_read->sc;
-    last = hsc->iters;
-    err = sweep_error(ctx, ctx->loop_read->ctl);
-    return hsc->done != 0;
-  };
-  if (graph && (rc = replay_iterations(ctx, loop_iterations(ctx), g1.ntiles > 0 ? 5 : 3, maxit + 2 * K, read, finished)) != XFP_OK) return rc;
+  auto done = [&] { return ctx->loop_read->sc.done != 0; };
+  if (graph && (rc = replay_iterations(ctx, loop_iterations(ctx), g1.ntiles > 0 ? 5 : 3, maxit + 2 * K, read, done)) != XFP_OK) return rc;
   for (int done_iters = 0; !graph;) {
     for (int q = 0; q < K; ++q) {
       const int it = done_iters + q + 1;   // this launch's PCG iteration (1-based)
@@ -284,12 +279,11 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
     done_iters += K;
     XFP_CUDA(ctx, read(st));
     XFP_CUDA(ctx, cudaStreamSynchronize(st));
-    int last;
-    const bool end = finished(rc, last);
-    if (rc != XFP_OK) return rc;
-    if (end) break;
+    if ((rc = sweep_error(ctx, ctx->loop_read->ctl)) != XFP_OK) return rc;
+    if (done()) break;
     if (done_iters > maxit + 2 * K) return fail(ctx, XFP_ERR_CUDA, "PCG loop did not terminate");
   }
+  *hsc = ctx->loop_read->sc;
   // the preconditioner's two sweeps, then two per iteration but the last (the
   // converged iteration skips its preconditioner): 2 * iterations did work;
   // the launches after them in the last chunk returned at once

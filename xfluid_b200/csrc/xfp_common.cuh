@@ -178,6 +178,14 @@ struct PcgScalars {
   unsigned int pad;
 };
 
+// Ends a solve.  The host may read the scalars beside the kernel that does: `done`
+// goes last, behind a fence, so that whoever sees it finds the others in place.
+__device__ __forceinline__ void end_solve(PcgScalars* sc, int status) {
+  sc->status = status;
+  __threadfence_system();
+  *(volatile int*)&sc->done = 1;
+}
+
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");

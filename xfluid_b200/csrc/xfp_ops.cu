@@ -862,14 +862,9 @@ __device__ __forceinline__ void update_xr_body(unsigned bid, unsigned nblk, VT* 
   if (threadIdx.x == 0) {
     sc->res = tot;
     sc->iters += 1;
-    if (tot <= sc->tolabs) {
-      sc->done = 1;
-      sc->status = 0;
-    } else if (sc->iters >= sc->maxit) {
-      sc->done = 1;
-      sc->status = 1;
-    }
     sc->red_count = 0;
+    if (tot <= sc->tolabs) end_solve(sc, 0);
+    else if (sc->iters >= sc->maxit) end_solve(sc, 1);
   }
 }
 template <typename VT>
@@ -1000,9 +995,9 @@ __device__ __forceinline__ void absmax_init_body(unsigned bid, unsigned nblk, co
     sc->iters = 0;
     sc->maxit = maxit;
     sc->status = 0;
-    sc->done = (tot == 0.0 || maxit <= 0) ? 1 : 0;
-    if (tot != 0.0 && maxit <= 0) sc->status = 1;
+    sc->done = 0;
     sc->red_count = 0;
+    if (tot == 0.0 || maxit <= 0) end_solve(sc, tot != 0.0 ? 1 : 0);
   }
 }
 template <typename VT>
@@ -1219,7 +1214,7 @@ __global__ void __launch_bounds__(1024) batch_bwd_reduce_kernel(const BatchSeg* 
   if (threadIdx.x != 0) return;
   if (mode == 0) {
     S->rho = rho_new;
-    if (rho_new == 0.0 || rho_new != rho_new) { S->status = -5; S->done = 1; }
+    if (rho_new == 0.0 || rho_new != rho_new) end_solve(S, -5);
   } else {
     S->beta = std::is_same<DT, float>::value ? (double)__fdiv_rn((float)rho_new, (float)S->rho)
                                              : __ddiv_rn(rho_new, S->rho);

@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
       PcgScalars* sc = g.scal;
       if (g.bwd_mode == 0) {
         sc->rho = rho_new;
-        if (rho_new == 0.0 || rho_new != rho_new) { sc->status = -5; sc->done = 1; }
+        if (rho_new == 0.0 || rho_new != rho_new) end_solve(sc, -5);
       } else {
         sc->beta = DOT32 ? (double)__fdiv_rn((float)rho_new, (float)sc->rho) : __ddiv_rn(rho_new, sc->rho);
         sc->rho = rho_new;
