@@ -29,3 +29,13 @@ def test_an_expired_wait_leaves_no_copies_behind():
     end = CODE[CODE.index("if (*(volatile int*)&s_broken != 0) {"):]
     assert end.index("mbar_try(") < end.index("cluster_sync();") < end.index("break;")
     assert "__nanosleep" not in CODE
+
+
+def test_free_slots_are_told_with_release_and_read_with_acquire():
+    """A block writes edge values into a neighbour's slot once the neighbour has told it
+    that the slot is free; what the neighbour read from the slot has to come first."""
+    assert "st.release.cta.shared::cluster" in CODE and "ld.acquire.cluster.shared" in CODE
+    told = [line for line in CODE.splitlines() if "if (told)" in line]
+    assert told and all("st_release_s32(" in line for line in told)
+    looks = re.findall(r"room = [^;]*(?:limit|freed)[^;]*;", CODE)
+    assert len(looks) >= 3 and all("ld_acquire_s32(" in look for look in looks)

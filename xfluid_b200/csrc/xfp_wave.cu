@@ -209,9 +209,18 @@ __device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank) {
 __device__ __forceinline__ void st_cluster_u32(unsigned a, unsigned v) {
   asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
+// A count of free slots, for another warp of the cluster (shared::cluster address), and
+// that warp's look: what was read from a slot before it was given back comes before
+// what is sent to it after.  The release is this CTA's: shared memory has one copy, so
+// its accesses are over for the cluster once they are for the CTA.  (One of the
+// cluster's scope holds the helper up for 0.2 us a group: 128^3 99 us against 64 in
+// FP32, 131 against 97 in FP64; the acquire and this release cost nothing measurable.)
+__device__ __forceinline__ void st_release_s32(unsigned a, int v) {
+  asm volatile("st.release.cta.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
 __device__ __forceinline__ int ld_acquire_s32(const int* p) {
   int v;
-  asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+  asm volatile("ld.acquire.cluster.shared.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
   return v;
 }
 __device__ __forceinline__ void cluster_sync() {
@@ -579,7 +588,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
             Spin sp;
             if (!warp_wait(
                     [&] {
-                      room = __shfl_sync(XFP_FULL, min(*(volatile int*)&sh.limit[0], *(volatile int*)&sh.limit[1]), 0);
+                      room = __shfl_sync(XFP_FULL, min(ld_acquire_s32(&sh.limit[0]), ld_acquire_s32(&sh.limit[1])), 0);
                       return q < room;
                     },
                     vote, [&] { return sp.step(near_limit); })) {
@@ -682,7 +691,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
           ++armed;
         }
         // the slot is the producers' again (all the rest at the end)
-        if (told) st_cluster_u32(tell, (unsigned)((q + 1 == me.ng ? INT_MAX / 2 : q + 1) + tell_ahead));
+        if (told) st_release_s32(tell, (q + 1 == me.ng ? INT_MAX / 2 : q + 1) + tell_ahead);
         if constexpr (REV) dot.add(z, rr);
       }
       if constexpr (REV) put_dot(1, dot);
@@ -786,7 +795,7 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
           bar = cluster_addr(smem_u32(&unit_at(is_j ? kt : kt + DIR)->full[0]), r);
         }
         unsigned long long* const pub = (is_j ? g.bj : g.bk) + ((size_t)mybase * 32 + (lane & 7) * 4) * P;
-        const volatile int* const limit = &sh.limit[is_j ? 0 : 1];
+        const int* const limit = &sh.limit[is_j ? 0 : 1];
         const int coef = wave_cell_slot<VT>(line_j, line_k, 0, is_j ? 1 : 2);
         constexpr int CELL_E = 128;              // from one step's cells to the next's
         const int edge_at = OUT + wave_line_slot(line_j, line_k);
@@ -808,8 +817,8 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
             if (near) {
               if (q >= room) {
                 // the consumer's slot may not be free yet
-                room = *limit;
-                for (Spin sp; q >= room; room = *limit) {
+                room = ld_acquire_s32(limit);
+                for (Spin sp; q >= room; room = ld_acquire_s32(limit)) {
                   if (!sp.step(near_limit)) {
                     give_up(4, q, (unsigned)room);
                     count = 0;   // it is not free: nothing more goes there
