@@ -147,7 +147,8 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S)
     // over single cells with the same blocks)
     g.blk_cells = (int)std::max<long long>(1, std::min<long long>((Ms / 4 + 255) / 256, NBLK_MAX));
     g.blk_cells_start = bc;
-    g.blk_groups = (int)spmv_block_count(Ms, NBLK_MAX);
+    // the SpMV's dot is summed over blocks: as many as a single scene's has
+    g.blk_groups = (int)spmv_block_count(Ms, ctx->vec_blocks);
     g.blk_groups_start = bg;
     g.blk_base = blk_base[s];
     g.line_base = line_base[s];
