@@ -123,6 +123,19 @@ int main(int argc, char** argv) {
     check(rc == XFP_ERR_TIMEOUT && ctx.err == "site 8", "the expired wait before the breakdown");
   } else if (what == "endless") {
     check(loop(ctx, [](int, bool, xfp_ctx::Read&) {}) == XFP_ERR_CUDA, "a loop that does not end");
+  } else if (what == "refused") {
+    // a capture that fails after one that did not leaves no executable graph behind
+    capture_result = cudaErrorStreamCaptureInvalidated;
+    check(!xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }), "a refused capture");
+    check(execs == 0 && ctx.loop_exec == nullptr, "the earlier graph given back");
+    capture_result = cudaSuccess;
+    check(!xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaErrorInvalidValue; }), "a refused launch");
+    check(execs == 0 && ctx.loop_exec == nullptr, "nothing kept");
+    check(xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }) && execs == 1, "a new graph");
+    update_result = cudaErrorGraphExecUpdateFailure;
+    check(xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }) && execs == 1, "one in its place");
+    instantiate_result = cudaErrorMemoryAllocation;
+    check(!xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }) && execs == 0, "no instance");
   } else {
     return 2;
   }

@@ -55,11 +55,11 @@ bool capture_iterations(xfp_ctx* ctx, int n, F&& iteration) {
     if (!ctx->loop_exec) e = cudaGraphInstantiate(&ctx->loop_exec, graph, 0);
   }
   if (graph) cudaGraphDestroy(graph);
-  if (e != cudaSuccess) {
-    ctx->loop_exec = nullptr;
-    cudaGetLastError();
-  }
-  return ctx->loop_exec != nullptr;
+  if (e == cudaSuccess) return ctx->loop_exec != nullptr;
+  if (ctx->loop_exec) cudaGraphExecDestroy(ctx->loop_exec);   // (an earlier call's)
+  ctx->loop_exec = nullptr;
+  cudaGetLastError();
+  return false;
 }
 
 // Launches the captured graph (n iterations of per_iter kernels) until done() says
