@@ -38,14 +38,7 @@ struct BatchState {
   long long M = 0;
 };
 
-void batch_state_free(BatchState* b) {
-  if (!b) return;
-  DevBuf* all[] = {&b->lines, &b->scene_tile_lists, &b->counters, &b->segs,
-                   &b->tile_scene, &b->scal, &b->scal2, &b->part,
-                   &b->tols, &b->maxits, &b->io, &b->pdense};
-  for (DevBuf* d : all) d->release();
-  delete b;
-}
+void batch_state_free(BatchState* b) { delete b; }
 
 namespace {
 

@@ -896,7 +896,6 @@ int debug_core(xfp_ctx* ctx, const CT* const Af[5], const VT* const Av[4], const
   XFP_CUDA(ctx, Fb.ensure((size_t)(M + 8) * 4 * sizeof(CT)));
   CT* F[4];
   for (int q = 0; q < 4; ++q) F[q] = Fb.as<CT>() + (size_t)(M + 8) * q;
-  struct Release { DevBuf& b; ~Release() { b.release(); } } release{Fb};
   if (ctx->ntiles > 0)
     XFP_CUDA(ctx, factor_lines<CT>(ctx->sw.as<CT>(), ctx->lines.as<Line>(), ctx->nj, ctx->nk,
                                    ctx->blks.as<WBlk>(), ctx->NJB, F, st));
@@ -1156,17 +1155,8 @@ int xfp_destroy(xfp_ctx* ctx) {
   if (!ctx) return XFP_OK;
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  DevBuf* all[] = {&ctx->io_mat, &ctx->io_u, &ctx->io_v, &ctx->io_w, &ctx->io_wu, &ctx->io_wv, &ctx->io_ww,
-                   &ctx->io_p, &ctx->io_gu, &ctx->io_gv, &ctx->io_gw, &ctx->lines, &ctx->line_sums,
-                   &ctx->blks, &ctx->tiles, &ctx->counters, &ctx->group_line, &ctx->group_nb, &ctx->gperm, &ctx->x64,
-                   &ctx->r64, &ctx->x32, &ctx->r32, &ctx->s32, &ctx->z32, &ctx->s64, &ctx->z64, &ctx->dense,
-                   &ctx->sw_sys, &ctx->sw, &ctx->edge, &ctx->ctl, &ctx->scal, &ctx->scal2, &ctx->partials,
-                   &ctx->tpartials};
-  for (DevBuf* b : all) b->release();
   batch_state_free(ctx->batch);
   ctx->batch = nullptr;
-  for (auto& b : ctx->A64) b.release();
-  for (auto& b : ctx->A32) b.release();
   for (auto& e : ctx->ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : ctx->sweep_ev)

@@ -16,10 +16,17 @@ namespace xfp_host {
 
 constexpr int NBLK_MAX = 148 * 8;   // blocks of the reduction kernels (partials slots)
 
-// A device allocation that only grows.
+// A device allocation that only grows; given back with its owner (on the owner's
+// device, which the caller has made the current one).
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  ~DevBuf() {
+    if (p) cudaFree(p);
+  }
   cudaError_t ensure(size_t bytes) {
     if (bytes <= cap && p) return cudaSuccess;
     if (p) cudaFree(p);
@@ -29,11 +36,6 @@ struct DevBuf {
     cudaError_t e = cudaMalloc(&p, want);
     if (e == cudaSuccess) cap = want;
     return e;
-  }
-  void release() {
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
   }
   template <typename T>
   T* as() const { return reinterpret_cast<T*>(p); }
