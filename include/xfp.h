@@ -69,7 +69,8 @@ typedef struct xfp_options {
   int precision;         /* XFP_PREC_* */
   int device_pointers;   /* 1: array arguments are device pointers */
   int device;            /* CUDA device ordinal */
-  int check_every;       /* PCG iterations per host convergence read (0: 8) */
+  int check_every;       /* PCG iterations between host convergence reads, at most (0: 8); as a CUDA
+                            graph the loop reads every min(check_every, 4), beside the next ones */
   double timeout_ms;     /* bound on the sweeps' waits for values of other thread-block clusters (0: 2000 ms); all
                             other device-side waits end with these */
   int max_refine;        /* mixed: iterative-refinement cycles (0: 20) */

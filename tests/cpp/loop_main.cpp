@@ -123,6 +123,12 @@ int main(int argc, char** argv) {
     check(rc == XFP_ERR_TIMEOUT && ctx.err == "site 8", "the expired wait before the breakdown");
   } else if (what == "endless") {
     check(loop(ctx, [](int, bool, xfp_ctx::Read&) {}) == XFP_ERR_CUDA, "a loop that does not end");
+  } else if (what == "check_every") {
+    // at most check_every iterations between reads, whether it is even or odd
+    for (int k : {0, 1, 2, 3, 4, 5, 6, 7, 8, 25, 32}) {
+      ctx.opt.check_every = k;
+      check(xfp_host::loop_iterations(&ctx) == (k == 0 || k > 4 ? 4 : k), "iterations of a graph");
+    }
   } else if (what == "refused") {
     // a capture that fails after one that did not leaves no executable graph behind
     capture_result = cudaErrorStreamCaptureInvalidated;

@@ -11,9 +11,9 @@
 //   * the vector kernels: one launch per kernel covers all scenes, each scene
 //     running the same block decomposition (and so the same reduction order)
 //     as its single-scene launch would.
-//   * the PCG iteration is captured once as a CUDA graph (check_every
-//     iterations: SpMV+dot, x/r update, forward, backward, rho/beta, s update)
-//     and replayed until every scene has converged or hit its cap.
+//   * a PCG loop's iterations (SpMV+dot, x/r update, forward, backward, rho/beta,
+//     s update) are captured as a CUDA graph of min(check_every, 4) of them and
+//     replayed until every scene has converged or hit its cap.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>

@@ -5,7 +5,8 @@
 //   assemble the variational system into the compact layout      (xfp_ops.cu)
 //   factor   MIC(0) in natural order                              (xfp_wave.cu)
 //   PCG      spmv+dot / x,r update / forward / backward+dot / s update per
-//            iteration, convergence read back every check_every iterations
+//            iteration, as a CUDA graph of min(check_every, 4) iterations whose
+//            scalars are read back while the next launch of it runs
 //   output   pressure scattered to the dense grid, velocity update (project)
 // Mixed precision wraps the FP32 PCG in FP64 iterative refinement.
 #include <algorithm>

@@ -12,9 +12,13 @@ extern thread_local long long g_kernel_launches;
 namespace xfp_host {
 
 // Iterations of a PCG loop's graph; its scalars are read after every launch of it.
+// options.check_every bounds them.  Since the read runs beside the next launch, more
+// than four only add launches past the end (two launches of the graph are on their
+// way when the last one is known), and fewer, or one of an odd check_every, a read an
+// iteration.
 inline int loop_iterations(const xfp_ctx* ctx) {
   const int K = ctx->opt.check_every > 0 ? ctx->opt.check_every : 8;
-  return K % 4 == 0 ? 4 : K % 2 == 0 ? 2 : 1;
+  return K < 4 ? K : 4;
 }
 
 // Captures n iterations of a PCG loop (iteration(stream) launches one) into
