@@ -96,16 +96,13 @@ int batch_layout(xfp_ctx* ctx, BatchState* B, const std::vector<DevScene<T>>& S)
   }
   if (base[n] >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "batch too large: more than 2^31 stored cells");
   if (group_base[n] * 256 >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "batch too large for the sweep layout");
-  // group -> line index (line numbers local to each scene's table; cells
-  // global) and group -> sweep element
-  XFP_CUDA(ctx, ctx->group_line.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(int)));
+  // group -> its neighbours (cells global) and group -> sweep element
   XFP_CUDA(ctx, ctx->gperm.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->group_nb.ensure((std::max<long long>(base[n], 4) / 4 + 8) * sizeof(GroupNb)));
   std::vector<TableScene> tables(n);
   for (int s = 0; s < n; ++s)
     tables[s] = {lines + line_base[s], ctx->blks.as<WBlk>() + blk_base[s], S[s].nj, S[s].nk, base[s], group_base[s]};
-  XFP_CUDA(ctx, layout_tables(tables.data(), n, ctx->group_line.as<int>(), ctx->group_nb.as<GroupNb>(),
-                              ctx->gperm.as<int>(), st));
+  XFP_CUDA(ctx, layout_tables(tables.data(), n, ctx->group_nb.as<GroupNb>(), ctx->gperm.as<int>(), st));
   // merge the scenes' block lists by wavefront level (each list is already in
   // its own topological order, which the merge keeps)
   long long ntl = 0;

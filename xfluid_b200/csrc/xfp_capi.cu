@@ -71,12 +71,10 @@ int build_layout(xfp_ctx* ctx, const uint8_t* dmat, int ni, int nj, int nk) {
   ctx->M = cnt[0]; ctx->rows = cnt[1]; ctx->nlines_act = cnt[2]; ctx->ntiles = cnt[3]; ctx->Gsw = cnt[4];
   ctx->nlines_all = nlines;
   if (ctx->Gsw * 256 >= (1LL << 31)) return fail(ctx, XFP_ERR_ARGS, "grid too large for the sweep layout");
-  XFP_CUDA(ctx, ctx->group_line.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->gperm.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(int)));
   XFP_CUDA(ctx, ctx->group_nb.ensure((std::max<long long>(ctx->M, 4) / 4 + 8) * sizeof(GroupNb)));
   const TableScene T{ctx->lines.as<Line>(), ctx->blks.as<WBlk>(), nj, nk, 0, 0};
-  XFP_CUDA(ctx, layout_tables(&T, 1, ctx->group_line.as<int>(), ctx->group_nb.as<GroupNb>(), ctx->gperm.as<int>(),
-                              ctx->stream));
+  XFP_CUDA(ctx, layout_tables(&T, 1, ctx->group_nb.as<GroupNb>(), ctx->gperm.as<int>(), ctx->stream));
   return XFP_OK;
 }
 
@@ -1108,7 +1106,6 @@ int xfp_create(xfp_ctx** out, const xfp_options* opt) {
     delete ctx;
     return XFP_ERR_ARGS;
   }
-  cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, o.device);
   if (o.stream) {
     ctx->stream = (cudaStream_t)o.stream;
   } else {

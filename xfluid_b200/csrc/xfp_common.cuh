@@ -186,24 +186,6 @@ __device__ __forceinline__ void end_solve(PcgScalars* sc, int status) {
   *(volatile int*)&sc->done = 1;
 }
 
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ double ld_relaxed(const double* p) {
-  double v;
-  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ float ld_relaxed(const float* p) {
-  float v;
-  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ unsigned int ld_volatile_u32(const unsigned int* p) {
   return *(const volatile unsigned int*)p;
 }
@@ -242,9 +224,4 @@ __device__ __forceinline__ void stg(double* p, const double (&v)[4]) {
   reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
   reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
 }
-template <typename T>
-__device__ __forceinline__ T shfl_up(T v, int d) { return __shfl_up_sync(XFP_FULL, v, d); }
-template <typename T>
-__device__ __forceinline__ T shfl_down(T v, int d) { return __shfl_down_sync(XFP_FULL, v, d); }
-
 }  // namespace xfp

@@ -52,12 +52,11 @@ struct xfp_ctx {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   std::string err;
-  int nsm = 148;
   using DevBuf = xfp_host::DevBuf;
   // I/O staging (host-pointer mode)
   DevBuf io_mat, io_u, io_v, io_w, io_wu, io_wv, io_ww, io_p, io_gu, io_gv, io_gw;
   // layout
-  DevBuf lines, line_sums, blks, tiles, counters, group_line, group_nb;
+  DevBuf lines, line_sums, blks, tiles, counters, group_nb;
   // compact arrays
   DevBuf A64[5];                  // diag, ax, ay, az, b (FP64)
   DevBuf A32[5];                  // same in FP32

@@ -96,17 +96,16 @@ struct LayoutScene {
   long long* counters;       // [5]
 };
 cudaError_t layout_build(const LayoutScene* scenes, int n, cudaStream_t st);
-// Per aligned 4-cell group: the line that stores it, its neighbours and its place in
-// the sweep layout; the grids' cells follow one another from `base` on, their groups of
-// the sweep layout from group_base on.  Line offsets are made global.
+// Per aligned 4-cell group: its neighbours and its place in the sweep layout.  The
+// grids' cells follow one another from `base` on, their groups of the sweep layout
+// from group_base on.  Line offsets are made global.
 struct TableScene {
   Line* lines;
   const WBlk* blks;
   int nj, nk;
   long long base, group_base;
 };
-cudaError_t layout_tables(const TableScene* scenes, int n, int* group_line, GroupNb* group_nb, int* gperm,
-                          cudaStream_t st);
+cudaError_t layout_tables(const TableScene* scenes, int n, GroupNb* group_nb, int* gperm, cudaStream_t st);
 
 // ---- assembly / apply / vector kernels (xfp_ops.cu) ----
 template <typename FT, typename AT>

@@ -258,15 +258,15 @@ __global__ void __launch_bounds__(1024) blk_scan_kernel(const __grid_constant__ 
   if (threadIdx.x == 0) counters[3] = carry;
 }
 
-// For the aligned 4-cell group of cell c, at c / 4 (cells counted over all grids):
-// its line (index in its grid's table; lines start at multiples of 4 and hold
-// multiples of 4 cells), where its y and z neighbours are, and the sweep element of
-// its first cell (its four cells are four consecutive elements).
+// For the aligned 4-cell group of cell c, at c / 4 (cells counted over all grids;
+// lines start at multiples of 4 and hold multiples of 4 cells): where its y and z
+// neighbours are, and the sweep element of its first cell (its four cells are four
+// consecutive elements).
 struct TableSet {
   TableScene s[LAYOUT_SCENES];
 };
-__global__ void group_tables_kernel(const __grid_constant__ TableSet set, int* __restrict__ group_line,
-                                    GroupNb* __restrict__ group_nb, int* __restrict__ gperm) {
+__global__ void group_tables_kernel(const __grid_constant__ TableSet set, GroupNb* __restrict__ group_nb,
+                                    int* __restrict__ gperm) {
   const TableScene& G = set.s[blockIdx.y];
   const Line* __restrict__ lines = G.lines;
   const int nj = G.nj, nk = G.nk;
@@ -294,7 +294,6 @@ __global__ void group_tables_kernel(const __grid_constant__ TableSet set, int* _
                 ((unsigned)(r & ~3) < (unsigned)N[n].len ? 1u : 0u) | ((unsigned)(4 * quad) < (unsigned)N[n].len ? 2u : 0u);
       }
       const int t = L.lo + 4 * q + j + k;
-      group_line[at] = (int)line;
       group_nb[at] = {nb[0], nb[1], nb[2], nb[3]};
       gperm[at] = (int)((G.group_base + b.goff + (t >> 2) - b.g0) * 256 + wave_line_slot(j, k));
     }
@@ -333,8 +332,7 @@ cudaError_t layout_build(const LayoutScene* scenes, int n, cudaStream_t st) {
   return cudaSuccess;
 }
 
-cudaError_t layout_tables(const TableScene* scenes, int n, int* group_line, GroupNb* group_nb, int* gperm,
-                          cudaStream_t st) {
+cudaError_t layout_tables(const TableScene* scenes, int n, GroupNb* group_nb, int* gperm, cudaStream_t st) {
   for (int first = 0; first < n; first += LAYOUT_SCENES) {
     TableSet set = {};
     const unsigned m = (unsigned)std::min(LAYOUT_SCENES, n - first);
@@ -347,7 +345,7 @@ cudaError_t layout_tables(const TableScene* scenes, int n, int* group_line, Grou
     }
     ++g_kernel_launches;
     group_tables_kernel<<<dim3((unsigned)std::min<long long>((nlines + 7) / 8, 65535LL * 8), m), 256, 0, st>>>(
-        set, group_line, group_nb, gperm);
+        set, group_nb, gperm);
     if (offset) {
       ++g_kernel_launches;
       offset_lines_kernel<<<dim3((unsigned)std::min<long long>((nlines + 255) / 256, 148LL * 8), m), 256, 0, st>>>(set);

@@ -49,9 +49,6 @@ __device__ __forceinline__ unsigned long long ld_gpu64(const unsigned long long*
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p));
   return v;
 }
-__device__ __forceinline__ void st_gpu64(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v));
-}
 
 // Turns of a wait: false after `limit`, and with ctl once another wait has run out.
 struct Spin {
