@@ -941,8 +941,10 @@ struct WaveLaunch {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = WAVE_CLUSTER;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeCooperative;
-    attr[1].val.cooperative = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    attr[2].id = cudaLaunchAttributeCooperative;
+    attr[2].val.cooperative = 1;
     cfg.blockDim = dim3(roles_of<OP>() * 32 * warps_of<OP>());
     cfg.gridDim = dim3(WAVE_CLUSTER);
     cfg.dynamicSmemBytes = smem;
@@ -960,9 +962,6 @@ struct WaveLaunch {
       if (n < 1) return cudaErrorLaunchOutOfResources;
       known[dev & 63] = resident = n;
     }
-    attr[2].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[2].val.programmaticStreamSerializationAllowed = 1;
-    cfg.numAttrs = 3;
     return cudaSuccess;
   }
 };
@@ -971,7 +970,12 @@ cudaError_t launch(const WaveArgs& g, cudaStream_t st) {
   WaveLaunch<OP, VT, CT> L;
   const cudaError_t e = L.prepare();
   if (e != cudaSuccess) return e;
-  L.cfg.gridDim = dim3(WAVE_CLUSTER * std::min(L.resident, g.ntiles));
+  const int clusters = std::min(L.resident, g.ntiles);
+  L.cfg.gridDim = dim3(WAVE_CLUSTER * clusters);
+  // Clusters that wait for one another have to be resident together; a lone one
+  // waits for none.  (ncu refuses cooperative cluster launches, "LaunchFailed", so grids
+  // of up to 32 x 32 lines are the ones that can be profiled.)
+  L.cfg.numAttrs = clusters > 1 ? 3 : 2;
   L.cfg.stream = st;
   ++g_kernel_launches;
   return cudaLaunchKernelEx(&L.cfg, wave_kernel<OP, VT, CT>, g);
