@@ -86,6 +86,7 @@
 #include <atomic>
 #include <climits>
 
+#include "xfp_edges.h"
 #include "xfp_sweep_util.cuh"
 #include "xfp_warp_wait.h"
 
@@ -383,15 +384,11 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
     const WBlk me = block_at(jb, ku);
     const WBlk pj = block_at(jb - DIR, ku), pk = block_at(jb, ku - DIR);
     const long long mybase = gbase + me.goff;
-    // Groups are numbered in sweep order from 0 in every block; the producer's
-    // number of the group at this block's group q is q + ahead (it holds one
-    // if that is in [0, ng)).  A block takes its groups as u = q + 1; u = 0
-    // carries only the producers' group before its first.
-    auto ahead = [&](const WBlk& p, const WBlk& c) { return REV ? p.g0 + p.ng - c.g0 - c.ng : c.g0 - p.g0; };
-    const int aj = ahead(pj, me) - 1, ak = ahead(pk, me) - 1;   // producer's group at u: u + aj, u + ak
+    auto shift = [&](const WBlk& p, const WBlk& c) { return edge_shift(REV, p.g0, p.ng, c.g0, c.ng); };
+    const int aj = shift(pj, me), ak = shift(pk, me);   // producer's group at u: u + aj, u + ak
     // the consumers' u of this block's group q is q - uj, q - uk
     const WBlk nj = block_at(jb + DIR, ku), nk = block_at(jb, ku + DIR);
-    const int uj = ahead(me, nj) - 1, uk = ahead(me, nk) - 1;
+    const int uj = shift(me, nj), uk = shift(me, nk);
     // the tables are the layout's; from here on, what the kernel before this one wrote
     if (first) {
       wait_previous();
@@ -442,8 +439,8 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
     };
     int armed = 0;   // (the helper's) slots filled in this tile
     // the range of own groups that each consumer takes
-    const int lo_j = uj, hi_j = nj.ng > 0 ? min(me.ng - 1, uj + nj.ng) : INT_MIN;
-    const int lo_k = uk, hi_k = nk.ng > 0 ? min(me.ng - 1, uk + nk.ng) : INT_MIN;
+    const int lo_j = uj, hi_j = last_sent(uj, me.ng, nj.ng);
+    const int lo_k = uk, hi_k = last_sent(uk, me.ng, nk.ng);
     if (!skip && me.ng > 0 && compute) {
       // ======================= compute warp =======================
       const bool edge_j = jl == (REV ? 0 : 7), edge_k = kl == (REV ? 0 : 3);
@@ -643,11 +640,11 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
       const ST* src = FACTOR ? static_cast<const ST*>(g.sys) + e0 * 4 * GE + half * 2 * GE : static_cast<const ST*>(g.sw) + e0 * WAVE_ROW;
       auto arm = [&](int n) {   // slot of group n, edge values u = n (the whole warp, n = 0, 1, ...)
         SL& d = sh.slot[n & (S - 1)];
-        const bool have_j = (unsigned)(n + aj) < (unsigned)pj.ng, have_k = (unsigned)(n + ak) < (unsigned)pk.ng;
+        const bool have_j = edge_comes(n, aj, pj.ng), have_k = edge_comes(n, ak, pk.ng);
         // a producer without such a group sends nothing: its edge values are zero
         // (and stay so, unless the slot's last use had some)
-        const bool clear_j = !have_j && (n < S || (unsigned)(n - S + aj) < (unsigned)pj.ng);
-        const bool clear_k = !have_k && (n < S || (unsigned)(n - S + ak) < (unsigned)pk.ng);
+        const bool clear_j = !have_j && (n < S || edge_comes(n - S, aj, pj.ng));
+        const bool clear_k = !have_k && (n < S || edge_comes(n - S, ak, pk.ng));
         if (clear_j || clear_k) {
           if (clear_j)
             for (int q = lane; q < (int)(sizeof(d.ej) / 16); q += 32) reinterpret_cast<uint4*>(&d.ej[0][0])[q] = make_uint4(0, 0, 0, 0);
@@ -706,9 +703,9 @@ __global__ void __launch_bounds__(roles_of<OP>() * 32 * warps_of<OP>(), OP != SW
         EdgeWords<X> w[FB];
       };
       Far fj, fk;
-      auto range = [&](Far& f, bool near, int a, const WBlk& p) {   // u with 0 <= u + a < ng
-        f.u = max(0, -a);
-        f.last = near || p.ng == 0 ? -1 : min(me.ng, p.ng - 1 - a);
+      auto range = [&](Far& f, bool near, int a, const WBlk& p) {
+        f.u = first_edge(a);
+        f.last = near ? -1 : last_edge(a, p.ng, me.ng);
 #pragma unroll
         for (int d = 0; d < FB; ++d)
 #pragma unroll
