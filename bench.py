@@ -266,21 +266,6 @@ def reference_arm(args, rank, world):
 
 
 # ---------------------------------------------------------------------------- our arm
-def sweep_traffic_per_row():
-    """DRAM bytes per unknown row of one sweep launch, from the committed ncu
-    summary (profiles/sweep_traffic.txt); None when absent."""
-    f = ROOT / "profiles" / "sweep_traffic.txt"
-    if not f.exists():
-        return None
-    for line in f.read_text().splitlines():
-        if line.startswith("dram_bytes_per_row_per_sweep:"):
-            try:
-                return float(line.split(":", 1)[1])
-            except ValueError:
-                return None
-    return None
-
-
 FULL_FIXTURE = ROOT / "tests" / "golden" / "full_blob256.npz"
 
 
@@ -517,12 +502,10 @@ def ours(args, rank, world):
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     peak = float(peaks.get("hbm_gbs", 6650.0))
     achieved = bytes_per_launch / avg_launch_s / 1e9 if avg_launch_s > 0 else None
-    tr = sweep_traffic_per_row()
     roofline = {"bound": "hbm", "kernel": "MIC(0) triangular solves (wave_kernel fwd/bwd, block wavefronts)",
                 "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650 GB/s",
                 "frac": (achieved / peak) if achieved else None,
-                "traffic": (tr * rows) if tr is not None else None,
                 "algorithmic_bytes_per_launch": bytes_per_launch, "avg_launch_ms": avg_launch_s * 1000,
                 # events sample every 16th iteration: the share scales the
                 # average launch by the launches that did work (two per
