@@ -93,13 +93,14 @@ struct xfp_ctx {
   int step_layers = 0;
   DevBuf xmarker;
   long long Gsw = 0, nlines_all = 0;   // groups and x-lines (one scene, or the whole batch)
-  // block cap of the PCG loop's SpMV: 148 x 4 measured best at 256^3 (37.4 us
-  // per launch, against 38.7 at 148 x 8 and 54.5 at 148 x 2).  XFP_VEC_BLOCKS
+  // block cap of the PCG loop's SpMV: 148 x 4 measured best at 256^3 (24.8 us per
+  // launch with its event pair, against 27.7 at 148 x 8 and 29.3 at 148 x 2; 128^3
+  // FP64: 16.7, 13.3 at 148; no difference at 48^3 and below).  XFP_VEC_BLOCKS
   // overrides, within [148, NBLK_MAX]; the dot's reduction order follows it.
   int vec_blocks = 148 * 4;
   // block cap of the x/r update (two groups in flight per thread): 148 x 2
-  // measured best at 256^3 (20.6 us, against 21.5 at 148 x 4 and 26.0 at
-  // 148 x 8).  Its |r|_inf is a max, the same in any order.  XFP_XR_BLOCKS
+  // measured best at 256^3 (21.1 us, against 26.3 at 148, 26.2 at 148 x 4 and 27.4
+  // at 148 x 8).  Its |r|_inf is a max, the same in any order.  XFP_XR_BLOCKS
   // overrides, within [148, NBLK_MAX].
   int xr_blocks = 148 * 2;
   // CUDA events around the PCG loop's solve and vector-kernel launches
@@ -110,9 +111,9 @@ struct xfp_ctx {
   int event_every = 0;
   int sweep_ord = 0;              // triangular-solve launches of the current PCG loop
   std::vector<int> sweep_ord_of;  // per timed sweep entry: its launch ordinal
-  // block cap of the PCG loop's s update: 148 x 8 measured best at 256^3
-  // (14.7 us per launch, against 17.0 at 148 x 16, with two groups in flight
-  // per thread).  XFP_S_BLOCKS overrides, within [148, 148 x 32].
+  // block cap of the PCG loop's s update: 148 x 8 at 256^3 (14.7 us per launch,
+  // against 13.8 at 148 x 4, 16.8 at 148 x 16 and 21.2 at 148, with two groups in
+  // flight per thread).  XFP_S_BLOCKS overrides, within [148, 148 x 32].
   int s_blocks = 148 * 8;
   // sizes of the current layout
   int ni = 0, nj = 0, nk = 0, NJB = 0, NKB = 0;

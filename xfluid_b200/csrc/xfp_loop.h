@@ -23,7 +23,7 @@ inline int loop_iterations(const xfp_ctx* ctx) {
 
 // Captures n iterations of a PCG loop (iteration(stream) launches one) into
 // ctx->loop_exec.  False if a graph is refused: the loop then launches directly.
-// A kernel of a graph starts 0.6 us after the one before it, one launched on a
+// A kernel of a graph starts 0.2 us after the one before it, one launched on a
 // stream 2.3 us; capturing 20 launches and updating the executable graph takes
 // 90 us on the host, while the device still works on what comes before the loop.
 template <typename F>

@@ -667,7 +667,7 @@ __device__ __forceinline__ DT partials_sum(const DT* partials, unsigned nblk, DT
 //
 // What bounds it: latency at small sizes (record, s, the reduction), the loads'
 // instructions and L2 above.  Per launch, FP32 at 256^3 half full (3.2 M cells) /
-// FP64 dam at 128^3 (0.44 M) / FP64 at 24^3: 19 / 10.9 / 4.4 us; with five line
+// FP64 dam at 128^3 (0.44 M) / FP64 at 24^3: 19 / 11.5 / 4.8 us; with five line
 // records a group and a scalar load per neighbour 30.5 / 14.8 / 5.8 us.
 // ---------------------------------------------------------------------------
 // A group's four neighbours in a line before it (j or k - 1) / after it; 0 where

@@ -67,17 +67,20 @@
 // chunks (one CTA alone reads 65,536 partials at 256^3).
 //
 // Measured (device time of a launch, full box of 128^3 / 256^3 cells): a solve
-// takes 62 / 159 us in FP32 and 90 / 285 us in FP64, the factorisation 0.21 / 0.64
-// ms (FP64 0.22 / 0.69); a launch costs 12 us to start and end, a group of four steps of a lone block
-// 0.25 (0.36) us, of which the steps are 0.13 (0.2) and the rest is waiting for a
-// slot, reading it and handing it on.
+// takes 64 / 171 us in FP32 and 94 / 301 us in FP64, the factorisation 0.24 / 0.67
+// ms; a launch costs 12 (FP64 14) us to start and end, a group of four steps of a
+// lone block 0.28 (0.41) us, of which the steps are 0.13 (0.2) and the rest is
+// waiting for a slot, reading it and handing it on.  Before waits were votes and
+// refills fenced: 62 / 159 and 90 / 285 us, 0.25 (0.36) us a group.  (The fence in the
+// sender instead, or one for two or four groups: the same within 2 %; waits that one
+// lane makes for its warp: 69 / 176 us.)
 // With the compute warp sending its edges and storing its results, as the
 // factorisation's does: 0.31 (0.39) us a group, 74 / 190 and 102 / 330 us.  With an
 // mbarrier each for operands and edge values, acknowledgements by the compute warp
 // and two or three copies a group: 0.43 (0.50) us, 83 / 214 and 114 / 365 us.
 // Before (one CTA per 32 x 15 lines, a CTA-wide barrier per step, tiles through
 // global memory): 263 us for the FP64 128^3 solve, 180 us for a half-full FP32
-// 256^3 one (now 80), 0.65 to 1.0 ms for the factorisation.  Tried on the way:
+// 256^3 one (now 65), 0.65 to 1.0 ms for the factorisation.  Tried on the way:
 // lockstep CTAs of 2 x 2 blocks (143 us where the first form took 81), blocks that
 // hand over through L2 words only (117 to 134), per-step instead of per-group
 // hand-over in the cluster (367 cycles a step), one warp as helper and courier with
