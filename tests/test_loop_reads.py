@@ -33,3 +33,10 @@ def test_done_is_the_kernels_last_store():
     common = (csrc / "xfp_common.cuh").read_text()
     body = common[common.index("void end_solve("):]
     assert body.index("sc->status = status;") < body.index("__threadfence_system();") < body.index("sc->done = 1;")
+
+
+def test_a_context_allocates_no_page_locked_memory():
+    """cudaHostAlloc takes longer than all else that creating a context does."""
+    capi = (ROOT / "xfluid_b200" / "csrc" / "xfp_capi.cu").read_text()
+    create = capi[capi.index("int xfp_create("):capi.index("int xfp_destroy(")]
+    assert "cudaHostAlloc" not in create and "cudaMallocHost" not in create

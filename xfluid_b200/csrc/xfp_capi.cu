@@ -97,8 +97,6 @@ int ensure_compact(xfp_ctx* ctx, int prec) {
     XFP_CUDA(ctx, ctx->s32.ensure(M * 4));
     XFP_CUDA(ctx, ctx->z32.ensure(M * 4));
   }
-  XFP_CUDA(ctx, ctx->ctl.ensure(sizeof(SweepCtl)));
-  XFP_CUDA(ctx, ctx->scal.ensure(sizeof(PcgScalars)));
   XFP_CUDA(ctx, ctx->scal2.ensure(sizeof(PcgScalars)));
   XFP_CUDA(ctx, ctx->partials.ensure(NBLK_MAX * sizeof(double)));
   // z.r partials: one per x-line
@@ -255,9 +253,7 @@ int pcg(xfp_ctx* ctx, const VT* const A[4], const VT* b, VT* x, VT* r, VT* s, VT
   const int K = ctx->opt.check_every > 0 ? ctx->opt.check_every : 8;
   DT* part = reinterpret_cast<DT*>(ctx->partials.p);
   auto read = [&](cudaStream_t cs) -> cudaError_t {
-    const cudaError_t e = cudaMemcpyAsync(&ctx->loop_read->sc, dsc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, cs);
-    if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(&ctx->loop_read->ctl, ctx->ctl.p, sizeof(SweepCtl), cudaMemcpyDeviceToHost, cs);
+    return cudaMemcpyAsync(ctx->loop_read, ctx->ctl.p, sizeof(xfp_ctx::LoopWords), cudaMemcpyDeviceToHost, cs);
   };
   auto done = [&] { return ctx->loop_read->sc.done != 0; };
   if (graph && (rc = replay_iterations(ctx, loop_iterations(ctx), g1.ntiles > 0 ? 5 : 3, maxit + 2 * K, read, done)) != XFP_OK) return rc;
@@ -335,7 +331,7 @@ int solve_core(xfp_ctx* ctx, int ni, int nj, int nk, const uint8_t* dmat, const 
   const Line* lines = ctx->lines.as<Line>();
   const long long M = ctx->M;
   ctx->iters = 0; ctx->refinements = 0; ctx->res = 0; ctx->bnorm = 0;
-  PcgScalars* dsc = ctx->scal.as<PcgScalars>();
+  PcgScalars* dsc = &ctx->ctl.as<xfp_ctx::LoopWords>()->sc;
   PcgScalars& hsc = ctx->host_sc;
   const double tol = ctx->opt.tol;
   const int maxit = ctx->opt.max_iter;
@@ -1136,12 +1132,7 @@ int xfp_create(xfp_ctx** out, const xfp_options* opt) {
   if (const char* e = getenv("XFP_XR_BLOCKS")) ctx->xr_blocks = std::max(148, std::min(xfp_host::NBLK_MAX, atoi(e)));
   if (const char* e = getenv("XFP_S_BLOCKS")) ctx->s_blocks = std::max(148, std::min(148 * 32, atoi(e)));
   if (const char* e = getenv("XFP_HOST_FACES")) ctx->host_sparse_ok = strcmp(e, "full") != 0;
-  if (cudaHostAlloc((void**)&ctx->loop_read, sizeof(*ctx->loop_read), cudaHostAllocDefault) != cudaSuccess) {
-    ctx->loop_read = nullptr;
-    xfp_destroy(ctx);
-    return XFP_ERR_NOMEM;
-  }
-  if (ctx->ctl.ensure(sizeof(SweepCtl)) != cudaSuccess) { xfp_destroy(ctx); return XFP_ERR_NOMEM; }
+  if (ctx->ctl.ensure(sizeof(xfp_ctx::LoopWords)) != cudaSuccess) { xfp_destroy(ctx); return XFP_ERR_NOMEM; }
   SweepCtl c0{};
   c0.gen = 1;
   cudaMemcpy(ctx->ctl.p, &c0, sizeof(c0), cudaMemcpyHostToDevice);
@@ -1171,7 +1162,6 @@ int xfp_destroy(xfp_ctx* ctx) {
   for (cudaEvent_t e : ctx->loop_ev)
     if (e) cudaEventDestroy(e);
   if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
-  if (ctx->loop_read) cudaFreeHost(ctx->loop_read);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return XFP_OK;

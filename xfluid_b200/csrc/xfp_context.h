@@ -62,7 +62,7 @@ struct xfp_ctx {
   DevBuf A32[5];                  // same in FP32
   DevBuf x64, r64, x32, r32, s32, z32, s64, z64, dense;
   // control
-  DevBuf ctl, scal, scal2, partials, tpartials;
+  DevBuf ctl, scal2, partials, tpartials;   // ctl: LoopWords
   // particle steps (xfp_particles.cu): staged particles and field, bin keys,
   // indices, boxes, positions, bin starts, box spans, sort/scan scratch
   DevBuf part_io, phi_io, part_key, part_idx, part_spos, part_start, part_span,
@@ -127,12 +127,14 @@ struct xfp_ctx {
   cudaGraphExec_t loop_exec = nullptr;
   cudaEvent_t loop_ev[2] = {};
   bool loop_graph = false;        // this call's loop ran as a graph
-  // pinned: what a loop reads back after some iterations
-  struct LoopRead {
-    xfp::PcgScalars sc;
+  // The sweeps' control block and the loop's scalars, on the device (ctl), and as a
+  // loop last read them: one copy, into ordinary memory (a page-locked allocation
+  // takes 2.4 ms, more than all else that a new context does).
+  struct LoopWords {
     xfp::SweepCtl ctl;
+    alignas(128) xfp::PcgScalars sc;
   };
-  LoopRead* loop_read = nullptr;
+  LoopWords loop_read_here{}, *loop_read = &loop_read_here;
   // stats
   double ms_setup = 0, ms_factor = 0, ms_solve = 0, ms_apply = 0;
   int iters = 0, refinements = 0;
