@@ -21,6 +21,7 @@ struct xfp_ctx {
   cudaStream_t stream = (cudaStream_t)1, cap_stream = nullptr;
   cudaGraphExec_t loop_exec = nullptr;
   cudaEvent_t loop_ev[2] = {};
+  bool loop_cooperative = false;
   struct Read {
     Scalars sc;
     Ctl ctl;
@@ -47,7 +48,7 @@ thread_local long long g_kernel_launches = 0;
 }
 
 // ---- the runtime ----
-static int execs = 0, launches = 0, drained = 0;   // live executables, graph launches, how many of them the host has waited for
+static int instances = 0, execs = 0, launches = 0, drained = 0;   // live executables, graph launches, how many of them the host has waited for
 static cudaError_t capture_result = cudaSuccess, instantiate_result = cudaSuccess, update_result = cudaSuccess;
 extern "C" {
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)8; return cudaSuccess; }
@@ -63,6 +64,7 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { --execs; return cudaSuccess;
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
   if (instantiate_result != cudaSuccess) return instantiate_result;
   ++execs;
+  ++instances;
   *e = (cudaGraphExec_t)32;
   return cudaSuccess;
 }
@@ -99,7 +101,7 @@ static int loop(xfp_ctx& ctx, const std::function<void(int, bool, xfp_ctx::Read&
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   xfp_ctx ctx;
-  check(xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }), "capture");
+  check(xfp_host::capture_iterations(&ctx, 4, true, [](cudaStream_t) { return cudaSuccess; }), "capture");
   if (what == "half") {
     // the third read meets the end of the solve half-way: the flag is there, the
     // count and the residual are an older iteration's
@@ -129,19 +131,25 @@ int main(int argc, char** argv) {
       ctx.opt.check_every = k;
       check(xfp_host::loop_iterations(&ctx) == (k == 0 || k > 4 ? 4 : k), "iterations of a graph");
     }
+  } else if (what == "kinds") {
+    // a graph of cooperative launches is not updated into one of plain launches
+    check(instances == 1 && xfp_host::capture_iterations(&ctx, 4, true, [](cudaStream_t) { return cudaSuccess; }), "updated");
+    check(instances == 1, "the same kind is updated");
+    check(xfp_host::capture_iterations(&ctx, 4, false, [](cudaStream_t) { return cudaSuccess; }), "the other kind");
+    check(instances == 2 && execs == 1, "the other kind is instantiated, and the first given back");
   } else if (what == "refused") {
     // a capture that fails after one that did not leaves no executable graph behind
     capture_result = cudaErrorStreamCaptureInvalidated;
-    check(!xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }), "a refused capture");
+    check(!xfp_host::capture_iterations(&ctx, 4, true, [](cudaStream_t) { return cudaSuccess; }), "a refused capture");
     check(execs == 0 && ctx.loop_exec == nullptr, "the earlier graph given back");
     capture_result = cudaSuccess;
-    check(!xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaErrorInvalidValue; }), "a refused launch");
+    check(!xfp_host::capture_iterations(&ctx, 4, true, [](cudaStream_t) { return cudaErrorInvalidValue; }), "a refused launch");
     check(execs == 0 && ctx.loop_exec == nullptr, "nothing kept");
-    check(xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }) && execs == 1, "a new graph");
+    check(xfp_host::capture_iterations(&ctx, 4, true, [](cudaStream_t) { return cudaSuccess; }) && execs == 1, "a new graph");
     update_result = cudaErrorGraphExecUpdateFailure;
-    check(xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }) && execs == 1, "one in its place");
+    check(xfp_host::capture_iterations(&ctx, 4, true, [](cudaStream_t) { return cudaSuccess; }) && execs == 1, "one in its place");
     instantiate_result = cudaErrorMemoryAllocation;
-    check(!xfp_host::capture_iterations(&ctx, 4, [](cudaStream_t) { return cudaSuccess; }) && execs == 0, "no instance");
+    check(!xfp_host::capture_iterations(&ctx, 4, true, [](cudaStream_t) { return cudaSuccess; }) && execs == 0, "no instance");
   } else {
     return 2;
   }

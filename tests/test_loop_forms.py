@@ -36,3 +36,24 @@ def test_a_capped_loop_reports_its_cap():
             assert st["status"] == 1 and st["iterations"] == cap
         finally:
             ctx.close()
+
+
+def test_one_context_for_grids_of_one_and_of_many_clusters():
+    """The loop's executable graph passes from plain to cooperative sweeps and back."""
+    scs = [scenes.blob_scene(dims=d, seed=5, fractional=False, dtype=np.float64) for d in ((24, 20, 22), (40, 65, 40))]
+    want = []
+    for sc in scs:
+        ctx = make_ctx("f64", tol=1e-8, max_iter=300)
+        try:
+            want.append(project(ctx, sc))
+        finally:
+            ctx.close()
+    ctx = make_ctx("f64", tol=1e-8, max_iter=300)
+    try:
+        for q in (0, 1, 0, 1, 1, 0):
+            got = project(ctx, scs[q])
+            assert got[0] == 0 and got[5]["graph"] == 1 and got[5]["iterations"] == want[q][5]["iterations"]
+            for a, b in zip(got[1:5], want[q][1:5]):
+                assert np.array_equal(a, b)
+    finally:
+        ctx.close()

@@ -17,7 +17,7 @@ def loop(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["half", "expired", "both", "endless", "refused", "check_every"])
+@pytest.mark.parametrize("case", ["half", "expired", "both", "endless", "refused", "kinds", "check_every"])
 def test_reads_beside_a_running_launch(loop, case):
     r = subprocess.run([str(loop), case], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stderr

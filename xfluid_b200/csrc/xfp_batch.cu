@@ -239,7 +239,7 @@ int batch_pcg(xfp_ctx* ctx, BatchState* B, const VT* const A[4], const VT* b, VT
   // iterations as a graph, read after every launch of it; if that is refused,
   // launch directly
   const int per = loop_iterations(ctx);
-  const bool graph = capture_iterations(ctx, per, iteration);
+  const bool graph = capture_iterations(ctx, per, B->ntiles > 1, iteration);
   ctx->loop_graph = graph;
   hsc.assign(n, PcgScalars{});
   int rc = XFP_OK;

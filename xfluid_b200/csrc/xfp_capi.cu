@@ -202,7 +202,7 @@ bool pcg_graph(xfp_ctx* ctx, const VT* const A[4], VT* x, VT* r, VT* s, VT* z, P
     }
     return wave_launch<VT, DT>(op, gl, cs);
   };
-  return capture_iterations(ctx, loop_iterations(ctx), [&](cudaStream_t cs) -> cudaError_t {
+  return capture_iterations(ctx, loop_iterations(ctx), ctx->ntiles > 1, [&](cudaStream_t cs) -> cudaError_t {
     cudaError_t e;
     if ((e = spmv_dot<VT, VT, DT>(A[0], A[1], A[2], A[3], s, z, ctx->group_nb.as<GroupNb>(), ctx->M, dsc,
                                   reinterpret_cast<DT*>(ctx->partials.p), ctx->vec_blocks, 0, cs)))

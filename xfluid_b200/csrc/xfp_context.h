@@ -126,6 +126,7 @@ struct xfp_ctx {
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t loop_exec = nullptr;
   cudaEvent_t loop_ev[2] = {};
+  bool loop_cooperative = false;  // the executable graph's sweeps are cooperative launches
   bool loop_graph = false;        // this call's loop ran as a graph
   // The sweeps' control block and the loop's scalars, on the device (ctl), and as a
   // loop last read them: one copy, into ordinary memory (a page-locked allocation

@@ -25,9 +25,11 @@ inline int loop_iterations(const xfp_ctx* ctx) {
 // ctx->loop_exec.  False if a graph is refused: the loop then launches directly.
 // A kernel of a graph starts 0.2 us after the one before it, one launched on a
 // stream 2.3 us; capturing 20 launches and updating the executable graph takes
-// 90 us on the host, while the device still works on what comes before the loop.
+// 90 us on the host, while the device still works on what comes before the loop.  An
+// update is not asked to change whether launches are cooperative: those of one cluster
+// are not (wave_launch), and a graph of the other kind is given back first.
 template <typename F>
-bool capture_iterations(xfp_ctx* ctx, int n, F&& iteration) {
+bool capture_iterations(xfp_ctx* ctx, int n, bool cooperative, F&& iteration) {
   for (cudaEvent_t& e : ctx->loop_ev)
     if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
       e = nullptr;
@@ -50,6 +52,11 @@ bool capture_iterations(xfp_ctx* ctx, int n, F&& iteration) {
   }
   xfp::g_kernel_launches = before;   // counted per launch of the graph
   if (e == cudaSuccess && graph) {
+    if (ctx->loop_exec && ctx->loop_cooperative != cooperative) {
+      cudaGraphExecDestroy(ctx->loop_exec);
+      ctx->loop_exec = nullptr;
+    }
+    ctx->loop_cooperative = cooperative;
     cudaGraphExecUpdateResultInfo info;
     if (ctx->loop_exec && cudaGraphExecUpdate(ctx->loop_exec, graph, &info) != cudaSuccess) {
       cudaGetLastError();
